@@ -20,10 +20,25 @@ template <class T> struct GemmDesc {
     int bias_mode = 0;              // 1: bias[i] (per row), 2: bias[j] (per column)
 };
 template <class T> void gemm(const GemmDesc<T> &d);
-// Up to three products of one shape whose operands are separate allocations (the q, k, v projections of an attention layer)
-// as one launch: `shape` gives sizes, strides, alpha, accumulate and bias_mode; A, B, C and bias come from the list.
-template <class T> struct GemmList { const T *A[3]; const T *B[3]; const T *bias[3]; T *C[3]; };
-template <class T> void gemm_list(const GemmDesc<T> &shape, const GemmList<T> &l, int count);
+// One member of a group of products that go out as one launch (tl_gemm_small.cu): a GemmDesc whose contraction may run over
+// `segs` segments of K each.  seg_list: segment s multiplies A[s] by B[s] (separate allocations, 3 at most); otherwise the
+// operands of segment s start at A[0] + s * a_ks and B[0] + s * b_ks.
+template <class T> struct GemmGroup {
+    const T *A[3] = {nullptr, nullptr, nullptr}; const T *B[3] = {nullptr, nullptr, nullptr}; T *C = nullptr;
+    int N = 0, M = 0, K = 0;
+    long long a_rs = 0, a_cs = 1, b_rs = 0, b_cs = 1, c_rs = 0, c_cs = 1;
+    int batch = 1; long long a_bs = 0, b_bs = 0, c_bs = 0;
+    int segs = 1, seg_list = 0; long long a_ks = 0, b_ks = 0;
+    float alpha = 1.f;
+    bool accumulate = false;
+    const T *bias = nullptr; int bias_mode = 0;
+    GemmGroup() {}
+    GemmGroup(const GemmDesc<T> &d) : C(d.C), N(d.N), M(d.M), K(d.K), a_rs(d.a_rs), a_cs(d.a_cs), b_rs(d.b_rs), b_cs(d.b_cs), c_rs(d.c_rs), c_cs(d.c_cs),
+        batch(d.batch), a_bs(d.a_bs), b_bs(d.b_bs), c_bs(d.c_bs), alpha(d.alpha), accumulate(d.accumulate), bias(d.bias), bias_mode(d.bias ? d.bias_mode : 0) { A[0] = d.A; B[0] = d.B; }
+};
+template <class T> void gemm_group(const GemmGroup<T> *list, int count);    // 6 at most, one launch
+// Independent products: those large enough for the tensor-core kernels one by one, the others as one group.
+template <class T> void gemm_many(const GemmGroup<T> *list, int count);
 
 // Reference-contract product: C[N x M] = A[N x K] * B, B is [K x M] or (trans_B) [M x K].
 template <class T> void mm_contract(const T *A, const T *B, T *C, int N, int K, int M, int trans_B, bool accumulate);

@@ -28,15 +28,15 @@ void mhsa_fw(Scope &sc, const MhsaDims &d, const T *x, const T *wq, const T *wk,
     const int L = d.L, E = d.E, F = d.F, NH = d.heads, H = F / NH;
     const float scaling = q_rsqrt_host((float)H);
 
-    // projections: q = Wq^T x (+ bq per row)  [ref: pulp_mhsa_fp32.c:87-158 and twins for k, v]
-    // the three are one launch (separate allocations, one shape): 192 tiles instead of three times 64 on 148 SMs
-    {
-        GemmDesc<T> g;
-        g.a_rs = 1; g.a_cs = F; g.b_rs = L; g.b_cs = 1; g.c_rs = L;
-        g.N = F; g.K = E; g.M = L; g.bias_mode = 1;
-        const GemmList<T> l = {{wq, wk, wv}, {x, x, x}, {bq, bk, bv}, {q, k, v}};
-        gemm_list<T>(g, l, 3);
+    // projections: q = Wq^T x (+ bq per row), the three as one launch  [ref: pulp_mhsa_fp32.c:87-158 and twins for k, v]
+    const T *ws[3] = {wq, wk, wv}, *bs[3] = {bq, bk, bv}; T *outs[3] = {q, k, v};
+    GemmGroup<T> proj[3];
+    for (int p = 0; p < 3; p++) {
+        GemmGroup<T> &g = proj[p];
+        g.A[0] = ws[p]; g.a_rs = 1; g.a_cs = F; g.B[0] = x; g.b_rs = L; g.b_cs = 1; g.C = outs[p]; g.c_rs = L;
+        g.N = F; g.K = E; g.M = L; g.bias = bs[p]; g.bias_mode = bs[p] ? 1 : 0;
     }
+    gemm_many<T>(proj, 3);
     if (attn_fused_ok(L, H) && gemm_path() != 1) {
         // scores, softmax and the product with v in one kernel per (head, query tile)   [ref: :348-560]
         attn_fw<T>(q, k, v, softmax, att, L, H, NH, scaling);
@@ -80,10 +80,14 @@ void mhsa_bw(Scope &sc, const MhsaDims &d, const T *x, const T *wq, const T *wk,
     const float scaling = q_rsqrt_host((float)H);
     const long long HL = (long long)H * L, LL = (long long)L * L;
 
-    // dWo = dY att^T   [ref: pulp_mhsa_fp32.c:704-760]
-    { GemmDesc<T> g; g.A = dy; g.a_rs = L; g.B = att; g.b_rs = 1; g.b_cs = L; g.C = dwo; g.c_rs = F; g.N = E; g.K = L; g.M = F; gemm<T>(g); }
-    // datt = Wo^T dY   [ref: :783-837]
-    { GemmDesc<T> g; g.A = wo; g.a_rs = 1; g.a_cs = F; g.B = dy; g.b_rs = L; g.C = datt; g.c_rs = L; g.N = F; g.K = E; g.M = L; gemm<T>(g); }
+    {
+        GemmGroup<T> l[2];
+        // dWo = dY att^T   [ref: pulp_mhsa_fp32.c:704-760]
+        { GemmGroup<T> &g = l[0]; g.A[0] = dy; g.a_rs = L; g.B[0] = att; g.b_rs = 1; g.b_cs = L; g.C = dwo; g.c_rs = F; g.N = E; g.K = L; g.M = F; }
+        // datt = Wo^T dY   [ref: :783-837]
+        { GemmGroup<T> &g = l[1]; g.A[0] = wo; g.a_rs = 1; g.a_cs = F; g.B[0] = dy; g.b_rs = L; g.C = datt; g.c_rs = L; g.N = F; g.K = E; g.M = L; }
+        gemm_many<T>(l, 2);
+    }
     const bool fused = attn_fused_ok(L, H) && gemm_path() != 1;
     if (fused) {
         // dP, dS (never stored), dq, dk, dv in two kernels   [ref: :842-1400]
@@ -109,18 +113,17 @@ void mhsa_bw(Scope &sc, const MhsaDims &d, const T *x, const T *wq, const T *wk,
     { GemmDesc<T> g; g.A = k; g.a_rs = L; g.a_bs = HL; g.B = dS; g.b_rs = 1; g.b_cs = L; g.b_bs = LL; g.C = dq; g.c_rs = L; g.c_bs = HL;
       g.N = H; g.K = L; g.M = L; g.batch = NH; g.alpha = scaling; gemm<T>(g); }
     }
-    // projection weight grads, stored F x E: dW = dproj x^T   [ref: :1426-1600]
-    const T *dps[3] = {dq, dk, dv}; const T *ws[3] = {wq, wk, wv};
-    {
-        GemmDesc<T> g; g.a_rs = L; g.b_rs = 1; g.b_cs = L; g.c_rs = E; g.N = F; g.K = L; g.M = E;                // one launch for the three
-        const GemmList<T> l = {{dq, dk, dv}, {x, x, x}, {nullptr, nullptr, nullptr}, {dwq, dwk, dwv}};
-        gemm_list<T>(g, l, 3);
-    }
-    // dx += Wq dq + Wk dk + Wv dv (the caller zeroes dx; same order as the reference)   [ref: :1605-1745]
+    // projection weight grads, stored F x E: dW = dproj x^T   [ref: :1426-1600], and
+    // dx += Wq dq + Wk dk + Wv dv (the caller zeroes dx): one product whose contraction runs over the three pairs   [ref: :1605-1745]
+    const T *dps[3] = {dq, dk, dv}; const T *ws[3] = {wq, wk, wv}; T *dws[3] = {dwq, dwk, dwv};
+    GemmGroup<T> l[4];
     for (int p = 0; p < 3; p++) {
-        GemmDesc<T> g; g.A = ws[p]; g.a_rs = F; g.B = dps[p]; g.b_rs = L; g.C = dx; g.c_rs = L; g.N = E; g.K = F; g.M = L; g.accumulate = true;
-        gemm<T>(g);
+        GemmGroup<T> &g = l[p];
+        g.A[0] = dps[p]; g.a_rs = L; g.B[0] = x; g.b_rs = 1; g.b_cs = L; g.C = dws[p]; g.c_rs = E; g.N = F; g.K = L; g.M = E;
+        l[3].A[p] = ws[p]; l[3].B[p] = dps[p];
     }
+    { GemmGroup<T> &g = l[3]; g.segs = 3; g.seg_list = 1; g.a_rs = F; g.b_rs = L; g.C = dx; g.c_rs = L; g.N = E; g.K = F; g.M = L; g.accumulate = true; }
+    gemm_many<T>(l, 4);
 }
 
 // Attention of the MobileBERT encoder block: token-major activations (x: L x E, bottleneck input xb: L x Kb, output
@@ -136,16 +139,17 @@ void mhsa_mobilebert_fw(Scope &sc, const MobileBertDims &d, const T *x, const T 
     const int L = d.L, E = d.E, Kb = d.Kb, F = d.F, No = d.No, NH = d.heads, H = F / NH;
     const float scaling = q_rsqrt_host((float)H);
     const T *ws[3] = {wq, wk, wv}; const T *bs[3] = {bq, bk, bv}; T *outs[3] = {q, k, v};
+    GemmGroup<T> proj[3];
     for (int p = 0; p < 3; p++) {
         const int K = p == 2 ? E : Kb;
-        GemmDesc<T> g;
-        g.A = ws[p]; g.a_rs = K; g.a_cs = 1;
-        g.B = p == 2 ? x : xb; g.b_rs = 1; g.b_cs = K;
+        GemmGroup<T> &g = proj[p];
+        g.A[0] = ws[p]; g.a_rs = K; g.a_cs = 1;
+        g.B[0] = p == 2 ? x : xb; g.b_rs = 1; g.b_cs = K;
         g.C = outs[p]; g.c_rs = L;
         g.N = F; g.K = K; g.M = L;
         if (bs[p]) { g.bias = bs[p]; g.bias_mode = 1; }
-        gemm<T>(g);
     }
+    gemm_many<T>(proj, 3);
     if (attn_fused_ok(L, H) && gemm_path() != 1) attn_fw<T>(q, k, v, softmax, att, L, H, NH, scaling);
     else {
         T *scores = sc.scratch<T>((size_t)NH * L * L);
@@ -174,8 +178,12 @@ void mhsa_mobilebert_bw(Scope &sc, const MobileBertDims &d, const T *x, const T 
     const float scaling = q_rsqrt_host((float)H);
     const long long HL = (long long)H * L, LL = (long long)L * L;
     // dWo[n][f] = sum_l dy[l][n] att[f][l];  datt[f][l] = sum_n Wo[n][f] dy[l][n]
-    { GemmDesc<T> g; g.A = dy; g.a_rs = 1; g.a_cs = No; g.B = att; g.b_rs = 1; g.b_cs = L; g.C = dwo; g.c_rs = F; g.N = No; g.K = L; g.M = F; gemm<T>(g); }
-    { GemmDesc<T> g; g.A = wo; g.a_rs = 1; g.a_cs = F; g.B = dy; g.b_rs = 1; g.b_cs = No; g.C = datt; g.c_rs = L; g.N = F; g.K = No; g.M = L; gemm<T>(g); }
+    {
+        GemmGroup<T> l[2];
+        { GemmGroup<T> &g = l[0]; g.A[0] = dy; g.a_rs = 1; g.a_cs = No; g.B[0] = att; g.b_rs = 1; g.b_cs = L; g.C = dwo; g.c_rs = F; g.N = No; g.K = L; g.M = F; }
+        { GemmGroup<T> &g = l[1]; g.A[0] = wo; g.a_rs = 1; g.a_cs = F; g.B[0] = dy; g.b_rs = 1; g.b_cs = No; g.C = datt; g.c_rs = L; g.N = F; g.K = No; g.M = L; }
+        gemm_many<T>(l, 2);
+    }
     if (attn_fused_ok(L, H) && gemm_path() != 1) {
         float *rowdot = sc.scratch<float>((size_t)NH * L);
         if (!rowdot) return;
@@ -194,14 +202,26 @@ void mhsa_mobilebert_bw(Scope &sc, const MobileBertDims &d, const T *x, const T 
           g.N = H; g.K = L; g.M = L; g.batch = NH; g.alpha = scaling; gemm<T>(g); }
     }
     const T *dps[3] = {dq, dk, dv}; T *dws[3] = {dwq, dwk, dwv}; const T *ws[3] = {wq, wk, wv};
+    GemmGroup<T> l[5];
+    int n = 3;
     for (int p = 0; p < 3; p++) {
-        const int K = p == 2 ? E : Kb;
         // dW[f][c] = sum_l dproj[f][l] in[l][c]
-        { GemmDesc<T> g; g.A = dps[p]; g.a_rs = L; g.a_cs = 1; g.B = p == 2 ? x : xb; g.b_rs = K; g.b_cs = 1; g.C = dws[p]; g.c_rs = K; g.N = F; g.K = L; g.M = K; gemm<T>(g); }
-        // din[l][c] += sum_f dproj[f][l] W[f][c]
-        T *din = p == 2 ? dx : dxb;
-        if (din) { GemmDesc<T> g; g.A = dps[p]; g.a_rs = 1; g.a_cs = L; g.B = ws[p]; g.b_rs = K; g.b_cs = 1; g.C = din; g.c_rs = K; g.N = L; g.K = F; g.M = K; g.accumulate = true; gemm<T>(g); }
+        const int K = p == 2 ? E : Kb;
+        GemmGroup<T> &g = l[p];
+        g.A[0] = dps[p]; g.a_rs = L; g.a_cs = 1; g.B[0] = p == 2 ? x : xb; g.b_rs = K; g.b_cs = 1; g.C = dws[p]; g.c_rs = K; g.N = F; g.K = L; g.M = K;
     }
+    // din[l][c] += sum_f dproj[f][l] W[f][c]: q and k into the bottleneck gradient, v into the input's; where the two are one
+    // buffer the contraction runs over all three pairs (two products of one launch must not add to the same matrix)
+    const bool one = dxb && dxb == dx;
+    for (int t = 0; t < 2; t++) {
+        T *din = t == 0 ? dxb : dx;
+        if (!din || (one && t == 1)) continue;
+        const int p0 = t == 0 ? 0 : 2, p1 = t == 0 ? (one ? 3 : 2) : 3, K = t == 0 ? Kb : E;
+        GemmGroup<T> &g = l[n++];
+        for (int p = p0; p < p1; p++) { g.A[p - p0] = dps[p]; g.B[p - p0] = ws[p]; }
+        g.segs = p1 - p0; g.seg_list = 1; g.a_rs = 1; g.a_cs = L; g.b_rs = K; g.b_cs = 1; g.C = din; g.c_rs = K; g.N = L; g.K = F; g.M = K; g.accumulate = true;
+    }
+    gemm_many<T>(l, n);
 }
 
 #define INST(T)                                                                                                        \
