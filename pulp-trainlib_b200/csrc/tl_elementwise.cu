@@ -5,6 +5,7 @@
 #include "tl_kernels.h"
 #include "tl_reduce.cuh"
 #include <cfloat>
+#include <algorithm>
 
 namespace tl {
 
@@ -753,6 +754,37 @@ template <class T> void batchnorm_fw(const T *x, T *y, const T *w, const T *b, i
     TL_LAUNCH((batchnorm_fw_kernel<T>), n * C, (B * HW) >= 256 ? 256 : 64, 0, x, y, w, b, B, C, HW, eps);
 }
 
+// Rows of up to 1024 elements: one warp per row, the row in registers (NV elements per lane), so every tensor is read once
+// and no CTA-wide barrier sits between the two sums and the output.
+template <class T, int NV> __device__ __forceinline__ void ln_load(const T *__restrict__ p, int width, int lane, float (&v)[NV])
+{
+#pragma unroll
+    for (int k = 0; k < NV; k++) { const int j = lane + 32 * k; v[k] = j < width ? ld(p + j) : 0.f; }
+}
+// mean and standard deviation of a row  [ref: lib/sources/pulp_layernorm_fp32.c:60-77]
+__device__ __forceinline__ void ln_stats(float s1, float s2, int width, float eps, float &mean, float &sv)
+{
+    mean = s1 / (float)width;
+    sv = sqrtf(__fadd_rn(__fadd_rn(__fdiv_rn(__fsub_rn(s2, __fmul_rn(__fmul_rn(2.f, s1), mean)), (float)width), __fmul_rn(mean, mean)), eps));
+}
+template <class T, int NV>
+__global__ void __launch_bounds__(256) layernorm_fw_warp_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ w,
+                                                                const T *__restrict__ b, int rows, int width, float eps)
+{
+    const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    float v[NV], wv[NV], bv[NV];
+    ln_load<T, NV>(x + (long long)row * width, width, lane, v);
+    ln_load<T, NV>(w, width, lane, wv); ln_load<T, NV>(b, width, lane, bv);
+    float s1 = 0.f, s2 = 0.f, mean, sv;
+#pragma unroll
+    for (int k = 0; k < NV; k++) { s1 += v[k]; s2 = fmaf(v[k], v[k], s2); }
+    ln_stats(warp_sum(s1), warp_sum(s2), width, eps, mean, sv);
+    T *yp = y + (long long)row * width;
+#pragma unroll
+    for (int k = 0; k < NV; k++) { const int j = lane + 32 * k; if (j < width) st(yp + j, __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(v[k], mean), sv), wv[k]), bv[k])); }
+}
+// wider rows: a CTA per row
 template <class T>
 __global__ void __launch_bounds__(128) layernorm_fw_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ w,
                                                            const T *__restrict__ b, int width, float eps)
@@ -760,19 +792,90 @@ __global__ void __launch_bounds__(128) layernorm_fw_kernel(const T *__restrict__
     __shared__ float red[33];
     const T *xp = x + (long long)blockIdx.x * width;
     T *yp = y + (long long)blockIdx.x * width;
-    float s1 = 0.f, s2 = 0.f;
+    float s1 = 0.f, s2 = 0.f, mean, sv;
     for (int j = threadIdx.x; j < width; j += blockDim.x) { float t = ld(xp + j); s1 += t; s2 = fmaf(t, t, s2); }
     s1 = block_sum(s1, red);
     s2 = block_sum(s2, red);
-    const float mean = s1 / (float)width;
-    const float sv = sqrtf(__fadd_rn(__fadd_rn(__fdiv_rn(__fsub_rn(s2, __fmul_rn(__fmul_rn(2.f, s1), mean)), (float)width), __fmul_rn(mean, mean)), eps));
+    ln_stats(s1, s2, width, eps, mean, sv);
     for (int j = threadIdx.x; j < width; j += blockDim.x)
         st(yp + j, __fadd_rn(__fmul_rn(__fdiv_rn(__fsub_rn(ld(xp + j), mean), sv), ld(w + j)), ld(b + j)));
 }
 // Backward of the layer norm above (the reference has no backward; derived from its forward formula):
 // xhat = (x - mean) / sv, g = w * dy;  dx = (g - mean_j(g) - xhat * mean_j(g * xhat)) / sv per row;
-// dw[j] = sum_rows dy * xhat, db[j] = sum_rows dy.  Kernel 1: one CTA per row writes dx and the row's (mean, 1/sv);
-// kernel 2: one thread per column adds over the rows in row order.
+// dw[j] = sum_rows dy * xhat, db[j] = sum_rows dy.
+//
+// Rows of up to 1024 elements, one launch: a CTA's eight warps take its rows in turn (a row in registers: dx and the lane's
+// columns of dw and db come from the same read), the warps' column sums meet in shared memory in warp order, and the CTA
+// that finishes last adds the CTAs' sums in CTA order.  A separate column kernel with a thread per column walked the rows
+// one after another on width / 128 CTAs: 16 us of the 19 us that 128 rows of 128 took; this one takes 4.
+static __device__ unsigned ln_ticket;                        // zero between launches
+template <class T, int NV>
+__global__ void __launch_bounds__(256) layernorm_bw_warp_kernel(const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ dy, T *__restrict__ dx,
+                                                                float *__restrict__ part, T *__restrict__ dw, T *__restrict__ db, int rows, int width,
+                                                                int rows_per_cta, float eps)
+{
+    constexpr int W = 32 * NV;
+    __shared__ float sm[8][W];
+    __shared__ unsigned ticket_s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * rows_per_cta, r1 = min(rows, r0 + rows_per_cta);
+    float wv[NV], ca[NV], cb[NV];
+    ln_load<T, NV>(w, width, lane, wv);
+#pragma unroll
+    for (int k = 0; k < NV; k++) ca[k] = cb[k] = 0.f;
+    for (int row = r0 + warp; row < r1; row += 8) {
+        float v[NV], g[NV];
+        ln_load<T, NV>(x + (long long)row * width, width, lane, v);
+        ln_load<T, NV>(dy + (long long)row * width, width, lane, g);
+        float s1 = 0.f, s2 = 0.f, mean, sv;
+#pragma unroll
+        for (int k = 0; k < NV; k++) { s1 += v[k]; s2 = fmaf(v[k], v[k], s2); }
+        ln_stats(warp_sum(s1), warp_sum(s2), width, eps, mean, sv);
+        const float inv = 1.f / sv;
+        float a = 0.f, b = 0.f;                              // sum g, sum g * xhat (elements past the row carry dy = w = 0)
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            v[k] = (v[k] - mean) * inv;
+            ca[k] = fmaf(g[k], v[k], ca[k]); cb[k] += g[k];
+            g[k] *= wv[k];
+            a += g[k]; b = fmaf(g[k], v[k], b);
+        }
+        const float ma = warp_sum(a) / (float)width, mb = warp_sum(b) / (float)width;
+        T *dp = dx + (long long)row * width;
+#pragma unroll
+        for (int k = 0; k < NV; k++) { const int j = lane + 32 * k; if (j < width) st(dp + j, (g[k] - ma - v[k] * mb) * inv); }
+    }
+    // column sums of the CTA: dw, then db
+    for (int half = 0; half < 2; half++) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) sm[warp][lane + 32 * k] = half ? cb[k] : ca[k];
+        __syncthreads();
+        for (int j = threadIdx.x; j < width; j += 256) {
+            float t = sm[0][j];
+#pragma unroll
+            for (int q = 1; q < 8; q++) t += sm[q][j];
+            if (gridDim.x == 1) st((half ? db : dw) + j, t);
+            else __stcg(part + ((size_t)blockIdx.x * 2 + half) * width + j, t);
+        }
+        __syncthreads();
+    }
+    if (gridDim.x == 1) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) ticket_s = atomicAdd(&ln_ticket, 1u);
+    __syncthreads();
+    if (ticket_s != gridDim.x - 1) return;
+    __threadfence();
+    for (int j = threadIdx.x; j < 2 * width; j += 256) {
+        float t = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < (int)gridDim.x; q++) t += __ldcg(part + (size_t)q * 2 * width + j);
+        if (j < width) st(dw + j, t); else st(db + j - width, t);
+    }
+    if (threadIdx.x == 0) ln_ticket = 0;
+}
+// wider rows.  Kernel 1: one CTA per row writes dx and the row's (mean, 1/sv); kernel 2: one thread per column adds over the
+// rows in row order.
 template <class T>
 __global__ void __launch_bounds__(128) layernorm_bw_rows_kernel(const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ dy,
                                                                 T *__restrict__ dx, float2 *__restrict__ stats, int width, float eps)
@@ -780,12 +883,11 @@ __global__ void __launch_bounds__(128) layernorm_bw_rows_kernel(const T *__restr
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const T *xp = x + row * width, *gp = dy + row * width;
-    float s1 = 0.f, s2 = 0.f;
+    float s1 = 0.f, s2 = 0.f, mean, sv;
     for (int j = threadIdx.x; j < width; j += blockDim.x) { float t = ld(xp + j); s1 += t; s2 = fmaf(t, t, s2); }
     s1 = block_sum(s1, red);
     s2 = block_sum(s2, red);
-    const float mean = s1 / (float)width;
-    const float sv = sqrtf(__fadd_rn(__fadd_rn(__fdiv_rn(__fsub_rn(s2, __fmul_rn(__fmul_rn(2.f, s1), mean)), (float)width), __fmul_rn(mean, mean)), eps));
+    ln_stats(s1, s2, width, eps, mean, sv);
     const float inv = 1.f / sv;
     float a = 0.f, b = 0.f;     // sum g, sum g * xhat
     for (int j = threadIdx.x; j < width; j += blockDim.x) {
@@ -819,6 +921,16 @@ __global__ void __launch_bounds__(128) layernorm_bw_cols_kernel(const T *__restr
 template <class T> void layernorm_bw(Scope &sc, const T *x, const T *w, const T *dy, T *dx, T *dw, T *db, int rows, int width, float eps)
 {
     if (rows <= 0) return;
+    if (width <= 1024) {
+        // a warp per row while that gives at most one CTA per two SMs (the last CTA adds that many sums), more rows per warp beyond
+        const int rows_per_cta = std::max(8, ceil_div(ceil_div(rows, sm_count() / 2), 8) * 8), ctas = ceil_div(rows, rows_per_cta);
+        float *part = sc.scratch<float>((size_t)ctas * 2 * width);
+        if (!part) return;
+#define TL_LN_BW(NV) TL_LAUNCH((layernorm_bw_warp_kernel<T, NV>), ctas, 256, 0, x, w, dy, dx, part, dw, db, rows, width, rows_per_cta, eps)
+        if (width <= 128) TL_LN_BW(4); else if (width <= 256) TL_LN_BW(8); else if (width <= 512) TL_LN_BW(16); else TL_LN_BW(32);
+#undef TL_LN_BW
+        return;
+    }
     float2 *stats = sc.scratch<float2>((size_t)rows);
     if (!stats) return;
     TL_LAUNCH((layernorm_bw_rows_kernel<T>), rows, 128, 0, x, w, dy, dx, stats, width, eps);
@@ -828,6 +940,13 @@ template <class T> void layernorm_bw(Scope &sc, const T *x, const T *w, const T 
 template <class T> void layernorm_fw(const T *x, T *y, const T *w, const T *b, int rows, int width, float eps)
 {
     if (rows <= 0) return;
+    if (width <= 1024) {
+        const int warps = rows >= 8 * sm_count() ? 8 : 2;    // few rows: spread them over the SMs
+#define TL_LN_FW(NV) TL_LAUNCH((layernorm_fw_warp_kernel<T, NV>), ceil_div(rows, warps), 32 * warps, 0, x, y, w, b, rows, width, eps)
+        if (width <= 128) TL_LN_FW(4); else if (width <= 256) TL_LN_FW(8); else if (width <= 512) TL_LN_FW(16); else TL_LN_FW(32);
+#undef TL_LN_FW
+        return;
+    }
     TL_LAUNCH((layernorm_fw_kernel<T>), rows, 128, 0, x, y, w, b, width, eps);
 }
 
@@ -854,23 +973,50 @@ template <class T> void mean_std(const T *x, T *mean, T *var, T *stdev, int D, f
 
 // ------------------------------------------------------------------ losses
 // MSE: loss = sum (1/dim) (t - y)^2; dy = (1/dim) * 2 * (y - t)   [ref: lib/sources/pulp_losses_fp32.c:214-275]
+// Long outputs of few streams are cut into `parts` pieces, one CTA each; the CTA of a stream that finishes last adds the
+// pieces in order (one CTA walked the 65 536 outputs of the encoder block in 60 us, 64 CTAs take 3).
+static __device__ unsigned mse_tickets[64];                  // one per stream; zero between launches
 template <class T>
-__global__ void __launch_bounds__(256) mse_fw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ loss, int dim)
+__global__ void __launch_bounds__(256) mse_fw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ loss, float *__restrict__ part, int dim, int parts)
 {
     __shared__ float red[33];
-    const T *yp = y + (long long)blockIdx.x * dim, *tp = t + (long long)blockIdx.x * dim;
+    __shared__ unsigned ticket_s;
+    const long long stream = blockIdx.y;
+    const T *yp = y + stream * dim, *tp = t + stream * dim;
     const float meanval = 1.0f / (float)dim;
+    const int per = (dim + parts - 1) / parts, i0 = blockIdx.x * per, i1 = min(dim, i0 + per);
     float s = 0.f;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) { float d = ld(tp + i) - ld(yp + i); s += meanval * d * d; }
+#pragma unroll 4
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) { float d = ld(tp + i) - ld(yp + i); s += meanval * d * d; }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) st(loss + blockIdx.x, s);
+    if (parts == 1) { if (threadIdx.x == 0) st(loss + stream, s); return; }
+    if (threadIdx.x == 0) {
+        __stcg(part + stream * parts + blockIdx.x, s);
+        __threadfence();
+        ticket_s = atomicAdd(&mse_tickets[stream], 1u);
+    }
+    __syncthreads();
+    if (ticket_s != (unsigned)(parts - 1)) return;
+    __threadfence();
+    s = threadIdx.x < parts ? __ldcg(part + stream * parts + threadIdx.x) : 0.f;
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) { st(loss + stream, s); mse_tickets[stream] = 0; }
 }
 template <class T> __global__ void mse_bw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ dy, int dim, long long total)
 {
     const float meanval = 1.0f / (float)dim;
     GRID_STRIDE(i, total) st(dy + i, __fmul_rn(__fmul_rn(meanval, 2.0f), __fsub_rn(ld(y + i), ld(t + i))));
 }
-template <class T> void mse_fw(const T *y, const T *t, T *loss, int dim, int n) { if (n > 0) TL_LAUNCH((mse_fw_kernel<T>), n, 256, 0, y, t, loss, dim); }
+template <class T> void mse_fw(const T *y, const T *t, T *loss, int dim, int n)
+{
+    if (n <= 0) return;
+    Scope sc;
+    int parts = n <= 64 ? std::min(ceil_div(dim, 1024), 128) : 1;
+    float *part = parts > 1 ? sc.scratch<float>((size_t)n * parts) : nullptr;
+    if (!part) parts = 1;
+    for (int s0 = 0; s0 < n; s0 += 65535)                   // a grid has 65 535 rows at most
+        TL_LAUNCH((mse_fw_kernel<T>), dim3(parts, std::min(n - s0, 65535)), 256, 0, y + (long long)s0 * dim, t + (long long)s0 * dim, loss + s0, part, dim, parts);
+}
 template <class T> void mse_bw(const T *y, const T *t, T *dy, int dim, int n)
 {
     long long total = (long long)dim * n;

@@ -10,7 +10,7 @@
 // its share of K; the partial tiles meet in shared memory in warp order).  Outputs with fewer tiles than SMs are further
 // split along K over CTAs; the CTA of a tile that finishes last adds the splits in order, so results do not depend on
 // scheduling.
-//   fp32: FFMA (full fp32 products and sums), 8 x 4 or 8 x 8 results per lane, operands read as 16-byte vectors along
+//   fp32: FFMA (full fp32 products and sums), 4 x 4 results per lane, operands read as 16-byte vectors along
 //         whichever of k / row is contiguous in memory: no transposition on the way into shared memory.
 //   fp16: mma.sync.m16n8k16 with fp32 accumulation, fragments by ldmatrix (plain for K-contiguous operands, .trans for
 //         row-contiguous ones).  A tcgen05 tile needs 128 rows and a barrier/TMEM set-up that costs more than these
@@ -463,14 +463,18 @@ template <class T> void gemm_group(const GemmGroup<T> *list, int count)
     if (!n) return;
     Scope sc;
     if (!sc.ok()) return;
-    // 64 x 64 tiles once they fill the GPU, 32 x 32 below; fp32 outputs with too few of those take 16 x 32
+    // Tiles by how many of them the group has (measured over 256^3, 300x400x500, 16x2048x4096, 17x3000x40, 2000x64x300 ...):
+    // small tiles while they are needed to occupy the SMs, larger ones as soon as they come to about one and a half per SM.
+    // fp32, us: 256^3 4.8 with 16 x 32 tiles, 6.1 with 32 x 32; 2000x50x2000 46 and 35.  fp16: 128x512x128 4.9 with 16 x 32,
+    // 5.7 with 32 x 32, 9.7 with 64 x 64; 1000x60x1000 11.8, 10.3, 6.4.  Four warps per CTA, several CTAs per SM: eight warps
+    // on one 32 x 32 fp32 tile cost 20 to 40 % more (shorter runs of FMAs between barriers).
     if constexpr (sizeof(T) == 2) {
         if (tiles64 >= sm_count()) gg_launch<T, 64, 64, 2, 2, 1, 64, 3, 3>(sc, live, n);
-        else gg_launch<T, 32, 32, 1, 1, 4, 128, 3, 4>(sc, live, n);
+        else if (tiles32 >= sm_count()) gg_launch<T, 32, 32, 1, 1, 4, 128, 3, 4>(sc, live, n);
+        else gg_launch<T, 16, 32, 1, 1, 4, 128, 3, 4>(sc, live, n);
     } else {
-        if (tiles64 >= sm_count()) gg_launch<T, 64, 64, 2, 2, 2, 32, 3, 2>(sc, live, n);
-        else if (tiles32 >= sm_count()) gg_launch<T, 32, 32, 1, 1, 8, 64, 3, 2>(sc, live, n);
-        else gg_launch<T, 16, 32, 1, 1, 8, 64, 3, 2>(sc, live, n);
+        if (2 * tiles32 >= 3 * sm_count()) gg_launch<T, 32, 32, 2, 1, 2, 64, 3, 4>(sc, live, n);
+        else gg_launch<T, 16, 32, 1, 1, 4, 64, 3, 4>(sc, live, n);
     }
 }
 template void gemm_group<float>(const GemmGroup<float> *, int);
