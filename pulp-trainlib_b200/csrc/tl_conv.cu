@@ -5,6 +5,8 @@
 // in shared memory, so no column buffer ever exists in global memory.  All kernels take
 // `n` independent batch-1 streams ([n][C][H][W] activations, shared weights).
 #include "tl_kernels.h"
+#include "tl_reduce.cuh"
+#include <algorithm>
 
 namespace tl {
 
@@ -406,7 +408,9 @@ template <> bool try_tc_ig<float>(Scope &sc, const ConvGeom &g, const float *dy,
 template <class T> void conv_fw(Scope &sc, const ConvGeom &g, const T *x, const T *w, const T *bias, T *y)
 {
     if (!g.depthwise && try_tc_fw<T>(sc, g, x, w, bias, y)) return;
+    if (!g.depthwise && conv_mma_fw<T>(g, x, w, bias, y)) { profile_add_flops(conv_flops(g)); return; }
     if (g.depthwise) {
+        if (dw_planes<T>(g, x, w, y, false)) return;
         long long total = (long long)g.n * g.Cin * g.Hout * g.Wout;
         int blocks = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 16);
         TL_LAUNCH((dw_fw_kernel<T>), blocks, 256, 0, g, x, w, y);
@@ -528,7 +532,9 @@ template <class T> void conv_ig_accumulate(Scope &sc, const ConvGeom &g, const T
 template <class T> void conv_ig(Scope &sc, const ConvGeom &g, const T *dy, const T *w, T *dx)
 {
     if (!g.depthwise && try_tc_ig<T>(sc, g, dy, w, dx)) return;
+    if (!g.depthwise && conv_mma_ig<T>(g, dy, w, dx)) { profile_add_flops(conv_flops(g)); return; }
     if (g.depthwise) {
+        if (dw_planes<T>(g, dy, w, dx, true)) return;
         long long total = (long long)g.n * g.Cin * g.Hin * g.Win;
         int blocks = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 16);
         TL_LAUNCH((dw_ig_kernel<T>), blocks, 256, 0, g, dy, w, dx);
@@ -913,21 +919,30 @@ __global__ void __launch_bounds__(256) conv_wg_direct_kernel(ConvGeom g, const T
     if (threadIdx.x == 0) st(dw + blockIdx.x, red[0]);
 }
 
-// db[co] = sum over streams and pixels of dY[co]   [ref: lib/sources/pulp_conv_naive_fp32.c:354-361]
+// db[co] = sum over streams and pixels of dY[co]   [ref: lib/sources/pulp_conv_naive_fp32.c:354-361]: the streams of a channel
+// are shared out to gridDim.y CTAs, the partial sums go through the fixed-order reduction (one CTA per channel took 108 us for
+// 48 channels of 28 x 28 x 128 streams).
 template <class T>
-__global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ dy, T *__restrict__ db, int n, int C, long long plane)
+__global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ dy, float *__restrict__ part, int n, int C, int plane)
 {
-    __shared__ float red[256];
-    const int c = blockIdx.x;
+    __shared__ float red[33];
+    const int c = blockIdx.x, per = (n + gridDim.y - 1) / gridDim.y, s0 = blockIdx.y * per, s1 = min(n, s0 + per);
     float acc = 0.f;
-    for (long long e = threadIdx.x; e < plane * n; e += blockDim.x) {
-        long long s = e / plane, p = e % plane;
-        acc += ld(dy + (s * C + c) * plane + p);
+    for (int s = s0; s < s1; s++) {
+        const T *p = dy + ((long long)s * C + c) * plane;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < plane; e += 256) acc += ld(p + e);
     }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) { if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o]; __syncthreads(); }
-    if (threadIdx.x == 0) st(db + c, red[0]);
+    acc = block_sum(acc, red);
+    if (threadIdx.x == 0) part[(long long)blockIdx.y * C + c] = acc;
+}
+template <class T> static void channel_sum(Scope &sc, const T *dy, T *db, int n, int C, int plane)
+{
+    const int groups = std::max(1, std::min(n, ceil_div(4 * sm_count(), C)));
+    float *part = sc.scratch<float>((size_t)groups * C);
+    if (!part) return;
+    TL_LAUNCH((channel_sum_kernel<T>), dim3(C, groups), 256, 0, dy, part, n, C, plane);
+    reduce_partials<T>(part, db, C, groups, false);
 }
 
 // tensor-core weight gradient (tl_conv_wgt.cu) where its geometry applies and the work is large enough to fill the GPU
@@ -968,11 +983,36 @@ template <> bool try_1x1_wg<float>(Scope &sc, const ConvGeom &g, const float *x,
     return true;
 }
 
+// weight gradient on mma.sync: per-CTA partials + the fixed-order reduction
+template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw)
+{
+    int groups = 0;
+    const long long nw = (long long)g.Cout * g.Cin * g.Hk * g.Wk;
+    const int most = (int)std::min<long long>(1 << 20, std::max<long long>(1, (64ll << 20) / nw));     // partial results: 256 MB at most
+    if (!conv_mma_wg<T>(g, x, dy, nullptr, most, &groups, true)) return false;
+    bool deferred;
+    float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred);
+    if (!part) return false;
+    if (!conv_mma_wg<T>(g, x, dy, part, most, &groups, false)) return false;
+    profile_add_flops(conv_flops(g));
+    reduce_partials<T>(part, dw, nw, groups, deferred);
+    return true;
+}
+
 template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw, T *dbias)
 {
-    if (dbias) TL_LAUNCH((channel_sum_kernel<T>), g.Cout, 256, 0, dy, dbias, g.n, g.Cout, (long long)g.Hout * g.Wout);
+    if (dbias) channel_sum<T>(sc, dy, dbias, g.n, g.Cout, g.Hout * g.Wout);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise) {
+        int groups = 0;
+        if (dw_wg_planes<T>(g, x, dy, nullptr, groups, true)) {
+            bool deferred;
+            float *part = partials_alloc<T>(sc, (size_t)groups * g.Cin * KK, deferred);
+            if (!part) return;
+            dw_wg_planes<T>(g, x, dy, part, groups, false);
+            reduce_partials<T>(part, dw, (long long)g.Cin * KK, groups, deferred);
+            return;
+        }
         TL_LAUNCH((dw_wg_kernel<T>), g.Cin * KK, 256, 0, g, x, dy, dw);
         return;
     }
@@ -981,6 +1021,9 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
     const bool k3 = g.Hk == 3 && g.Wk == 3 && g.padL == 1, k1 = g.Hk == 1 && g.Wk == 1 && g.padL == 0 && g.padU == 0;
     if (try_tc_wg<T>(sc, g, x, dy, dw)) return;
     if (try_1x1_wg<T>(sc, g, x, dy, dw)) return;
+    // the register-tiled FFMA kernel below keeps 3x3 fp32 layers of 8, 16 and 32 pixel rows (100 streams of 16 -> 32 on 32 x 32: 31 us
+    // against 34 us on mma.sync)
+    if (!(sizeof(T) == 4 && k3) && try_mma_wg<T>(sc, g, x, dy, dw)) return;
     if ((k3 || k1) && g.sh == g.sw && (g.sh == 1 || g.sh == 2) && g.Win == g.sw * g.Wout && (g.Wout == 8 || g.Wout == 16 || g.Wout == 32)) {
         // about 256 (stride 1) or 128 (stride 2) pixels per item: whole output rows, two streams for 8-pixel rows.
         // The item shape is part of the kernel type: (TW, TH, S_T) = (32, 8, 1), (16, 16, 1), (8, 8, 2) for stride 1
@@ -1023,6 +1066,7 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
             return;
         }
     }
+    if (sizeof(T) == 4 && k3 && try_mma_wg<T>(sc, g, x, dy, dw)) return;
     // pixel tile: whole rows, about 256 pixels
     int TW = g.Wout < 64 ? g.Wout : 64;
     int TH = 256 / TW; if (TH < 1) TH = 1; if (TH > g.Hout) TH = g.Hout;

@@ -141,6 +141,13 @@ template <class T> inline float *partials_alloc(Scope &sc, size_t floats, bool &
 bool conv1x1s_fw(const ConvGeom &g, const float *x, const float *w, const float *bias, float *y);
 bool conv1x1s_ig(const ConvGeom &g, const float *dy, const float *w, float *dx);   // dX += gradient
 bool conv1x1s_wg(const ConvGeom &g, const float *x, const float *dy, float *part, int part_groups, int *groups_out, bool dry_run);
+// any-shape convolutions on mma.sync, fp16 and 3xTF32 (tl_conv_mma.cu); false = geometry not covered, nothing launched
+template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, const T *bias, T *y);
+template <class T> bool conv_mma_ig(const ConvGeom &g, const T *dy, const T *w, T *dx);
+template <class T> bool conv_mma_wg(const ConvGeom &g, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry_run);
+// depthwise planes through shared memory (tl_conv_dw.cu)
+template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T *dst, bool ig);
+template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy, float *part, int &groups, bool dry_run);
 // tensor-core weight gradient (tl_conv_wgt.cu): partial results per CTA into `part`; false = geometry not covered
 bool conv_wgt_run(const float *x, const float *dy, float *part, int part_groups, int *groups_out, long long *group_floats_out, int n, int Cin, int Cout, int H,
                   int W, int stride, bool dry_run);
