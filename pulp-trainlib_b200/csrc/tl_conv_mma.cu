@@ -30,43 +30,101 @@ __device__ __forceinline__ void cm_ldsm(uint32_t (&r)[4], uint32_t addr) { asm v
 __device__ __forceinline__ void cm_ldsm_t(uint32_t (&r)[4], uint32_t addr) { asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr)); }
 __device__ __forceinline__ void cm_hmma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void cm_tmma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t cm_lds32(uint32_t addr) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr)); return v; }
 
 // A patch of the source plane(s), channels-last: `streams` x rows x cols pixels of `chans` channels (a multiple of 8 fp16 / 4
 // fp32; channels at or past c_left read as zero).  One item = one pixel x 16 bytes of channels: neighbouring threads take
-// neighbouring pixels, so the per-channel loads are coalesced and the 16-byte store is conflict-free.
+// neighbouring pixels, so the per-channel loads are coalesced and the 16-byte store is conflict-free.  Addresses are a
+// CTA-uniform base plus a 32-bit byte offset (the host keeps a tile's span below 4 GB).
 template <class T, int NT>
-__device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams, int streams_left, int rows, int cols, CmDiv dcols, CmDiv drc, CmDiv dpix,
-                                         int row0, int col0, int H, int W, int chans, int c_left, long long cstride, long long sstride, uint32_t pitch)
+__device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams, int streams_left, int rows, int cols, CmDiv dcols,
+                                         int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch)
 {
-    constexpr int G = 16 / (int)sizeof(T);
-    const int pix = streams * rows * cols, items = pix * (chans / G);
-    for (int e = threadIdx.x; e < items; e += NT) {
-        const int g = cm_quot(e, dpix), p = e - g * pix;                   // channel group, pixel of the patch
-        const int st = cm_quot(p, drc), rc = p - st * drc.d, r = cm_quot(rc, dcols), c = rc - r * cols;
-        const int h = row0 + r, w = col0 + c;
-        const bool ok = st < streams_left && (unsigned)h < (unsigned)H && (unsigned)w < (unsigned)W;
-        const T *s = src + st * sstride + (long long)(g * G) * cstride + (ok ? h * W + w : 0);
-        uint32_t v[4];
+    constexpr int SZ = (int)sizeof(T);
+    const char *base = reinterpret_cast<const char *>(src);
+    const int groups = chans >> 3, lane = threadIdx.x & 31;
+    const uint32_t cs = cstride * SZ;
+    // Blocks of 32 items and groups of eight channels, warp by warp (both uniform in a warp); all loads of an item are issued
+    // before its first store.
+    if ((W & 1) == 0 && ((cstride | sstride) & 1) == 0 && (reinterpret_cast<uintptr_t>(base) & (2 * SZ - 1)) == 0) {
+        // even rows: an item is two neighbouring pixels from an even column (both inside the image or both outside), one load per
+        // channel for the two
+        const int w_even = col0 & ~1, half = (col0 + cols + 1 - w_even) >> 1, rc_n = rows * half, items = streams * rc_n;
+        const CmDiv dhalf = cm_div_dev(half);
+        const int blocks = (items + 31) >> 5;
+        int g = 0, blk = threadIdx.x >> 5;
+        while (blk >= blocks) { blk -= blocks; g++; }
+        for (; g < groups;) {
+            const int p = blk * 32 + lane;
+            int st = 0, rc = p;
+            if (streams > 1) { st = p / rc_n; rc = p - st * rc_n; }
+            const int r = rows > 1 ? cm_quot(rc, dhalf) : 0, w = w_even + 2 * (rc - r * half), h = row0 + r, c = w - col0;
+            const bool in = p < items;
+            const bool ok = in && st < streams_left && (unsigned)h < (unsigned)H && (unsigned)w < (unsigned)W;
+            uint32_t off = ok ? ((uint32_t)st * sstride + (uint32_t)(h * W + w)) * SZ + (uint32_t)(g * 8) * cs : 0u;
+            const int left = ok ? c_left - g * 8 : 0;
+            const uint32_t to = sm + (uint32_t)((st * rows + r) * cols + c) * pitch + (uint32_t)g * (8u * SZ);
+            if constexpr (sizeof(T) == 2) {
+                uint32_t e[8], v0[4], v1[4];
+#pragma unroll
+                for (int q = 0; q < 8; q++, off += cs) e[q] = q < left ? *reinterpret_cast<const uint32_t *>(base + off) : 0u;
+#pragma unroll
+                for (int q = 0; q < 4; q++) { v0[q] = __byte_perm(e[2 * q], e[2 * q + 1], 0x5410); v1[q] = __byte_perm(e[2 * q], e[2 * q + 1], 0x7632); }
+                if (in && c >= 0) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(v0[0]), "r"(v0[1]), "r"(v0[2]), "r"(v0[3]) : "memory");
+                if (in && c + 1 < cols) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + pitch), "r"(v1[0]), "r"(v1[1]), "r"(v1[2]), "r"(v1[3]) : "memory");
+            } else {
+                float2 e[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++, off += cs) e[q] = q < left ? *reinterpret_cast<const float2 *>(base + off) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    if (in && c >= 0) asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 16u * q), "f"(e[4 * q].x), "f"(e[4 * q + 1].x), "f"(e[4 * q + 2].x), "f"(e[4 * q + 3].x) : "memory");
+                    if (in && c + 1 < cols) asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + pitch + 16u * q), "f"(e[4 * q].y), "f"(e[4 * q + 1].y), "f"(e[4 * q + 2].y), "f"(e[4 * q + 3].y) : "memory");
+                }
+            }
+            blk += NT / 32;
+            while (blk >= blocks) { blk -= blocks; g++; }
+        }
+        return;
+    }
+    const int rc_n = rows * cols, pix = streams * rc_n, blocks = (pix + 31) >> 5;
+    int g = 0, blk = threadIdx.x >> 5;
+    while (blk >= blocks) { blk -= blocks; g++; }
+    while (g < groups) {
+        const int p = blk * 32 + lane;
+        int st = 0, rc = p;
+        if (streams > 1) { st = p / rc_n; rc = p - st * rc_n; }
+        const int r = rows > 1 ? cm_quot(rc, dcols) : 0, c = rc - r * cols, h = row0 + r, w = col0 + c;
+        const bool ok = p < pix && st < streams_left && (unsigned)h < (unsigned)H && (unsigned)w < (unsigned)W;
+        uint32_t off = ok ? ((uint32_t)st * sstride + (uint32_t)(h * W + w)) * SZ + (uint32_t)(g * 8) * cs : 0u;
+        const int left = ok ? c_left - g * 8 : 0;
+        constexpr int R = 2 * SZ;                                          // 32-bit registers of an item
+        uint32_t v[R];
         if constexpr (sizeof(T) == 2) {
-            unsigned short u[8];
+            unsigned short e[8];
 #pragma unroll
-            for (int q = 0; q < 8; q++) u[q] = (ok && g * G + q < c_left) ? *reinterpret_cast<const unsigned short *>(s + q * cstride) : (unsigned short)0;
+            for (int q = 0; q < 8; q++, off += cs) e[q] = q < left ? *reinterpret_cast<const unsigned short *>(base + off) : (unsigned short)0;
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = (uint32_t)u[2 * q] | ((uint32_t)u[2 * q + 1] << 16);
+            for (int q = 0; q < 4; q++) v[q] = (uint32_t)e[2 * q] | ((uint32_t)e[2 * q + 1] << 16);
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = (ok && g * G + q < c_left) ? *reinterpret_cast<const uint32_t *>(s + q * cstride) : 0u;
+            for (int q = 0; q < 8; q++, off += cs) v[q] = q < left ? *reinterpret_cast<const uint32_t *>(base + off) : 0u;
         }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sm + (uint32_t)p * pitch + (uint32_t)g * 16u), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+        if (p < pix) {
+#pragma unroll
+            for (int q = 0; q < R / 4; q++)
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sm + (uint32_t)p * pitch + (uint32_t)g * (8u * SZ) + 16u * q), "r"(v[4 * q]), "r"(v[4 * q + 1]), "r"(v[4 * q + 2]), "r"(v[4 * q + 3]) : "memory");
+        }
+        blk += NT / 32;
+        while (blk >= blocks) { blk -= blocks; g++; }
     }
 }
 
@@ -74,7 +132,7 @@ __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams,
 // dst[m][oy0 + i osy][ox0 + j osx] = sum over taps t and source channels k of src[k][i S + dr_t][j S + dc_t] W[m][k][t].
 // Forward: S = the stride, one class.  Input gradient: a class per parity (oy0, ox0) of the input pixels (osy = osx = the
 // stride, S = 1), whose taps are the ones that reach that parity; the weights are read with the channel roles swapped.
-struct CmClass { int Hc, Wc, oy0, ox0, tap0, ntaps, dr_min, dc_min, cols; CmDiv dW, dcols; };
+struct CmClass { int Hc, Wc, oy0, ox0, tap0, ntaps, dr_min, dc_min, cols, wide_cols; CmDiv dW, dcols; };
 struct CmFwd {
     const void *src, *w, *bias; void *dst;
     int n, Cs, Hs, Ws, Cd, oH, oW, S, osy, osx, KK;
@@ -84,7 +142,7 @@ struct CmFwd {
     int st_tile;                             // streams per tile (planes smaller than a tile), else 1
     int CKS, groups, cblk, resident;         // channels staged at a time, how often, k-steps per chain; weights loaded once per CTA
     uint32_t pitch, wpitch, w_off;           // bytes: pixel, weight row; offset of the weights behind the patch
-    int rows_max;
+    int rows_max, linear, pairs;
 };
 
 template <class T, int MT, int WM, int WN, int WK, int BN>
@@ -101,58 +159,76 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
     const int m0 = blockIdx.y * BM;
     const uint32_t patch = (uint32_t)__cvta_generic_to_shared(cm_smem), wsm = patch + p.w_off;
     const int P = c.Hc * c.Wc, ntaps = c.ntaps;
-    const int tiles_s = P < BN ? 1 : (P + BN - 1) / BN;                     // tiles of one stream
+    // rows longer than a tile are cut into tiles of their own: a tile then stages its columns only
+    const bool wide = c.Wc > BN;
+    const int tiles_r = wide ? (c.Wc + BN - 1) / BN : 0;
+    const int tiles_s = P < BN ? 1 : wide ? c.Hc * tiles_r : (P + BN - 1) / BN;      // tiles of one stream
+    const int cols = wide ? c.wide_cols : c.cols;
     const int tiles = (P < BN ? (p.n + p.st_tile - 1) / p.st_tile : p.n * tiles_s);
     if ((int)blockIdx.x >= tiles) return;
 
     for (int t = tid; t < p.KK; t += NT) tap_of[t] = -1;
     __syncthreads();
     for (int t = tid; t < ntaps; t += NT) {
-        tap_off[t] = ((p.dr[c.tap0 + t] - c.dr_min) * c.cols + (p.dc[c.tap0 + t] - c.dc_min)) * (int)p.pitch;
+        tap_off[t] = ((p.dr[c.tap0 + t] - c.dr_min) * cols + (p.dc[c.tap0 + t] - c.dc_min)) * (int)p.pitch;
         tap_of[p.widx[c.tap0 + t]] = t;
     }
     __syncthreads();
 
-    // weights of channels k0 .. k0 + kc as [tap][BM][wpitch], one contiguous source run per row (or per contraction channel)
+    // Weights of channels k0 .. k0 + kc as [tap][BM][wpitch].  A thread takes one (m, k) pair (fp16: two neighbouring k), walks
+    // its taps, which are contiguous in memory, nine loads in flight, and stores each to its tap's matrix: one or two
+    // instructions per weight.  (Dealing single weights to threads cost twenty: a third of the kernel's time.)
     auto load_weights = [&](int k0, int kc) {
+        constexpr int V = HALF ? 2 : 1;
+        const int kp = kc / V, items = kp * BM, KK = p.KK;
+        const bool m_first = p.wm < p.wk;                                           // neighbouring threads take neighbouring memory
+        const CmDiv dq = cm_div_dev(m_first ? BM : kp);
+        const uint32_t s_tap = (uint32_t)BM * p.wpitch;
         const T *w = reinterpret_cast<const T *>(p.w);
-        const CmDiv dKK = cm_div_dev(p.KK);
-        if (p.wk == p.KK) {
-            const int run = kc * p.KK, live = min(kc, p.Cs - k0) * p.KK;
-            for (int m = warp; m < BM; m += NT / 32) {
-                const T *row = w + (long long)(m0 + m) * p.wm + (long long)k0 * p.KK;
-                const bool in = m0 + m < p.Cd;
-                for (int e = lane; e < run; e += 32) {
-                    const int k = cm_quot(e, dKK), t = tap_of[e - k * p.KK];
-                    const T v = (in && e < live) ? row[e] : T(0.f);
-                    if (t >= 0) *reinterpret_cast<T *>(cm_smem + p.w_off + (size_t)((t * BM + m) * (int)p.wpitch + k * SZ)) = v;
-                }
-            }
-        } else {
-            const int run = BM * p.KK, live = min(BM, p.Cd - m0) * p.KK;
-            for (int k = warp; k < kc; k += NT / 32) {
-                const T *row = w + (long long)(k0 + k) * p.wk + (long long)m0 * p.KK;
-                const bool in = k0 + k < p.Cs;
-                for (int e = lane; e < run; e += 32) {
-                    const int m = cm_quot(e, dKK), t = tap_of[e - m * p.KK];
-                    const T v = (in && e < live) ? row[e] : T(0.f);
-                    if (t >= 0) *reinterpret_cast<T *>(cm_smem + p.w_off + (size_t)((t * BM + m) * (int)p.wpitch + k * SZ)) = v;
+        for (int e = tid; e < items; e += NT) {
+            const int eq = cm_quot(e, dq), er = e - eq * dq.d, m = m_first ? er : eq, k = (m_first ? eq : er) * V;
+            const bool ok0 = m0 + m < p.Cd && k0 + k < p.Cs, ok1 = ok0 && k0 + k + 1 < p.Cs;
+            const T *src = ok0 ? w + (long long)(m0 + m) * p.wm + (long long)(k0 + k) * p.wk : w;
+            const uint32_t to = wsm + (uint32_t)m * p.wpitch + (uint32_t)(k * SZ);
+            for (int t0 = 0; t0 < KK; t0 += 9) {
+                if constexpr (HALF) {
+                    unsigned short lo[9], hi[9];
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        const bool in = t0 + u < KK;
+                        lo[u] = in && ok0 ? *reinterpret_cast<const unsigned short *>(src + t0 + u) : (unsigned short)0;
+                        hi[u] = in && ok1 ? *reinterpret_cast<const unsigned short *>(src + p.wk + t0 + u) : (unsigned short)0;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        const int t = t0 + u < KK ? tap_of[t0 + u] : -1;
+                        if (t >= 0) asm volatile("st.shared.b32 [%0], %1;" ::"r"(to + (uint32_t)t * s_tap), "r"((uint32_t)lo[u] | ((uint32_t)hi[u] << 16)) : "memory");
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 9; u++) {
+                        const int t = t0 + u < KK ? tap_of[t0 + u] : -1;
+                        if (t >= 0) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + (uint32_t)t * s_tap), "l"(ok0 ? src + t0 + u : src), "r"(ok0 ? 4 : 0) : "memory");
+                    }
                 }
             }
         }
+        if constexpr (!HALF) asm volatile("cp.async.wait_all;" ::: "memory");
     };
     if (p.resident) load_weights(0, p.groups * p.CKS);
 
-    const CmDiv dcols = c.dcols, dW = c.dW;
+    const CmDiv dcols = wide ? cm_div_dev(cols) : c.dcols, dW = c.dW;
     const long long src_plane = (long long)p.Hs * p.Ws, dst_plane = (long long)p.oH * p.oW;
 
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int s0 = P < BN ? tile * p.st_tile : tile / tiles_s, p0 = P < BN ? 0 : (tile % tiles_s) * BN;
+        const int s0 = P < BN ? tile * p.st_tile : tile / tiles_s, ts = tile % tiles_s;
+        const int row_t = wide ? ts / tiles_r : 0, col_t = wide ? (ts - row_t * tiles_r) * BN : 0;
+        const int p0 = P < BN ? 0 : wide ? row_t * c.Wc + col_t : ts * BN;
         const int st_n = P < BN ? p.st_tile : 1;
-        const int i0 = cm_quot(p0, dW);
-        const int live = P < BN ? min(st_n, p.n - s0) * P : min(BN, P - p0);        // output pixels of this tile
-        const int last = P < BN ? P - 1 : min(p0 + BN, P) - 1;
-        const int rows = (cm_quot(last, dW) - i0) * p.S + p.rows_max;               // rows_max: rows that one output row needs
+        const int i0 = wide ? row_t : cm_quot(p0, dW);
+        const int live = P < BN ? min(st_n, p.n - s0) * P : wide ? min(BN, c.Wc - col_t) : min(BN, P - p0);        // output pixels of this tile
+        const int last = P < BN ? P - 1 : p0 + live - 1;
+        const int rows = ((wide ? i0 : cm_quot(last, dW)) - i0) * p.S + p.rows_max; // rows_max: rows that one output row needs
         // start addresses (in the patch) of the pixels this lane supplies fragments for
         constexpr int NB = HALF ? N8 / 2 : N8;
         uint32_t pix[NB];
@@ -162,8 +238,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
             if (q >= live) q = 0;
             int st = 0, pp = p0 + q;
             if (P < BN) { st = q / P; pp = q - st * P; }
-            const int i = cm_quot(pp, dW), jj = pp - i * c.Wc;
-            pix[j] = patch + (uint32_t)(((st * rows + (i - i0) * p.S) * c.cols + jj * p.S) * (int)p.pitch) + (HALF ? (uint32_t)((lane >> 3) & 1) * 16u : (uint32_t)(lane & 3) * 4u);
+            const int i = wide ? i0 : cm_quot(pp, dW), jj = pp - i * c.Wc - col_t;
+            pix[j] = patch + (uint32_t)(((st * rows + (i - i0) * p.S) * cols + jj * p.S) * (int)p.pitch) + (HALF ? (uint32_t)((lane >> 3) & 1) * 16u : (uint32_t)(lane & 3) * 4u);
         }
         float acc[MT][N8][4];
 #pragma unroll
@@ -177,9 +253,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
             __syncthreads();                                                        // the patch (and the weights) are free again
             const int k0 = g * p.CKS;
             if (!p.resident) load_weights(k0, p.CKS);
-            const CmDiv drc = cm_div_dev(rows * c.cols), dpix = cm_div_dev(st_n * rows * c.cols);
-            cm_stage<T, NT>(patch, reinterpret_cast<const T *>(p.src) + ((long long)s0 * p.Cs + k0) * src_plane, st_n, p.n - s0, rows, c.cols, dcols, drc, dpix,
-                            i0 * p.S + c.dr_min, c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0, src_plane, (long long)p.Cs * src_plane, p.pitch);
+            cm_stage<T, NT>(patch, reinterpret_cast<const T *>(p.src) + ((long long)s0 * p.Cs + k0) * src_plane, st_n, p.n - s0, rows, cols, dcols,
+                            i0 * p.S + c.dr_min, col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0, (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
             __syncthreads();
             const uint32_t wg = wsm + (uint32_t)(p.resident ? k0 * SZ : 0);
             const int nck = p.CKS / CK, nblk = (nck + p.cblk - 1) / p.cblk;
@@ -217,14 +292,18 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
 #pragma unroll
                             for (int q = 0; q < 4; q++)                             // a0 (r, k), a1 (r + 8, k), a2 (r, k + 4), a3 (r + 8, k + 4)
                                 tc::split_tf32_fast(__uint_as_float(cm_lds32(wa + (uint32_t)(i * 16 + (q & 1) * 8) * p.wpitch + ck * 32u + (q >> 1) * 16u)), ah[i][q], al[i][q]);
+                        uint32_t bh[N8][2], bl[N8][2];
 #pragma unroll
-                        for (int j = 0; j < N8; j++) {
-                            uint32_t bh0, bl0, bh1, bl1;
-                            tc::split_tf32_fast(__uint_as_float(cm_lds32(pix[j] + toff + ck * 32u)), bh0, bl0);
-                            tc::split_tf32_fast(__uint_as_float(cm_lds32(pix[j] + toff + ck * 32u + 16u)), bh1, bl1);
+                        for (int j = 0; j < N8; j++)
 #pragma unroll
-                            for (int i = 0; i < MT; i++) { cm_tmma(tmp[i][j], al[i], bh0, bh1); cm_tmma(tmp[i][j], ah[i], bl0, bl1); cm_tmma(tmp[i][j], ah[i], bh0, bh1); }
-                        }
+                            for (int h = 0; h < 2; h++) tc::split_tf32_fast(__uint_as_float(cm_lds32(pix[j] + toff + ck * 32u + h * 16u)), bh[j][h], bl[j][h]);
+                        // the three terms of a product go to one accumulator: neighbouring instructions take different ones
+#pragma unroll
+                        for (int term = 0; term < 3; term++)
+#pragma unroll
+                            for (int j = 0; j < N8; j++)
+#pragma unroll
+                                for (int i = 0; i < MT; i++) cm_tmma(tmp[i][j], term == 0 ? al[i] : ah[i], term == 1 ? bl[j][0] : bh[j][0], term == 1 ? bl[j][1] : bh[j][1]);
                     }
 #pragma unroll
                     for (int i = 0; i < MT; i++)
@@ -260,35 +339,46 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
             if (wk > 0) continue;
         }
         // results: a lane holds pixel pairs of two rows (output channels) per 16 x 8 fragment
-        T *dst = reinterpret_cast<T *>(p.dst);
+        T *dst = reinterpret_cast<T *>(p.dst) + (long long)s0 * p.Cd * dst_plane + (long long)c.oy0 * p.oW + c.ox0;
         const T *bias = reinterpret_cast<const T *>(p.bias);
+        float bv[MT][2];
+        T *row[MT][2];
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int m = m0 + wm * 16 * MT + i * 16 + (lane >> 2) + h * 8;
+                row[i][h] = m < p.Cd ? dst + m * dst_plane : nullptr;
+                bv[i][h] = bias && m < p.Cd ? ld(bias + m) : 0.f;
+            }
 #pragma unroll
         for (int j = 0; j < N8; j++) {
             const int q0 = wn * TN + 8 * j + 2 * (lane & 3);
-            long long off[2];
+            if (q0 >= live) continue;
+            int off[2];
+            const bool second = q0 + 1 < live;
+            if (p.linear && P >= BN) { off[0] = p0 + q0; off[1] = off[0] + 1; }          // the class is the whole plane, pixels in memory order
+            else
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int q = min(q0 + h, live - 1);
-                int st = 0, pp = p0 + q;
-                if (P < BN) { st = q / P; pp = q - st * P; }
-                const int i = cm_quot(pp, dW), jj = pp - i * c.Wc;
-                off[h] = ((long long)(s0 + st) * p.Cd) * dst_plane + (long long)(c.oy0 + i * p.osy) * p.oW + c.ox0 + jj * p.osx;
-            }
+                for (int h = 0; h < 2; h++) {
+                    int st = 0, pp = p0 + q0 + (second ? h : 0);
+                    if (P < BN) { st = pp / P; pp -= st * P; }
+                    const int i = cm_quot(pp, dW), jj = pp - i * c.Wc;
+                    off[h] = st * p.Cd * (int)dst_plane + i * p.osy * p.oW + jj * p.osx;
+                }
+            const bool pair = p.pairs && off[1] == off[0] + 1;                          // (pairs: even planes and an aligned tensor)
 #pragma unroll
             for (int i = 0; i < MT; i++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int m = m0 + wm * 16 * MT + i * 16 + (lane >> 2) + h * 8;
-                    if (m >= p.Cd || q0 >= live) continue;
-                    const float bv = bias ? ld(bias + m) : 0.f;
-                    const float v0 = acc[i][j][2 * h] + bv, v1 = acc[i][j][2 * h + 1] + bv;
-                    T *d0 = dst + off[0] + m * dst_plane;
-                    if (q0 + 1 < live && off[1] == off[0] + 1 && (((uintptr_t)d0) & (2 * SZ - 1)) == 0) {
-                        if constexpr (HALF) *reinterpret_cast<__half2 *>(d0) = __floats2half2_rn(v0, v1);
-                        else *reinterpret_cast<float2 *>(d0) = make_float2(v0, v1);
+                    if (!row[i][h]) continue;
+                    const float v0 = acc[i][j][2 * h] + bv[i][h], v1 = acc[i][j][2 * h + 1] + bv[i][h];
+                    if (pair) {
+                        if constexpr (HALF) *reinterpret_cast<__half2 *>(row[i][h] + off[0]) = __floats2half2_rn(v0, v1);
+                        else *reinterpret_cast<float2 *>(row[i][h] + off[0]) = make_float2(v0, v1);
                     } else {
-                        st(d0, v0);
-                        if (q0 + 1 < live) st(dst + off[1] + m * dst_plane, v1);
+                        st(row[i][h] + off[0], v0);
+                        if (second) st(row[i][h] + off[1], v1);
                     }
                 }
         }
@@ -305,10 +395,13 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
     for (int i = 0; i < p.ncls; i++) {
         const CmClass &c = p.cls[i];
         const int P = c.Hc * c.Wc;
-        const int rows = (P < BN ? c.Hc - 1 : (BN + c.Wc - 2) / c.Wc) * p.S + p.rows_max;
-        pix = std::max(pix, (long long)p.st_tile * rows * c.cols);
+        const bool wide = c.Wc > BN;
+        if (!(wide && p.linear) && (long long)P * c.Wc >= (1ll << 32)) return false;          // (range of the quotients by multiplication)
+        p.cls[i].wide_cols = (BN - 1) * p.S + c.cols - (c.Wc - 1) * p.S;
+        const int rows = (wide ? 0 : P < BN ? c.Hc - 1 : (BN + c.Wc - 2) / c.Wc) * p.S + p.rows_max;
+        pix = std::max(pix, (long long)p.st_tile * rows * (wide ? p.cls[i].wide_cols : c.cols));
         taps = std::max(taps, c.ntaps);
-        tiles_max = std::max(tiles_max, P < BN ? ceil_div(p.n, p.st_tile) : (int)std::min<long long>((long long)p.n * ceil_div(P, BN), 1 << 30));
+        tiles_max = std::max(tiles_max, P < BN ? ceil_div(p.n, p.st_tile) : (int)std::min<long long>((long long)p.n * (wide ? (long long)c.Hc * ceil_div(c.Wc, BN) : ceil_div(P, BN)), 1 << 30));
     }
     const size_t red = WK > 1 ? (size_t)(WK - 1) * WM * WN * MT * (BN / WN / 8) * 512 : 0;
     auto plan = [&](int cks, bool resident, size_t limit) {
@@ -337,8 +430,8 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
     static size_t attr = 0;
     if (smem > attr) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM_MAX); attr = CM_SMEM_MAX; }
     const int co_tiles = ceil_div(p.Cd, BM);
-    const int slots = std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls));
-    const int rounds = ceil_div(tiles_max, slots), gx = ceil_div(tiles_max, rounds);
+    // every CTA slot taken: co-resident CTAs share an SM, so a last round that only some of them have costs less than idle slots
+    const int gx = std::min(tiles_max, std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls)));
     TL_LAUNCH((conv_mma_kernel<T, MT, WM, WN, WK, BN>), dim3(gx, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p);
     return true;
 }
@@ -347,6 +440,10 @@ template <class T> static bool conv_mma_dispatch(CmFwd &p)
 {
     constexpr int CK = sizeof(T) == 2 ? 16 : 8;
     const int cpad = ceil_div(p.Cs, CK) * CK;
+    // 32-bit offsets inside a tile
+    if ((long long)p.Cs * p.Hs * p.Ws * 16 >= (1ll << 29) || (long long)p.Cd * p.oH * p.oW * 16 >= (1ll << 29)) return false;
+    p.linear = p.ncls == 1 && p.osx == 1 && p.osy == 1;
+    p.pairs = p.linear && (p.oW * p.oH) % 2 == 0 && ((uintptr_t)p.dst) % (2 * sizeof(T)) == 0;
     long long tiles = 0;                                                   // 128-pixel tiles
     for (int i = 0; i < p.ncls; i++) tiles += ((long long)p.n * p.cls[i].Hc * p.cls[i].Wc + 127) / 128;
     // Few tiles (single streams): 16 x 32 result tiles whose taps and channels are dealt to four warps each, so that a layer of
@@ -357,9 +454,17 @@ template <class T> static bool conv_mma_dispatch(CmFwd &p)
     return conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
 }
 
-// false = not covered, nothing launched
-template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, const T *bias, T *y)
+// A pointwise layer of stride 1 is a product over the flattened plane: one long row, so tiles stage no pixel twice.
+static ConvGeom cm_flat(ConvGeom g)
 {
+    if (g.Hk == 1 && g.Wk == 1 && g.sh == 1 && g.sw == 1 && g.padU == 0 && g.padL == 0 && g.Hin == g.Hout && g.Win == g.Wout) { g.Win *= g.Hin; g.Wout = g.Win; g.Hin = g.Hout = 1; }
+    return g;
+}
+
+// false = not covered, nothing launched
+template <class T> bool conv_mma_fw(const ConvGeom &geom, const T *x, const T *w, const T *bias, T *y)
+{
+    const ConvGeom g = cm_flat(geom);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise || gemm_path() == 1 || KK > CM_MAXTAPS || g.sh != g.sw || (long long)g.Hin * g.Win >= (1ll << 31)) return false;
     CmFwd p;
@@ -373,8 +478,9 @@ template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, c
     p.rows_max = g.Hk;
     return conv_mma_dispatch<T>(p);
 }
-template <class T> bool conv_mma_ig(const ConvGeom &g, const T *dy, const T *w, T *dx)
+template <class T> bool conv_mma_ig(const ConvGeom &geom, const T *dy, const T *w, T *dx)
 {
+    const ConvGeom g = cm_flat(geom);
     const int KK = g.Hk * g.Wk, s = g.sh;
     if (g.depthwise || gemm_path() == 1 || KK > CM_MAXTAPS || g.sh != g.sw || s > 3 || g.padU > 100 || g.padL > 100) return false;
     CmFwd p;
@@ -416,7 +522,7 @@ INST(__half)
 struct CmWg {
     const void *x, *dy; float *part;
     int n, Ci, H, W, Co, Ho, Wo, S, KK, Wk, padU, padL, tap0, ntaps;
-    int st_tile, tiles, tiles_s, rows_max, cols, ci_tiles, steps;
+    int st_tile, tiles, tiles_s, tiles_r, rows_max, cols, ci_tiles, steps;       // tiles_r: tiles of a row longer than a tile
     CmDiv dW, dcols;
     uint32_t xpitch, dpitch, d_off, t_off;      // bytes: pixel of X / of dY; offsets of the dY tile and of the address table
 };
@@ -436,7 +542,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     const uint32_t xs = (uint32_t)__cvta_generic_to_shared(cm_smem), ds = xs + p.d_off;
     int *table = reinterpret_cast<int *>(cm_smem + p.t_off);
     const int P = p.Ho * p.Wo, cols = p.cols;
-    const bool multi = P < BN;
+    const bool multi = P < BN, wide = p.Wo > BN;
     const CmDiv dW = p.dW, dcols = p.dcols;
 
     float acc[TAPS][MI][NI][4];
@@ -454,28 +560,29 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     // pixels of the tile that no stream covers stay zero in the dY tile
     for (uint32_t e = tid * 16; e < BN * p.dpitch; e += NT * 16) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ds + e), "r"(0) : "memory");
 
-    const int per = (p.tiles + gridDim.y - 1) / gridDim.y, t_begin = blockIdx.y * per, t_end = min(p.tiles, t_begin + per);
+    const int t_begin = (int)((long long)p.tiles * blockIdx.y / gridDim.y), t_end = (int)((long long)p.tiles * (blockIdx.y + 1) / gridDim.y);
     const long long xplane = (long long)p.H * p.W;
     for (int tile = t_begin; tile < t_end; tile++) {
-        const int s0 = multi ? tile * p.st_tile : tile / p.tiles_s, p0 = multi ? 0 : (tile % p.tiles_s) * BN;
+        const int s0 = multi ? tile * p.st_tile : tile / p.tiles_s, ts = tile % p.tiles_s;
+        const int row_t = wide ? ts / p.tiles_r : 0, col_t = wide ? (ts - row_t * p.tiles_r) * BN : 0;      // a tile within one long row
+        const int p0 = multi ? 0 : wide ? row_t * p.Wo + col_t : ts * BN;
         const int st_n = multi ? p.st_tile : 1;
-        const int i0 = cm_quot(p0, dW), last = multi ? P - 1 : min(p0 + BN, P) - 1;
-        const int rows = (cm_quot(last, dW) - i0) * p.S + p.rows_max;
+        const int i0 = wide ? row_t : cm_quot(p0, dW), last = multi ? P - 1 : wide ? p0 + min(BN, p.Wo - col_t) - 1 : min(p0 + BN, P) - 1;
+        const int rows = ((wide ? i0 : cm_quot(last, dW)) - i0) * p.S + p.rows_max;
         __syncthreads();
         if (tid < BN) {
             const int live = multi ? st_n * P : last + 1 - p0, q = tid < live ? tid : 0;
             int st = 0, pp = p0 + q;
             if (multi) { st = q / P; pp = q - st * P; }
-            const int i = cm_quot(pp, dW), j = pp - i * p.Wo;
+            const int i = wide ? i0 : cm_quot(pp, dW), j = pp - i * p.Wo - col_t;
             table[tid] = ((st * rows + (i - i0) * p.S) * cols + j * p.S) * (int)p.xpitch;
         }
-        const CmDiv drc = cm_div_dev(rows * cols), dpix = cm_div_dev(st_n * rows * cols);
-        cm_stage<T, NT>(xs, reinterpret_cast<const T *>(p.x) + ((long long)s0 * p.Ci + ci0) * xplane, st_n, p.n - s0, rows, cols, dcols, drc, dpix,
-                        i0 * p.S - p.padU, -p.padL, p.H, p.W, CI, p.Ci - ci0, xplane, (long long)p.Ci * xplane, p.xpitch);
+        cm_stage<T, NT>(xs, reinterpret_cast<const T *>(p.x) + ((long long)s0 * p.Ci + ci0) * xplane, st_n, p.n - s0, rows, cols, dcols,
+                        i0 * p.S - p.padU, col_t * p.S - p.padL, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
         const int run = multi ? P : BN;
-        const CmDiv drun = cm_div_dev(run), dall = cm_div_dev(st_n * run);
-        cm_stage<T, NT>(ds, reinterpret_cast<const T *>(p.dy) + ((long long)s0 * p.Co + co0) * P, st_n, p.n - s0, 1, run, drun, drun, dall,
-                        0, p0, 1, P, CO, p.Co - co0, P, (long long)p.Co * P, p.dpitch);
+        const CmDiv drun = cm_div_dev(run);
+        cm_stage<T, NT>(ds, reinterpret_cast<const T *>(p.dy) + ((long long)s0 * p.Co + co0) * P, st_n, p.n - s0, 1, run, drun,
+                        0, p0, 1, multi ? P : last + 1, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
         __syncthreads();
         for (int s = wk * KCH; s < p.steps; s += WK * KCH) {
             uint32_t a[KCH][MI][4], al[HALF ? 1 : KCH][HALF ? 1 : MI][4], xa[KCH][HALF ? 1 : 2];
@@ -517,14 +624,17 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
                             for (int i = 0; i < MI; i++) { cm_hmma(tmp[i][2 * j], a[c][i], b[0], b[1]); cm_hmma(tmp[i][2 * j + 1], a[c][i], b[2], b[3]); }
                         }
                     } else {
+                        uint32_t bh[NI][2], bl[NI][2];
 #pragma unroll
-                        for (int j = 0; j < NI; j++) {
-                            uint32_t bh0, bl0, bh1, bl1;
-                            tc::split_tf32_fast(__uint_as_float(cm_lds32(xa[c][0] + toff[t] + j * 32u)), bh0, bl0);
-                            tc::split_tf32_fast(__uint_as_float(cm_lds32(xa[c][1] + toff[t] + j * 32u)), bh1, bl1);
+                        for (int j = 0; j < NI; j++)
 #pragma unroll
-                            for (int i = 0; i < MI; i++) { cm_tmma(tmp[i][j], al[c][i], bh0, bh1); cm_tmma(tmp[i][j], a[c][i], bl0, bl1); cm_tmma(tmp[i][j], a[c][i], bh0, bh1); }
-                        }
+                            for (int h = 0; h < 2; h++) tc::split_tf32_fast(__uint_as_float(cm_lds32(xa[c][h] + toff[t] + j * 32u)), bh[j][h], bl[j][h]);
+#pragma unroll
+                        for (int term = 0; term < 3; term++)
+#pragma unroll
+                            for (int j = 0; j < NI; j++)
+#pragma unroll
+                                for (int i = 0; i < MI; i++) cm_tmma(tmp[i][j], term == 0 ? al[c][i] : a[c][i], term == 1 ? bl[j][0] : bh[j][0], term == 1 ? bl[j][1] : bh[j][1]);
                     }
                 }
 #pragma unroll
@@ -568,12 +678,15 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     constexpr int BN = 128, SZ = (int)sizeof(T), CO = 16 * MI * WM, CI = 8 * NI * WN, PAD = SZ == 2 ? 16 : 32;
     const int P = p.Ho * p.Wo;
     p.st_tile = P < BN ? std::max(1, std::min(BN / P, p.n)) : 1;
-    p.tiles_s = ceil_div(P, BN);
+    const bool wide = p.Wo > BN;
+    p.tiles_r = ceil_div(p.Wo, BN); p.tiles_s = wide ? p.Ho * p.tiles_r : ceil_div(P, BN);
+    if (wide) { p.cols = (BN - 1) * p.S + p.cols - (p.Wo - 1) * p.S; p.dcols = cm_div(p.cols); }
+    else if ((long long)P * p.Wo >= (1ll << 32)) return false;
     const long long tiles = P < BN ? ceil_div(p.n, p.st_tile) : (long long)p.n * p.tiles_s;
-    if (tiles >= (1 << 30)) return false;
+    if (tiles >= (1 << 30) || ((long long)p.Ci * p.H * p.W + (long long)p.Co * P) * 16 >= (1ll << 29)) return false;      // 32-bit offsets inside a tile
     p.tiles = (int)tiles;
     p.steps = ceil_div(P < BN ? p.st_tile * P : BN, SZ == 2 ? 16 : 8);
-    const int rows = (P < BN ? p.Ho - 1 : (BN + p.Wo - 2) / p.Wo) * p.S + p.rows_max;
+    const int rows = (wide ? 0 : P < BN ? p.Ho - 1 : (BN + p.Wo - 2) / p.Wo) * p.S + p.rows_max;
     p.xpitch = CI * SZ + PAD; p.dpitch = CO * SZ + PAD;
     const size_t xb = ((size_t)p.st_tile * rows * p.cols * p.xpitch + 15) & ~(size_t)15, db = (size_t)BN * p.dpitch;
     p.d_off = (uint32_t)xb; p.t_off = (uint32_t)(xb + db);
@@ -583,7 +696,6 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     const int ctiles = p.ci_tiles * ceil_div(p.Co, CO);
     int groups = std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / ctiles);
     groups = std::min(std::min(groups, p.tiles), part_groups);
-    groups = ceil_div(p.tiles, ceil_div(p.tiles, groups));
     *groups_out = groups;
     if (dry) return true;
     auto kern = conv_mma_wg_kernel<T, TAPS, MI, NI, WM, WN, WK>;
@@ -597,8 +709,9 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
 }
 
 // Partial results per CTA into `part`; false = geometry not covered.  dry_run: only the number of groups.
-template <class T> bool conv_mma_wg(const ConvGeom &g, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry)
+template <class T> bool conv_mma_wg(const ConvGeom &geom, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry)
 {
+    const ConvGeom g = cm_flat(geom);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise || gemm_path() == 1 || KK > CM_MAXTAPS || g.sh != g.sw || (long long)g.Hin * g.Win >= (1ll << 31)) return false;
     CmWg p;
@@ -609,6 +722,7 @@ template <class T> bool conv_mma_wg(const ConvGeom &g, const T *x, const T *dy, 
         return conv_mma_wg_launch<T, 1, 1, 4, 2, 1, 4>(p, part_groups, groups_out, dry);
     }
     // channel tiles of 16 or 32 by what the layer has; the warps that a narrow layer leaves over share the pixels
+    if (g.Cin > 16 && g.Cout > 32) return conv_mma_wg_launch<T, 9, 1, 2, 4, 2, 1>(p, part_groups, groups_out, dry);
     if (g.Cin > 16 && g.Cout > 16) return conv_mma_wg_launch<T, 9, 1, 2, 2, 2, 2>(p, part_groups, groups_out, dry);
     if (g.Cout > 16) return conv_mma_wg_launch<T, 9, 1, 2, 2, 1, 4>(p, part_groups, groups_out, dry);
     if (g.Cin > 16) return conv_mma_wg_launch<T, 9, 1, 2, 1, 2, 4>(p, part_groups, groups_out, dry);
