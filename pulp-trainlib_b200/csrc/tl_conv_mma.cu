@@ -128,6 +128,36 @@ __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams,
     }
 }
 
+// The same patch by asynchronous 4-byte copies (fp32 only): nothing waits, the next tile's patch arrives while this one is
+// multiplied.  The caller commits and waits.
+template <int NT>
+__device__ __forceinline__ void cm_stage_async(uint32_t sm, const float *src, int streams, int streams_left, int rows, int cols, CmDiv dcols,
+                                               int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch)
+{
+    const char *base = reinterpret_cast<const char *>(src);
+    const int groups = chans >> 3, lane = threadIdx.x & 31, rc_n = rows * cols, pix = streams * rc_n, blocks = (pix + 31) >> 5;
+    const uint32_t cs = cstride * 4;
+    int g = 0, blk = threadIdx.x >> 5;
+    while (blk >= blocks) { blk -= blocks; g++; }
+    while (g < groups) {
+        const int p = blk * 32 + lane;
+        int st = 0, rc = p;
+        if (streams > 1) { st = p / rc_n; rc = p - st * rc_n; }
+        const int r = rows > 1 ? cm_quot(rc, dcols) : 0, c = rc - r * cols, h = row0 + r, w = col0 + c;
+        const bool ok = st < streams_left && (unsigned)h < (unsigned)H && (unsigned)w < (unsigned)W;
+        uint32_t off = ok ? ((uint32_t)st * sstride + (uint32_t)(h * W + w)) * 4u + (uint32_t)(g * 8) * cs : 0u;
+        const int left = ok ? c_left - g * 8 : 0;
+        const uint32_t to = sm + (uint32_t)p * pitch + (uint32_t)g * 32u;
+        if (p < pix) {
+#pragma unroll
+            for (int q = 0; q < 8; q++, off += cs)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + 4u * q), "l"(base + (q < left ? off : 0u)), "r"(q < left ? 4 : 0) : "memory");
+        }
+        blk += NT / 32;
+        while (blk >= blocks) { blk -= blocks; g++; }
+    }
+}
+
 // ---------------------------------------------------------------- forward and input gradient
 // dst[m][oy0 + i osy][ox0 + j osx] = sum over taps t and source channels k of src[k][i S + dr_t][j S + dc_t] W[m][k][t].
 // Forward: S = the stride, one class.  Input gradient: a class per parity (oy0, ox0) of the input pixels (osy = osx = the
@@ -141,7 +171,7 @@ struct CmFwd {
     signed char dr[CM_MAXTAPS], dc[CM_MAXTAPS]; unsigned char widx[CM_MAXTAPS];
     int st_tile;                             // streams per tile (planes smaller than a tile), else 1
     int CKS, groups, cblk, resident;         // channels staged at a time, how often, k-steps per chain; weights loaded once per CTA
-    uint32_t pitch, wpitch, w_off;           // bytes: pixel, weight row; offset of the weights behind the patch
+    uint32_t pitch, wpitch, w_off, patch2;   // bytes: pixel, weight row; offset of the weights behind the patch; of the second patch (0: none)
     int rows_max, linear, pairs;
 };
 
@@ -220,15 +250,40 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
     const CmDiv dcols = wide ? cm_div_dev(cols) : c.dcols, dW = c.dW;
     const long long src_plane = (long long)p.Hs * p.Ws, dst_plane = (long long)p.oH * p.oW;
 
+    struct Geo { int s0, p0, i0, col_t, live, rows; };
+    const int st_n = P < BN ? p.st_tile : 1;
+    auto geometry = [&](int tile) {
+        Geo q;
+        const int ts = tile % tiles_s, row_t = wide ? ts / tiles_r : 0;
+        q.s0 = P < BN ? tile * p.st_tile : tile / tiles_s;
+        q.col_t = wide ? (ts - row_t * tiles_r) * BN : 0;
+        q.p0 = P < BN ? 0 : wide ? row_t * c.Wc + q.col_t : ts * BN;
+        q.i0 = wide ? row_t : cm_quot(q.p0, dW);
+        q.live = P < BN ? min(st_n, p.n - q.s0) * P : wide ? min(BN, c.Wc - q.col_t) : min(BN, P - q.p0);      // output pixels of the tile
+        const int last = P < BN ? P - 1 : q.p0 + q.live - 1;
+        q.rows = ((wide ? q.i0 : cm_quot(last, dW)) - q.i0) * p.S + p.rows_max;                                 // rows_max: rows that one output row needs
+        return q;
+    };
+    auto stage = [&](const Geo &q, int g, uint32_t to, bool async) {
+        const int k0 = g * p.CKS;
+        const T *src = reinterpret_cast<const T *>(p.src) + ((long long)q.s0 * p.Cs + k0) * src_plane;
+        if constexpr (!HALF)
+            if (async) {
+                cm_stage_async<NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
+                                   (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
+                return;
+            }
+        cm_stage<T, NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
+                        (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
+    };
+    // two patches (fp32, weights resident): the next tile's channels are on their way while this tile is multiplied
+    const bool two = !HALF && p.patch2 != 0;
+    uint32_t cur = 0;
+    if (two) stage(geometry(blockIdx.x), 0, patch, true);
+
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int s0 = P < BN ? tile * p.st_tile : tile / tiles_s, ts = tile % tiles_s;
-        const int row_t = wide ? ts / tiles_r : 0, col_t = wide ? (ts - row_t * tiles_r) * BN : 0;
-        const int p0 = P < BN ? 0 : wide ? row_t * c.Wc + col_t : ts * BN;
-        const int st_n = P < BN ? p.st_tile : 1;
-        const int i0 = wide ? row_t : cm_quot(p0, dW);
-        const int live = P < BN ? min(st_n, p.n - s0) * P : wide ? min(BN, c.Wc - col_t) : min(BN, P - p0);        // output pixels of this tile
-        const int last = P < BN ? P - 1 : p0 + live - 1;
-        const int rows = ((wide ? i0 : cm_quot(last, dW)) - i0) * p.S + p.rows_max; // rows_max: rows that one output row needs
+        const Geo geo = geometry(tile);
+        const int s0 = geo.s0, p0 = geo.p0, i0 = geo.i0, col_t = geo.col_t, live = geo.live, rows = geo.rows;
         // start addresses (in the patch) of the pixels this lane supplies fragments for
         constexpr int NB = HALF ? N8 / 2 : N8;
         uint32_t pix[NB];
@@ -250,17 +305,25 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
                 for (int q = 0; q < 4; q++) acc[i][j][q] = 0.f;
 
         for (int g = 0; g < p.groups; g++) {
-            __syncthreads();                                                        // the patch (and the weights) are free again
             const int k0 = g * p.CKS;
-            if (!p.resident) load_weights(k0, p.CKS);
-            cm_stage<T, NT>(patch, reinterpret_cast<const T *>(p.src) + ((long long)s0 * p.Cs + k0) * src_plane, st_n, p.n - s0, rows, cols, dcols,
-                            i0 * p.S + c.dr_min, col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0, (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
-            __syncthreads();
+            uint32_t poff = 0;
+            if (two) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncthreads();                                                    // this patch has landed, the other one is free
+                poff = cur; cur ^= p.patch2;
+                if (g + 1 < p.groups) stage(geo, g + 1, patch + cur, true);
+                else if (tile + (int)gridDim.x < tiles) stage(geometry(tile + gridDim.x), 0, patch + cur, true);
+            } else {
+                __syncthreads();                                                    // the patch (and the weights) are free again
+                if (!p.resident) load_weights(k0, p.CKS);
+                stage(geo, g, patch, false);
+                __syncthreads();
+            }
             const uint32_t wg = wsm + (uint32_t)(p.resident ? k0 * SZ : 0);
             const int nck = p.CKS / CK, nblk = (nck + p.cblk - 1) / p.cblk;
             for (int u = wk; u < ntaps * nblk; u += WK) {
                 const int t = nblk == 1 ? u : u / nblk, ck0 = nblk == 1 ? 0 : (u - t * nblk) * p.cblk, ck1 = min(nck, ck0 + p.cblk);
-                const uint32_t toff = (uint32_t)tap_off[t];
+                const uint32_t toff = (uint32_t)tap_off[t] + poff;
                 const uint32_t wrow = wg + (uint32_t)((t * BM + wm * 16 * MT) * (int)p.wpitch);
                 if constexpr (HALF) {
                     const uint32_t wa = wrow + (uint32_t)((lane & 7) + ((lane >> 3) & 1) * 8) * p.wpitch + (uint32_t)(lane >> 4) * 16u;
@@ -404,20 +467,23 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
         tiles_max = std::max(tiles_max, P < BN ? ceil_div(p.n, p.st_tile) : (int)std::min<long long>((long long)p.n * (wide ? (long long)c.Hc * ceil_div(c.Wc, BN) : ceil_div(P, BN)), 1 << 30));
     }
     const size_t red = WK > 1 ? (size_t)(WK - 1) * WM * WN * MT * (BN / WN / 8) * 512 : 0;
-    auto plan = [&](int cks, bool resident, size_t limit) {
+    auto plan = [&](int cks, bool resident, size_t limit, bool two) {
         p.CKS = cks; p.groups = ceil_div(cpad, cks); p.resident = resident;
         p.pitch = (uint32_t)(cks * SZ + 16); p.wpitch = (uint32_t)((resident ? p.groups * cks : cks) * SZ + 16);
         const size_t pb = std::max<size_t>(((size_t)pix * p.pitch + 15) & ~(size_t)15, red);
-        p.w_off = (uint32_t)pb;
-        return pb + (size_t)taps * BM * p.wpitch <= limit;
+        p.patch2 = two ? (uint32_t)pb : 0u; p.w_off = (uint32_t)(two ? 2 * pb : pb);
+        return p.w_off + (size_t)taps * BM * p.wpitch <= limit;
     };
     // everything resident in half of an SM's shared memory if it fits (two CTAs overlap staging and arithmetic), else fewer
     // channels at a time, else all of it, else weights reloaded with every group of channels
     bool ok = false;
     for (size_t limit : {(size_t)110 * 1024, (size_t)CM_SMEM_MAX}) {
-        for (int parts = 1; !ok && parts <= cpad / CK; parts *= 2) ok = plan(ceil_div(ceil_div(cpad, parts), CK) * CK, true, limit);
+        if (sizeof(T) == 4 && WK == 1)                                     // (the K shares of WK > 1 meet where the patches lie)
+            for (int parts = 1; !ok && parts <= cpad / CK; parts *= 2) ok = plan(ceil_div(ceil_div(cpad, parts), CK) * CK, true, limit, true);
         if (ok) break;
-        for (int parts = 1; !ok && parts <= cpad / CK; parts *= 2) ok = plan(ceil_div(ceil_div(cpad, parts), CK) * CK, false, limit);
+        for (int parts = 1; !ok && parts <= cpad / CK; parts *= 2) ok = plan(ceil_div(ceil_div(cpad, parts), CK) * CK, true, limit, false);
+        if (ok) break;
+        for (int parts = 1; !ok && parts <= cpad / CK; parts *= 2) ok = plan(ceil_div(ceil_div(cpad, parts), CK) * CK, false, limit, false);
         if (ok) break;
     }
     if (!ok) return false;
@@ -522,9 +588,9 @@ INST(__half)
 struct CmWg {
     const void *x, *dy; float *part;
     int n, Ci, H, W, Co, Ho, Wo, S, KK, Wk, padU, padL, tap0, ntaps;
-    int st_tile, tiles, tiles_s, tiles_r, rows_max, cols, ci_tiles, steps;       // tiles_r: tiles of a row longer than a tile
+    int bn, st_tile, tiles, tiles_s, tiles_r, rows_max, cols, ci_tiles, steps;       // tiles_r: tiles of a row longer than a tile
     CmDiv dW, dcols;
-    uint32_t xpitch, dpitch, d_off, t_off;      // bytes: pixel of X / of dY; offsets of the dY tile and of the address table
+    uint32_t xpitch, dpitch, d_off, t_off, buf2;    // bytes: pixel of X / of dY; offsets of the dY tile, of the address tables, of the second tiles (0: none)
 };
 
 template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK>
@@ -542,7 +608,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     const uint32_t xs = (uint32_t)__cvta_generic_to_shared(cm_smem), ds = xs + p.d_off;
     int *table = reinterpret_cast<int *>(cm_smem + p.t_off);
     const int P = p.Ho * p.Wo, cols = p.cols;
-    const bool multi = P < BN, wide = p.Wo > BN;
+    const int bn = p.bn;                                                   // pixels of a tile, at most BN
+    const bool multi = P < bn, wide = p.Wo > bn;
     const CmDiv dW = p.dW, dcols = p.dcols;
 
     float acc[TAPS][MI][NI][4];
@@ -558,50 +625,75 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
 #pragma unroll
     for (int t = 0; t < TAPS; t++) { const int tt = p.tap0 + min(t, p.ntaps - 1); toff[t] = ((tt / p.Wk) * cols + tt % p.Wk) * (int)p.xpitch; }
     // pixels of the tile that no stream covers stay zero in the dY tile
-    for (uint32_t e = tid * 16; e < BN * p.dpitch; e += NT * 16) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ds + e), "r"(0) : "memory");
+    for (uint32_t e = tid * 16; e < BN * p.dpitch; e += NT * 16) {
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ds + e), "r"(0) : "memory");
+        if (p.buf2) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ds + p.buf2 + e), "r"(0) : "memory");
+    }
 
     const int t_begin = (int)((long long)p.tiles * blockIdx.y / gridDim.y), t_end = (int)((long long)p.tiles * (blockIdx.y + 1) / gridDim.y);
     const long long xplane = (long long)p.H * p.W;
-    for (int tile = t_begin; tile < t_end; tile++) {
+    const int st_n = multi ? p.st_tile : 1;
+    auto stage = [&](int tile, uint32_t buf, bool async) {
         const int s0 = multi ? tile * p.st_tile : tile / p.tiles_s, ts = tile % p.tiles_s;
-        const int row_t = wide ? ts / p.tiles_r : 0, col_t = wide ? (ts - row_t * p.tiles_r) * BN : 0;      // a tile within one long row
-        const int p0 = multi ? 0 : wide ? row_t * p.Wo + col_t : ts * BN;
-        const int st_n = multi ? p.st_tile : 1;
-        const int i0 = wide ? row_t : cm_quot(p0, dW), last = multi ? P - 1 : wide ? p0 + min(BN, p.Wo - col_t) - 1 : min(p0 + BN, P) - 1;
+        const int row_t = wide ? ts / p.tiles_r : 0, col_t = wide ? (ts - row_t * p.tiles_r) * bn : 0;      // a tile within one long row
+        const int p0 = multi ? 0 : wide ? row_t * p.Wo + col_t : ts * bn;
+        const int i0 = wide ? row_t : cm_quot(p0, dW), last = multi ? P - 1 : wide ? p0 + min(bn, p.Wo - col_t) - 1 : min(p0 + bn, P) - 1;
         const int rows = ((wide ? i0 : cm_quot(last, dW)) - i0) * p.S + p.rows_max;
-        __syncthreads();
         if (tid < BN) {
             const int live = multi ? st_n * P : last + 1 - p0, q = tid < live ? tid : 0;
             int st = 0, pp = p0 + q;
             if (multi) { st = q / P; pp = q - st * P; }
             const int i = wide ? i0 : cm_quot(pp, dW), j = pp - i * p.Wo - col_t;
-            table[tid] = ((st * rows + (i - i0) * p.S) * cols + j * p.S) * (int)p.xpitch;
+            table[(buf ? BN : 0) + tid] = ((st * rows + (i - i0) * p.S) * cols + j * p.S) * (int)p.xpitch;
         }
-        cm_stage<T, NT>(xs, reinterpret_cast<const T *>(p.x) + ((long long)s0 * p.Ci + ci0) * xplane, st_n, p.n - s0, rows, cols, dcols,
-                        i0 * p.S - p.padU, col_t * p.S - p.padL, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
-        const int run = multi ? P : BN;
+        const T *xp = reinterpret_cast<const T *>(p.x) + ((long long)s0 * p.Ci + ci0) * xplane, *dp = reinterpret_cast<const T *>(p.dy) + ((long long)s0 * p.Co + co0) * P;
+        const int run = multi ? P : bn, row0 = i0 * p.S - p.padU, col0 = col_t * p.S - p.padL, d_end = multi ? P : last + 1;
         const CmDiv drun = cm_div_dev(run);
-        cm_stage<T, NT>(ds, reinterpret_cast<const T *>(p.dy) + ((long long)s0 * p.Co + co0) * P, st_n, p.n - s0, 1, run, drun,
-                        0, p0, 1, multi ? P : last + 1, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
-        __syncthreads();
+        if constexpr (!HALF)
+            if (async) {
+                cm_stage_async<NT>(xs + buf, xp, st_n, p.n - s0, rows, cols, dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
+                cm_stage_async<NT>(ds + buf, dp, st_n, p.n - s0, 1, run, drun, 0, p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
+                return;
+            }
+        cm_stage<T, NT>(xs + buf, xp, st_n, p.n - s0, rows, cols, dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
+        cm_stage<T, NT>(ds + buf, dp, st_n, p.n - s0, 1, run, drun, 0, p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
+    };
+    // two sets of tiles (fp32): the next tile arrives by asynchronous copies while this one is multiplied
+    const bool two = !HALF && p.buf2 != 0;
+    uint32_t cur = 0;
+    __syncthreads();                                                       // the zeros of the dY tiles are in place
+    if (two && t_begin < t_end) stage(t_begin, 0, true);
+    for (int tile = t_begin; tile < t_end; tile++) {
+        uint32_t off = 0;
+        if (two) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            off = cur; cur ^= p.buf2;
+            if (tile + 1 < t_end) stage(tile + 1, cur, true);
+        } else {
+            __syncthreads();
+            stage(tile, 0, false);
+            __syncthreads();
+        }
+        const int *tab = table + (off ? BN : 0);
         for (int s = wk * KCH; s < p.steps; s += WK * KCH) {
             uint32_t a[KCH][MI][4], al[HALF ? 1 : KCH][HALF ? 1 : MI][4], xa[KCH][HALF ? 1 : 2];
 #pragma unroll
             for (int c = 0; c < KCH; c++) {
                 const int k0 = (s + c) * KS;
                 if constexpr (HALF) {
-                    xa[c][0] = xs + (uint32_t)table[k0 + (lane & 7) + ((lane >> 3) & 1) * 8] + (uint32_t)(wn * NI * 8 + (lane >> 4) * 8) * 2u;
+                    xa[c][0] = xs + off + (uint32_t)tab[k0 + (lane & 7) + ((lane >> 3) & 1) * 8] + (uint32_t)(wn * NI * 8 + (lane >> 4) * 8) * 2u;
 #pragma unroll
                     for (int i = 0; i < MI; i++)
-                        cm_ldsm_t(a[c][i], ds + (uint32_t)(k0 + (lane & 7) + (lane >> 4) * 8) * p.dpitch + (uint32_t)((wm * MI + i) * 16 + ((lane >> 3) & 1) * 8) * 2u);
+                        cm_ldsm_t(a[c][i], ds + off + (uint32_t)(k0 + (lane & 7) + (lane >> 4) * 8) * p.dpitch + (uint32_t)((wm * MI + i) * 16 + ((lane >> 3) & 1) * 8) * 2u);
                 } else {
 #pragma unroll
-                    for (int h = 0; h < 2; h++) xa[c][h] = xs + (uint32_t)table[k0 + (lane & 3) + 4 * h] + (uint32_t)(wn * NI * 8 + (lane >> 2)) * 4u;
+                    for (int h = 0; h < 2; h++) xa[c][h] = xs + off + (uint32_t)tab[k0 + (lane & 3) + 4 * h] + (uint32_t)(wn * NI * 8 + (lane >> 2)) * 4u;
 #pragma unroll
                     for (int i = 0; i < MI; i++)
 #pragma unroll
                         for (int q = 0; q < 4; q++)
-                            tc::split_tf32_fast(__uint_as_float(cm_lds32(ds + (uint32_t)(k0 + (lane & 3) + (q >> 1) * 4) * p.dpitch + (uint32_t)((wm * MI + i) * 16 + (lane >> 2) + (q & 1) * 8) * 4u)), a[c][i][q], al[c][i][q]);
+                            tc::split_tf32_fast(__uint_as_float(cm_lds32(ds + off + (uint32_t)(k0 + (lane & 3) + (q >> 1) * 4) * p.dpitch + (uint32_t)((wm * MI + i) * 16 + (lane >> 2) + (q & 1) * 8) * 4u)), a[c][i][q], al[c][i][q]);
                 }
             }
 #pragma unroll
@@ -676,24 +768,36 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
 template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool conv_mma_wg_launch(CmWg &p, int part_groups, int *groups_out, bool dry)
 {
     constexpr int BN = 128, SZ = (int)sizeof(T), CO = 16 * MI * WM, CI = 8 * NI * WN, PAD = SZ == 2 ? 16 : 32;
-    const int P = p.Ho * p.Wo;
-    p.st_tile = P < BN ? std::max(1, std::min(BN / P, p.n)) : 1;
-    const bool wide = p.Wo > BN;
-    p.tiles_r = ceil_div(p.Wo, BN); p.tiles_s = wide ? p.Ho * p.tiles_r : ceil_div(P, BN);
-    if (wide) { p.cols = (BN - 1) * p.S + p.cols - (p.Wo - 1) * p.S; p.dcols = cm_div(p.cols); }
-    else if ((long long)P * p.Wo >= (1ll << 32)) return false;
-    const long long tiles = P < BN ? ceil_div(p.n, p.st_tile) : (long long)p.n * p.tiles_s;
-    if (tiles >= (1 << 30) || ((long long)p.Ci * p.H * p.W + (long long)p.Co * P) * 16 >= (1ll << 29)) return false;      // 32-bit offsets inside a tile
-    p.tiles = (int)tiles;
-    p.steps = ceil_div(P < BN ? p.st_tile * P : BN, SZ == 2 ? 16 : 8);
-    const int rows = (wide ? 0 : P < BN ? p.Ho - 1 : (BN + p.Wo - 2) / p.Wo) * p.S + p.rows_max;
-    p.xpitch = CI * SZ + PAD; p.dpitch = CO * SZ + PAD;
-    const size_t xb = ((size_t)p.st_tile * rows * p.cols * p.xpitch + 15) & ~(size_t)15, db = (size_t)BN * p.dpitch;
-    p.d_off = (uint32_t)xb; p.t_off = (uint32_t)(xb + db);
-    const size_t smem = std::max(xb + db + BN * 4, (size_t)WK * CO * CI * 4);
-    if (smem > CM_SMEM_MAX) return false;
+    const int P = p.Ho * p.Wo, cols0 = p.cols;
     p.ci_tiles = ceil_div(p.Ci, CI);
     const int ctiles = p.ci_tiles * ceil_div(p.Co, CO);
+    const int slots = std::max(1, std::min(2 * sm_count() / ctiles, part_groups));
+    auto tiles_of = [&](int bn) -> long long { return P < bn ? ceil_div(p.n, std::max(1, std::min(bn / P, p.n))) : p.Wo > bn ? (long long)p.n * p.Ho * ceil_div(p.Wo, bn) : (long long)p.n * ceil_div(P, bn); };
+    // pixels per tile: what makes the fewest pixels of the longest CTA (planes and rounds come out even), halo rows included
+    double best = 1e30;
+    for (int bn = BN; bn >= BN / 2; bn -= SZ == 2 ? 16 : 8) {
+        const int halo = bn + 2 * std::min(p.Wo, bn) * (p.rows_max - 1) / 3;
+        const double cost = (double)ceil_div(tiles_of(bn), slots) * halo;
+        if (cost < 0.98 * best) { best = cost; p.bn = bn; }
+    }
+    const int bn = p.bn;
+    p.st_tile = P < bn ? std::max(1, std::min(bn / P, p.n)) : 1;
+    const bool wide = p.Wo > bn;
+    p.tiles_r = ceil_div(p.Wo, bn); p.tiles_s = wide ? p.Ho * p.tiles_r : ceil_div(P, bn);
+    if (wide) { p.cols = (bn - 1) * p.S + cols0 - (p.Wo - 1) * p.S; p.dcols = cm_div(p.cols); }
+    else if ((long long)P * p.Wo >= (1ll << 32)) return false;
+    const long long tiles = tiles_of(bn);
+    if (tiles >= (1 << 30) || ((long long)p.Ci * p.H * p.W + (long long)p.Co * P) * 16 >= (1ll << 29)) return false;      // 32-bit offsets inside a tile
+    p.tiles = (int)tiles;
+    p.steps = ceil_div(P < bn ? p.st_tile * P : bn, SZ == 2 ? 16 : 8);
+    const int rows = (wide ? 0 : P < bn ? p.Ho - 1 : (bn + p.Wo - 2) / p.Wo) * p.S + p.rows_max;
+    p.xpitch = CI * SZ + PAD; p.dpitch = CO * SZ + PAD;
+    const size_t xb = ((size_t)p.st_tile * rows * p.cols * p.xpitch + 15) & ~(size_t)15, db = (size_t)BN * p.dpitch;
+    p.d_off = (uint32_t)xb;
+    const bool two = SZ == 4 && 2 * (xb + db) + 8 * BN <= 110 * 1024;
+    p.buf2 = two ? (uint32_t)(xb + db) : 0u; p.t_off = (uint32_t)((xb + db) * (two ? 2 : 1));
+    const size_t smem = std::max((size_t)p.t_off + 8 * BN, (size_t)WK * CO * CI * 4);
+    if (smem > CM_SMEM_MAX) return false;
     int groups = std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / ctiles);
     groups = std::min(std::min(groups, p.tiles), part_groups);
     *groups_out = groups;
@@ -722,7 +826,7 @@ template <class T> bool conv_mma_wg(const ConvGeom &geom, const T *x, const T *d
         return conv_mma_wg_launch<T, 1, 1, 4, 2, 1, 4>(p, part_groups, groups_out, dry);
     }
     // channel tiles of 16 or 32 by what the layer has; the warps that a narrow layer leaves over share the pixels
-    if (g.Cin > 16 && g.Cout > 32) return conv_mma_wg_launch<T, 9, 1, 2, 4, 2, 1>(p, part_groups, groups_out, dry);
+    if (sizeof(T) == 2 && g.Cin > 16 && g.Cout > 32) return conv_mma_wg_launch<T, 9, 1, 2, 4, 2, 1>(p, part_groups, groups_out, dry);
     if (g.Cin > 16 && g.Cout > 16) return conv_mma_wg_launch<T, 9, 1, 2, 2, 2, 2>(p, part_groups, groups_out, dry);
     if (g.Cout > 16) return conv_mma_wg_launch<T, 9, 1, 2, 2, 1, 4>(p, part_groups, groups_out, dry);
     if (g.Cin > 16) return conv_mma_wg_launch<T, 9, 1, 2, 1, 2, 4>(p, part_groups, groups_out, dry);
