@@ -82,6 +82,7 @@ template <class T>
 __global__ void __launch_bounds__(ATT_THREADS) attn_fw_kernel(const T *__restrict__ q, const T *__restrict__ k, const T *__restrict__ v,
                                                               T *__restrict__ P, T *__restrict__ att, int L, int H, float scaling)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float att_smem[];
     const int Lp = L + 1, head = blockIdx.y, t0 = blockIdx.x * ATT_TQ, nt = min(ATT_TQ, L - t0);
     float *a_tile = att_smem, *tile = att_smem + H * ATT_TQ;
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_query_kernel(const T *__r
                                                                     const T *__restrict__ P, T *__restrict__ dP, float *__restrict__ rowdot,
                                                                     T *__restrict__ dq, int L, int H, float scaling)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float att_smem[];
     const int Lp = L + 1, head = blockIdx.y, t0 = blockIdx.x * ATT_TQ, nt = min(ATT_TQ, L - t0);
     float *a_tile = att_smem, *tile = att_smem + H * ATT_TQ;
@@ -158,6 +160,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_key_kernel(const T *__res
                                                                   const T *__restrict__ dP, const float *__restrict__ rowdot,
                                                                   T *__restrict__ dk, T *__restrict__ dv, int L, int H, float scaling)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float att_smem[];
     const int Lp = L + 1, head = blockIdx.y, k0 = blockIdx.x * ATT_TQ, nk = min(ATT_TQ, L - k0);
     float *p_tile = att_smem, *ds_tile = att_smem + ATT_TQ * Lp;        // [key][query]

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
 conv_fw_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ bias,
                T *__restrict__ y, int TH, int TW, int S_T, int CC, int tiles_w, int tiles_h)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     const int PH = (TH - 1) * g.sh + g.Hk, PW = (TW - 1) * g.sw + g.Wk;
     const int PWp = PW | 1;                                  // odd row pitch: fewer bank conflicts
@@ -111,6 +112,7 @@ conv_fw_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ w, con
 template <class T>
 __global__ void dw_fw_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ w, T *__restrict__ y)
 {
+    pdl_wait();
     long long total = (long long)g.n * g.Cin * g.Hout * g.Wout;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         int wo = e % g.Wout, ho = (e / g.Wout) % g.Hout;
@@ -135,6 +137,7 @@ __global__ void dw_fw_kernel(ConvGeom g, const T *__restrict__ x, const T *__res
 template <class T>
 __global__ void dw_ig_kernel(ConvGeom g, const T *__restrict__ dy, const T *__restrict__ w, T *__restrict__ dx)
 {
+    pdl_wait();
     long long total = (long long)g.n * g.Cin * g.Hin * g.Win;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         int wi = e % g.Win, hi = (e / g.Win) % g.Hin;
@@ -164,6 +167,7 @@ __global__ void dw_ig_kernel(ConvGeom g, const T *__restrict__ dy, const T *__re
 template <class T>
 __global__ void __launch_bounds__(256) dw_wg_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ dy, T *__restrict__ dw)
 {
+    pdl_wait();
     __shared__ float red[256];
     const int tap = blockIdx.x % (g.Hk * g.Wk), ch = blockIdx.x / (g.Hk * g.Wk);
     const int kh = tap / g.Wk, kw = tap % g.Wk;
@@ -211,6 +215,7 @@ template <> bool try_tc_fw<float>(Scope &sc, const ConvGeom &g, const float *x, 
 __global__ void __launch_bounds__(256) conv_dilate_dy_kernel(const float *__restrict__ dy, float *__restrict__ dil, unsigned total4,
                                                             int Hout, int Wout, int Hin, int Win, int sh, int sw)
 {
+    pdl_wait();
     // 32-bit index arithmetic throughout (the host checks the element count)
     const unsigned W4 = (unsigned)Win / 4u;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < total4; e += gridDim.x * blockDim.x) {
@@ -246,6 +251,7 @@ __global__ void __launch_bounds__(256) conv_dilate_dy_kernel(const float *__rest
 template <int PX, bool ACC>
 __global__ void __launch_bounds__(PX) conv1x1_strided_ig_kernel(ConvGeom g, const float *__restrict__ dy, const float *__restrict__ w, float *__restrict__ dx)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float sm1[];
     float *ws = sm1;                                 // [Cout][Cin]
     float *dys = sm1 + g.Cout * g.Cin;               // [Cout][PX]
@@ -293,6 +299,7 @@ __global__ void __launch_bounds__(PX) conv1x1_strided_ig_kernel(ConvGeom g, cons
 // zero fill of dX before the scattered samples are written (16-byte stores)
 __global__ void __launch_bounds__(256) zero_f4_kernel(float4 *__restrict__ p, size_t n4)
 {
+    pdl_wait();
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n4; e += (size_t)gridDim.x * blockDim.x) p[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
@@ -434,6 +441,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
 conv_ig_kernel(ConvGeom g, const T *__restrict__ dy, const T *__restrict__ w, T *__restrict__ dx,
                int TH, int TW, int S_T, int CC, int tiles_w, int tiles_h, int PH, int PW)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     const int PWp = PW | 1;
     const int KK = g.Hk * g.Wk;
@@ -574,6 +582,7 @@ __global__ void __launch_bounds__(CONV_THREADS)
 conv_wg_partial_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part,
                        int TH, int TW, int tiles_w, int tiles_h, int ci_tiles)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     const int PH = (TH - 1) * g.sh + g.Hk, PW = (TW - 1) * g.sw + g.Wk;
     const int PWp = PW | 1;
@@ -667,6 +676,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
 conv_wg3x3_partial_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part,
                           int tiles_h, int ci_tiles, int vec, int nstage)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     typedef WgShape<S, TW, K, TH, S_T> WS;
     constexpr int WIN = WS::WIN, RW = WS::RW, W4 = WS::W4, KK = WS::KK, VOFF = WS::VOFF, PH = WS::PH, PLANE = WS::PLANE;
@@ -856,6 +866,7 @@ conv_wg3x3_partial_kernel(ConvGeom g, const T *__restrict__ x, const T *__restri
 template <class T>
 __global__ void __launch_bounds__(1024) reduce_partials_kernel(const float *__restrict__ part, T *__restrict__ out, long long n, int groups)
 {
+    pdl_wait();
     __shared__ float sm[32][33];
     const int wx = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const long long i = (long long)blockIdx.x * 32 + wx;
@@ -875,6 +886,7 @@ __global__ void __launch_bounds__(1024) reduce_partials_kernel(const float *__re
 // fp32 results: 512 consecutive weights per CTA, 16-byte loads (partial_sums_quad; the deferred mode uses the same function)
 __global__ void __launch_bounds__(1024) reduce_partials_f32_kernel(const float *__restrict__ part, float *__restrict__ out, long long n, int groups)
 {
+    pdl_wait();
     __shared__ float4 sm[8][128];
     const long long i = (long long)blockIdx.x * PSUM_ELEMS + (threadIdx.x & 127) * 4;
     float4 t;
@@ -900,6 +912,7 @@ template <class T> static void reduce_partials(const float *part, T *out, long l
 template <class T>
 __global__ void __launch_bounds__(256) conv_wg_direct_kernel(ConvGeom g, const T *__restrict__ x, const T *__restrict__ dy, T *__restrict__ dw)
 {
+    pdl_wait();
     __shared__ float red[256];
     const int KK = g.Hk * g.Wk;
     const int tap = blockIdx.x % KK, ci = (blockIdx.x / KK) % g.Cin, co = blockIdx.x / (KK * g.Cin);
@@ -925,6 +938,7 @@ __global__ void __launch_bounds__(256) conv_wg_direct_kernel(ConvGeom g, const T
 template <class T>
 __global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ dy, float *__restrict__ part, int n, int C, int plane)
 {
+    pdl_wait();
     __shared__ float red[33];
     const int c = blockIdx.x, per = (n + gridDim.y - 1) / gridDim.y, s0 = blockIdx.y * per, s1 = min(n, s0 + per);
     float acc = 0.f;
@@ -1109,6 +1123,7 @@ template <class T>
 __global__ void im2row_kernel(const T *__restrict__ src, T *__restrict__ buf, int C, int H, int W, int Hk, int Wk,
                               int Ho, int Wo, int sh, int sw, int padU, int padL, int mode_ig, int hwc, int transposed)
 {
+    pdl_wait();
     // mode 0: rows = output pixels (Ho x Wo), columns = (c,hk,wk) [CHW] or (hk,wk,c) [HWC], source = input.
     // mode 1: rows = input pixels (H x W), columns = (co,hk,wk) / (hk,wk,co), source = output gradient of
     //         size C x Ho x Wo, "full" correlation window starting at (hi-(Hk-1), wi-(Wk-1)).
@@ -1144,6 +1159,7 @@ void im2row(const T *src, T *buf, int C, int H, int W, int Hk, int Wk, int Ho, i
 template <class T>
 __global__ void blocktransp_kernel(const T *__restrict__ w, T *__restrict__ bt, int Cin, int Cout, int Hk, int Wk, int hwc)
 {
+    pdl_wait();
     const int HW = Hk * Wk;
     const long long total = (long long)Cin * Cout * HW;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {

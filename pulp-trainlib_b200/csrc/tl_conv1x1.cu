@@ -150,6 +150,7 @@ template <int KT, int MTW, bool IG>
 __global__ void __launch_bounds__(C1_THREADS, (KT * MTW <= 4) ? 4 : 2) conv1x1s_mma_kernel(Conv1x1Params p, const float *__restrict__ src, const float *__restrict__ w,
                                                                   const float *__restrict__ bias, float *__restrict__ dst)
 {
+    pdl_wait();
     constexpr int LD = C1_LDK, K = KT * 8;
     extern __shared__ __align__(16) float c1_smem[];
     const uint32_t smem_s = (uint32_t)__cvta_generic_to_shared(c1_smem);
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(C1_THREADS, (KT * MTW <= 4) ? 4 : 2) conv1x1s_
 template <int MTW, int NT>
 __global__ void __launch_bounds__(C1_THREADS, (MTW * NT <= 4) ? 4 : 2) conv1x1s_wg_kernel(Conv1x1Params p, const float *__restrict__ x, const float *__restrict__ dy, float *__restrict__ part)
 {
+    pdl_wait();
     constexpr int LD = C1_LDM;
     extern __shared__ __align__(16) float c1_smem[];
     const uint32_t smem_s = (uint32_t)__cvta_generic_to_shared(c1_smem);

@@ -26,6 +26,7 @@ struct DwParams {
 template <class T, int K>
 __global__ void __launch_bounds__(256) dw_plane_kernel(const __grid_constant__ DwParams p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
 {
+    pdl_wait();
     extern __shared__ float dw_smem[];
     const int KH = K ? K : p.Hk, KW = K ? K : p.Wk, KK = KH * KW;
     const int pl0 = blockIdx.x * p.G, np = min(p.G, p.planes - pl0), P = p.PH * p.PW, O = p.Ho * p.Wo;
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(256) dw_plane_kernel(const __grid_constant__ D
 template <class T, int K>
 __global__ void __launch_bounds__(256) dw_wg_plane_kernel(const __grid_constant__ DwParams p, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part, int n)
 {
+    pdl_wait();
     extern __shared__ float dw_smem[];
     __shared__ float red[8][K * K];
     const int ch = blockIdx.x, P = p.PH * p.PW, O = p.Ho * p.Wo;
@@ -165,6 +167,7 @@ template <int PADL> __device__ __forceinline__ void dw3_row(const float *row, fl
 template <class T, int PADL>
 __global__ void __launch_bounds__(128) dw3_kernel(const __grid_constant__ Dw3Params p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float dw_smem[];
     const int P = p.PH * p.PW, pl0 = blockIdx.x * p.G, np = min(p.G, p.planes - pl0), O = p.Ho * p.Wo, per = p.Ho * p.O4;
     float *ws = dw_smem + p.G * P;
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(128) dw3_kernel(const __grid_constant__ Dw3Par
 template <class T, int PADL>
 __global__ void __launch_bounds__(128) dw3_wg_kernel(const __grid_constant__ Dw3Params p, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part, int n)
 {
+    pdl_wait();
     extern __shared__ __align__(16) float dw_smem[];
     __shared__ float red[4][9];
     const int ch = blockIdx.x, P = p.PH * p.PW, O = p.Ho * p.Wo, per = p.Ho * p.O4;

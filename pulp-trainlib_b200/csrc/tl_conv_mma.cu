@@ -178,6 +178,7 @@ struct CmFwd {
 template <class T, int MT, int WM, int WN, int WK, int BN>
 __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __grid_constant__ CmFwd p)
 {
+    pdl_wait();
     constexpr int NT = 32 * WM * WN * WK, BM = 16 * MT * WM, TN = BN / WN, N8 = TN / 8;
     constexpr int CK = sizeof(T) == 2 ? 16 : 8, SZ = (int)sizeof(T);
     constexpr bool HALF = sizeof(T) == 2;
@@ -429,7 +430,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __
                     const int i = cm_quot(pp, dW), jj = pp - i * c.Wc;
                     off[h] = st * p.Cd * (int)dst_plane + i * p.osy * p.oW + jj * p.osx;
                 }
-            const bool pair = p.pairs && off[1] == off[0] + 1;                          // (pairs: even planes and an aligned tensor)
+            // one store for two pixels: even planes and an aligned tensor (pairs), from an even pixel (a tile inside a long row may start odd)
+            const bool pair = p.pairs && second && off[1] == off[0] + 1 && (off[0] & 1) == 0;
 #pragma unroll
             for (int i = 0; i < MT; i++)
 #pragma unroll
@@ -596,6 +598,7 @@ struct CmWg {
 template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK>
 __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const __grid_constant__ CmWg p)
 {
+    pdl_wait();
     constexpr int NT = 32 * WM * WN * WK, BN = 128;
     constexpr bool HALF = sizeof(T) == 2;
     constexpr int KS = HALF ? 16 : 8, STEPS = BN / KS;

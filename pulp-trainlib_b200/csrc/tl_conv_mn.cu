@@ -83,6 +83,7 @@ template <int WK, int PADL, bool UP = false>
 __global__ void __launch_bounds__(MN_MAX_THREADS, 1)
 conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
 {
+    pdl_wait();
     extern __shared__ unsigned char smem_dyn[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NI = p.NI;

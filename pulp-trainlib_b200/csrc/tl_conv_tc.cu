@@ -113,6 +113,7 @@ template <int PLANE_B>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 conv_tc_kernel(const __grid_constant__ CUtensorMap tmap, const ConvTcParams p)
 {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NT = p.NT, N2 = 2 * NT;

@@ -68,6 +68,7 @@ static constexpr int WGT_SLOT = 1024;           // 8 channels x 32 pixels x 4 by
 __global__ void __launch_bounds__(WGT_THREADS, 1)
 conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_dy, const WgtParams p)
 {
+    pdl_wait();
     extern __shared__ unsigned char smem_dyn[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int NISS = p.MB * p.KS;
@@ -281,6 +282,7 @@ int *tc_status_word();
 __global__ void __launch_bounds__(1024) wgt_reduce_kernel(const float *__restrict__ part, float *__restrict__ dw, int groups, int Cin, int Cout,
                                                           int s2, int xg, int cigs, int ncopy, int MB)
 {
+    pdl_wait();
     __shared__ float4 sm[8][128];
     const int NBc = ncopy * Cout;
     const long long nn = (long long)MB * 128 * NBc, i = (long long)blockIdx.x * PSUM_ELEMS + (threadIdx.x & 127) * 4;

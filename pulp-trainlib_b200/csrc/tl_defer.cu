@@ -44,6 +44,7 @@ static struct {
 // loads are in flight (the immediate mode takes two passes there).
 __global__ void __launch_bounds__(1024) deferred_reduce_kernel(const __grid_constant__ DeferBatch b)
 {
+    pdl_wait();
     __shared__ float4 sm4[8][128];
     int j = 0;
     while (j + 1 < b.count && (int)blockIdx.x >= b.job[j + 1].first_cta) j++;

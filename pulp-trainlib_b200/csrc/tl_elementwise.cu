@@ -43,6 +43,7 @@ __device__ __forceinline__ float act_apply(int kind, float x, float slope)
 
 template <class T> __global__ void act_fw_kernel(int kind, const T *__restrict__ x, T *__restrict__ y, long long n, float slope)
 {
+    pdl_wait();
     GRID_STRIDE(i, n) st(y + i, act_apply(kind, ld(x + i), slope));
 }
 
@@ -52,6 +53,7 @@ template <class T>
 __global__ void act_bw_kernel(int kind, const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ dy,
                               T *__restrict__ dx, long long n, float slope)
 {
+    pdl_wait();
     GRID_STRIDE(i, n) {
         float g = ld(dy + i), r;
         if (kind == ACT_RELU) r = ld(x + i) > 0.f ? g : 0.f;
@@ -93,6 +95,7 @@ template <class T>
 __global__ void __launch_bounds__(128) softmax_fw_kernel(const T *__restrict__ in, T *__restrict__ out,
                                                          T *__restrict__ maxes, T *__restrict__ sums, int width, int rows_per_batch)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const T *ip = in + row * width;
@@ -116,6 +119,7 @@ template <class T>
 __global__ void __launch_bounds__(128) softmax_bw_kernel(const T *__restrict__ out, const T *__restrict__ dout,
                                                          T *__restrict__ din, T *__restrict__ sums, int width, int rows_per_batch)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const T *op = out + row * width, *gp = dout + row * width;
@@ -140,6 +144,7 @@ template <class T> void softmax_bw(const T *out, const T *dout, T *din, T *sums,
 
 template <class T> __global__ void row_max_kernel(const T *__restrict__ in, T *__restrict__ maxes, int width)
 {
+    pdl_wait();
     __shared__ float red[33];
     const T *ip = in + (long long)blockIdx.x * width;
     float m = ld(maxes + blockIdx.x);                  // reference semantics: running maximum
@@ -149,6 +154,7 @@ template <class T> __global__ void row_max_kernel(const T *__restrict__ in, T *_
 }
 template <class T> __global__ void exp_sum_kernel(const T *__restrict__ in, T *__restrict__ out, const T *__restrict__ maxes, T *__restrict__ sums, int width)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     float m = ld(maxes + row), s = 0.f;
@@ -162,6 +168,7 @@ template <class T> __global__ void exp_sum_kernel(const T *__restrict__ in, T *_
 }
 template <class T> __global__ void row_div_kernel(T *__restrict__ io, const T *__restrict__ sums, int width, long long n)
 {
+    pdl_wait();
     GRID_STRIDE(i, n) st(io + i, __fdiv_rn(ld(io + i), ld(sums + i / width)));
 }
 template <class T> void row_max(const T *in, T *maxes, int rows, int width) { if (rows > 0) TL_LAUNCH((row_max_kernel<T>), rows, 128, 0, in, maxes, width); }
@@ -181,6 +188,7 @@ __global__ void __launch_bounds__(256) instnorm_fw_kernel(const T *__restrict__ 
                                                           T *__restrict__ mean_o, T *__restrict__ var_o, T *__restrict__ std_o,
                                                           int C, int D, int frozen, float eps)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long plane = blockIdx.x;
     const int ch = (int)(plane % C);
@@ -215,6 +223,7 @@ __global__ void __launch_bounds__(256) instnorm_bw_input_kernel(const T *__restr
                                                                 const T *__restrict__ gamma, const T *__restrict__ mean_i,
                                                                 const T *__restrict__ var_i, const T *__restrict__ std_i, int C, int D)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long plane = blockIdx.x;
     const int ch = (int)(plane % C);
@@ -241,6 +250,7 @@ template <class T>
 __global__ void __launch_bounds__(256) instnorm_bw_param_kernel(const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part,
                                                                 const T *__restrict__ mean_i, const T *__restrict__ std_i, int D)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long plane = blockIdx.x;
     const T *xp = x + plane * D, *gp = dy + plane * D;
@@ -258,6 +268,7 @@ __global__ void __launch_bounds__(256) instnorm_bw_param_kernel(const T *__restr
 template <class T>
 __global__ void __launch_bounds__(256) column_partial_kernel(const T *__restrict__ in, float *__restrict__ part, int n, int dim, int rows_per_slice)
 {
+    pdl_wait();
     __shared__ float sm[8][33];
     const int c = threadIdx.x & 31, r = threadIdx.x >> 5, j = blockIdx.x * 32 + c;
     const int begin = blockIdx.y * rows_per_slice, end = min(n, begin + rows_per_slice);
@@ -277,6 +288,7 @@ __global__ void __launch_bounds__(256) column_partial_kernel(const T *__restrict
 template <class TI, class TO>
 __global__ void __launch_bounds__(1024) column_direct_kernel(const TI *__restrict__ in, TO *__restrict__ out, int n, int dim, int pairs)
 {
+    pdl_wait();
     // 32 columns x 32 row lanes; a lane walks rows r, r + 32, ... four at a time (independent loads in flight, the four partial
     // sums are then added in a fixed order), the 32 lane sums of a column are added in lane order: one fixed summation tree.
     __shared__ float sm[32][33];
@@ -302,6 +314,7 @@ __global__ void __launch_bounds__(1024) column_direct_kernel(const TI *__restric
 template <class T>
 __global__ void __launch_bounds__(128) column_final_kernel(const float *__restrict__ part, T *__restrict__ out, int slices, int dim, int pairs)
 {
+    pdl_wait();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= dim) return;
     float s = 0.f;
@@ -341,6 +354,7 @@ __global__ void __launch_bounds__(256) instnorm_fw_warp_kernel(const float *__re
                                                                float *__restrict__ mean_o, float *__restrict__ var_o, float *__restrict__ std_o,
                                                                long long planes, int C, int D, int frozen, float eps, const float *__restrict__ skip)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long plane = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (plane >= planes) return;
@@ -400,6 +414,7 @@ __global__ void __launch_bounds__(256) instnorm_bw_warp_kernel(const float *__re
                                                                const float *__restrict__ mean_i, const float *__restrict__ var_i,
                                                                const float *__restrict__ std_i, long long planes, int C, int D, const float *__restrict__ dy2)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long plane = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (plane >= planes) return;
@@ -454,6 +469,7 @@ __global__ void __launch_bounds__(256) instnorm_fw_half_kernel(const float *__re
                                                                float *__restrict__ mean_o, float *__restrict__ var_o, float *__restrict__ std_o,
                                                                long long planes, int C, int D, int frozen, float eps, const float *__restrict__ skip)
 {
+    pdl_wait();
     const int l16 = threadIdx.x & 15;
     const long long plane = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const bool live = plane < planes;
@@ -494,6 +510,7 @@ __global__ void __launch_bounds__(256) instnorm_bw_half_kernel(const float *__re
                                                                const float *__restrict__ mean_i, const float *__restrict__ var_i,
                                                                const float *__restrict__ std_i, long long planes, int C, int D, const float *__restrict__ dy2)
 {
+    pdl_wait();
     const int l16 = threadIdx.x & 15;
     const long long plane = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     const bool live = plane < planes;
@@ -528,6 +545,7 @@ __global__ void __launch_bounds__(256) instnorm_bw_pair_kernel(const float *__re
                                                                const float *__restrict__ mean_i, const float *__restrict__ var_i,
                                                                const float *__restrict__ std_i, long long planes, int C, int D, const float *__restrict__ dy2)
 {
+    pdl_wait();
     __shared__ float2 sums[4][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = warp >> 1, half = warp & 1;
     const long long plane = (long long)blockIdx.x * 4 + slot;
@@ -727,6 +745,7 @@ template <class T>
 __global__ void __launch_bounds__(256) batchnorm_fw_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ w,
                                                            const T *__restrict__ b, int B, int C, int HW, float eps)
 {
+    pdl_wait();
     __shared__ float red[33];
     const int c = blockIdx.x % C;
     const long long s = blockIdx.x / C;                  // stream
@@ -771,6 +790,7 @@ template <class T, int NV>
 __global__ void __launch_bounds__(256) layernorm_fw_warp_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ w,
                                                                 const T *__restrict__ b, int rows, int width, float eps)
 {
+    pdl_wait();
     const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     float v[NV], wv[NV], bv[NV];
@@ -789,6 +809,7 @@ template <class T>
 __global__ void __launch_bounds__(128) layernorm_fw_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ w,
                                                            const T *__restrict__ b, int width, float eps)
 {
+    pdl_wait();
     __shared__ float red[33];
     const T *xp = x + (long long)blockIdx.x * width;
     T *yp = y + (long long)blockIdx.x * width;
@@ -814,6 +835,7 @@ __global__ void __launch_bounds__(256) layernorm_bw_warp_kernel(const T *__restr
                                                                 float *__restrict__ part, T *__restrict__ dw, T *__restrict__ db, int rows, int width,
                                                                 int rows_per_cta, float eps)
 {
+    pdl_wait();
     constexpr int W = 32 * NV;
     __shared__ float sm[8][W];
     __shared__ unsigned ticket_s;
@@ -880,6 +902,7 @@ template <class T>
 __global__ void __launch_bounds__(128) layernorm_bw_rows_kernel(const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ dy,
                                                                 T *__restrict__ dx, float2 *__restrict__ stats, int width, float eps)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const T *xp = x + row * width, *gp = dy + row * width;
@@ -907,6 +930,7 @@ template <class T>
 __global__ void __launch_bounds__(128) layernorm_bw_cols_kernel(const T *__restrict__ x, const T *__restrict__ dy, const float2 *__restrict__ stats,
                                                                 T *__restrict__ dw, T *__restrict__ db, int rows, int width)
 {
+    pdl_wait();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= width) return;
     float a = 0.f, b = 0.f;
@@ -952,6 +976,7 @@ template <class T> void layernorm_fw(const T *x, T *y, const T *w, const T *b, i
 
 template <class T> __global__ void mean_std_kernel(const T *__restrict__ x, T *mean, T *var, T *stdev, int D, float eps)
 {
+    pdl_wait();
     __shared__ float red[33];
     float s = 0.f, q = 0.f;
     for (int d = threadIdx.x; d < D; d += blockDim.x) { float t = ld(x + d); s += t; q = fmaf(t, t, q); }
@@ -979,6 +1004,7 @@ static __device__ unsigned mse_tickets[64];                  // one per stream; 
 template <class T>
 __global__ void __launch_bounds__(256) mse_fw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ loss, float *__restrict__ part, int dim, int parts)
 {
+    pdl_wait();
     __shared__ float red[33];
     __shared__ unsigned ticket_s;
     const long long stream = blockIdx.y;
@@ -1004,6 +1030,7 @@ __global__ void __launch_bounds__(256) mse_fw_kernel(const T *__restrict__ y, co
 }
 template <class T> __global__ void mse_bw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ dy, int dim, long long total)
 {
+    pdl_wait();
     const float meanval = 1.0f / (float)dim;
     GRID_STRIDE(i, total) st(dy + i, __fmul_rn(__fmul_rn(meanval, 2.0f), __fsub_rn(ld(y + i), ld(t + i))));
 }
@@ -1029,6 +1056,7 @@ template <class T> void mse_bw(const T *y, const T *t, T *dy, int dim, int n)
 template <class T>
 __global__ void ce_kernel(const T *__restrict__ z, const T *__restrict__ t, T *__restrict__ loss, T *__restrict__ dz, int dim, int n)
 {
+    pdl_wait();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const T *zp = z + (long long)s * dim, *tp = t + (long long)s * dim;
@@ -1053,6 +1081,7 @@ template <class T> void ce_bw(const T *z, const T *t, T *dz, int dim, int n) { i
 // does in place [ref: lib/sources/pulp_optimizers_fp32.c:48-62].
 template <class T> __global__ void sgd_kernel(T *__restrict__ w, T *__restrict__ g, long long n, float lr, float lambda)
 {
+    pdl_wait();
     GRID_STRIDE(i, n) {
         float wv = ld(w + i), gv = ld(g + i);
         if (lambda != 0.f) { gv = __fadd_rn(gv, __fmul_rn(lambda, wv)); st(g + i, gv); }
@@ -1061,17 +1090,18 @@ template <class T> __global__ void sgd_kernel(T *__restrict__ w, T *__restrict__
 }
 template <class T> void sgd(T *w, T *g, long long n, float lr, float lambda) { if (n > 0) TL_LAUNCH((sgd_kernel<T>), grid_for(n), 256, 0, w, g, n, lr, lambda); }
 
-template <class T> __global__ void add_kernel(const T *a, const T *b, T *c, long long n) { GRID_STRIDE(i, n) st(c + i, __fadd_rn(ld(a + i), ld(b + i))); }
+template <class T> __global__ void add_kernel(const T *a, const T *b, T *c, long long n) { pdl_wait(); GRID_STRIDE(i, n) st(c + i, __fadd_rn(ld(a + i), ld(b + i))); }
 template <class T> void add(const T *a, const T *b, T *c, long long n) { if (n > 0) TL_LAUNCH((add_kernel<T>), grid_for(n), 256, 0, a, b, c, n); }
-template <class T> __global__ void copy_kernel(const T *__restrict__ f, T *__restrict__ t, long long n) { GRID_STRIDE(i, n) t[i] = f[i]; }
+template <class T> __global__ void copy_kernel(const T *__restrict__ f, T *__restrict__ t, long long n) { pdl_wait(); GRID_STRIDE(i, n) t[i] = f[i]; }
 template <class T> void copy_n(const T *from, T *to, long long n) { if (n > 0 && from != to) TL_LAUNCH((copy_kernel<T>), grid_for(n), 256, 0, from, to, n); }
-template <class T> __global__ void fill_kernel(T *t, float v, long long n) { GRID_STRIDE(i, n) st(t + i, v); }
+template <class T> __global__ void fill_kernel(T *t, float v, long long n) { pdl_wait(); GRID_STRIDE(i, n) st(t + i, v); }
 template <class T> void fill(T *to, float v, long long n) { if (n > 0) TL_LAUNCH((fill_kernel<T>), grid_for(n), 256, 0, to, v, n); }
-template <class T> __global__ void scale_kernel(T *x, float s, long long n) { GRID_STRIDE(i, n) st(x + i, __fmul_rn(ld(x + i), s)); }
+template <class T> __global__ void scale_kernel(T *x, float s, long long n) { pdl_wait(); GRID_STRIDE(i, n) st(x + i, __fmul_rn(ld(x + i), s)); }
 template <class T> void scale(T *x, float s, long long n) { if (n > 0) TL_LAUNCH((scale_kernel<T>), grid_for(n), 256, 0, x, s, n); }
 // mat[H x W] += bias: per_row -> bias[row] [ref: lib/sources/pulp_train_utils_fp32.c:1286-1327], else bias[col]
 template <class T> __global__ void bias_add_kernel(T *mat, const T *bias, int W, long long n, int per_row)
 {
+    pdl_wait();
     GRID_STRIDE(i, n) st(mat + i, __fadd_rn(ld(mat + i), ld(bias + (per_row ? i / W : i % W))));
 }
 template <class T> void bias_add_rows(T *mat, const T *bias, int H, int W, int per_row)
@@ -1079,8 +1109,8 @@ template <class T> void bias_add_rows(T *mat, const T *bias, int H, int W, int p
     long long n = (long long)H * W;
     if (n > 0) TL_LAUNCH((bias_add_kernel<T>), grid_for(n), 256, 0, mat, bias, W, n, per_row);
 }
-__global__ void cast_h2f_kernel(const __half *s, float *d, long long n) { GRID_STRIDE(i, n) d[i] = __half2float(s[i]); }
-__global__ void cast_f2h_kernel(const float *s, __half *d, long long n) { GRID_STRIDE(i, n) d[i] = __float2half_rn(s[i]); }
+__global__ void cast_h2f_kernel(const __half *s, float *d, long long n) { pdl_wait(); GRID_STRIDE(i, n) d[i] = __half2float(s[i]); }
+__global__ void cast_f2h_kernel(const float *s, __half *d, long long n) { pdl_wait(); GRID_STRIDE(i, n) d[i] = __float2half_rn(s[i]); }
 void cast_h2f(const __half *src, float *dst, long long n) { if (n > 0) TL_LAUNCH(cast_h2f_kernel, grid_for(n), 256, 0, src, dst, n); }
 void cast_f2h(const float *src, __half *dst, long long n) { if (n > 0) TL_LAUNCH(cast_f2h_kernel, grid_for(n), 256, 0, src, dst, n); }
 
@@ -1090,6 +1120,7 @@ template <class T>
 __global__ void avgpool_fw_kernel(const T *__restrict__ x, T *__restrict__ y, long long total, int H, int W, int Ho, int Wo,
                                   int Hk, int Wk, int sh, int sw)
 {
+    pdl_wait();
     GRID_STRIDE(e, total) {
         int wo = e % Wo, ho = (e / Wo) % Ho;
         long long plane = e / ((long long)Wo * Ho);
@@ -1104,6 +1135,7 @@ template <class T>
 __global__ void avgpool_bw_kernel(const T *__restrict__ dy, T *__restrict__ dx, long long total, int H, int W, int Ho, int Wo,
                                   int Hk, int Wk, int sh, int sw)
 {
+    pdl_wait();
     GRID_STRIDE(e, total) {
         int wi = e % W, hi = (e / W) % H;
         long long plane = e / ((long long)W * H);
@@ -1127,6 +1159,7 @@ __global__ void avgpool_bw_kernel(const T *__restrict__ dy, T *__restrict__ dx, 
 // in the reference's order from 16-byte loads; backward writes dy / count with 16-byte stores.
 __global__ void __launch_bounds__(256) avgpool_global_fw_kernel(const float *__restrict__ x, float *__restrict__ y, long long planes, int hw4, float cnt)
 {
+    pdl_wait();
     const long long pl = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (pl >= planes) return;
     const float4 *xp = reinterpret_cast<const float4 *>(x) + pl * hw4;
@@ -1137,6 +1170,7 @@ __global__ void __launch_bounds__(256) avgpool_global_fw_kernel(const float *__r
 }
 __global__ void __launch_bounds__(256) avgpool_global_bw_kernel(const float *__restrict__ dy, float4 *__restrict__ dx, long long total4, int hw4, float cnt)
 {
+    pdl_wait();
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total4; e += (long long)gridDim.x * blockDim.x) {
         const float v = __fdiv_rn(dy[e / hw4], cnt);
         dx[e] = make_float4(v, v, v, v);
@@ -1174,6 +1208,7 @@ struct Shape8 { int n; int d[8]; long long s[8]; };   // extents and source stri
 // out = in.transpose(axes): out extent i = dims[axes[i]]  [ref: lib/sources/pulp_train_utils_fp32.c:79-185]
 template <class T> __global__ void transpose_kernel(const T *__restrict__ in, T *__restrict__ out, Shape8 sh, long long total)
 {
+    pdl_wait();
     GRID_STRIDE(e, total) {
         long long rem = e, src = 0;
 #pragma unroll
@@ -1186,6 +1221,7 @@ template <class T> __global__ void transpose_kernel(const T *__restrict__ in, T 
 // 2-D case: 32x32 tiles through shared memory so that both sides are coalesced.
 template <class T> __global__ void transpose2d_kernel(const T *__restrict__ in, T *__restrict__ out, int R, int Ccols)
 {
+    pdl_wait();
     __shared__ T tile[32][33];
     int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     for (int r = threadIdx.y; r < 32; r += blockDim.y)
@@ -1221,6 +1257,7 @@ template <class T> void transpose_nd(const T *in, T *out, const int *dims, const
 struct Bcast8 { int n; int d[8]; long long sa[8]; long long sb[8]; };
 template <class T> __global__ void broadcast_add_kernel(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ c, Bcast8 bc, long long total)
 {
+    pdl_wait();
     GRID_STRIDE(e, total) {
         long long rem = e, ia = 0, ib = 0;
 #pragma unroll
@@ -1258,6 +1295,7 @@ template <class T> void broadcast_add(const T *a, const T *b, T *c, const int *d
 template <class T>
 __global__ void pad_kernel(const T *__restrict__ src, T *__restrict__ dst, int C, int H, int W, int padL, int padU, int Ho, int Wo, int hwc, long long total)
 {
+    pdl_wait();
     GRID_STRIDE(e, total) {
         int c, ht, wt;
         if (!hwc) { wt = e % Wo; ht = (e / Wo) % Ho; c = e / ((long long)Wo * Ho); }

@@ -22,6 +22,7 @@ static inline int fam_grid(long long n, int per_block = 256, int waves = 16)
 template <class T, bool BERHU>
 __global__ void __launch_bounds__(256) l1_fw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ loss, int dim, float alpha)
 {
+    pdl_wait();
     __shared__ float red[33];
     const T *yp = y + (long long)blockIdx.x * dim, *tp = t + (long long)blockIdx.x * dim;
     const float meanval = 1.0f / (float)dim;
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(256) l1_fw_kernel(const T *__restrict__ y, con
 template <class T, bool BERHU>
 __global__ void __launch_bounds__(256) l1_bw_kernel(const T *__restrict__ y, const T *__restrict__ t, T *__restrict__ dy, int dim, float alpha)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long base = (long long)blockIdx.x * dim;
     const float meanval = 1.0f / (float)dim;
@@ -80,6 +82,7 @@ template <class T>
 __global__ void maxpool_fw_kernel(const T *__restrict__ x, T *__restrict__ y, long long total, int H, int W, int Ho, int Wo,
                                   int Hk, int Wk, int Hs, int Ws)
 {
+    pdl_wait();
     FAM_STRIDE(i, total) {
         const int wo = (int)(i % Wo), ho = (int)((i / Wo) % Ho);
         const long long plane = i / ((long long)Wo * Ho);
@@ -94,6 +97,7 @@ template <class T>
 __global__ void maxpool_bw_kernel(const T *__restrict__ x, const T *__restrict__ dy, T *__restrict__ dx, long long total, int H, int W,
                                   int Ho, int Wo, int Hk, int Wk, int Hs, int Ws)
 {
+    pdl_wait();
     FAM_STRIDE(i, total) {
         const int w = (int)(i % W), h = (int)((i / W) % H);
         const long long plane = i / ((long long)W * H);
@@ -136,6 +140,7 @@ template <class T> void maxpool_bw(const T *x, const T *dy, T *dx, long long pla
 template <class T>
 __global__ void nonorm_kernel(const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ b, T *__restrict__ y, long long total, int width)
 {
+    pdl_wait();
     FAM_STRIDE(i, total) { const int j = (int)(i % width); st(y + i, __fadd_rn(__fmul_rn(ld(x + i), ld(w + j)), ld(b + j))); }
 }
 template <class T> void nonorm_fw(const T *x, const T *w, const T *b, T *y, long long rows, int width)
@@ -148,6 +153,7 @@ template <class T> void nonorm_fw(const T *x, const T *w, const T *b, T *y, long
 template <class T>
 __global__ void weighted_scaling_kernel(const T *__restrict__ x, const T *__restrict__ w, T *__restrict__ y, long long n, float sf, const T *__restrict__ sumsq)
 {
+    pdl_wait();
     if (sumsq) {
         float ss = __fdiv_rn(ld(sumsq), (float)n);
         ss = __fadd_rn(ss, 1e-5f);
@@ -165,6 +171,7 @@ template <class T> void weighted_scaling(const T *x, const T *w, T *y, long long
 template <class T>
 __global__ void __launch_bounds__(1024) sum_of_squares_kernel(const T *__restrict__ x, T *__restrict__ out, long long n)
 {
+    pdl_wait();
     __shared__ float red[33];
     float s = 0.f;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) { const float v = ld(x + i); s = fmaf(v, v, s); }
@@ -179,6 +186,7 @@ template <class T> void sum_of_squares(const T *x, T *out, long long n)
 template <class T>
 __global__ void swiglu_kernel(const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y, long long n)
 {
+    pdl_wait();
     FAM_STRIDE(i, n) {
         float v = ld(a + i);
         v = __fmul_rn(v, __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-v))));
@@ -195,6 +203,7 @@ template <class T> void swiglu(const T *a, const T *b, T *y, long long n)
 // maxes[0] = max of a W-long vector (one core's share = all of it)   [ref: lib/sources/pulp_train_utils_fp32.c:987-1006]
 template <class T> __global__ void __launch_bounds__(1024) vec_max_kernel(const T *__restrict__ x, T *__restrict__ out, long long n)
 {
+    pdl_wait();
     __shared__ float red[33];
     float m = -FLT_MAX;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, ld(x + i));
@@ -206,6 +215,7 @@ template <class T> void vec_max(const T *x, T *out, long long n) { if (n > 0) TL
 // output[i] = exp(input[i] - max); sums[0] = their sum   [ref: lib/sources/pulp_train_utils_fp32.c:1730-1756]
 template <class T> __global__ void __launch_bounds__(1024) vec_exp_sum_kernel(const T *__restrict__ x, T *__restrict__ y, T *__restrict__ sum, long long n, float mx)
 {
+    pdl_wait();
     __shared__ float red[33];
     float s = 0.f;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) {
@@ -221,6 +231,7 @@ template <class T> void vec_exp_sum(const T *x, T *y, T *sum, long long n, float
 // out = exp(in - max) / sum over one vector   [ref: lib/sources/pulp_act_fp32.c:651-685]
 template <class T> __global__ void __launch_bounds__(1024) vector_softmax_kernel(const T *__restrict__ x, T *__restrict__ y, long long n)
 {
+    pdl_wait();
     __shared__ float red[33];
     float m = -FLT_MAX;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, ld(x + i));
@@ -232,7 +243,7 @@ template <class T> __global__ void __launch_bounds__(1024) vector_softmax_kernel
 }
 template <class T> void vector_softmax(const T *x, T *y, long long n) { if (n > 0) TL_LAUNCH((vector_softmax_kernel<T>), 1, 1024, 0, x, y, n); }
 // io[i] /= d   [ref: lib/sources/pulp_train_utils_fp32.c:1250-1264]
-template <class T> __global__ void vec_div_kernel(T *__restrict__ io, long long n, float d) { FAM_STRIDE(i, n) st(io + i, __fdiv_rn(ld(io + i), d)); }
+template <class T> __global__ void vec_div_kernel(T *__restrict__ io, long long n, float d) { pdl_wait(); FAM_STRIDE(i, n) st(io + i, __fdiv_rn(ld(io + i), d)); }
 template <class T> void vec_div(T *io, long long n, float d) { if (n > 0) TL_LAUNCH((vec_div_kernel<T>), fam_grid(n), 256, 0, io, n, d); }
 
 // The reference's polynomial stand-in for 2^-x: 0 from 3.14 on   [ref: lib/sources/pulp_train_utils_fp32.c:1009-1027]
@@ -250,6 +261,7 @@ __device__ __forceinline__ float threshold_dev(float x)
 // output[i][j] = threshold(maxes[i] - input[i][j]); sums[i] = row sum, dim x dim   [ref: pulp_train_utils_fp32.c:1193-1220]
 template <class T> __global__ void __launch_bounds__(128) shift_sum_kernel(const T *__restrict__ x, const T *__restrict__ maxes, T *__restrict__ y, T *__restrict__ sums, int dim)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const float m = ld(maxes + row);
@@ -263,6 +275,7 @@ template <class T> void shift_sum(const T *x, const T *maxes, T *y, T *sums, int
 // S[i] = sum_j A[i][j] B[i][j];  out[i][j] = (A[i][j] - S[i]) B[i][j]   [ref: pulp_train_utils_fp32.c:1136-1189]
 template <class T> __global__ void __launch_bounds__(128) sm_bw_op1_kernel(const T *__restrict__ A, const T *__restrict__ B, T *__restrict__ S, int W)
 {
+    pdl_wait();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     float s = 0.f;
@@ -272,6 +285,7 @@ template <class T> __global__ void __launch_bounds__(128) sm_bw_op1_kernel(const
 }
 template <class T> __global__ void sm_bw_op2_kernel(const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ S, T *__restrict__ out, long long total, int W)
 {
+    pdl_wait();
     FAM_STRIDE(i, total) st(out + i, __fmul_rn(__fsub_rn(ld(A + i), ld(S + i / W)), ld(B + i)));
 }
 template <class T> void sm_bw_op1(const T *A, const T *B, T *S, int H, int W) { if (H > 0 && W > 0) TL_LAUNCH((sm_bw_op1_kernel<T>), H, 128, 0, A, B, S, W); }

@@ -16,6 +16,7 @@ template <class T, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_ffma_kernel(GemmDesc<T> d)
 {
+    pdl_wait();
     const int b = blockIdx.z;
     const T *A = d.A + (long long)b * d.a_bs;
     const T *B = d.B + (long long)b * d.b_bs;
@@ -222,6 +223,7 @@ template <class T, int VEC>
 __global__ void __launch_bounds__(256) linear_fw_kernel(const T *__restrict__ W, const T *__restrict__ x,
                                                         const T *__restrict__ bias, T *__restrict__ y, int out, int in, int parts)
 {
+    pdl_wait();
     // a row is cut into `parts` segments (a multiple of 128 elements each), one warp per segment, so that layers with
     // few rows still put enough loads in flight; the segment sums of a row are added in segment order
     __shared__ float seg[8];
@@ -268,6 +270,7 @@ template <class T>
 __global__ void __launch_bounds__(256) linear_wg_kernel(const T *__restrict__ dy, const T *__restrict__ x,
                                                         T *__restrict__ dW, int out, int in)
 {
+    pdl_wait();
     constexpr int V = 16 / sizeof(T);
     const long long total = (long long)out * in;
     const bool vec_ok = (in % V == 0) && (((uintptr_t)dW & 15) == 0) && (((uintptr_t)x & 15) == 0);
@@ -305,6 +308,7 @@ template <class T>
 __global__ void __launch_bounds__(256) linear_wg_streams_partial_kernel(const T *__restrict__ dy, const T *__restrict__ x, float *__restrict__ part,
                                                                         int n, int out, int in, int per)
 {
+    pdl_wait();
     const int s0 = blockIdx.y * per, s1 = min(n, s0 + per);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= out * in) return;
@@ -316,6 +320,7 @@ __global__ void __launch_bounds__(256) linear_wg_streams_partial_kernel(const T 
 template <class T>
 __global__ void linear_wg_streams_reduce_kernel(const float *__restrict__ part, T *__restrict__ dW, int count, int blocks)
 {
+    pdl_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
     float acc = 0.f;
@@ -352,6 +357,7 @@ template <class T>
 __global__ void __launch_bounds__(128) linear_ig_partial_kernel(const T *__restrict__ W, const T *__restrict__ dy,
                                                                 float *__restrict__ part, int out, int in, int rows_per_slab)
 {
+    pdl_wait();
     constexpr int V = 16 / sizeof(T);
     const int slab = blockIdx.y;
     const int o_begin = slab * rows_per_slab;
@@ -398,6 +404,7 @@ __global__ void __launch_bounds__(128) linear_ig_partial_kernel(const T *__restr
 template <class T>
 __global__ void __launch_bounds__(1024) linear_ig_reduce_kernel(const float *__restrict__ part, T *__restrict__ dx, int in, int slabs)
 {
+    pdl_wait();
     __shared__ float sm[32][33];
     const int cx = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + cx;
@@ -445,6 +452,7 @@ __global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_fused_kernel
                                                                                  T *__restrict__ dW, float *__restrict__ part, T *__restrict__ dx,
                                                                                  int out, int in, int rows_per_slab, int slabs)
 {
+    pdl_wait();
     constexpr int V = 16 / sizeof(T);
     __shared__ float red[LBW_LANES][LBW_STRIPS][V + 1];
     __shared__ unsigned ticket_s;

@@ -200,6 +200,7 @@ template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST> struc
 template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC>
 __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(const __grid_constant__ GgParams<T> g)
 {
+    pdl_wait();
     typedef GgCfg<T, BM, BN, WM, WN, WK, KC, ST> Cfg;
     constexpr int NT = Cfg::NT, PAD = Cfg::PAD, PK = Cfg::PK, PA_R = Cfg::PA_R, PB_R = Cfg::PB_R;
     extern __shared__ __align__(16) unsigned char gg_smem[];

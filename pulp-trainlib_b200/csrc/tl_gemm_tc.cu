@@ -111,6 +111,7 @@ __device__ __forceinline__ void gt_stage(const T *__restrict__ base, long long r
 template <class T>
 __global__ void __launch_bounds__(GT_THREADS) gemm_tc_kernel(GtParams p)
 {
+    pdl_wait();
     typedef GtCfg<T> Cfg;
     constexpr int BN = Cfg::BN;
     constexpr uint32_t A_BYTES = gt_block_bytes(GT_BM), B_BYTES = gt_block_bytes(BN);

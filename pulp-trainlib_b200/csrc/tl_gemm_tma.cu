@@ -63,6 +63,7 @@ template <class T>
 __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensorMap a1,
                                                               const __grid_constant__ CUtensorMap b0, const __grid_constant__ CUtensorMap b1, TmParams p)
 {
+    pdl_wait();
     typedef TmCfg<T> Cfg;
     constexpr int BN = Cfg::BN, BK = Cfg::BK, ST = Cfg::STAGES;
     constexpr uint32_t A_BYTES = TM_BM * 128u, B_BYTES = BN * 128u;                // one 128-byte row per tile row
@@ -199,6 +200,7 @@ template <class T>
 __global__ void __launch_bounds__(256) pack_kmajor_kernel(const T *__restrict__ src, long long rs, long long cs, long long bs,
                                                           T *__restrict__ dst, T *__restrict__ dst_lo, int rows, int K, int Kp)
 {
+    pdl_wait();
     __shared__ float tile[32][33];
     const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32, b = blockIdx.z;
     const T *s = src + (long long)b * bs;

@@ -1,0 +1,109 @@
+"""Shapes at the edges of the kernels' tiles and dispatch rules (partial tiles, odd strides, several streams per tile, rows
+longer than a tile, split contractions), fp32 and fp16, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from abi_runner import AbiRunner
+from metrics import FP16_TOL, FP32_TOL, assert_close, seeded
+from oracle_bind import geom, out_hw
+
+pytestmark = pytest.mark.gpu
+F = np.float32
+
+
+@pytest.fixture(params=[False, True], ids=["fp32", "fp16"])
+def run(pkg, gpulib, request):
+    gpulib.trainlib_set_streams(1)
+    r = AbiRunner(pkg, gpulib, device=True, half=request.param)
+    yield r
+    r.close()
+    gpulib.trainlib_set_streams(1)
+
+
+def rounded(r, a):
+    return a.astype(r.dt).astype(F)
+
+
+CONV = [(28, 14, 45, 28, 3, 1, 1), (3, 33, 41, 70, 5, 2, 3), (6, 42, 13, 81, 5, 1, 1), (40, 9, 11, 64, 3, 1, 5), (16, 5, 5, 8, 3, 1, 40), (20, 3, 200, 24, 3, 1, 2),
+        (17, 12, 130, 33, 3, 2, 2), (64, 7, 7, 96, 1, 1, 30), (24, 28, 28, 48, 3, 1, 60), (33, 11, 12, 17, 3, 3, 2), (1, 6, 6, 4, 1, 1, 2), (70, 10, 10, 12, 7, 1, 1),
+        (12, 8, 9, 16, 1, 2, 3), (64, 12, 12, 64, 5, 1, 4)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", CONV)
+def test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n):
+    g = geom(cin, h, w, cout, k, stride=stride, pad=k // 2)
+    Ho, Wo = out_hw(g)
+    rng = seeded(cin + 3 * h + 5 * w + n)
+    x, wt, b = rounded(run, rng.uniform(-1, 1, (n, cin, h, w))), rounded(run, rng.uniform(-1, 1, (cout, cin, k, k))), rounded(run, rng.standard_normal(cout))
+    dy = rounded(run, rng.standard_normal((n, cout, Ho, Wo)) / 8)
+    run.lib.trainlib_set_streams(n)
+    X, W_, dY, B = run.t(x), run.t(wt), run.t(dy), run.t(b)
+    Y, dX, dW, dB, one = run.zeros(n, cout, Ho, Wo), run.zeros(*x.shape), run.zeros(*wt.shape), run.zeros(cout), run.zeros(4)
+    a = run.args(run.sname("Conv2D_args"), input=run.blob(X, dX, C=cin, H=h, W=w), coeff=run.blob(W_, dW, C=cin, H=k, W=k, dim=wt.size), bias=run.blob(B, dB, dim=cout, W=cout),
+                 output=run.blob(Y, dY, C=cout, H=Ho, W=Wo), Lpad=k // 2, Rpad=k // 2, Upad=k // 2, Dpad=k // 2, stride_h=stride, stride_w=stride,
+                 i2c_buffer=one, bt_buffer=one, USE_BIASES=1, USE_IM2COL=0, HWC=0)
+    for f in ("fw", "bw_param_grads", "bw_input_grads"):
+        run.call(run.fname("pulp_conv2d_fp32_%s_cl" % f), a)
+    tol = FP16_TOL if run.half else FP32_TOL
+    y, dx = Y.get().astype(F), dX.get().astype(F)
+    for s in range(n):
+        assert_close(y[s], oracle.conv2d_fw(x[s], wt, b, g), tol, "fw stream %d" % s)
+        assert_close(dx[s], oracle.conv2d_ig(dy[s], wt, g), tol, "ig stream %d" % s)
+    want = sum(oracle.conv2d_wg(x[s], dy[s], g)[0].astype(np.float64) for s in range(n)).astype(F)
+    assert_close(dW.get().astype(F), want, tol, "wg")
+    assert_close(dB.get().astype(F), dy.astype(np.float64).sum(axis=(0, 2, 3)).astype(F), tol, "bias gradient")
+
+
+@pytest.mark.parametrize("c,h,w,k,pad,n", [(5, 9, 7, 3, 1, 3), (64, 28, 28, 3, 1, 4), (3, 33, 18, 3, 0, 2), (8, 6, 6, 5, 2, 9), (2, 40, 41, 3, 2, 1), (7, 4, 4, 3, 1, 700), (4, 12, 12, 4, 1, 2)])
+def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n):
+    g = geom(c, h, w, c, k, pad=pad)
+    Ho, Wo = out_hw(g)
+    rng = seeded(c + h + w + n)
+    x, wt, dy = rounded(run, rng.standard_normal((n, c, h, w))), rounded(run, rng.standard_normal((c, k, k)) / k), rounded(run, rng.standard_normal((n, c, Ho, Wo)) / 4)
+    run.lib.trainlib_set_streams(n)
+    X, W_, dY = run.t(x), run.t(wt), run.t(dy)
+    Y, dX, dW = run.zeros(n, c, Ho, Wo), run.zeros(*x.shape), run.zeros(*wt.shape)
+    fields = {} if run.half else dict(stride_h=1, stride_w=1)
+    a = run.args(run.sname("DepthWise_Conv_args"), input=run.blob(X, dX, C=c, H=h, W=w), coeff=run.blob(W_, dW, C=c, H=k, W=k), output=run.blob(Y, dY, C=c, H=Ho, W=Wo),
+                 Lpad=pad, Rpad=pad, Upad=pad, Dpad=pad, skip_wg_grad=0, skip_in_grad=0, HWC=0, **fields)
+    run.call(run.fname("pulp_conv_dw_fp32_fw_cl"), a); run.call(run.fname("pulp_conv_dw_fp32_bw_cl"), a)
+    tol = FP16_TOL if run.half else FP32_TOL
+    y, dx = Y.get().astype(F), dX.get().astype(F)
+    for s in range(0, n, max(1, n // 5)):
+        assert_close(y[s], oracle.dw_fw(x[s], wt, g), tol, "fw stream %d" % s)
+        assert_close(dx[s], oracle.dw_ig(dy[s], wt, g), tol, "ig stream %d" % s)
+    want = sum(oracle.dw_wg(x[s], dy[s], g).astype(np.float64) for s in range(n)).astype(F)
+    assert_close(dW.get().astype(F), want, tol, "wg")
+
+
+@pytest.mark.parametrize("N,K,M", [(1, 1, 1), (17, 3001, 41), (16, 2048, 300), (33, 64, 31), (130, 7, 130), (64, 129, 65), (500, 40, 333), (1000, 60, 520), (128, 512, 128)])
+@pytest.mark.parametrize("trans_B", [0, 1])
+def test_products_of_small_groups(run, N, K, M, trans_B):
+    rng = seeded(N + K + M)
+    A, B = rounded(run, rng.standard_normal((N, K)) / np.sqrt(K)), rounded(run, rng.standard_normal((M, K) if trans_B else (K, M)))
+    want = (A.astype(np.float64) @ (B.T if trans_B else B).astype(np.float64)).astype(F)
+    assert_close(run.mm(A, B, N, K, M, trans_B=trans_B).astype(F), want, FP16_TOL if run.half else FP32_TOL, "mm")
+
+
+@pytest.mark.parametrize("rows,width", [(1, 1), (7, 33), (200, 128), (700, 250), (300, 512), (5, 1024), (9, 1500)])
+def test_layernorm_shapes(run, oracle, rows, width):
+    rng = seeded(rows + width)
+    x, w, b, dy = (rounded(run, a) for a in (rng.standard_normal((rows, width)), rng.standard_normal(width), rng.standard_normal(width), rng.standard_normal((rows, width)) / 16))
+    eps = float(np.asarray(1e-3, run.dt))
+    got = run.layernorm_ext(x, w, b, dy, rows, width, eps)
+    tol = FP16_TOL if run.half else FP32_TOL
+    assert_close(got["y"].astype(F), oracle.layernorm_fw(x, w, b, rows, width, eps), tol, "y")
+    dx, dw, db = oracle.layernorm_bw(x, w, dy, rows, width, eps)
+    for k, v in (("dx", dx), ("dw", dw), ("db", db)):
+        if np.abs(v).max() > 1e-6:                          # (a row of one element has no gradient)
+            assert_close(got[k].astype(F), v, tol, k)
+
+
+@pytest.mark.parametrize("dim", [1, 5, 1023, 1025, 70001, 400000])
+def test_mse_lengths(run, oracle, dim):
+    rng = seeded(dim)
+    y, t = rounded(run, rng.standard_normal(dim)), rounded(run, rng.standard_normal(dim))
+    loss, dy = run.loss("MSELoss", y, t)
+    tol = FP16_TOL if run.half else FP32_TOL
+    assert_close(np.asarray([loss], F), np.asarray([np.mean((t.astype(np.float64) - y) ** 2)], F), tol, "loss")
+    assert_close(dy.astype(F) * dim, (2.0 * (y.astype(np.float64) - t)).astype(F), tol if dim < 5000 or not run.half else 0.1, "dy")
