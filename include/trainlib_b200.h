@@ -135,14 +135,14 @@ void  trainlib_conv2d_fp16_bw_input_grads_acc_cl(void *Conv2D_args_fp16);
  * before anything outside the library (a collective, a kernel of your own, a cudaMemcpy) reads a gradient.  The values
  * are those of the immediate mode (same summation trees).  The arena is sized at a flush from what the calls since the
  * previous flush asked for: the first pass of a workload in this mode still sums at once, and so does any call whose
- * partial results do not fit (after a graph capture the arena is never moved again). */
+ * partial results do not fit (an arena that a captured graph uses stays where it is until the last graph is destroyed). */
 void  trainlib_set_deferred_reductions(int on);
 void  trainlib_flush_reductions(void);
 
 /* ---- CUDA graphs.  Entry-point calls made between begin and end are recorded instead of executed (device pointers
  * only: a host pointer would need a synchronous copy); the handle replays them with one launch on the library's
  * stream.  The recorded launches keep the addresses they saw, including library scratch: run the same calls once
- * before capturing so that the scratch arena has its final size; it is never shrunk or moved afterwards.
+ * before capturing so that the scratch arena has its final size; it is not shrunk or moved while a graph lives.
  * trainlib_kernel_launches() advances by the number of recorded kernels on every replay. */
 int   trainlib_graph_begin(void);
 void *trainlib_graph_end(void);               /* NULL on failure (see trainlib_last_error) */

@@ -96,7 +96,8 @@ private:
 };
 
 bool is_device_pointer(const void *p);
-bool arena_pinned();                // a captured graph holds addresses of library-owned device memory: never move it again
+bool arena_pinned();                // a captured graph holds addresses of library-owned device memory: it must stay where it is
+bool capturing();                   // between trainlib_graph_begin and _end
 
 // deferred reductions (tl_defer.cu): partial results kept until one batched launch sums them all
 bool defer_enabled();
@@ -105,6 +106,7 @@ void defer_plain(const float *part, float *out, long long n, int groups);
 void defer_columns(const float *part, float *out, int rows, int dim, int pairs);
 void defer_wgt(const float *part, float *out, int groups, long long group_floats, int Cin, int Cout, int s2, int xg, int cigs, int ncopy);
 void defer_flush();
+void defer_release();               // the last captured graph is gone
 
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 

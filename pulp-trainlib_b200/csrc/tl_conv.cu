@@ -204,10 +204,21 @@ static bool conv_fw_plan(const ConvGeom &g, int &TH, int &TW, int &S_T, int &CC,
     return smem <= 200 * 1024;
 }
 
+// Small fp32 layers: the tcgen05 kernels pay 7 us and about 0.3 ns per weight (barriers, tensor memory, the weight operand)
+// before the first tile, the mma.sync kernels 4.5 us but 0.075 us per million multiply-adds; this is where the lines cross.
+// (us, forward + input gradient: 16 -> 32 on 32 x 32, one stream 20.5 / 11.1, ten 21.2 / 22.3; 64 -> 64 on 8 x 8, 30 streams
+// 35.1 / 22.9, 100 streams 35.6 / 46.9; 32 -> 48 on 16 x 16 with 5 x 5 filters, one stream 42.2 / 24.4)
+static bool mma_beats_tcgen05(const ConvGeom &g)
+{
+    if (gemm_path() != 0) return false;
+    const double w = (double)g.Cin * g.Cout * g.Hk * g.Wk, ch = (double)((g.Cin + 7) / 8 * 8) * ((g.Cout + 7) / 8 * 8);
+    return ch * g.Hk * g.Wk * g.Hout * g.Wout * g.n < 30e6 + 4000.0 * w;
+}
 template <class T> static bool try_tc_fw(Scope &, const ConvGeom &, const T *, const T *, const T *, T *) { return false; }
 template <> bool try_tc_fw<float>(Scope &sc, const ConvGeom &g, const float *x, const float *w, const float *bias, float *y)
 {
-    if (conv1x1s_fw(g, x, w, bias, y)) return true;          // strided 1x1: memory-bound, CUDA cores
+    if (conv1x1s_fw(g, x, w, bias, y)) return true;          // strided 1x1: memory-bound
+    if (mma_beats_tcgen05(g) && conv_mma_fw<float>(g, x, w, bias, y)) { profile_add_flops(conv_flops(g)); return true; }
     return conv_tc_run(sc, x, w, bias, y, g.n, g.Cin, g.Hin, g.Win, g.Cout, g.Hout, g.Wout, g.Hk, g.Wk, g.sh, g.sw, g.padU, g.padL, g.Cout, g.Cin, false);
 }
 // dY of a strided convolution spread onto the input grid: dil[s][co][h][w] = dY[s][co][h/sh][w/sw] where both
@@ -336,6 +347,7 @@ template <> bool try_tc_ig<float>(Scope &sc, const ConvGeom &g, const float *dy,
 {
     // dX is a stride-1 convolution of dY with the rotated filters and padding k-1-pad
     if (g.Hk - 1 - g.padU < 0 || g.Wk - 1 - g.padL < 0) return false;
+    if (!(g.Hk == 1 && g.Wk == 1 && g.sh > 1) && mma_beats_tcgen05(g) && conv_mma_ig<float>(g, dy, w, dx)) { profile_add_flops(conv_flops(g)); return true; }
     if (g.sh == 1 && g.sw == 1)
         return conv_tc_run(sc, dy, w, (const float *)nullptr, dx, g.n, g.Cout, g.Hout, g.Wout, g.Cin, g.Hin, g.Win, g.Hk, g.Wk, 1, 1,
                            g.Hk - 1 - g.padU, g.Wk - 1 - g.padL, g.Cout, g.Cin, true);
@@ -1035,9 +1047,9 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
     const bool k3 = g.Hk == 3 && g.Wk == 3 && g.padL == 1, k1 = g.Hk == 1 && g.Wk == 1 && g.padL == 0 && g.padU == 0;
     if (try_tc_wg<T>(sc, g, x, dy, dw)) return;
     if (try_1x1_wg<T>(sc, g, x, dy, dw)) return;
-    // the register-tiled FFMA kernel below keeps 3x3 fp32 layers of 8, 16 and 32 pixel rows (100 streams of 16 -> 32 on 32 x 32: 31 us
-    // against 34 us on mma.sync)
-    if (!(sizeof(T) == 4 && k3) && try_mma_wg<T>(sc, g, x, dy, dw)) return;
+    // the register-tiled FFMA kernel below keeps stride-1 3x3 fp32 layers with few input channels on 8, 16 and 32 pixel rows (ten streams of 16 -> 32 on
+    // 32 x 32: 14.5 us against 16.4 us on mma.sync) unless the layer is small (one stream of it: 13.2 us against 9.3)
+    if (!(sizeof(T) == 4 && k3 && g.sh == 1 && g.Cin < 32 && conv_flops(g) > 3e7) && try_mma_wg<T>(sc, g, x, dy, dw)) return;
     if ((k3 || k1) && g.sh == g.sw && (g.sh == 1 || g.sh == 2) && g.Win == g.sw * g.Wout && (g.Wout == 8 || g.Wout == 16 || g.Wout == 32)) {
         // about 256 (stride 1) or 128 (stride 2) pixels per item: whole output rows, two streams for 8-pixel rows.
         // The item shape is part of the kernel type: (TW, TH, S_T) = (32, 8, 1), (16, 16, 1), (8, 8, 2) for stride 1

@@ -516,7 +516,7 @@ template <class T> static bool conv_mma_dispatch(CmFwd &p)
     for (int i = 0; i < p.ncls; i++) tiles += ((long long)p.n * p.cls[i].Hc * p.cls[i].Wc + 127) / 128;
     // Few tiles (single streams): 16 x 32 result tiles whose taps and channels are dealt to four warps each, so that a layer of
     // 32 channels on 32 x 32 pixels still occupies 64 CTAs; otherwise 128 pixels by 16, 32 or 64 channels.
-    if (tiles * ceil_div(p.Cd, p.Cd > 32 ? 64 : 32) < sm_count()) return conv_mma_launch<T, 1, 1, 2, 4, 32>(p, cpad, false);
+    if (2 * tiles * ceil_div(p.Cd, p.Cd > 32 ? 64 : 32) < sm_count()) return conv_mma_launch<T, 1, 1, 2, 4, 32>(p, cpad, false);
     if (p.Cd > 32) return conv_mma_launch<T, 2, 2, 4, 1, 128>(p, cpad, false) || conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
     if (p.Cd > 16) return conv_mma_launch<T, 2, 1, 8, 1, 128>(p, cpad, false) || conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
     return conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
@@ -741,12 +741,14 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
             }
         }
     }
-    // pixel shares of the warps added in warp order, one tap at a time; then this CTA's partial
+    // pixel shares of the warps meet in shared memory in the order of dW (taps innermost) and are added in warp order on the way
+    // out: one barrier and contiguous stores (tap by tap it was two barriers each and every store its own sector)
+    constexpr int RP = CI * TAPS + 4;
     float *red = reinterpret_cast<float *>(cm_smem);
     float *out = p.part + (size_t)blockIdx.y * p.Co * p.Ci * p.KK;
+    __syncthreads();
 #pragma unroll
-    for (int t = 0; t < TAPS; t++) {
-        __syncthreads();
+    for (int t = 0; t < TAPS; t++)
 #pragma unroll
         for (int i = 0; i < MI; i++)
 #pragma unroll
@@ -754,17 +756,19 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
                     const int r = (wm * MI + i) * 16 + (lane >> 2) + (q >> 1) * 8, c = wn * NI * 8 + j * 8 + 2 * (lane & 3) + (q & 1);
-                    red[(wk * CO + r) * CI + c] = acc[t][i][j][q];
+                    red[(wk * CO + r) * RP + c * TAPS + t] = acc[t][i][j][q];
                 }
-        __syncthreads();
-        if (t < p.ntaps)
-            for (int e = tid; e < CO * CI; e += NT) {
-                const int r = e / CI, c = e % CI;
-                float v = red[e];
+    __syncthreads();
+    for (int r = warp; r < CO; r += NT / 32) {
+        if (co0 + r >= p.Co) break;
+        float *row = out + ((long long)(co0 + r) * p.Ci + ci0) * p.KK + p.tap0;
+        for (int e = lane; e < CI * TAPS; e += 32) {
+            float v = red[r * RP + e];
 #pragma unroll
-                for (int k = 1; k < WK; k++) v += red[k * CO * CI + e];
-                if (co0 + r < p.Co && ci0 + c < p.Ci) out[((long long)(co0 + r) * p.Ci + ci0 + c) * p.KK + p.tap0 + t] = v;
-            }
+            for (int k = 1; k < WK; k++) v += red[(k * CO + r) * RP + e];
+            const int c = e / TAPS, t = e - c * TAPS;
+            if (ci0 + c < p.Ci && t < p.ntaps) row[c * p.KK + t] = v;
+        }
     }
 }
 
@@ -778,7 +782,7 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     auto tiles_of = [&](int bn) -> long long { return P < bn ? ceil_div(p.n, std::max(1, std::min(bn / P, p.n))) : p.Wo > bn ? (long long)p.n * p.Ho * ceil_div(p.Wo, bn) : (long long)p.n * ceil_div(P, bn); };
     // pixels per tile: what makes the fewest pixels of the longest CTA (planes and rounds come out even), halo rows included
     double best = 1e30;
-    for (int bn = BN; bn >= BN / 2; bn -= SZ == 2 ? 16 : 8) {
+    for (int bn = BN; bn >= BN / 4; bn -= SZ == 2 ? 16 : 8) {
         const int halo = bn + 2 * std::min(p.Wo, bn) * (p.rows_max - 1) / 3;
         const double cost = (double)ceil_div(tiles_of(bn), slots) * halo;
         if (cost < 0.98 * best) { best = cost; p.bn = bn; }
@@ -799,7 +803,7 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     p.d_off = (uint32_t)xb;
     const bool two = SZ == 4 && 2 * (xb + db) + 8 * BN <= 110 * 1024;
     p.buf2 = two ? (uint32_t)(xb + db) : 0u; p.t_off = (uint32_t)((xb + db) * (two ? 2 : 1));
-    const size_t smem = std::max((size_t)p.t_off + 8 * BN, (size_t)WK * CO * CI * 4);
+    const size_t smem = std::max((size_t)p.t_off + 8 * BN, (size_t)WK * CO * (CI * TAPS + 4) * 4);
     if (smem > CM_SMEM_MAX) return false;
     int groups = std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / ctiles);
     groups = std::min(std::min(groups, p.tiles), part_groups);

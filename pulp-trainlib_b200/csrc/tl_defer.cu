@@ -35,6 +35,7 @@ static struct {
     char *base = nullptr;
     size_t cap = 0, off = 0, need = 0;   // bytes; `need` = what this epoch asked for, granted or not
     DeferBatch batch = {};
+    std::vector<char *> outgrown;        // earlier blocks that captured graphs still use
 } d;
 
 // A CTA serves one job.  Weight-gradient partials (PLAIN, WGT): 512 consecutive elements through partial_sums_quad, the
@@ -112,17 +113,28 @@ void defer_flush()
         TL_LAUNCH(deferred_reduce_kernel, d.batch.ctas, 1024, 0, d.batch);
         d.batch.count = 0; d.batch.ctas = 0;
     }
-    // grow to what the last epoch asked for, unless a captured graph holds addresses inside the arena
-    if (d.need > d.cap && !arena_pinned()) {
+    // Grow to what the last epoch asked for.  Captured graphs may hold addresses inside the old block: it is then kept beside the
+    // new one until the last graph is destroyed.  (A graph of a small network used to freeze the arena at its size, and every
+    // later sum of a larger one ran at once: 25 launches and 100 us of a 4096-stream step.)
+    if (d.need > d.cap && !capturing()) {
         const size_t want = d.need + d.need / 4;
+        char *p = nullptr;
         cudaStreamSynchronize(stream());
+        if (d.base && arena_pinned()) { d.outgrown.push_back(d.base); d.base = nullptr; }
         if (d.base) cudaFree(d.base);
         d.base = nullptr; d.cap = 0;
-        char *p = nullptr;
         if (cudaMalloc(&p, want) == cudaSuccess) { d.base = p; d.cap = want; }
         else cudaGetLastError();                                    // no arena: every sum runs at once, as without the mode
     }
     d.off = 0; d.need = 0;
+}
+
+void defer_release()
+{
+    if (d.outgrown.empty()) return;
+    cudaStreamSynchronize(stream());
+    for (char *p : d.outgrown) cudaFree(p);
+    d.outgrown.clear();
 }
 
 // room for partial results that a deferred sum will read; nullptr = not now (the caller sums at once from its own scratch)

@@ -25,7 +25,8 @@ struct Context {
     long long launches = 0;
     std::vector<Chunk> chunks;     // staging arena; normally exactly one chunk
     int scope_depth = 0;
-    bool arena_pinned = false;     // a captured graph holds arena addresses: never free or merge chunks again
+    int live_graphs = 0;           // captured graphs hold arena addresses: while one lives (or is being recorded) no chunk is freed or merged
+    bool capturing = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int err = TL_OK;
     bool cuda_sticky = false;      // the context is lost: TL_ERR_CUDA cannot be cleared
@@ -176,7 +177,8 @@ bool is_device_pointer(const void *p)
 }
 
 // ---------------------------------------------------------------- arena
-bool arena_pinned() { return g.arena_pinned; }
+bool arena_pinned() { return g.live_graphs > 0 || g.capturing; }
+bool capturing() { return g.capturing; }
 
 static size_t arena_mark()
 {
@@ -191,7 +193,7 @@ static void arena_release(size_t mark)
     size_t idx = mark >> 48, off = mark & (((size_t)1 << 48) - 1);
     if (g.scope_depth == 0) {
         // top level: merge a fragmented arena into one chunk of the total size
-        if (g.chunks.size() > 1 && !g.arena_pinned) {
+        if (g.chunks.size() > 1 && !arena_pinned()) {
             size_t total = 0;
             cudaStreamSynchronize(g.cur_stream);
             for (auto &c : g.chunks) { total += c.cap; cudaFree(c.base); }
@@ -403,28 +405,27 @@ long long trainlib_kernel_launches(void) { return g.launches; }
 // ---- CUDA graphs: capture the entry-point calls queued between begin and end, replay them with one launch
 struct TlGraph { cudaGraphExec_t exec; cudaGraph_t graph; long long kernels; };
 static long long g_capture_launches0 = 0;
-static bool g_capturing = false;
-static bool g_capturing_now() { return g_capturing; }
+static bool g_capturing_now() { return g.capturing; }
 int trainlib_graph_begin(void)
 {
     if (!ready()) return g.err;
-    if (g_capturing) { set_error(TL_ERR_BAD_ARGS, "trainlib_graph_begin: a capture is already open"); return TL_ERR_BAD_ARGS; }
+    if (g.capturing) { set_error(TL_ERR_BAD_ARGS, "trainlib_graph_begin: a capture is already open"); return TL_ERR_BAD_ARGS; }
     defer_flush();                                  // sums pending from before the capture run now, outside the graph
     if (!TL_CUDA(cudaStreamBeginCapture(g.cur_stream, cudaStreamCaptureModeRelaxed))) return g.err;
-    g_capturing = true; g_capture_launches0 = g.launches;
-    g.arena_pinned = true;
+    g.capturing = true; g_capture_launches0 = g.launches;
     return TL_OK;
 }
 void *trainlib_graph_end(void)
 {
-    if (!ready() || !g_capturing) return nullptr;
+    if (!ready() || !g.capturing) return nullptr;
     defer_flush();                                  // sums pending from the captured calls become the graph's last node
-    g_capturing = false;
+    g.capturing = false;
     cudaGraph_t graph = nullptr;
     if (!TL_CUDA(cudaStreamEndCapture(g.cur_stream, &graph)) || !graph) return nullptr;
     cudaGraphExec_t exec = nullptr;
     if (!TL_CUDA(cudaGraphInstantiate(&exec, graph, 0))) { cudaGraphDestroy(graph); return nullptr; }
     TlGraph *t = new TlGraph{exec, graph, g.launches - g_capture_launches0};
+    g.live_graphs++;
     g.launches = g_capture_launches0;        // nothing ran during the capture
     return t;
 }
@@ -443,6 +444,7 @@ void trainlib_graph_destroy(void *handle)
     if (!t) return;
     cudaGraphExecDestroy(t->exec); cudaGraphDestroy(t->graph);
     delete t;
+    if (g.live_graphs > 0 && --g.live_graphs == 0 && !g.capturing) defer_release();      // nothing holds addresses of outgrown arenas any more
 }
 void trainlib_profile(int on)
 {
