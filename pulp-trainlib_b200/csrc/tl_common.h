@@ -56,6 +56,27 @@ template <class... P, class... A> inline void launch_kernel(void (*kernel)(P...)
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream(); cfg.attrs = &attr; cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+// The same as clusters of `cluster` blocks.
+template <class... P, class... A> inline void launch_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, int cluster, A &&...args)
+{
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream(); cfg.attrs = attr; cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+#define TL_LAUNCH_CLUSTER(kernel, grid, block, smem, cluster, ...)                  \
+    do {                                                                            \
+        const bool tl_prof_ = ::tl::profiling();                                    \
+        if (tl_prof_) ::tl::profile_begin(#kernel);                                 \
+        ::tl::launch_clusters(kernel, dim3(grid), dim3(block), (size_t)(smem), cluster, __VA_ARGS__); \
+        if (tl_prof_) ::tl::profile_end();                                          \
+        ::tl::count_launch();                                                       \
+        ::tl::cuda_ok(cudaGetLastError(), #kernel);                                 \
+    } while (0)
 #define TL_LAUNCH(kernel, grid, block, smem, ...)                                   \
     do {                                                                            \
         const bool tl_prof_ = ::tl::profiling();                                    \

@@ -85,6 +85,13 @@ def test_products_of_small_groups(run, N, K, M, trans_B):
     assert_close(run.mm(A, B, N, K, M, trans_B=trans_B).astype(F), want, FP16_TOL if run.half else FP32_TOL, "mm")
 
 
+# the tcgen05 kernel: one CTA per tile, CTA pairs, split contractions; operands in place (multiples of 16 bytes) and packed
+@pytest.mark.parametrize("N,K,M", [(257, 512, 1030), (129, 200, 4100), (300, 2048, 912), (1000, 1001, 700), (2504, 1304, 2600), (2600, 1800, 5001), (2560, 1800, 5008)])
+@pytest.mark.parametrize("trans_B", [0, 1])
+def test_products_of_tiles(run, N, K, M, trans_B):
+    test_products_of_small_groups(run, N, K, M, trans_B)
+
+
 @pytest.mark.parametrize("rows,width", [(1, 1), (7, 33), (200, 128), (700, 250), (300, 512), (5, 1024), (9, 1500)])
 def test_layernorm_shapes(run, oracle, rows, width):
     rng = seeded(rows + width)
