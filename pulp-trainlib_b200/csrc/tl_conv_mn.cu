@@ -85,7 +85,7 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
 {
     pdl_wait();
     extern __shared__ unsigned char smem_dyn[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // a warp-uniform value to the compiler too
     const int NI = p.NI;
     const int first_issuer = 4 * p.NE, tma_warp = first_issuer + NI, first_conv = tma_warp + 1;
     const int nthreads = blockDim.x;
@@ -166,7 +166,7 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
     const uint32_t stages_u32 = smem_u32(stages);
     if (warp == tma_warp) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             uint32_t k = 0;                                     // chunk counter (tile, channel group)
             const uint32_t chunk_tx = (uint32_t)p.NSLOT * (uint32_t)MN_SLOT;
             bool ok = true;
@@ -174,9 +174,11 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
                 const int s0 = (t / p.tiles_per_image) * p.P, y0 = (t % p.tiles_per_image) * p.VR;
                 for (int g = 0; g < p.cigs; g++, k++) {
                     const int st = k % p.nstage;
-                    if (!wait_or_abort(&stage_empty[st], ((k / p.nstage) & 1) ^ 1, abort_flag, p.status, 11, 128u)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&raw_full[st], chunk_tx);
-                    tma_load_4d(stages + (size_t)st * 2 * half_bytes, &tmap, &raw_full[st], 0, s0, g * 8, y0 - p.padU);
+                    if (!warp_wait_or_abort(&stage_empty[st], ((k / p.nstage) & 1) ^ 1, abort_flag, p.status, 11, 128u, lane)) { ok = false; break; }
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&raw_full[st], chunk_tx);
+                        tma_load_4d(stages + (size_t)st * 2 * half_bytes, &tmap, &raw_full[st], 0, s0, g * 8, y0 - p.padU);
+                    }
                 }
             }
         }
@@ -217,7 +219,7 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
         }
     } else if (warp >= first_issuer) {
         // ------------------------------------------------------------ MMA issuers: issuer j owns m-block j of every tile
-        if (lane == 0) {
+        {
             const int j = warp - first_issuer;
             const uint32_t idesc_nb = mma_idesc(FMT_TF32, 128, (uint32_t)p.NB);
             // Descriptors as (low word, high word): only the start-address field (low word, units of 16 bytes) moves between
@@ -233,7 +235,7 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
             for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, tseq++) {
                 const int dbuf = (tseq % p.NBUF) * NI + j;
                 const uint32_t use = tseq / p.NBUF;
-                if (!wait_or_abort(&d_empty[dbuf], (use & 1) ^ 1, abort_flag, p.status, 12, nap_iss)) break;
+                if (!warp_wait_or_abort(&d_empty[dbuf], (use & 1) ^ 1, abort_flag, p.status, 12, nap_iss, lane)) break;
                 tc_fence_after();                               // the epilogue's tensor-memory loads of this accumulator come first
                 const uint32_t d_addr = tmem_base + (uint32_t)(dbuf * p.NB);
                 uint32_t acc = 0;
@@ -241,20 +243,22 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
                 for (int g = 0; g < p.cigs; g++, k++) {
                     const int st = k % p.nstage;
                     // (shared-memory operands: the converters' fence.proxy.async and the barrier order them, no tensor-core fence)
-                    if (!wait_or_abort(&a_full[st], (k / p.nstage) & 1, abort_flag, p.status, 13, nap_iss)) { ok = false; break; }
+                    if (!warp_wait_or_abort(&a_full[st], (k / p.nstage) & 1, abort_flag, p.status, 13, nap_iss, lane)) { ok = false; break; }
                     uint32_t aw = a_loword + a_base16 + (uint32_t)st * 2u * half16;
                     for (int a = 0; a < p.Hk; a++, aw += MN_SLOT / 16, bw += b_step16) {
                         const uint64_t a_hi = ((uint64_t)a_hiword << 32) | aw, a_lo = ((uint64_t)a_hiword << 32) | (aw + half16);
                         const uint64_t b_hi = ((uint64_t)b_hiword << 32) | bw, b_lo = ((uint64_t)b_hiword << 32) | (bw + b_lo16);
-                        mma_tf32_ss(d_addr, a_hi, b_hi, idesc_nb, acc);
-                        mma_tf32_ss(d_addr, a_hi, b_lo, idesc_nb, 1u);
-                        mma_tf32_ss(d_addr, a_lo, b_hi, idesc_nb, 1u);
+                        if (elect_one()) {
+                            mma_tf32_ss(d_addr, a_hi, b_hi, idesc_nb, acc);
+                            mma_tf32_ss(d_addr, a_hi, b_lo, idesc_nb, 1u);
+                            mma_tf32_ss(d_addr, a_lo, b_hi, idesc_nb, 1u);
+                        }
                         acc = 1u;
                     }
-                    mma_commit(&stage_empty[st]);
+                    if (elect_one()) mma_commit(&stage_empty[st]);
                 }
                 if (!ok) break;
-                mma_commit(&d_full[dbuf]);
+                if (elect_one()) mma_commit(&d_full[dbuf]);
             }
         }
     } else {

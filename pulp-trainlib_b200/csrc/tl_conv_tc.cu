@@ -76,23 +76,9 @@ static constexpr int MAX_ND = 4;            // accumulator buffers (2 when 4 wou
 // polls when every failed attempt slept 32 ns): the first attempt is bare, later ones sleep NAP_FAST / NAP_SLOW ns in
 // between, and the abort flag is only looked at every 16th attempt.
 static constexpr uint32_t NAP_FAST = 128u, NAP_SLOW = 512u;
-__device__ __forceinline__ bool tc_wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int id)
-{
-    // ids 3..5 sit on the critical path and sleep least; about a second of attempts bounds the wait
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint32_t nap = (id == 3 || id == 4 || id == 5) ? NAP_FAST : NAP_SLOW;
-    for (uint32_t i = 0; i < 4000000u; i++) {
-        __nanosleep(nap);
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 15u) == 15u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    atomicCAS(status, 0, id);
-    return false;
-}
-
-// Whole-warp variant for callers that go on to warp-collective tcgen05 instructions: every lane polls the same
-// barrier in the same instruction, so the warp stays converged and all lanes get the same answer.
+// Every lane polls the same barrier in the same instruction, so the warp stays converged (it goes on to warp-collective
+// tcgen05 instructions or elects the lane that issues them) and all lanes get the same answer.  Ids 3..5 sit on the critical
+// path and sleep least; about a second of attempts bounds the wait.
 __device__ __forceinline__ bool tc_warp_wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int id, int lane)
 {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
@@ -115,7 +101,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap, const ConvTcParams p)
 {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // a warp-uniform value to the compiler too
     const int NT = p.NT, N2 = 2 * NT;
     const int patch_floats = p.S_T * 16 * p.PH * p.PWB;
     const uint32_t patch_bytes = (uint32_t)patch_floats * 4u;
@@ -181,21 +167,24 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap, const ConvTcParams p)
 
     if (warp == TMA_WARP) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        {
             uint32_t pc = 0;
-            for (int t = blockIdx.x; t < p.n_tiles && !*abort_flag; t += gridDim.x) {
+            bool ok = true;
+            for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
                 const int tw0 = (t % p.tiles_w) * p.TW, th0 = ((t / p.tiles_w) % p.tiles_h) * p.TH, s0 = (t / tiles_per_stream_group) * p.S_T;
                 for (int g = 0; g < p.groups; g++, pc++) {
                     const int slot = pc % PS;
-                    if (!tc_wait_or_abort(&patch_empty[slot], ((pc / PS) & 1) ^ 1, abort_flag, p.status, 1)) break;
-                    mbar_arrive_expect_tx(&patch_full[slot], patch_bytes);
-                    tma_load_4d(patch + slot * patch_stride, &tmap, &patch_full[slot], p.x_base + tw0 * p.sw, p.y_base + th0 * p.sh, g * 16, s0);
+                    if (!tc_warp_wait_or_abort(&patch_empty[slot], ((pc / PS) & 1) ^ 1, abort_flag, p.status, 1, lane)) { ok = false; break; }
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&patch_full[slot], patch_bytes);
+                        tma_load_4d(patch + slot * patch_stride, &tmap, &patch_full[slot], p.x_base + tw0 * p.sw, p.y_base + th0 * p.sh, g * 16, s0);
+                    }
                 }
             }
         }
     } else if (warp >= FIRST_ISSUER && warp < FIRST_CONV) {
         // ------------------------------------------------------------ MMA issuers
-        if (lane == 0) {
+        {
             const int me = warp - FIRST_ISSUER;
             const uint32_t idesc_2n = mma_idesc(FMT_TF32, 128, N2), idesc_n = mma_idesc(FMT_TF32, 128, NT);
             const uint32_t bs_addr = smem_u32(Bs);
@@ -206,31 +195,33 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap tmap, const ConvTcParams p)
             int rb = 0; uint32_t rph = 0;       // ring position and phase of this group's next chunk
             uint32_t cbase = 0;                 // chunks dealt so far (all groups), mod GROUPS
             bool ok = true;
-            for (int t = blockIdx.x; t < p.n_tiles && ok && !*abort_flag; t += gridDim.x, tcnt++) {
+            for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, tcnt++) {
                 const int dbuf = tcnt & (p.nd - 1);
-                if (!tc_wait_or_abort(&d_empty[dbuf], (tcnt >> p.nd_log2) & 1, abort_flag, p.status, 2)) break;
+                if (!tc_warp_wait_or_abort(&d_empty[dbuf], (tcnt >> p.nd_log2) & 1, abort_flag, p.status, 2, lane)) break;
                 tc_fence_after();
                 const uint32_t d_addr = d_col0 + dbuf * N2;
                 for (int g = 0; g < p.groups && ok; g++, cbase = (cbase + p.taps) & (GROUPS - 1)) {
                     for (int tap = (me - cbase) & (GROUPS - 1); tap < p.taps; tap += GROUPS) {
                         const int abuf = me * p.ring + rb;
-                        if (!tc_wait_or_abort(&a_full[abuf], rph, abort_flag, p.status, 3)) { ok = false; break; }
+                        if (!tc_warp_wait_or_abort(&a_full[abuf], rph, abort_flag, p.status, 3, lane)) { ok = false; break; }
                         if (++rb == p.ring) { rb = 0; rph ^= 1u; }
                         tc_fence_after();
                         const uint32_t a_addr = a_col0 + abuf * 32;
                         // descriptor of this tap's weights: the start-address field (bits 0..13, units of 16 bytes) moves, the rest stays
                         const uint64_t b_tap = bdesc0 + (uint64_t)(((uint32_t)(g * p.taps + tap) * tap_bytes) >> 4);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 2; kk++) {
-                            const uint64_t bdesc = b_tap + (uint64_t)((kk * 2 * lbo) >> 4);
-                            mma_tf32_ts(d_addr, a_addr + kk * 8, bdesc, idesc_2n, 1u);
-                            mma_tf32_ts(d_addr, a_addr + 16 + kk * 8, bdesc, idesc_n, 1u);
+                            for (int kk = 0; kk < 2; kk++) {
+                                const uint64_t bdesc = b_tap + (uint64_t)((kk * 2 * lbo) >> 4);
+                                mma_tf32_ts(d_addr, a_addr + kk * 8, bdesc, idesc_2n, 1u);
+                                mma_tf32_ts(d_addr, a_addr + 16 + kk * 8, bdesc, idesc_n, 1u);
+                            }
+                            mma_commit(&a_empty[abuf]);
                         }
-                        mma_commit(&a_empty[abuf]);
                     }
                 }
                 if (!ok) break;
-                mma_commit(&d_full[dbuf]);       // one arrival per issuer: the tile is complete when all have landed
+                if (elect_one()) mma_commit(&d_full[dbuf]);       // one arrival per issuer: the tile is complete when all have landed
             }
         }
     } else if (warp >= FIRST_CONV) {

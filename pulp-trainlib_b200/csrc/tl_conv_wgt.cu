@@ -70,7 +70,7 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
 {
     pdl_wait();
     extern __shared__ unsigned char smem_dyn[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // a warp-uniform value to the compiler too
     const int NISS = p.MB * p.KS;
     constexpr int first_issuer = WGT_CONV_WARPS, tma_warp = WGT_CONV_WARPS + WGT_MAX_ISS;
 
@@ -103,16 +103,18 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
 
     if (warp == tma_warp) {
         // ------------------------------------------------------------ TMA producer: one copy of X rows, one of dY rows per tile
-        if (lane == 0) {
+        {
             uint32_t k = 0;
             for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, k++) {
                 const int rs = k % p.NR;
-                if (!wait_or_abort(&raw_empty[rs], ((k / p.NR) & 1) ^ 1, abort_flag, p.status, 21, 128u)) break;
+                if (!warp_wait_or_abort(&raw_empty[rs], ((k / p.NR) & 1) ^ 1, abort_flag, p.status, 21, 128u, lane)) break;
                 const int s0 = (t / p.tiles_per_image) * p.P, y0 = (t % p.tiles_per_image) * p.T;
                 unsigned char *rb = raws + (size_t)rs * p.raw_bytes;
-                mbar_arrive_expect_tx(&raw_full[rs], p.raw_bytes);
-                tma_load_4d(rb, &tmap_x, &raw_full[rs], 0, s0, 0, rowstep * y0 - 1);
-                tma_load_4d(rb + xraw_bytes, &tmap_dy, &raw_full[rs], 0, s0, 0, y0);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&raw_full[rs], p.raw_bytes);
+                    tma_load_4d(rb, &tmap_x, &raw_full[rs], 0, s0, 0, rowstep * y0 - 1);
+                    tma_load_4d(rb + xraw_bytes, &tmap_dy, &raw_full[rs], 0, s0, 0, y0);
+                }
             }
         }
     } else if (warp < WGT_CONV_WARPS) {
@@ -227,7 +229,7 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     } else if (warp >= first_issuer && warp < tma_warp) {
         // ------------------------------------------------------------ MMA issuers: issuer (m, qs) owns M-block m and the k-steps = qs (mod KS)
         const int j = warp - first_issuer;
-        if (lane == 0 && j < NISS) {
+        if (j < NISS) {
             const int m = j % p.MB, qs = j / p.MB;
             const uint32_t n_nb = (uint32_t)(p.ncopy * p.Cout), n_wide = p.stack ? 2u * n_nb : n_nb;
             const uint32_t idesc_wide = mma_idesc(FMT_TF32, 128, n_wide), idesc_nb = mma_idesc(FMT_TF32, 128, n_nb);
@@ -239,7 +241,7 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
             bool ok = true;
             for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, k++) {
                 const int cs = k % p.NC;
-                if (!wait_or_abort(&conv_full[cs], (k / p.NC) & 1, abort_flag, p.status, 23, 0u)) { ok = false; break; }
+                if (!warp_wait_or_abort(&conv_full[cs], (k / p.NC) & 1, abort_flag, p.status, 23, 0u, lane)) { ok = false; break; }
                 const uint32_t sb = conv_u32 + (uint32_t)cs * p.conv_bytes;
                 for (int r = 0; r < p.T; r++) {
                     const uint32_t a16 = (sb + (uint32_t)(r * rowstep) * x_row_bytes + (uint32_t)m * 16u * WGT_SLOT) >> 4;   // three consecutive rows of X = input rows y-1, y, y+1 (2y-1, 2y, 2y+1)
@@ -248,11 +250,12 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                         if ((int)(kstep % (uint32_t)p.KS) != qs) continue;
                         const uint64_t a_hi = ((uint64_t)hiword << 32) | (loword + a16 + 2u * kk), a_lo = ((uint64_t)hiword << 32) | (loword + a16 + (p.xh_bytes >> 4) + 2u * kk);
                         const uint64_t b_hi = ((uint64_t)hiword << 32) | (loword + b16 + 2u * kk);
-                        if (p.stack) {
+                        const uint64_t b_lo = ((uint64_t)hiword << 32) | (loword + b16 + (((uint32_t)p.ncopy * p.cogs * WGT_SLOT) >> 4) + 2u * kk);
+                        if (!elect_one()) {
+                        } else if (p.stack) {
                             mma_tf32_ss(d_addr, a_hi, b_hi, idesc_wide, acc);
                             mma_tf32_ss(d_addr, a_lo, b_hi, idesc_nb, 1u);
                         } else {
-                            const uint64_t b_lo = ((uint64_t)hiword << 32) | (loword + b16 + (((uint32_t)p.ncopy * p.cogs * WGT_SLOT) >> 4) + 2u * kk);
                             mma_tf32_ss(d_addr, a_hi, b_hi, idesc_nb, acc);
                             mma_tf32_ss(d_addr, a_hi, b_lo, idesc_nb, 1u);
                             mma_tf32_ss(d_addr, a_lo, b_hi, idesc_nb, 1u);
@@ -260,9 +263,9 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                         acc = 1u;
                     }
                 }
-                mma_commit(&conv_empty[cs]);
+                if (elect_one()) mma_commit(&conv_empty[cs]);
             }
-            if (ok) mma_commit(all_done);
+            if (ok && elect_one()) mma_commit(all_done);
         }
     }
     // ---------------------------------------------------------------- teardown
