@@ -106,11 +106,12 @@ public:
     bool may_defer() const { return !staged_ && !no_defer_; }
     void no_deferral() { no_defer_ = true; }
 private:
-    struct Entry { void *host; void *dev; size_t bytes; bool write_back; bool copied_in; };
+    struct Entry { void *host; void *dev; void *pinned; size_t bytes; bool write_back; bool copied_in; };
+    bool upload(Entry &e);
     void *map(void *p, size_t bytes, bool copy_in, bool copy_out);
     void *alloc(size_t bytes);
     std::vector<Entry> entries_;
-    size_t arena_mark_;
+    size_t arena_mark_, pinned_mark_;
     bool ok_;
     bool staged_;
     bool no_defer_ = false;

@@ -228,7 +228,56 @@ static void *arena_alloc(size_t bytes)
     return base;
 }
 
-Scope::Scope() : arena_mark_(0), ok_(true), staged_(false)
+// ---------------------------------------------------------------- staging of small host buffers
+// A copy of pageable memory costs the host 10 to 20 us whatever its size, and one by a copy engine costs the GPU two hand-overs
+// between engines.  Buffers of up to PINNED_MAX bytes go through a page-locked block instead: the host copies them there and a
+// kernel of the library's stream fetches them over the bus (the next one is being copied meanwhile); on the way back one
+// kernel delivers all results of the call.  The block is small enough to stay in the host's cache, past which the driver's own
+// staging is faster (measured, bytes in + two thirds of that out: 4 KB 24 -> 18 us, 192 KB 50 -> 41, 512 KB 81 -> 71,
+// 1 MB 129 -> 146).  Not while a graph is recorded: it would replay the block's content of that moment.
+static constexpr size_t PINNED_BLOCK = (size_t)1536 << 10, PINNED_MAX = (size_t)384 << 10;
+static char *g_pinned = nullptr;
+static size_t g_pinned_off = 0;
+
+static void *pinned_alloc(const void *host, size_t bytes)
+{
+    if (bytes > PINNED_MAX || g.capturing) return nullptr;
+    cudaPointerAttributes attr;             // "everything is host memory" is the caller's word: the driver's copies check it, memcpy would not
+    if (g.mem_mode == TL_MEM_HOST && (cudaPointerGetAttributes(&attr, host) != cudaSuccess || attr.type == cudaMemoryTypeDevice)) { cudaGetLastError(); return nullptr; }
+    if (!g_pinned && cudaMallocHost(&g_pinned, PINNED_BLOCK) != cudaSuccess) { cudaGetLastError(); g_pinned = nullptr; return nullptr; }
+    bytes = (bytes + 255) & ~(size_t)255;
+    if (g_pinned_off + bytes > PINNED_BLOCK) return nullptr;
+    void *p = g_pinned + g_pinned_off;
+    g_pinned_off += bytes;
+    return p;
+}
+
+// whole 16-byte pieces: both sides of a staged buffer are 256-byte aligned and padded
+struct StageJob { const uint4 *src; uint4 *dst; int count, first; };
+struct StageJobs { StageJob job[8]; int jobs; };
+__global__ void __launch_bounds__(256) stage_kernel(const __grid_constant__ StageJobs s)
+{
+    pdl_wait();
+    int j = 0;
+    while (j + 1 < s.jobs && (int)blockIdx.x >= s.job[j + 1].first) j++;
+    const int i = ((int)blockIdx.x - s.job[j].first) * 256 + threadIdx.x;
+    if (i < s.job[j].count) s.job[j].dst[i] = s.job[j].src[i];
+}
+static bool stage_run(StageJobs &s, int blocks)
+{
+    if (s.jobs == 0) return true;
+    launch_kernel(stage_kernel, dim3(blocks), dim3(256), 0, s);
+    s.jobs = 0;
+    return TL_CUDA(cudaGetLastError());
+}
+static void stage_add(StageJobs &s, int &blocks, const void *src, void *dst, size_t bytes)
+{
+    const int count = (int)((bytes + 15) / 16);
+    s.job[s.jobs++] = {(const uint4 *)src, (uint4 *)dst, count, blocks};
+    blocks += ceil_div(count, 256);
+}
+
+Scope::Scope() : arena_mark_(0), pinned_mark_(g_pinned_off), ok_(true), staged_(false)
 {
     ok_ = ready();
     arena_mark_ = arena_mark();
@@ -242,6 +291,18 @@ void *Scope::alloc(size_t bytes)
     return p;
 }
 
+bool Scope::upload(Entry &e)
+{
+    e.copied_in = true;
+    if (!e.pinned) return TL_CUDA(cudaMemcpyAsync(e.dev, e.host, e.bytes, cudaMemcpyHostToDevice, g.cur_stream));
+    memcpy(e.pinned, e.host, e.bytes);
+    StageJobs s;
+    int blocks = 0;
+    s.jobs = 0;
+    stage_add(s, blocks, e.pinned, e.dev, e.bytes);
+    return stage_run(s, blocks);
+}
+
 void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
 {
     if (p == nullptr || !ok_) return nullptr;
@@ -249,10 +310,7 @@ void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
     for (auto &e : entries_) {
         if (e.host == p && e.bytes >= bytes) {
             // same host range again: one mirror.  It was filled only if some earlier mapping asked for it.
-            if (copy_in && !e.copied_in) {
-                if (!TL_CUDA(cudaMemcpyAsync(e.dev, p, e.bytes, cudaMemcpyHostToDevice, g.cur_stream))) ok_ = false;
-                e.copied_in = true;
-            }
+            if (copy_in && !e.copied_in && !upload(e)) ok_ = false;
             e.write_back |= copy_out;
             return e.dev;
         }
@@ -268,22 +326,30 @@ void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
     void *d = arena_alloc(bytes);
     if (!d) { ok_ = false; return nullptr; }
     staged_ = true;
-    if (copy_in) {
-        if (!TL_CUDA(cudaMemcpyAsync(d, p, bytes, cudaMemcpyHostToDevice, g.cur_stream))) ok_ = false;
-    }
-    entries_.push_back({p, d, bytes, copy_out, copy_in});
+    entries_.push_back({p, d, pinned_alloc(p, bytes), bytes, copy_out, false});
+    if (copy_in && !upload(entries_.back())) ok_ = false;
     return d;
 }
 
 Scope::~Scope()
 {
     if (staged_) {
-        for (auto &e : entries_)
-            if (e.write_back) TL_CUDA(cudaMemcpyAsync(e.host, e.dev, e.bytes, cudaMemcpyDeviceToHost, g.cur_stream));
-        TL_CUDA(cudaStreamSynchronize(g.cur_stream));
+        StageJobs s;
+        int blocks = 0;
+        s.jobs = 0;
+        for (auto &e : entries_) {
+            if (!e.write_back) continue;
+            if (!e.pinned) { TL_CUDA(cudaMemcpyAsync(e.host, e.dev, e.bytes, cudaMemcpyDeviceToHost, g.cur_stream)); continue; }
+            if (s.jobs == 8) { stage_run(s, blocks); blocks = 0; }
+            stage_add(s, blocks, e.dev, e.pinned, e.bytes);
+        }
+        stage_run(s, blocks);
+        if (TL_CUDA(cudaStreamSynchronize(g.cur_stream)))
+            for (auto &e : entries_) if (e.write_back && e.pinned) memcpy(e.host, e.pinned, e.bytes);
     }
     g.scope_depth--;
     arena_release(arena_mark_);
+    g_pinned_off = pinned_mark_;
 }
 
 } // namespace tl

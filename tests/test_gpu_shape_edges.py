@@ -92,6 +92,17 @@ def test_products_of_tiles(run, N, K, M, trans_B):
     test_products_of_small_groups(run, N, K, M, trans_B)
 
 
+# host arrays: odd byte counts, at and past the size that goes through the page-locked block, and more than the block holds
+@pytest.mark.parametrize("N,K,M", [(1, 3, 5), (96, 1024, 7), (97, 1024, 3), (300, 320, 330), (330, 297, 1)])
+def test_products_of_host_arrays(pkg, gpulib, N, K, M):
+    r = AbiRunner(pkg, gpulib, device=False)
+    rng = seeded(N + K + M)
+    A, B = (rng.standard_normal(s).astype(F) for s in ((N, K), (K, M)))
+    want = (A.astype(np.float64) @ B.astype(np.float64)).astype(F)
+    assert_close(r.mm(A, B, N, K, M), want, FP32_TOL, "mm")
+    r.close()
+
+
 @pytest.mark.parametrize("rows,width", [(1, 1), (7, 33), (200, 128), (700, 250), (300, 512), (5, 1024), (9, 1500)])
 def test_layernorm_shapes(run, oracle, rows, width):
     rng = seeded(rows + width)
