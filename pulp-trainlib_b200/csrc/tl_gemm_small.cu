@@ -396,6 +396,7 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
     GgParams<T> g;
     g.count = count;
     long long tiles_all = 0, tile_steps = 0;
+    int shortest = 1 << 30;
     for (int i = 0; i < count; i++) {
         const GemmGroup<T> &s = list[i];
         GgProb<T> &p = g.p[i];
@@ -416,6 +417,7 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
         p.chunks = p.segs * ceil_div(p.K, KC);
         p.splits = 1; p.part = nullptr; p.ticket0 = 0;
         tiles_all += (long long)p.tiles_nm * s.batch;
+        shortest = std::min(shortest, p.chunks);
         tile_steps += (long long)p.tiles_nm * s.batch * p.chunks;
     }
     // Split K over CTAs while the group leaves SMs idle: enough CTAs for two per SM, never less than 256 of K each (a
@@ -427,8 +429,11 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
     for (int i = 0; i < count; i++) {
         GgProb<T> &p = g.p[i];
         const long long tiles = (long long)p.tiles_nm * list[i].batch;
-        if (tiles_all < sm_count() && p.chunks >= 2 * MIN_CH) {
-            long long s = (want * p.chunks + tile_steps - 1) / tile_steps;     // this product's share of the wanted CTAs, per tile
+        // this product's share of the wanted CTAs, per tile; in a group that fills the SMs, a contraction much longer than the
+        // shortest one (three segments beside products of one) is cut to about that length
+        long long s = tiles_all < sm_count() ? (want * p.chunks + tile_steps - 1) / tile_steps
+                                             : (tiles_all < 4 * sm_count() && p.chunks >= 2 * shortest ? p.chunks / std::max(shortest, MIN_CH) : 1);
+        if (s > 1 && p.chunks >= 2 * MIN_CH) {
             s = std::min<long long>(std::min<long long>(s, p.chunks / MIN_CH), 64);
             if (s > 1 && ticket + tiles <= 16384) {
                 const int per = ceil_div(p.chunks, (int)s);
