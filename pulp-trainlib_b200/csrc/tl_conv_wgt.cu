@@ -35,6 +35,7 @@
 // naive kernel [ref: lib/sources/pulp_conv_naive_fp32.c:302-408].
 #include "tl_kernels.h"
 #include "tl_tc.cuh"
+#include <algorithm>
 
 namespace tl {
 
@@ -274,6 +275,217 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     if (warp == tma_warp) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, 512u); }
 }
 
+// ------------------------------------------------------------------ 8 or 16 channels on either side, stride 1
+// With M = (filter row, ci) a layer of 16 channels fills 48 of the 128 rows of an MMA, and what an MMA costs here is the
+// shared-memory traffic of its operands: 4 KB of A per 8 pixels whatever its useful rows.  So both halves of the split go
+// into ONE instruction: M = (part of dY, filter column b, co), up to 96 rows, N = (filter row a, part of X, ci), up to 96
+// columns; the four part products lie in blocks of their own and are added at the end (the one of the two low parts comes
+// for nothing).  28 KB of operand reads per dY row instead of 50.  Two more differences from the kernel above: one elected
+// thread issues everything, and the accumulators are drained into registers every WGY_ROWS rows (two banks of two, so that
+// the products go on meanwhile): the tensor core's accumulation truncates, and a CTA's whole run of a large batch would lose
+// digit or two (relative error of 4096 streams 4e-7; 1.2e-6 with drains every 32 rows).  Measured, 16 -> 16 on 32 x 32: 4096
+// streams 250 us against 431 us of the FFMA kernel and 441 us of the kernel above; 200 streams 18.5 against 32.6 us, 16 streams
+// 7.1 against 12.0 us.
+//
+// status ids of this kernel's waits: 41 raw stage free (TMA), 42 raw landed, 43 operand stage free (converters), 44 operands
+// ready, 45 bank free (issuer), 46 bank complete (epilogue)
+struct WgyParams {
+    int n, W, P, T, NR, NC, tiles_per_image, n_tiles, flush;        // flush: tiles between two drains
+    uint32_t raw_bytes, conv_bytes;
+    float *part;                                                    // [gridDim.x][Cout][Cin][3][3]
+    int *status;
+};
+static constexpr int WGY_CONV_WARPS = 8, WGY_ROWS = 8;
+static constexpr int WGY_THREADS = 32 * (4 + WGY_CONV_WARPS + 2);  // warps 0-3: epilogue, then the converters, the issuer, the TMA producer
+
+template <int CIG, int COG>
+__global__ void __launch_bounds__(WGY_THREADS, 1)
+conv_wgy_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_dy, const WgyParams p)
+{
+    pdl_wait();
+    constexpr int N = 48 * CIG, CIN = 8 * CIG, COUT = 8 * COG;
+    constexpr int issuer_warp = 4 + WGY_CONV_WARPS, tma_warp = issuer_warp + 1;
+    constexpr uint32_t dy_row = 6u * COG * WGT_SLOT, x_row = 2u * CIG * WGT_SLOT;       // operand bytes of a dY row [part][b][co group] and an X row [part][ci group]
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ uint64_t raw_full[WGT_MAX_NR], raw_empty[WGT_MAX_NR], conv_full[WGT_MAX_NC], conv_empty[WGT_MAX_NC], bank_full[2], bank_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_s;
+    volatile int *abort_flag = &abort_s;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t base_u32 = smem_u32(smem_dyn);
+    const uint32_t pad = ((base_u32 + 1023u) & ~1023u) - base_u32;
+    unsigned char *conv = smem_dyn + pad;                                   // NC x [dY rows | X rows]; the M rows past the last dY row overrun into the X rows
+    unsigned char *raws = conv + (size_t)p.NC * p.conv_bytes;               // NR x [X rows | dY rows]
+    const uint32_t x_at = (uint32_t)p.T * dy_row, xraw_bytes = (uint32_t)(p.T + 2) * CIG * WGT_SLOT;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < p.NR; i++) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], WGY_CONV_WARPS); }
+        for (int i = 0; i < p.NC; i++) { mbar_init(&conv_full[i], WGY_CONV_WARPS); mbar_init(&conv_empty[i], 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(&bank_full[i], 1); mbar_init(&bank_empty[i], 4); }
+        abort_s = 0;
+        fence_barrier_init();
+        tma_prefetch_desc(&tmap_x); tma_prefetch_desc(&tmap_dy);
+    }
+    if (warp == tma_warp) { tmem_alloc(&tmem_slot, 512u); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_slot;
+
+    if (warp == tma_warp) {
+        uint32_t k = 0;
+        for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, k++) {
+            const int rs = k % p.NR;
+            if (!warp_wait_or_abort(&raw_empty[rs], ((k / p.NR) & 1) ^ 1, abort_flag, p.status, 41, 128u, lane)) break;
+            if (elect_one()) {
+                const int s0 = (t / p.tiles_per_image) * p.P, y0 = (t % p.tiles_per_image) * p.T;
+                unsigned char *rb = raws + (size_t)rs * p.raw_bytes;
+                mbar_arrive_expect_tx(&raw_full[rs], p.raw_bytes);
+                tma_load_4d(rb, &tmap_x, &raw_full[rs], 0, s0, 0, y0 - 1);
+                tma_load_4d(rb + xraw_bytes, &tmap_dy, &raw_full[rs], 0, s0, 0, y0);
+            }
+            __syncwarp();
+        }
+    } else if (warp == issuer_warp) {
+        constexpr uint32_t idesc = mma_idesc(FMT_TF32, 128, N);
+        const uint64_t tmpl = smem_desc_kmajor_sw128(0u, WGT_SLOT);
+        const uint32_t conv_u32 = smem_u32(conv);
+        uint32_t k = 0, bank = 0, in_bank = 0, drained = 0, fresh = 0;      // fresh: sets of the bank that were written
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, k++) {
+            if (in_bank == 0) {
+                if (!warp_wait_or_abort(&bank_empty[bank], ((drained >> 1) & 1) ^ 1, abort_flag, p.status, 45, 20u, lane)) { ok = false; break; }
+                fresh = 0;
+            }
+            const int cs = k % p.NC;
+            if (!warp_wait_or_abort(&conv_full[cs], (k / p.NC) & 1, abort_flag, p.status, 44, 0u, lane)) { ok = false; break; }
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t sb = conv_u32 + (uint32_t)cs * p.conv_bytes;
+                uint32_t done = fresh;
+                for (int r = 0; r < p.T; r++) {
+                    const uint64_t da = tmpl + ((sb + (uint32_t)r * dy_row) >> 4), db = tmpl + ((sb + x_at + (uint32_t)r * x_row) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++) {
+                        mma_tf32_ss(tmem_base + bank * 256u + (kk & 1) * 128u, da + 2u * kk, db + 2u * kk, idesc, done);
+                        if (kk & 1) done = 1u;
+                    }
+                }
+                mma_commit(&conv_empty[cs]);
+            }
+            __syncwarp();
+            fresh = 1u;
+            if (++in_bank == (uint32_t)p.flush || t + (int)gridDim.x >= p.n_tiles) {
+                if (elect_one()) mma_commit(&bank_full[bank]);
+                __syncwarp();
+                in_bank = 0; bank ^= 1u; drained++;
+            }
+        }
+    } else if (warp >= 4) {
+        // converters, as in conv_wgt_kernel: 16-byte chunk q of slot row R goes to chunk q ^ R
+        const int cw = warp - 4;
+        const int R0 = lane >> 3, q = lane & 7;
+        const int d0 = R0 * 8 + (q ^ R0), d1 = (R0 + 4) * 8 + (q ^ (R0 + 4));
+        const int cpw = p.W / 4;
+        const bool left_edge = (q % cpw) == 0, right_edge = (q % cpw) == cpw - 1;
+        uint32_t k = 0;
+        for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, k++) {
+            const int rs = k % p.NR, cs = k % p.NC;
+            if (!warp_wait_or_abort(&raw_full[rs], (k / p.NR) & 1, abort_flag, p.status, 42, 32u, lane)) break;
+            if (!warp_wait_or_abort(&conv_empty[cs], ((k / p.NC) & 1) ^ 1, abort_flag, p.status, 43, 32u, lane)) break;
+            const unsigned char *rb = raws + (size_t)rs * p.raw_bytes;
+            unsigned char *cb = conv + (size_t)cs * p.conv_bytes;
+            const int ndy = p.T * COG, nx = (p.T + 2) * CIG;
+            for (int sl = cw; sl < ndy + nx; sl += WGY_CONV_WARPS) {
+                if (sl >= ndy) {
+                    const int xs = sl - ndy, row = xs / CIG, cig = xs % CIG;
+                    const float4 *r4 = reinterpret_cast<const float4 *>(rb + (size_t)xs * WGT_SLOT);
+                    float4 *h = reinterpret_cast<float4 *>(cb + x_at + (size_t)row * x_row + (size_t)cig * WGT_SLOT), *l = h + CIG * (WGT_SLOT / 16);
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {
+                        const float4 v = r4[lane + 32 * half];
+                        uint32_t a0, a1, a2, a3, b0, b1, b2, b3;
+                        split_tf32_fast(v.x, a0, b0); split_tf32_fast(v.y, a1, b1); split_tf32_fast(v.z, a2, b2); split_tf32_fast(v.w, a3, b3);
+                        h[half ? d1 : d0] = make_float4(__uint_as_float(a0), __uint_as_float(a1), __uint_as_float(a2), __uint_as_float(a3));
+                        l[half ? d1 : d0] = make_float4(__uint_as_float(b0), __uint_as_float(b1), __uint_as_float(b2), __uint_as_float(b3));
+                    }
+                } else {
+                    const int row = sl / COG, cog = sl % COG;
+                    const float4 *raw = reinterpret_cast<const float4 *>(rb + xraw_bytes + (size_t)sl * WGT_SLOT);
+                    float4 *hh = reinterpret_cast<float4 *>(cb + (size_t)row * dy_row + (size_t)cog * WGT_SLOT);
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {
+                        const float4 v = raw[lane + 32 * half];
+                        // the values are split once; the three copies shift the parts
+                        uint32_t h0, h1, h2, h3, l0, l1, l2, l3;
+                        split_tf32_fast(v.x, h0, l0); split_tf32_fast(v.y, h1, l1); split_tf32_fast(v.z, h2, l2); split_tf32_fast(v.w, h3, l3);
+                        const int dst = half ? d1 : d0;
+                        auto copies = [&](float4 *o, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+                            uint32_t lft = __shfl_up_sync(0xffffffffu, w, 1), rgt = __shfl_down_sync(0xffffffffu, x, 1);
+                            if (left_edge) lft = 0u;
+                            if (right_edge) rgt = 0u;
+                            o[dst] = make_float4(__uint_as_float(y), __uint_as_float(z), __uint_as_float(w), __uint_as_float(rgt));                                            // b = 0: dY[x + 1]
+                            o[COG * (WGT_SLOT / 16) + dst] = make_float4(__uint_as_float(x), __uint_as_float(y), __uint_as_float(z), __uint_as_float(w));
+                            o[2 * COG * (WGT_SLOT / 16) + dst] = make_float4(__uint_as_float(lft), __uint_as_float(x), __uint_as_float(y), __uint_as_float(z));                // b = 2: dY[x - 1]
+                        };
+                        copies(hh, h0, h1, h2, h3);
+                        copies(hh + 3 * COG * (WGT_SLOT / 16), l0, l1, l2, l3);
+                    }
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&conv_full[cs]); mbar_arrive(&raw_empty[rs]); }
+        }
+    } else {
+        // epilogue: thread = accumulator row; drains the banks into registers, then adds the parts and writes this CTA's dW
+        const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+        float acc[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) acc[i] = 0.f;
+        const int mine = (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, drains = (mine + p.flush - 1) / p.flush;
+        bool ok = true;
+        for (int f = 0; f < drains; f++) {
+            if (!warp_wait_or_abort(&bank_full[f & 1], (f >> 1) & 1, abort_flag, p.status, 46, 256u, lane)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int set = 0; set < 2; set++)
+#pragma unroll
+                for (int c0 = 0; c0 < N; c0 += 16) {
+                    uint32_t v[16];
+                    tmem_ld16w(tmem_base + lane_addr + (uint32_t)((f & 1) * 256 + set * 128 + c0), v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; i++) acc[c0 + i] += __uint_as_float(v[i]);
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bank_empty[f & 1]);
+        }
+        // (every product of this CTA has completed: the operand stages are free)
+        float *sm = reinterpret_cast<float *>(conv);
+        constexpr int PITCH = 3 * CIN + 1;
+        const int m = warp * 32 + lane;
+        if (ok && m < 6 * COUT) {
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int c = 0; c < CIN; c++) sm[m * PITCH + a * CIN + c] = acc[a * 2 * CIN + c] + acc[(a * 2 + 1) * CIN + c];
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (ok) {
+            float *out = p.part + (long long)blockIdx.x * (COUT * CIN * 9);
+            for (int e = threadIdx.x; e < COUT * CIN * 9; e += 128) {
+                const int b = e % 3, a = (e / 3) % 3, ci = (e / 9) % CIN, co = e / (9 * CIN), r = b * COUT + co, c = a * CIN + ci;
+                out[e] = sm[r * PITCH + c] + sm[(3 * COUT + r) * PITCH + c];
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == tma_warp) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, 512u); }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -390,6 +602,53 @@ bool conv_wgt_run(const float *x, const float *dy, float *part, int part_groups,
     TL_LAUNCH(conv_wgt_kernel, ctas, WGT_THREADS, smem, tx, tdy, p);
     profile_add_flops(2.0 * n * Cout * Cin * 9.0 * H * W);          // H x W = the dY plane for either stride
     *groups_out = ctas;
+    return true;
+}
+
+// conv_wgy_kernel: partial results of Cout * Cin * 9 floats each in dW's own order; otherwise the contract of conv_wgt_run.
+bool conv_wgy_run(const float *x, const float *dy, float *part, int part_groups, int *groups_out, int n, int Cin, int Cout, int H, int W, bool dry_run)
+{
+    EncodeTiledFn enc = (EncodeTiledFn)tc_encode_tiled_fn();
+    if (!enc) return false;
+    if (W != 32 && W != 16 && W != 8) return false;
+    if ((Cin != 8 && Cin != 16) || (Cout != 8 && Cout != 16) || n < 1) return false;
+    if ((((uintptr_t)x | (uintptr_t)dy) & 15) != 0) return false;
+    const int cigs = Cin / 8, cogs = Cout / 8;
+    WgyParams p;
+    p.n = n; p.W = W; p.P = 32 / W;
+    p.T = H % 4 == 0 ? 4 : H % 2 == 0 ? 2 : 1;
+    p.raw_bytes = (uint32_t)((p.T + 2) * cigs + p.T * cogs) * WGT_SLOT;
+    p.conv_bytes = (uint32_t)(p.T * 6 * cogs + (p.T + 2) * 2 * cigs) * WGT_SLOT;
+    p.NC = 2;
+    p.NR = std::min<int>(WGT_MAX_NR, (int)((224u * 1024 - p.NC * p.conv_bytes) / p.raw_bytes));
+    p.tiles_per_image = H / p.T;
+    p.n_tiles = ceil_div(n, p.P) * p.tiles_per_image;
+    p.flush = WGY_ROWS / p.T;
+    const int ctas = std::min(sm_count(), p.n_tiles);
+    if (ctas > part_groups) return false;
+    *groups_out = ctas;
+    if (dry_run) return true;
+    CUtensorMap tx, tdy;
+    auto map = [&](CUtensorMap *m, const float *base, int C, int rows) {
+        cuuint64_t gstr[3] = {(cuuint64_t)W * H * C * 4, (cuuint64_t)W * H * 4, (cuuint64_t)W * 4};
+        cuuint64_t gdim[4] = {(cuuint64_t)W, (cuuint64_t)n, (cuuint64_t)C, (cuuint64_t)H};
+        cuuint32_t box[4] = {(cuuint32_t)W, (cuuint32_t)p.P, (cuuint32_t)C, (cuuint32_t)rows};
+        cuuint32_t estr[4] = {1, 1, 1, 1};
+        return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)base, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!map(&tx, x, Cin, p.T + 2) || !map(&tdy, dy, Cout, p.T)) return false;
+    p.part = part;
+    p.status = tc_status_word();
+    if (!p.status) return false;
+    const size_t smem = 1024 + (size_t)p.NC * p.conv_bytes + (size_t)p.NR * p.raw_bytes;
+    auto launch = [&](auto kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        TL_LAUNCH(kern, ctas, WGY_THREADS, smem, tx, tdy, p);
+    };
+    if (cigs == 2) { if (cogs == 2) launch(conv_wgy_kernel<2, 2>); else launch(conv_wgy_kernel<2, 1>); }
+    else { if (cogs == 2) launch(conv_wgy_kernel<1, 2>); else launch(conv_wgy_kernel<1, 1>); }
+    profile_add_flops(2.0 * n * Cout * Cin * 9.0 * H * W);
     return true;
 }
 

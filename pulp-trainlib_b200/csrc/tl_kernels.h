@@ -149,6 +149,7 @@ template <class T> bool conv_mma_wg(const ConvGeom &g, const T *x, const T *dy, 
 template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T *dst, bool ig);
 template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy, float *part, int &groups, bool dry_run);
 // tensor-core weight gradient (tl_conv_wgt.cu): partial results per CTA into `part`; false = geometry not covered
+bool conv_wgy_run(const float *x, const float *dy, float *part, int part_groups, int *groups_out, int n, int Cin, int Cout, int H, int W, bool dry_run);
 bool conv_wgt_run(const float *x, const float *dy, float *part, int part_groups, int *groups_out, long long *group_floats_out, int n, int Cin, int Cout, int H,
                   int W, int stride, bool dry_run);
 void conv_wgt_reduce(const float *part, float *dw, int groups, int Cin, int Cout, int stride, bool deferred);   // deferred: noted for the batched launch
