@@ -284,8 +284,9 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
 // thread issues everything, and the accumulators are drained into registers every WGY_ROWS rows (two banks of two, so that
 // the products go on meanwhile): the tensor core's accumulation truncates, and a CTA's whole run of a large batch would lose
 // digit or two (relative error of 4096 streams 4e-7; 1.2e-6 with drains every 32 rows).  Measured, 16 -> 16 on 32 x 32: 4096
-// streams 250 us against 431 us of the FFMA kernel and 441 us of the kernel above; 200 streams 18.5 against 32.6 us, 16 streams
-// 7.1 against 12.0 us.
+// streams 223 us (250 with eight converter warps) against 431 us of the FFMA kernel and 441 us of the kernel above; 200 streams
+// 17.4 against 32.6 us, 16 streams
+// 6.8 against 12.0 us. A second issuer with accumulators of its own changed nothing (238 us).
 //
 // status ids of this kernel's waits: 41 raw stage free (TMA), 42 raw landed, 43 operand stage free (converters), 44 operands
 // ready, 45 bank free (issuer), 46 bank complete (epilogue)
@@ -295,7 +296,7 @@ struct WgyParams {
     float *part;                                                    // [gridDim.x][Cout][Cin][3][3]
     int *status;
 };
-static constexpr int WGY_CONV_WARPS = 8, WGY_ROWS = 8;
+static constexpr int WGY_CONV_WARPS = 12, WGY_ROWS = 8;
 static constexpr int WGY_THREADS = 32 * (4 + WGY_CONV_WARPS + 2);  // warps 0-3: epilogue, then the converters, the issuer, the TMA producer
 
 template <int CIG, int COG>
@@ -440,9 +441,9 @@ conv_wgy_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     } else {
         // epilogue: thread = accumulator row; drains the banks into registers, then adds the parts and writes this CTA's dW
         const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
-        float acc[N];
+        float acc[N / 2];                                                   // [filter row][ci], the parts of X added
 #pragma unroll
-        for (int i = 0; i < N; i++) acc[i] = 0.f;
+        for (int i = 0; i < N / 2; i++) acc[i] = 0.f;
         const int mine = (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, drains = (mine + p.flush - 1) / p.flush;
         bool ok = true;
         for (int f = 0; f < drains; f++) {
@@ -456,7 +457,7 @@ conv_wgy_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     tmem_ld16w(tmem_base + lane_addr + (uint32_t)((f & 1) * 256 + set * 128 + c0), v);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; i++) acc[c0 + i] += __uint_as_float(v[i]);
+                    for (int i = 0; i < 16; i++) acc[(c0 + i) / (2 * CIN) * CIN + (c0 + i) % CIN] += __uint_as_float(v[i]);
                 }
             tc_fence_before();
             __syncwarp();
@@ -468,9 +469,7 @@ conv_wgy_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         const int m = warp * 32 + lane;
         if (ok && m < 6 * COUT) {
 #pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int c = 0; c < CIN; c++) sm[m * PITCH + a * CIN + c] = acc[a * 2 * CIN + c] + acc[(a * 2 + 1) * CIN + c];
+            for (int c = 0; c < N / 2; c++) sm[m * PITCH + c] = acc[c];
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (ok) {
