@@ -285,8 +285,7 @@ conv_wgt_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
 // the products go on meanwhile): the tensor core's accumulation truncates, and a CTA's whole run of a large batch would lose
 // digit or two (relative error of 4096 streams 4e-7; 1.2e-6 with drains every 32 rows).  Measured, 16 -> 16 on 32 x 32: 4096
 // streams 223 us (250 with eight converter warps) against 431 us of the FFMA kernel and 441 us of the kernel above; 200 streams
-// 17.4 against 32.6 us, 16 streams
-// 6.8 against 12.0 us. A second issuer with accumulators of its own changed nothing (238 us).
+// 17.4 against 32.6 us, 16 streams 6.8 against 12.0 us.  A second issuer with accumulators of its own changed nothing (238 us).
 //
 // status ids of this kernel's waits: 41 raw stage free (TMA), 42 raw landed, 43 operand stage free (converters), 44 operands
 // ready, 45 bank free (issuer), 46 bank complete (epilogue)

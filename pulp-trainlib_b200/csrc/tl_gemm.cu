@@ -119,7 +119,6 @@ gemm_ffma_kernel(GemmDesc<T> d)
 
 // Tensor-core path (tl_gemm_tc.cu); returns false when the shape/layout does not qualify.
 template <class T> bool gemm_tensor_core(const GemmDesc<T> &d);
-template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d);
 
 // Products that the tensor-core kernels decline go to the group kernel (tl_gemm_small.cu) as a group of one.
 template <class T> void gemm(const GemmDesc<T> &d)

@@ -14,8 +14,8 @@
 //   fp32: 3xTF32 on packed (hi, lo) pairs.  B_hi and B_lo lie behind each other: D0 += A_hi [B_hi | B_lo]^T is one instruction of
 //         N = 2 BN (A_hi is read once), D1 += A_lo B_hi^T a second one; the epilogue adds the three parts, whose accumulation
 //         chains are a third as long as one common chain (the accumulator truncates).
-// Measured, whole call: fp16 4096^3 173 -> 101 us, fp16 2048^3 29 -> 18 us, fp32 2048^3 118 -> 99 us, fp32 1000 x 600 x 1300
-// (B transposed) 31 -> 21.5 us, fp32 300 x 2050 x 914 67 -> 27 us.
+// Measured, whole call: fp16 4096^3 173 -> 101 us, fp16 2048^3 29 -> 17.5 us, fp32 2048^3 118 -> 89 us, fp32 1000 x 600 x 1300
+// (B transposed) 31 -> 20.3 us, fp32 300 x 2050 x 914 67 -> 26 us.
 // Few tiles: `splits` CTAs share the K steps of a tile and write partial tiles; tm_reduce_kernel adds them in order.
 // No multicast loads.  Every wait is bounded and reports through the status word.
 #include "tl_kernels.h"
@@ -47,7 +47,7 @@ struct TmParams {
     int N, M, K;
     long long c_rs, c_cs, c_bs;
     float alpha; int accumulate, bias_mode;
-    int BN, tiles_m, tiles_n, tiles, ksteps, splits, stages, pair, a_mn, b_mn;
+    int BN, tiles_m, tiles_n, tiles, ksteps, splits, stages, pair, a_mn, b_mn, b_one;      // b_one: all products of a batch share B
     uint32_t stage_bytes;
     int *status;
 };
@@ -194,23 +194,23 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
         for (int tile = first; tile < p.tiles && ok; tile += step) {
             int b, rb, cb;
             tm_locate(p, tile, b, rb, cb);
-            const int row0 = rb * ROWS + row_of_tile, col0 = cb * BN + (PAIR ? rank * BNL : 0);
+            const int row0 = rb * ROWS + row_of_tile, col0 = cb * BN + (PAIR ? rank * BNL : 0), zb = p.b_one ? 0 : b;
             for (int kt = ks0; kt < ks1; kt++) {
                 if (!tm_wait(&empty[s], phase, failed)) { ok = false; break; }
                 if (elect_one()) {
                     const uint32_t st = sbase + s * p.stage_bytes, sb = st + Cfg::PARTS * A_BYTES;
                     const uint32_t bar = full0 + 8u * s;
-                    auto load = [&](uint32_t dst, const CUtensorMap *m, int x, int y) {
-                        if constexpr (PAIR) tma_load_3d_pair(dst, m, bar, x, y, b);
-                        else tma_load_3d(dst, m, &full[s], x, y, b);
+                    auto load = [&](uint32_t dst, const CUtensorMap *m, int x, int y, int z) {
+                        if constexpr (PAIR) tma_load_3d_pair(dst, m, bar, x, y, z);
+                        else tma_load_3d(dst, m, &full[s], x, y, z);
                     };
                     if (!PAIR || rank == 0) mbar_arrive_expect_tx(&full[s], PAIR ? 2 * p.stage_bytes : p.stage_bytes);
-                    if (HALF && p.a_mn) { for (int j = 0; j < 2; j++) load(st + j * 8192u, &a0, row0 + 64 * j, kt * BK); }
-                    else load(st, &a0, kt * BK, row0);
-                    if (!HALF) load(st + A_BYTES, &a1, kt * BK, row0);
-                    if (HALF && p.b_mn) { for (int j = 0; j < BNL / 64; j++) load(sb + j * 8192u, &b0, col0 + 64 * j, kt * BK); }
-                    else load(sb, &b0, kt * BK, col0);
-                    if (!HALF) load(sb + B_BYTES, &b1, kt * BK, col0);
+                    if (HALF && p.a_mn) { for (int j = 0; j < 2; j++) load(st + j * 8192u, &a0, row0 + 64 * j, kt * BK, b); }
+                    else load(st, &a0, kt * BK, row0, b);
+                    if (!HALF) load(st + A_BYTES, &a1, kt * BK, row0, b);
+                    if (HALF && p.b_mn) { for (int j = 0; j < BNL / 64; j++) load(sb + j * 8192u, &b0, col0 + 64 * j, kt * BK, zb); }
+                    else load(sb, &b0, kt * BK, col0, zb);
+                    if (!HALF) load(sb + B_BYTES, &b1, kt * BK, col0, zb);
                 }
                 __syncwarp();
                 if (++s == ST) { s = 0; phase ^= 1u; }
@@ -295,19 +295,38 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
                     for (int j = 0; j < 32; j += 4)
                         *reinterpret_cast<float4 *>(mine + c0 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
                 } else if (row < p.N) {
-                    const bool v8 = HALF && vec && p.bias_mode != 2 && col0 + c0 + 32 <= p.M;
-                    if (v8) {
-                        const float brow = p.bias_mode == 1 ? ld(reinterpret_cast<const T *>(p.bias) + row) : 0.f;
-                        uint4 *dst = reinterpret_cast<uint4 *>(crow + col0 + c0);
+                    // whole groups of 32 columns: straight-line stores, 16 bytes along the row, or element by element where the rows are
+                    // the contiguous index (neighbouring lanes then write neighbouring elements)
+                    const bool whole = !p.accumulate && col0 + c0 + 32 <= p.M;
+                    if (whole && (vec || p.c_rs == 1)) {
+                        const T *bias = reinterpret_cast<const T *>(p.bias);
+                        const float brow = p.bias_mode == 1 ? ld(bias + row) : 0.f;
 #pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            uint32_t w[4];
+                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(p.alpha * __uint_as_float(v[j]) + brow);
+                        if (p.bias_mode == 2) {
 #pragma unroll
-                            for (int q = 0; q < 4; q++) {
-                                const __half2 h = __floats2half2_rn(p.alpha * __uint_as_float(v[j + 2 * q]) + brow, p.alpha * __uint_as_float(v[j + 2 * q + 1]) + brow);
-                                w[q] = *reinterpret_cast<const uint32_t *>(&h);
+                            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + ld(bias + col0 + c0 + j));
+                        }
+                        if (!vec) {
+                            T *dst = crow + (long long)(col0 + c0) * p.c_cs;
+#pragma unroll
+                            for (int j = 0; j < 32; j++, dst += p.c_cs) st(dst, __uint_as_float(v[j]));
+                        } else if constexpr (HALF) {
+                            uint4 *dst = reinterpret_cast<uint4 *>(crow + col0 + c0);
+#pragma unroll
+                            for (int j = 0; j < 32; j += 8) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int q = 0; q < 4; q++) {
+                                    const __half2 h = __floats2half2_rn(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
+                                    w[q] = *reinterpret_cast<const uint32_t *>(&h);
+                                }
+                                dst[j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
                             }
-                            dst[j / 8] = make_uint4(w[0], w[1], w[2], w[3]);
+                        } else {
+                            uint4 *dst = reinterpret_cast<uint4 *>(crow + col0 + c0);
+#pragma unroll
+                            for (int j = 0; j < 32; j += 4) dst[j / 4] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                         }
                     } else {
 #pragma unroll
@@ -351,8 +370,10 @@ template <class T> __global__ void __launch_bounds__(256) tm_reduce_kernel(const
 
 // ---------------------------------------------------------------- operand packing
 // dst[(b * rows + r) * Kp + k] = src[b*bs + r*rs + k*cs] for k < K (columns K..Kp-1 are never read: the tensor map ends at K).
-// fp32: hi part to dst, lo part to lo.  One launch for both operands of a product.  A block moves 32 rows x 64 k: K-contiguous
-// sources go straight through registers, eight k per thread; the others through a shared-memory tile read along the rows.
+// fp32: hi part to dst, lo part to lo.  One launch for both operands of a product.  K-contiguous sources go straight through
+// registers, 32 rows x 64 k per block and eight k per thread; the others through a shared-memory tile of 32 k x 64 rows, read
+// as vectors along the rows where they are contiguous and aligned, written as whole 128-byte rows of 32 k (64 x [64 x 784]
+// transposed and split: 15.5 us with scalar reads of 32 rows, 9.2 us so).
 template <class T> struct PackOp { const T *src; T *dst, *lo; long long rs, cs, bs; int rows, K, Kp, nk, nr, first, straight, vec; };
 template <class T> struct PackOps { PackOp<T> op[2]; int count; };
 
@@ -362,11 +383,59 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(const __grid_constant_
     pdl_wait();
     __shared__ float tile[32][65];
     const PackOp<T> &o = ops.op[ops.count > 1 && (int)blockIdx.x >= ops.op[1].first ? 1 : 0];
-    const int t = (int)blockIdx.x - o.first, k0 = (t % o.nk) * 64, r0 = ((t / o.nk) % o.nr) * 32, b = t / (o.nk * o.nr);
+    const int t = (int)blockIdx.x - o.first, tr = t / o.nk, b = tr / o.nr;
+    if (!o.straight) {
+        const int k0 = (t - tr * o.nk) * 32, r0 = (tr - b * o.nr) * 64, left = o.rows - r0;
+        const T *s = o.src + (long long)b * o.bs + (long long)r0 * o.rs;
+        if (sizeof(T) == 4 && o.vec) {
+            const int rq = (threadIdx.x & 15) * 4, kk = threadIdx.x >> 4;
+            float4 v[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const T *p = s + rq + (long long)(k0 + kk + 16 * q) * o.cs;
+                v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k0 + kk + 16 * q < o.K) {
+                    if (rq + 4 <= left) v[q] = *reinterpret_cast<const float4 *>(p);
+                    else { if (rq < left) v[q].x = ld(p); if (rq + 1 < left) v[q].y = ld(p + 1); if (rq + 2 < left) v[q].z = ld(p + 2); }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) { float *d = &tile[kk + 16 * q][rq]; d[0] = v[q].x; d[1] = v[q].y; d[2] = v[q].z; d[3] = v[q].w; }
+        } else {
+            const int rr = threadIdx.x & 63, kk = threadIdx.x >> 6;
+            const T *p = s + (long long)rr * o.rs + (long long)(k0 + kk) * o.cs;
+            float v[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++, p += 4 * o.cs) v[q] = rr < left && k0 + kk + 4 * q < o.K ? ld(p) : 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) tile[kk + 4 * q][rr] = v[q];
+        }
+        __syncthreads();
+        const int kq = (threadIdx.x & 7) * 4;
+        if (k0 + kq >= o.Kp) return;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int row = (threadIdx.x >> 3) + 32 * h;
+            if (row >= left) return;
+            const long long at = ((long long)b * o.rows + r0 + row) * o.Kp + k0 + kq;
+            if constexpr (sizeof(T) == 4) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) split_tf32(tile[kq + q][row], hi[q], lo[q]);
+                *reinterpret_cast<uint4 *>(o.dst + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4 *>(o.lo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            } else {
+                const __half2 x = __floats2half2_rn(tile[kq][row], tile[kq + 1][row]), y = __floats2half2_rn(tile[kq + 2][row], tile[kq + 3][row]);
+                *reinterpret_cast<uint2 *>(o.dst + at) = make_uint2(*reinterpret_cast<const uint32_t *>(&x), *reinterpret_cast<const uint32_t *>(&y));
+            }
+        }
+        return;
+    }
+    const int k0 = (t - tr * o.nk) * 64, r0 = (tr - b * o.nr) * 32;
     const T *s = o.src + (long long)b * o.bs;
     const int r = threadIdx.x >> 3, kq = (threadIdx.x & 7) * 8;
     float v[8];
-    if (o.straight) {
+    {
         const T *p = s + (long long)(r0 + r) * o.rs + k0 + kq;
         if (o.vec && r0 + r < o.rows && k0 + kq + 8 <= o.K) {
             if constexpr (sizeof(T) == 4) {
@@ -380,16 +449,6 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(const __grid_constant_
 #pragma unroll
             for (int q = 0; q < 8; q++) v[q] = (r0 + r < o.rows && k0 + kq + q < o.K) ? ld(p + q) : 0.f;
         }
-    } else {
-        const int rr = threadIdx.x & 31, kk = threadIdx.x >> 5;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const int k = k0 + kk + 8 * q;
-            tile[rr][kk + 8 * q] = (r0 + rr < o.rows && k < o.K) ? ld(s + (long long)(r0 + rr) * o.rs + (long long)k * o.cs) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = tile[r][kq + q];
     }
     if (r0 + r >= o.rows || k0 + kq >= o.Kp) return;
     const long long at = ((long long)b * o.rows + r0 + r) * o.Kp + k0 + kq;          // Kp is a multiple of 16 bytes
@@ -455,7 +514,7 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     typedef TmCfg<T> Cfg;
     if (d.N < 1 || d.M < 1 || d.K < 1 || d.batch < 1) return false;
     if (gemm_path() != 3) {      // 3 = forced (tests): every shape, the tails come from the tensor maps' zero fill
-        if (d.N < TM_BM || d.M < TM_BM / 2 || d.K < 2 * Cfg::BK) return false;
+        if (d.N < TM_BM || d.M < TM_BM / 2 || d.K < (d.batch > 1 ? 1 : 2) * Cfg::BK) return false;
         if ((long long)d.N * d.M * d.K * d.batch < (1ll << 26)) return false;
     }
     EncodeTiledFn enc = (EncodeTiledFn)tc_encode_tiled_fn();
@@ -470,22 +529,24 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     PackOps<T> pack;
     pack.count = 0;
     int blocks = 0;
-    auto prepare = [&](const T *src, long long rs, long long cs, long long bs, int rows, Op &o) -> bool {
-        const bool aligned = sizeof(T) == 2 && ((uintptr_t)src & 15) == 0 && (d.batch == 1 || bs % EB == 0);
+    auto prepare = [&](const T *src, long long rs, long long cs, long long bs, int rows, int batch, Op &o) -> bool {
+        const bool aligned = sizeof(T) == 2 && ((uintptr_t)src & 15) == 0 && (batch == 1 || bs % EB == 0);
         if (aligned && cs == 1 && rs % EB == 0 && rs >= d.K) { o = {src, nullptr, rs, bs, 0}; return true; }
         if (aligned && rs == 1 && cs % EB == 0 && cs >= rows) { o = {src, nullptr, cs, bs, 1}; return true; }
-        const size_t count = (size_t)d.batch * rows * Kp;
+        const size_t count = (size_t)batch * rows * Kp;
         T *hi = sc.scratch<T>(count), *lo = sizeof(T) == 4 ? sc.scratch<T>(count) : nullptr;
         if (!hi || (sizeof(T) == 4 && !lo)) return false;
         PackOp<T> &q = pack.op[pack.count++];
-        q = {src, hi, lo, rs, cs, bs, rows, d.K, Kp, ceil_div(Kp, 64), ceil_div(rows, 32), blocks, cs == 1, cs == 1 && rs % EB == 0 && (d.batch == 1 || bs % EB == 0) && ((uintptr_t)src & 15) == 0};
-        blocks += q.nk * q.nr * d.batch;
+        const bool straight = cs == 1;
+        q = {src, hi, lo, rs, cs, bs, rows, d.K, Kp, ceil_div(Kp, straight ? 64 : 32), ceil_div(rows, straight ? 32 : 64), blocks, straight, (straight ? rs : rs == 1 ? cs : 1) % EB == 0 && (batch == 1 || bs % EB == 0) && ((uintptr_t)src & 15) == 0};
+        blocks += q.nk * q.nr * batch;
         o = {hi, lo, Kp, (long long)rows * Kp, 0};
         return true;
     };
     Op a, b;
-    if (!prepare(d.A, d.a_rs, d.a_cs, d.a_bs, d.N, a)) return false;
-    if (!prepare(d.B, d.b_cs, d.b_rs, d.b_bs, d.M, b)) return false;     // row of the B operand = column of C
+    const int b_batch = d.b_bs == 0 ? 1 : d.batch;
+    if (!prepare(d.A, d.a_rs, d.a_cs, d.a_bs, d.N, d.batch, a)) return false;
+    if (!prepare(d.B, d.b_cs, d.b_rs, d.b_bs, d.M, b_batch, b)) return false;     // row of the B operand = column of C
     TmParams p;
     p.ksteps = ceil_div(d.K, Cfg::BK);
     p.BN = sizeof(T) == 2 ? 256 : 128; p.splits = 1; p.pair = 0;
@@ -493,20 +554,20 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     p.C = d.C; p.bias = d.bias; p.N = d.N; p.M = d.M; p.K = d.K;
     p.c_rs = d.c_rs; p.c_cs = d.c_cs; p.c_bs = d.c_bs;
     p.alpha = d.alpha; p.accumulate = d.accumulate ? 1 : 0; p.bias_mode = d.bias ? d.bias_mode : 0;
-    p.status = status; p.a_mn = a.mn; p.b_mn = b.mn;
+    p.status = status; p.a_mn = a.mn; p.b_mn = b.mn; p.b_one = b_batch < d.batch;
     p.tiles_m = ceil_div(d.M, p.BN); p.tiles_n = ceil_div(d.N, p.pair ? 2 * TM_BM : TM_BM); p.tiles = p.tiles_m * p.tiles_n * d.batch;
     p.part = nullptr;
     if (p.splits > 1 && !(p.part = sc.scratch<float>((size_t)p.tiles * p.splits * TM_BM * p.BN))) return false;
     const int b_rows = p.pair ? p.BN / 2 : p.BN;
     p.stage_bytes = Cfg::PARTS * (TM_BM * 128u + (uint32_t)b_rows * 128u);
     p.stages = std::min<int>(TM_MAX_STAGES, TM_RING / p.stage_bytes);
-    auto map = [&](CUtensorMap *m, const T *base, const Op &o, int rows, int box_rows) {
-        return o.mn ? make_map<T>(enc, m, base, rows, d.K, d.batch, o.os, o.bs, 64, 64) : make_map<T>(enc, m, base, d.K, rows, d.batch, o.os, o.bs, Cfg::BK, box_rows);
+    auto map = [&](CUtensorMap *m, const T *base, const Op &o, int rows, int batch, int box_rows) {
+        return o.mn ? make_map<T>(enc, m, base, rows, d.K, batch, o.os, o.bs, 64, 64) : make_map<T>(enc, m, base, d.K, rows, batch, o.os, o.bs, Cfg::BK, box_rows);
     };
     CUtensorMap ma0, ma1, mb0, mb1;
-    if (!map(&ma0, a.hi, a, d.N, TM_BM) || !map(&mb0, b.hi, b, d.M, b_rows)) return false;
+    if (!map(&ma0, a.hi, a, d.N, d.batch, TM_BM) || !map(&mb0, b.hi, b, d.M, b_batch, b_rows)) return false;
     ma1 = ma0; mb1 = mb0;
-    if (sizeof(T) == 4 && (!map(&ma1, a.lo, a, d.N, TM_BM) || !map(&mb1, b.lo, b, d.M, b_rows))) return false;
+    if (sizeof(T) == 4 && (!map(&ma1, a.lo, a, d.N, d.batch, TM_BM) || !map(&mb1, b.lo, b, d.M, b_batch, b_rows))) return false;
     if (pack.count) TL_LAUNCH((pack_kmajor_kernel<T>), blocks, 256, 0, pack);
     const size_t smem = (size_t)p.stages * p.stage_bytes + 1024;
     static bool attr_set = false;

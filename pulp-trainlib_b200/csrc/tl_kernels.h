@@ -20,6 +20,7 @@ template <class T> struct GemmDesc {
     int bias_mode = 0;              // 1: bias[i] (per row), 2: bias[j] (per column)
 };
 template <class T> void gemm(const GemmDesc<T> &d);
+template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d);      // false: not a product for it, nothing launched
 // One member of a group of products that go out as one launch (tl_gemm_small.cu): a GemmDesc whose contraction may run over
 // `segs` segments of K each.  seg_list: segment s multiplies A[s] by B[s] (separate allocations, 3 at most); otherwise the
 // operands of segment s start at A[0] + s * a_ks and B[0] + s * b_ks.
