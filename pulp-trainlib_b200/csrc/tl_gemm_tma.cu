@@ -16,7 +16,8 @@
 //         chains are a third as long as one common chain (the accumulator truncates).
 // Measured, whole call: fp16 4096^3 173 -> 101 us, fp16 2048^3 29 -> 17.5 us, fp32 2048^3 118 -> 89 us, fp32 1000 x 600 x 1300
 // (B transposed) 31 -> 20.3 us, fp32 300 x 2050 x 914 67 -> 26 us.
-// Few tiles: `splits` CTAs share the K steps of a tile and write partial tiles; tm_reduce_kernel adds them in order.
+// Few tiles: `splits` CTAs share the K steps of a tile and write partial tiles; tm_reduce_kernel adds them in order.  A contraction
+// may run over several segments (the streams of a batch), which the tensor maps' third index selects, as it selects a batch.
 // No multicast loads.  Every wait is bounded and reports through the status word.
 #include "tl_kernels.h"
 #include "tl_tc.cuh"
@@ -47,7 +48,7 @@ struct TmParams {
     int N, M, K;
     long long c_rs, c_cs, c_bs;
     float alpha; int accumulate, bias_mode;
-    int BN, tiles_m, tiles_n, tiles, ksteps, splits, stages, pair, a_mn, b_mn, b_one;      // b_one: all products of a batch share B
+    int BN, tiles_m, tiles_n, tiles, ksteps, kps, splits, stages, pair, a_mn, b_mn, b_one;      // b_one: all products of a batch share B
     uint32_t stage_bytes;
     int *status;
 };
@@ -194,8 +195,10 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
         for (int tile = first; tile < p.tiles && ok; tile += step) {
             int b, rb, cb;
             tm_locate(p, tile, b, rb, cb);
-            const int row0 = rb * ROWS + row_of_tile, col0 = cb * BN + (PAIR ? rank * BNL : 0), zb = p.b_one ? 0 : b;
-            for (int kt = ks0; kt < ks1; kt++) {
+            const int row0 = rb * ROWS + row_of_tile, col0 = cb * BN + (PAIR ? rank * BNL : 0);
+            int seg = ks0 / p.kps, kt = ks0 - seg * p.kps;                          // segment of the contraction, K step inside it
+            for (int k = ks0; k < ks1; k++) {
+                const int za = b + seg, zb = (p.b_one ? 0 : b) + seg;
                 if (!tm_wait(&empty[s], phase, failed)) { ok = false; break; }
                 if (elect_one()) {
                     const uint32_t st = sbase + s * p.stage_bytes, sb = st + Cfg::PARTS * A_BYTES;
@@ -205,14 +208,15 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
                         else tma_load_3d(dst, m, &full[s], x, y, z);
                     };
                     if (!PAIR || rank == 0) mbar_arrive_expect_tx(&full[s], PAIR ? 2 * p.stage_bytes : p.stage_bytes);
-                    if (HALF && p.a_mn) { for (int j = 0; j < 2; j++) load(st + j * 8192u, &a0, row0 + 64 * j, kt * BK, b); }
-                    else load(st, &a0, kt * BK, row0, b);
-                    if (!HALF) load(st + A_BYTES, &a1, kt * BK, row0, b);
+                    if (HALF && p.a_mn) { for (int j = 0; j < 2; j++) load(st + j * 8192u, &a0, row0 + 64 * j, kt * BK, za); }
+                    else load(st, &a0, kt * BK, row0, za);
+                    if (!HALF) load(st + A_BYTES, &a1, kt * BK, row0, za);
                     if (HALF && p.b_mn) { for (int j = 0; j < BNL / 64; j++) load(sb + j * 8192u, &b0, col0 + 64 * j, kt * BK, zb); }
                     else load(sb, &b0, kt * BK, col0, zb);
                     if (!HALF) load(sb + B_BYTES, &b1, kt * BK, col0, zb);
                 }
                 __syncwarp();
+                if (++kt == p.kps) { kt = 0; seg++; }
                 if (++s == ST) { s = 0; phase ^= 1u; }
             }
         }
@@ -350,19 +354,34 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
     } else if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// C from the partial tiles of a split contraction: one thread per four neighbouring columns, parts added in order.
-template <class T> __global__ void __launch_bounds__(256) tm_reduce_kernel(const __grid_constant__ TmParams p)
+// C from the partial tiles of a split contraction: a thread per four neighbouring columns; PARTS threads share the partial tiles
+// of a quad where there are many (their sums are added in order).
+template <class T, int PARTS> __global__ void __launch_bounds__(256) tm_reduce_kernel(const __grid_constant__ TmParams p)
 {
     pdl_wait();
-    const int quads = p.BN / 4, per = TM_BM * quads, e = blockIdx.x * 256 + threadIdx.x;          // (per is a multiple of 256: a block stays inside one tile)
+    constexpr int Q = 256 / PARTS;                                                  // quads of a block
+    __shared__ float4 sums[PARTS > 1 ? PARTS : 1][Q];
+    const int quads = p.BN / 4, per = TM_BM * quads, part = threadIdx.x / Q, e = blockIdx.x * Q + threadIdx.x % Q;    // (per is a multiple of 256: a block stays inside one tile)
     const int tile = e / per, in = e - tile * per, r = in / quads, c = (in - r * quads) * 4;
     int b, rb, cb;
     tm_locate(p, tile, b, rb, cb);
     const int row = rb * TM_BM + r, col = cb * p.BN + c;
-    if (row >= p.N || col >= p.M) return;
+    const bool live = row < p.N && col < p.M;
     const float4 *src = reinterpret_cast<const float4 *>(p.part + (long long)tile * p.splits * TM_BM * p.BN) + in;
-    float4 t = src[0];
-    for (int k = 1; k < p.splits; k++) { const float4 u = src[(long long)k * per]; t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+    const int k0 = p.splits * part / PARTS, k1 = p.splits * (part + 1) / PARTS;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) {
+#pragma unroll 8
+        for (int k = k0; k < k1; k++) { const float4 u = src[(long long)k * per]; t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+    }
+    if constexpr (PARTS > 1) {
+        sums[part][threadIdx.x % Q] = t;
+        __syncthreads();
+        if (part > 0) return;
+#pragma unroll
+        for (int k = 1; k < PARTS; k++) { const float4 u = sums[k][threadIdx.x]; t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w; }
+    }
+    if (!live) return;
     T *crow = reinterpret_cast<T *>(p.C) + (long long)b * p.c_bs + (long long)row * p.c_rs;
     const float v[4] = {t.x, t.y, t.z, t.w};
     tm_store4<T>(p, crow, row, col, v, p.c_cs == 1 && !p.accumulate && ((uintptr_t)crow & (4 * sizeof(T) - 1)) == 0);
@@ -487,7 +506,7 @@ template <class T> static bool make_map(EncodeTiledFn enc, CUtensorMap *m, const
 // pass over the partial tiles of a split contraction a launch and their bytes.  So pairs take the products of several rounds of
 // tiles with long contractions (fp16 4096^3: 97 us against 105 us) and single CTAs the rest (fp16 2048^3: 17.6 us against
 // 19.1 us, fp32 1000 x 600 x 1300: 16.2 us against 19.5 us).
-template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int &BN, int &splits, int &pair)
+template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int most_splits, int &BN, int &splits, int &pair)
 {
     constexpr bool HALF = sizeof(T) == 2;
     double best = 1e30;
@@ -496,7 +515,7 @@ template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int 
         const bool two = i == 3;
         const int bn = HALF ? bns_h[i] : bns_f[i], rows = two ? 2 * TM_BM : TM_BM;
         const long long tiles = (long long)ceil_div(N, rows) * ceil_div(M, bn) * batch;
-        for (int s = 1; s <= (two ? 1 : 8); s++) {
+        for (int s = 1; s <= (two ? 1 : most_splits); s++) {
             if (s > 1 && (ksteps < 2 * s || tiles * s > sm_count())) break;
             const long long ctas = tiles * s * (two ? 2 : 1);
             const double tensor = (HALF ? 2.0 : 6.0) * bn * (two ? 4.0 / 3.0 : 1.0);
@@ -512,10 +531,10 @@ template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int 
 template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
 {
     typedef TmCfg<T> Cfg;
-    if (d.N < 1 || d.M < 1 || d.K < 1 || d.batch < 1) return false;
+    if (d.N < 1 || d.M < 1 || d.K < 1 || d.batch < 1 || d.segs < 1 || (d.batch > 1 && d.segs > 1)) return false;
     if (gemm_path() != 3) {      // 3 = forced (tests): every shape, the tails come from the tensor maps' zero fill
-        if (d.N < TM_BM || d.M < TM_BM / 2 || d.K < (d.batch > 1 ? 1 : 2) * Cfg::BK) return false;
-        if ((long long)d.N * d.M * d.K * d.batch < (1ll << 26)) return false;
+        if (d.segs == 1 && (d.N < TM_BM || d.M < TM_BM / 2 || d.K < (d.batch > 1 ? 1 : 2) * Cfg::BK)) return false;
+        if ((long long)d.N * d.M * d.K * d.batch * d.segs < (1ll << 26)) return false;
     }
     EncodeTiledFn enc = (EncodeTiledFn)tc_encode_tiled_fn();
     int *status = tc_status_word();
@@ -544,17 +563,17 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
         return true;
     };
     Op a, b;
-    const int b_batch = d.b_bs == 0 ? 1 : d.batch;
-    if (!prepare(d.A, d.a_rs, d.a_cs, d.a_bs, d.N, d.batch, a)) return false;
-    if (!prepare(d.B, d.b_cs, d.b_rs, d.b_bs, d.M, b_batch, b)) return false;     // row of the B operand = column of C
+    const int copies = d.batch * d.segs, b_batch = d.segs == 1 && d.b_bs == 0 ? 1 : copies;      // a batch and the segments of a contraction are walked alike
+    if (!prepare(d.A, d.a_rs, d.a_cs, d.segs > 1 ? d.a_ks : d.a_bs, d.N, copies, a)) return false;
+    if (!prepare(d.B, d.b_cs, d.b_rs, d.segs > 1 ? d.b_ks : d.b_bs, d.M, b_batch, b)) return false;     // row of the B operand = column of C
     TmParams p;
-    p.ksteps = ceil_div(d.K, Cfg::BK);
+    p.kps = ceil_div(d.K, Cfg::BK); p.ksteps = p.kps * d.segs;
     p.BN = sizeof(T) == 2 ? 256 : 128; p.splits = 1; p.pair = 0;
-    tm_plan<T>(d.N, d.M, d.batch, p.ksteps, p.BN, p.splits, p.pair);
+    tm_plan<T>(d.N, d.M, d.batch, p.ksteps, d.segs > 1 ? 1 << 20 : 8, p.BN, p.splits, p.pair);
     p.C = d.C; p.bias = d.bias; p.N = d.N; p.M = d.M; p.K = d.K;
     p.c_rs = d.c_rs; p.c_cs = d.c_cs; p.c_bs = d.c_bs;
     p.alpha = d.alpha; p.accumulate = d.accumulate ? 1 : 0; p.bias_mode = d.bias ? d.bias_mode : 0;
-    p.status = status; p.a_mn = a.mn; p.b_mn = b.mn; p.b_one = b_batch < d.batch;
+    p.status = status; p.a_mn = a.mn; p.b_mn = b.mn; p.b_one = b_batch < copies;
     p.tiles_m = ceil_div(d.M, p.BN); p.tiles_n = ceil_div(d.N, p.pair ? 2 * TM_BM : TM_BM); p.tiles = p.tiles_m * p.tiles_n * d.batch;
     p.part = nullptr;
     if (p.splits > 1 && !(p.part = sc.scratch<float>((size_t)p.tiles * p.splits * TM_BM * p.BN))) return false;
@@ -565,9 +584,9 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
         return o.mn ? make_map<T>(enc, m, base, rows, d.K, batch, o.os, o.bs, 64, 64) : make_map<T>(enc, m, base, d.K, rows, batch, o.os, o.bs, Cfg::BK, box_rows);
     };
     CUtensorMap ma0, ma1, mb0, mb1;
-    if (!map(&ma0, a.hi, a, d.N, d.batch, TM_BM) || !map(&mb0, b.hi, b, d.M, b_batch, b_rows)) return false;
+    if (!map(&ma0, a.hi, a, d.N, copies, TM_BM) || !map(&mb0, b.hi, b, d.M, b_batch, b_rows)) return false;
     ma1 = ma0; mb1 = mb0;
-    if (sizeof(T) == 4 && (!map(&ma1, a.lo, a, d.N, d.batch, TM_BM) || !map(&mb1, b.lo, b, d.M, b_batch, b_rows))) return false;
+    if (sizeof(T) == 4 && (!map(&ma1, a.lo, a, d.N, copies, TM_BM) || !map(&mb1, b.lo, b, d.M, b_batch, b_rows))) return false;
     if (pack.count) TL_LAUNCH((pack_kmajor_kernel<T>), blocks, 256, 0, pack);
     const size_t smem = (size_t)p.stages * p.stage_bytes + 1024;
     static bool attr_set = false;
@@ -580,7 +599,9 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     else if (p.splits == 1) TL_LAUNCH((gemm_tma_kernel<T, false>), (unsigned)std::min(p.tiles, sm_count()), TM_THREADS, smem, ma0, ma1, mb0, mb1, p);
     else {
         TL_LAUNCH((gemm_tma_kernel<T, false>), (unsigned)(p.tiles * p.splits), TM_THREADS, smem, ma0, ma1, mb0, mb1, p);
-        TL_LAUNCH((tm_reduce_kernel<T>), (unsigned)((long long)p.tiles * TM_BM * p.BN / 1024), 256, 0, p);
+        const long long quads = (long long)p.tiles * TM_BM * p.BN / 4;
+        if (p.splits <= 16) TL_LAUNCH((tm_reduce_kernel<T, 1>), (unsigned)(quads / 256), 256, 0, p);
+        else TL_LAUNCH((tm_reduce_kernel<T, 8>), (unsigned)(quads / 32), 256, 0, p);
     }
     return true;
 }

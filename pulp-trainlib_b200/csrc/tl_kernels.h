@@ -14,6 +14,7 @@ template <class T> struct GemmDesc {
     int N = 0, M = 0, K = 0;
     long long a_rs = 0, a_cs = 1, b_rs = 0, b_cs = 1, c_rs = 0, c_cs = 1;
     int batch = 1; long long a_bs = 0, b_bs = 0, c_bs = 0;
+    int segs = 1; long long a_ks = 0, b_ks = 0;     // gemm_tensor_core_tma only (batch 1): the contraction runs over `segs` segments of K, strides between them
     float alpha = 1.f;
     bool accumulate = false;        // C += result instead of C = result
     const T *bias = nullptr;        // added after the product

@@ -26,7 +26,7 @@ def rounded(r, a):
 
 CONV = [(28, 14, 45, 28, 3, 1, 1), (3, 33, 41, 70, 5, 2, 3), (6, 42, 13, 81, 5, 1, 1), (40, 9, 11, 64, 3, 1, 5), (16, 5, 5, 8, 3, 1, 40), (20, 3, 200, 24, 3, 1, 2),
         (17, 12, 130, 33, 3, 2, 2), (64, 7, 7, 96, 1, 1, 30), (24, 28, 28, 48, 3, 1, 60), (33, 11, 12, 17, 3, 3, 2), (1, 6, 6, 4, 1, 1, 2), (70, 10, 10, 12, 7, 1, 1),
-        (12, 8, 9, 16, 1, 2, 3), (64, 12, 12, 64, 5, 1, 4), (16, 7, 8, 8, 3, 1, 150), (8, 10, 16, 16, 3, 1, 63), (16, 32, 32, 16, 3, 1, 9), (8, 12, 32, 8, 3, 1, 30), (64, 16, 17, 64, 1, 1, 70), (36, 13, 15, 100, 1, 1, 100), (64, 40, 40, 72, 1, 1, 10), (72, 12, 12, 64, 1, 1, 110)]
+        (12, 8, 9, 16, 1, 2, 3), (64, 12, 12, 64, 5, 1, 4), (16, 7, 8, 8, 3, 1, 150), (8, 10, 16, 16, 3, 1, 63), (16, 32, 32, 16, 3, 1, 9), (8, 12, 32, 8, 3, 1, 30), (64, 16, 17, 64, 1, 1, 70), (36, 13, 15, 100, 1, 1, 100), (64, 40, 40, 72, 1, 1, 10), (72, 12, 12, 64, 1, 1, 110), (33, 9, 8, 130, 1, 1, 230)]
 
 
 @pytest.mark.parametrize("cin,h,w,cout,k,stride,n", CONV)
