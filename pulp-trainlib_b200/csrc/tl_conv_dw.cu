@@ -317,8 +317,9 @@ template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy,
     if (dw3_params(g, q, x, dy, (int)sizeof(T), false)) {
         groups = std::max(1, std::min(ceil_div(8 * sm_count(), g.Cin), g.n));
         if (dry) return true;
-        q.G = std::max(1, std::min(256 / (q.Ho * q.O4), ceil_div(g.n, groups)));
-        while (q.G > 1 && (size_t)q.G * q.PH * q.PW * 4 > 48 * 1024) q.G--;
+        // all planes of a CTA at once while eight CTAs fit an SM's shared memory: one wait for memory instead of one per plane
+        q.G = ceil_div(g.n, groups);
+        while (q.G > 1 && (size_t)q.G * q.PH * q.PW * 4 > 24 * 1024) q.G--;
         const size_t smem = (size_t)q.G * q.PH * q.PW * 4;
         const dim3 grid(g.Cin, groups);
         if (q.padL == 1) TL_LAUNCH((dw3_wg_kernel<T, 1>), grid, 128, smem, q, x, dy, part, g.n);
