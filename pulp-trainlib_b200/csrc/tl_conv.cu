@@ -1052,7 +1052,11 @@ template <> bool try_tc_wg<float>(Scope &sc, const ConvGeom &g, const float *x, 
         reduce_partials<float>(part, dw, nw, small, deferred);
         return true;
     }
-    if (gemm_path() != 2 && (work < (1ll << 28) || g.Cin < (g.sh == 2 ? 16 : 32))) return false;
+    // What the tensor-core kernel pays below is its partial results, one dW per SM, so the line lies by their size (us with the sum,
+    // against mma.sync): 16 -> 32 stride 2, 20 streams 12.5 / 14.0, 200 streams 20.6 / 29.3; 32 -> 32 on 16 x 16, 50 streams 16.1 /
+    // 20.8; 32 -> 64 stride 2, 50 streams 16.4 / 16.0, 200 streams 20.7 / 27.8; 64 -> 64 on 8 x 8, 100 streams 25.2 / 23.6.
+    const int pair = g.Cin * g.Cout;
+    if (gemm_path() != 2 && (work < (1ll << (pair <= 1024 ? 24 : pair <= 2048 ? 26 : 28)) || g.Cin < (g.sh == 2 ? 16 : 32))) return false;
     int groups = 0;
     long long group_floats = 0;
     if (!conv_wgt_run(x, dy, nullptr, sm_count(), &groups, &group_floats, g.n, g.Cin, g.Cout, g.Hout, g.Wout, g.sh, true)) return false;
