@@ -105,14 +105,26 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(d_empty + 2 * MN_MAX_NI);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < p.nstage; i++) { mbar_init(&raw_full[i], 1); mbar_init(&a_full[i], MN_CONV_WARPS); mbar_init(&stage_empty[i], NI); }
-        for (int i = 0; i < NI * p.NBUF; i++) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4); }
-        *abort_flag = 0;
-        fence_barrier_init();
-        tma_prefetch_desc(&tmap);
+    // Copies of chunk k (channel group k mod cigs of the CTA's tile k / cigs)
+    const int my_chunks = ((p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * p.cigs, early = min(p.nstage, my_chunks);
+    auto load_chunk = [&](int k) {
+        const int st = k % p.nstage, tile = k / p.cigs, g = k - tile * p.cigs, t = (int)blockIdx.x + tile * (int)gridDim.x;
+        const int s0 = (t / p.tiles_per_image) * p.P, y0 = (t % p.tiles_per_image) * p.VR;
+        mbar_arrive_expect_tx(&raw_full[st], (uint32_t)p.NSLOT * (uint32_t)MN_SLOT);
+        tma_load_4d(stages + (size_t)st * 2 * half_bytes, &tmap, &raw_full[st], 0, s0, g * 8, y0 - p.padU);
+    };
+    if (warp == tma_warp) {
+        // the first round of copies leaves before the weights are built: the two waits for memory overlap
+        if (elect_one()) {
+            for (int i = 0; i < p.nstage; i++) { mbar_init(&raw_full[i], 1); mbar_init(&a_full[i], MN_CONV_WARPS); mbar_init(&stage_empty[i], NI); }
+            for (int i = 0; i < NI * p.NBUF; i++) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], 4); }
+            *abort_flag = 0;
+            fence_barrier_init();
+            for (int k = 0; k < early; k++) load_chunk(k);
+        }
+        __syncwarp();
+        tmem_alloc(tmem_slot, 512u); tmem_relinquish();
     }
-    if (warp == tma_warp) { tmem_alloc(tmem_slot, 512u); tmem_relinquish(); }
     // B operand (weights of this CTA's output-channel slice), K-major core matrices of 8 rows x 16 bytes:
     // step (g, a) = channel group g, window row a; inside a step [k4 = 0..1][row r = 0..2NB-1][j = 0..3].
     // Row r = chunk*(WK*16) + b*16 + c holds hi(w) and row NB + r lo(w) of output channel slice*NT + chunk*16 + c,
@@ -127,7 +139,8 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
         // times did not change with the dealing, the filters come from L1 / L2 either way.)
         const int taps = p.Hk * WK, items = taps * p.cigs * p.NT;
         const bool by_group = !p.cls && !p.flip;
-        for (int it = threadIdx.x; it < items; it += nthreads) {
+        const int me = warp == tma_warp ? items : warp > tma_warp ? (int)threadIdx.x - 32 : (int)threadIdx.x;     // (the copying warp has none)
+        for (int it = me; it < items; it += nthreads - 32) {
             const int tap = it % taps, rest = it / taps;
             const int a = tap / WK, b = tap % WK;
             const int g = by_group ? rest % p.cigs : rest / p.NT, c = by_group ? rest / p.cigs : rest % p.NT;
@@ -166,21 +179,10 @@ conv_mn_kernel(const __grid_constant__ CUtensorMap tmap, const ConvMnParams p)
     const uint32_t stages_u32 = smem_u32(stages);
     if (warp == tma_warp) {
         // ------------------------------------------------------------ TMA producer
-        {
-            uint32_t k = 0;                                     // chunk counter (tile, channel group)
-            const uint32_t chunk_tx = (uint32_t)p.NSLOT * (uint32_t)MN_SLOT;
-            bool ok = true;
-            for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
-                const int s0 = (t / p.tiles_per_image) * p.P, y0 = (t % p.tiles_per_image) * p.VR;
-                for (int g = 0; g < p.cigs; g++, k++) {
-                    const int st = k % p.nstage;
-                    if (!warp_wait_or_abort(&stage_empty[st], ((k / p.nstage) & 1) ^ 1, abort_flag, p.status, 11, 128u, lane)) { ok = false; break; }
-                    if (elect_one()) {
-                        mbar_arrive_expect_tx(&raw_full[st], chunk_tx);
-                        tma_load_4d(stages + (size_t)st * 2 * half_bytes, &tmap, &raw_full[st], 0, s0, g * 8, y0 - p.padU);
-                    }
-                }
-            }
+        for (int k = early; k < my_chunks; k++) {
+            if (!warp_wait_or_abort(&stage_empty[k % p.nstage], ((k / p.nstage) & 1) ^ 1, abort_flag, p.status, 11, 128u, lane)) break;
+            if (elect_one()) load_chunk(k);
+            __syncwarp();
         }
     } else if (warp >= first_conv) {
         // ------------------------------------------------------------ converters: raw -> hi in place, lo beside it
