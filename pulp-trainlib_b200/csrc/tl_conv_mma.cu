@@ -175,8 +175,12 @@ struct CmFwd {
     int rows_max, linear, pairs;
 };
 
+// CTAs per SM.  What bounds these kernels is issue at few warps, so a third one helps where the registers allow it without loss: fp16
+// tiles of 16 and 32 channels (400 streams of 8 -> 20 on 9 x 11: 12.4 -> 10.0 us a direction; 50 of 30 -> 13, 5 x 5: 19.5 -> 16.7).
+// The 64-channel tiles lose the overlap of their fragment loads (88 -> 96 us), the fp32 ones up to 6 %.
+template <class T, int WM> constexpr int cm_ctas() { return sizeof(T) == 2 && WM == 1 ? 3 : 2; }
 template <class T, int MT, int WM, int WN, int WK, int BN>
-__global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_kernel(const __grid_constant__ CmFwd p)
+__global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_kernel(const __grid_constant__ CmFwd p)
 {
     pdl_wait();
     constexpr int NT = 32 * WM * WN * WK, BM = 16 * MT * WM, TN = BN / WN, N8 = TN / 8;
@@ -499,7 +503,7 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
     if (smem > attr) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM_MAX); attr = CM_SMEM_MAX; }
     const int co_tiles = ceil_div(p.Cd, BM);
     // every CTA slot taken: co-resident CTAs share an SM, so a last round that only some of them have costs less than idle slots
-    const int gx = std::min(tiles_max, std::max(1, sm_count() * (smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls)));
+    const int gx = std::min(tiles_max, std::max(1, sm_count() * (cm_ctas<T, WM>() == 3 && smem <= 74 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls)));
     TL_LAUNCH((conv_mma_kernel<T, MT, WM, WN, WK, BN>), dim3(gx, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p);
     return true;
 }
