@@ -488,18 +488,19 @@ template <class F> bool linear_bw_both(void *args)
     const int in = a->input->dim, out = a->output->dim;
     if (streams() != 1 || in <= 0 || out <= 0 || gemm_path() == 1) return false;
     const bool ub = (a->use_biases == 1) && a->bias;
-    // what the kernel needs is checked before anything is staged: 16-byte strips (host buffers get aligned device mirrors)
-    if (in % (16 / (int)sizeof(T)) != 0 || in / (16 / (int)sizeof(T)) > 8192 * 32) return false;
+    // what the kernel needs is checked before anything is staged: all buffers, and 8192 column blocks of 32 strips at most (rows
+    // longer than that only in 16-byte strips; host buffers get aligned device mirrors)
     const void *ptrs[4] = {a->coeff->data, a->coeff->diff, a->input->data, a->input->diff};
+    constexpr int V = 16 / (int)sizeof(T), most = 8192 * 32;
+    if (in > most && (in % V != 0 || in / V > most)) return false;
     for (const void *q : ptrs)
-        if (!q || (is_device_pointer(q) && (((uintptr_t)q) & 15) != 0)) return false;
+        if (!q || (in > most && is_device_pointer(q) && (((uintptr_t)q) & 15) != 0)) return false;
     Scope sc;
     const T *dy = sc.in(a->output->diff, (size_t)out), *x = sc.in(a->input->data, (size_t)in), *w = sc.in(a->coeff->data, (size_t)out * in);
     T *dw = sc.out(a->coeff->diff, (size_t)out * in), *dx = sc.out(a->input->diff, (size_t)in);
     T *db = ub ? sc.out(a->bias->diff, (size_t)out) : nullptr;
     if (!sc.ok()) return true;                                     // the error is set; the separate calls would fail the same way
-    if (!linear_bw_fused<T>(sc, w, dy, x, dw, dx, out, in)) return true;   // only a failed scratch allocation is left: the error is set
-    if (db) column_sum<T>(sc, dy, db, 1, out);
+    linear_bw_fused<T>(sc, w, dy, x, dw, dx, db, out, in);         // false: a failed scratch allocation, the error is set
     return true;
 }
 

@@ -197,6 +197,7 @@ template <> __device__ __forceinline__ float dot_row<float, 4>(const float *__re
         s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
     }
     s = (s + s1) + (s2 + s3);
+#pragma unroll 8
     for (int t = n4 * 4 + lane; t < n; t += 32) s = fmaf(w[t], x[t], s);
     return s;
 }
@@ -214,6 +215,7 @@ template <> __device__ __forceinline__ float dot_row<__half, 8>(const __half *__
             s = fmaf(af.x, bf.x, s); s = fmaf(af.y, bf.y, s);
         }
     }
+#pragma unroll 8
     for (int i = n8 * 8 + lane; i < n; i += 32) s = fmaf(__half2float(w[i]), __half2float(x[i]), s);
     return s;
 }
@@ -437,37 +439,67 @@ template <class T> void linear_ig_gemv(Scope &sc, const T *W, const T *dy, T *dx
 }
 
 // Both gradients of a batch-1 Linear layer in one launch [ref: lib/sources/pulp_linear_fp32.c:60-180, the two halves of
-// pulp_linear_fp32_bw_cl].  A CTA owns 32 column strips of 16 bytes in one row slab; its four warps take every fourth
+// pulp_linear_fp32_bw_cl].  A CTA owns 32 column strips of V elements (16 bytes; rows that do not step in multiples of 16 bytes:
+// 4 bytes or one element, still neighbouring addresses per warp) in one row slab; its four warps take every fourth
 // row: for every row a thread loads its strip of W once, adds W * dy[o] to its dX partial and stores dy[o] * x[strip]
 // to dW (a warp moves 512 contiguous bytes each way per row).  The four warps' partials are added in warp order, the
 // slab's partial goes to `part`, and the CTA of a column block that finishes last (a ticket per column block) adds the
 // slabs' partials, always in the same order, so the result does not depend on which CTA that is: one launch instead of
-// three, W read once.
+// three, W read once.  The bias gradient, a copy of dy, leaves with the first column block.  Measured, whole step with bias, odd
+// rows: 21 -> 1398 fp32 20 us with five launches, 11 us with two; 3999 -> 4000 fp32 83 -> 42 us.
 static __device__ unsigned tl_linear_tickets[8192];                 // one per column block; zero between launches
 static constexpr int LBW_STRIPS = 32, LBW_LANES = 4;
 
-template <class T>
-__global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_fused_kernel(const T *__restrict__ W, const T *__restrict__ dy, const T *__restrict__ x,
-                                                                                 T *__restrict__ dW, float *__restrict__ part, T *__restrict__ dx,
-                                                                                 int out, int in, int rows_per_slab, int slabs)
+template <class T> struct LbwParams { const T *W, *dy, *x; T *dW; float *part; T *dx, *db; int out, in, rows_per_slab, slabs; };
+template <class T, int V> __device__ __forceinline__ void linear_bw_body(const LbwParams<T> &p)
 {
-    pdl_wait();
-    constexpr int V = 16 / sizeof(T);
+    const T *__restrict__ W = p.W, *__restrict__ dy = p.dy, *__restrict__ x = p.x;
+    T *__restrict__ dW = p.dW, *__restrict__ dx = p.dx, *__restrict__ db = p.db;
+    float *__restrict__ part = p.part;
+    const int out = p.out, in = p.in, rows_per_slab = p.rows_per_slab, slabs = p.slabs;
     __shared__ float red[LBW_LANES][LBW_STRIPS][V + 1];
     __shared__ unsigned ticket_s;
     const int cx = threadIdx.x % LBW_STRIPS, ry = threadIdx.x / LBW_STRIPS, slab = blockIdx.y;
     const int o_end = min(out, (slab + 1) * rows_per_slab);
     const int col0 = (blockIdx.x * LBW_STRIPS + cx) * V;
     const bool live = col0 < in;                                    // in % V == 0 (host): a strip is inside or outside as a whole
+    if (db && blockIdx.x == 0)
+        for (int o = slab * rows_per_slab + (int)threadIdx.x; o < o_end; o += LBW_STRIPS * LBW_LANES) db[o] = dy[o];
     float acc[V], xv[V];
 #pragma unroll
     for (int q = 0; q < V; q++) { acc[q] = 0.f; xv[q] = live ? ld(x + col0 + q) : 0.f; }
-    if (live) {
+    if (live && V <= 2) {
+        // narrow strips: the elements of sixteen rows are on their way before the first is used
+        constexpr int U = 16;
+        for (int o0 = slab * rows_per_slab + ry; o0 < o_end; o0 += U * LBW_LANES) {
+            T w[U][V];
+            float g[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int o = o0 + u * LBW_LANES;
+                const T *p = W + (long long)min(o, o_end - 1) * in + col0;
+                if constexpr (V == 2 && sizeof(T) == 2) *reinterpret_cast<__half2 *>(w[u]) = __ldcs(reinterpret_cast<const __half2 *>(p));
+                else w[u][0] = __ldcs(p);
+                g[u] = o < o_end ? ld(dy + o) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (o0 + u * LBW_LANES >= o_end) break;
+                T *d = dW + (long long)(o0 + u * LBW_LANES) * in + col0;
+#pragma unroll
+                for (int q = 0; q < V; q++) acc[q] = fmaf((float)w[u][q], g[u], acc[q]);
+                if constexpr (V == 2 && sizeof(T) == 2) __stcs(reinterpret_cast<__half2 *>(d), __floats2half2_rn(g[u] * xv[0], g[u] * xv[1]));
+                else st(d, g[u] * xv[0]);
+            }
+        }
+    }
+    if (live && V > 2) {
 #pragma unroll 8
         for (int o = slab * rows_per_slab + ry; o < o_end; o += LBW_LANES) {
             const float g = ld(dy + o);
             const long long e = (long long)o * in + col0;
-            if (sizeof(T) == 4) {
+            if constexpr (V <= 2) {
+            } else if constexpr (sizeof(T) == 4) {
                 const float4 w = __ldcs((const float4 *)(W + e));
                 acc[0] = fmaf(w.x, g, acc[0]); acc[1] = fmaf(w.y, g, acc[1]); acc[2] = fmaf(w.z, g, acc[2]); acc[3] = fmaf(w.w, g, acc[3]);
                 __stcs((float4 *)(dW + e), make_float4(g * xv[0], g * xv[1], g * xv[2], g * xv[3]));
@@ -502,11 +534,17 @@ __global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_fused_kernel
 #pragma unroll
     for (int q = 0; q < V; q++) t[q] = 0.f;
     if (live)
+#pragma unroll 8
         for (int b = ry; b < slabs; b += LBW_LANES)                 // lane r adds slabs r, r + 4, ...
+            if constexpr (V % 4 == 0) {
 #pragma unroll
-            for (int q = 0; q < V; q += 4) {
-                const float4 v = __ldcg((const float4 *)(part + (long long)b * in + col0 + q));
-                t[q] += v.x; t[q + 1] += v.y; t[q + 2] += v.z; t[q + 3] += v.w;
+                for (int q = 0; q < V; q += 4) {
+                    const float4 v = __ldcg((const float4 *)(part + (long long)b * in + col0 + q));
+                    t[q] += v.x; t[q + 1] += v.y; t[q + 2] += v.z; t[q + 3] += v.w;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < V; q++) t[q] += __ldcg(part + (long long)b * in + col0 + q);
             }
 #pragma unroll
     for (int q = 0; q < V; q++) red[ry][cx][q] = t[q];
@@ -518,13 +556,24 @@ __global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_fused_kernel
     if (threadIdx.x == 0) tl_linear_tickets[blockIdx.x] = 0;        // ready for the next launch on this device
 }
 
-// false: shape or alignment not covered (the caller issues the two separate kernels)
-template <class T> bool linear_bw_fused(Scope &sc, const T *W, const T *dy, const T *x, T *dW, T *dx, int out, int in)
+template <class T> __global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_fused_kernel(const __grid_constant__ LbwParams<T> p)
 {
-    constexpr int V = 16 / sizeof(T);
-    if (in % V != 0 || ((((uintptr_t)W) | ((uintptr_t)dW) | ((uintptr_t)x) | ((uintptr_t)dx)) & 15) != 0) return false;
+    pdl_wait();
+    linear_bw_body<T, 16 / sizeof(T)>(p);
+}
+template <class T, int V> __global__ void __launch_bounds__(LBW_STRIPS * LBW_LANES) linear_bw_narrow_kernel(const __grid_constant__ LbwParams<T> p)
+{
+    pdl_wait();
+    linear_bw_body<T, V>(p);
+}
+
+// false: the scratch for the slabs' partials could not be had (the error is set).  db: the bias gradient, or null
+template <class T> bool linear_bw_fused(Scope &sc, const T *W, const T *dy, const T *x, T *dW, T *dx, T *db, int out, int in)
+{
+    constexpr int V16 = 16 / sizeof(T);
+    const uintptr_t at = (uintptr_t)W | (uintptr_t)dW | (uintptr_t)x | (uintptr_t)dx;
+    const int V = in % V16 == 0 && at % 16 == 0 ? V16 : sizeof(T) == 2 && in % 2 == 0 && at % 4 == 0 ? 2 : 1;
     const int col_blocks = ceil_div(in / V, LBW_STRIPS);
-    if (col_blocks > 8192) return false;
     // about four CTAs per SM, at least 8 rows each
     int slabs = ceil_div(4 * sm_count(), col_blocks);
     if (slabs > ceil_div(out, 8)) slabs = ceil_div(out, 8);
@@ -533,11 +582,15 @@ template <class T> bool linear_bw_fused(Scope &sc, const T *W, const T *dy, cons
     slabs = ceil_div(out, rows_per_slab);
     float *part = sc.scratch<float>((size_t)slabs * in);
     if (!part) return false;
-    TL_LAUNCH((linear_bw_fused_kernel<T>), dim3(col_blocks, slabs), LBW_STRIPS * LBW_LANES, 0, W, dy, x, dW, part, dx, out, in, rows_per_slab, slabs);
+    const dim3 grid(col_blocks, slabs);
+    const LbwParams<T> p = {W, dy, x, dW, part, dx, db, out, in, rows_per_slab, slabs};
+    if (V == V16) TL_LAUNCH((linear_bw_fused_kernel<T>), grid, LBW_STRIPS * LBW_LANES, 0, p);
+    else if (V == 2) TL_LAUNCH((linear_bw_narrow_kernel<T, sizeof(T) == 2 ? 2 : 1>), grid, LBW_STRIPS * LBW_LANES, 0, p);
+    else TL_LAUNCH((linear_bw_narrow_kernel<T, 1>), grid, LBW_STRIPS * LBW_LANES, 0, p);
     return true;
 }
-template bool linear_bw_fused<float>(Scope &, const float *, const float *, const float *, float *, float *, int, int);
-template bool linear_bw_fused<__half>(Scope &, const __half *, const __half *, const __half *, __half *, __half *, int, int);
+template bool linear_bw_fused<float>(Scope &, const float *, const float *, const float *, float *, float *, float *, int, int);
+template bool linear_bw_fused<__half>(Scope &, const __half *, const __half *, const __half *, __half *, __half *, __half *, int, int);
 
 } // namespace tl
 

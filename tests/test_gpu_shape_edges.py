@@ -103,6 +103,17 @@ def test_products_of_host_arrays(pkg, gpulib, N, K, M):
     r.close()
 
 
+# both gradients and the bias gradient of one stream, rows that are no multiple of 16 bytes
+@pytest.mark.parametrize("inn,out", [(1, 1), (21, 1398), (1001, 70), (34, 3001), (3, 9000), (2050, 33)])
+def test_linear_rows_of_any_length(run, oracle, inn, out):
+    rng = seeded(inn + out)
+    W, x = rounded(run, rng.standard_normal((out, inn)) / np.sqrt(inn)), rounded(run, rng.standard_normal(inn))
+    dy, bias = rounded(run, rng.standard_normal(out)), rounded(run, rng.standard_normal(out))
+    want, got = oracle.linear(W, x, dy, bias), run.linear(W, x, dy, bias, one_backward_call=True)
+    for k in ("y", "dW", "dx", "db"):
+        assert_close(got[k].astype(F).reshape(want[k].shape), want[k], FP16_TOL if run.half else FP32_TOL, k)
+
+
 @pytest.mark.parametrize("rows,width", [(1, 1), (7, 33), (200, 128), (700, 250), (300, 512), (5, 1024), (9, 1500)])
 def test_layernorm_shapes(run, oracle, rows, width):
     rng = seeded(rows + width)
