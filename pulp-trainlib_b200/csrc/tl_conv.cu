@@ -983,7 +983,7 @@ __global__ void __launch_bounds__(256) conv_wg_direct_kernel(ConvGeom g, const T
 // 48 channels of 28 x 28 x 128 streams).  What bounds it is bytes in flight: a thread walks the pieces of all its CTA's planes,
 // eight 16-byte loads at a time where the planes allow (fp16, that size: 8.9 us element by element, 4.8 us so).
 template <class T, int V>
-__global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ dy, float *__restrict__ part, int n, int C, int plane)
+__global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ dy, float *__restrict__ part, T *__restrict__ db, int n, int C, int plane)
 {
     pdl_wait();
     __shared__ float red[33];
@@ -1016,7 +1016,8 @@ __global__ void __launch_bounds__(256) channel_sum_kernel(const T *__restrict__ 
         }
     }
     acc = block_sum(acc, red);
-    if (threadIdx.x == 0) part[(long long)blockIdx.y * C + c] = acc;
+    if (threadIdx.x != 0) return;
+    if (gridDim.y == 1) st(db + c, acc); else part[(long long)blockIdx.y * C + c] = acc;
 }
 template <class T> static void channel_sum(Scope &sc, const T *dy, T *db, int n, int C, int plane)
 {
@@ -1024,9 +1025,9 @@ template <class T> static void channel_sum(Scope &sc, const T *dy, T *db, int n,
     float *part = sc.scratch<float>((size_t)groups * C);
     if (!part) return;
     constexpr int V = 16 / (int)sizeof(T);
-    if (plane % V == 0 && ((uintptr_t)dy & 15) == 0) TL_LAUNCH((channel_sum_kernel<T, V>), dim3(C, groups), 256, 0, dy, part, n, C, plane);
-    else TL_LAUNCH((channel_sum_kernel<T, 1>), dim3(C, groups), 256, 0, dy, part, n, C, plane);
-    reduce_partials<T>(part, db, C, groups, false);
+    if (plane % V == 0 && ((uintptr_t)dy & 15) == 0) TL_LAUNCH((channel_sum_kernel<T, V>), dim3(C, groups), 256, 0, dy, part, db, n, C, plane);
+    else TL_LAUNCH((channel_sum_kernel<T, 1>), dim3(C, groups), 256, 0, dy, part, db, n, C, plane);
+    if (groups > 1) reduce_partials<T>(part, db, C, groups, false);           // (one group writes the sums itself)
 }
 
 // tensor-core weight gradient (tl_conv_wgt.cu) where its geometry applies and the work is large enough to fill the GPU
