@@ -745,17 +745,20 @@ template <class F> void sgd_impl(void *args)
     const float lr = F::f(a->learning_rate), lambda = F::f(a->weight_decay_lambda);
     if (ready()) defer_flush();                                   // the gradients read here may have their sums pending
     Scope sc;
-    {
-        const size_t n = (size_t)a->weights->dim;
-        T *w = sc.inout(a->weights->data, n);
-        T *g = lambda != 0.f ? sc.inout(a->weights->diff, n) : (T *)sc.in(a->weights->diff, n);
-        if (sc.ok()) sgd<T>(w, g, (long long)n, lr, lambda);
-    }
-    if (a->use_biases == 1 && a->biases) {
-        const size_t n = (size_t)a->biases->dim;
-        T *w = sc.inout(a->biases->data, n);
-        T *g = lambda != 0.f ? sc.inout(a->biases->diff, n) : (T *)sc.in(a->biases->diff, n);
-        if (sc.ok()) sgd<T>(w, g, (long long)n, lr, lambda);
+    auto map = [&](typename F::blob_t *b, SgdTensor<T> &t) {
+        t.n = b->dim;
+        t.w = sc.inout(b->data, (size_t)t.n);
+        t.g = lambda != 0.f ? sc.inout(b->diff, (size_t)t.n) : (T *)sc.in(b->diff, (size_t)t.n);
+        return sc.ok();
+    };
+    SgdTensor<T> w, b;
+    const bool both = a->use_biases == 1 && a->biases, w_ok = map(a->weights, w), b_ok = both && map(a->biases, b);
+    // one launch for both, unless they share memory (then the second update sees the first)
+    auto apart = [](const T *p, long long np, const T *q, long long nq) { return p + np <= q || q + nq <= p; };
+    if (w_ok && b_ok && apart(w.w, w.n, b.w, b.n) && apart(w.w, w.n, b.g, b.n) && apart(w.g, w.n, b.w, b.n) && apart(w.g, w.n, b.g, b.n)) sgd<T>(w, &b, lr, lambda);
+    else {
+        if (w_ok) sgd<T>(w, nullptr, lr, lambda);
+        if (b_ok) sgd<T>(b, nullptr, lr, lambda);
     }
 }
 template <class F> void residual_impl(void *args, int which)

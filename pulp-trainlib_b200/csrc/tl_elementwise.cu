@@ -1079,16 +1079,24 @@ template <class T> void ce_bw(const T *z, const T *t, T *dz, int dim, int n) { i
 // ------------------------------------------------------------------ SGD and vector ops
 // w -= lr*g; with weight decay the gradient is first replaced by g + lambda*w, as the reference
 // does in place [ref: lib/sources/pulp_optimizers_fp32.c:48-62].
-template <class T> __global__ void sgd_kernel(T *__restrict__ w, T *__restrict__ g, long long n, float lr, float lambda)
+// w -= lr * (g + lambda w); a second tensor (a layer's biases) rides in the same launch
+template <class T> __global__ void sgd_kernel(SgdTensor<T> a, SgdTensor<T> b, float lr, float lambda)
 {
     pdl_wait();
-    GRID_STRIDE(i, n) {
+    GRID_STRIDE(e, a.n + b.n) {
+        const bool second = e >= a.n;
+        T *w = second ? b.w : a.w, *g = second ? b.g : a.g;
+        const long long i = second ? e - a.n : e;
         float wv = ld(w + i), gv = ld(g + i);
         if (lambda != 0.f) { gv = __fadd_rn(gv, __fmul_rn(lambda, wv)); st(g + i, gv); }
         st(w + i, __fsub_rn(wv, __fmul_rn(lr, gv)));
     }
 }
-template <class T> void sgd(T *w, T *g, long long n, float lr, float lambda) { if (n > 0) TL_LAUNCH((sgd_kernel<T>), grid_for(n), 256, 0, w, g, n, lr, lambda); }
+template <class T> void sgd(const SgdTensor<T> &a, const SgdTensor<T> *b, float lr, float lambda)
+{
+    const SgdTensor<T> second = b ? *b : SgdTensor<T>{nullptr, nullptr, 0};
+    if (a.n + second.n > 0) TL_LAUNCH((sgd_kernel<T>), grid_for(a.n + second.n), 256, 0, a, second, lr, lambda);
+}
 
 template <class T> __global__ void add_kernel(const T *a, const T *b, T *c, long long n) { pdl_wait(); GRID_STRIDE(i, n) st(c + i, __fadd_rn(ld(a + i), ld(b + i))); }
 template <class T> void add(const T *a, const T *b, T *c, long long n) { if (n > 0) TL_LAUNCH((add_kernel<T>), grid_for(n), 256, 0, a, b, c, n); }
@@ -1333,7 +1341,7 @@ template <class T> void pad2d(const T *src, T *dst, int C, int H, int W, int pad
     template void mse_bw<T>(const T *, const T *, T *, int, int);                                                  \
     template void ce_fw<T>(const T *, const T *, T *, int, int);                                                   \
     template void ce_bw<T>(const T *, const T *, T *, int, int);                                                   \
-    template void sgd<T>(T *, T *, long long, float, float);                                                       \
+    template void sgd<T>(const SgdTensor<T> &, const SgdTensor<T> *, float, float);                                                       \
     template void add<T>(const T *, const T *, T *, long long);                                                    \
     template void copy_n<T>(const T *, T *, long long);                                                            \
     template void fill<T>(T *, float, long long);                                                                  \

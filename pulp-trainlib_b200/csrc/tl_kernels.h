@@ -187,7 +187,8 @@ template <class T> void mse_fw(const T *y, const T *t, T *loss, int dim, int n);
 template <class T> void mse_bw(const T *y, const T *t, T *dy, int dim, int n);
 template <class T> void ce_fw(const T *z, const T *t, T *loss, int dim, int n);
 template <class T> void ce_bw(const T *z, const T *t, T *dz, int dim, int n);
-template <class T> void sgd(T *w, T *g, long long n, float lr, float lambda);
+template <class T> struct SgdTensor { T *w, *g; long long n; };
+template <class T> void sgd(const SgdTensor<T> &a, const SgdTensor<T> *b, float lr, float lambda);       // b: a second tensor, or null
 template <class T> void add(const T *a, const T *b, T *c, long long n);
 template <class T> void copy_n(const T *from, T *to, long long n);
 template <class T> void fill(T *to, float v, long long n);
