@@ -27,6 +27,10 @@ struct Context {
     int scope_depth = 0;
     int live_graphs = 0;           // captured graphs hold arena addresses: while one lives (or is being recorded) no chunk is freed or merged
     bool capturing = false;
+    bool scratch_used = false;     // since the stream was last set: calls of two streams share the arena and the kernels' ticket counters
+    bool track_scratch = false;    // the caller has changed between streams of its own: every use of scratch is followed by an event
+    bool scratch_ev_set = false;
+    cudaEvent_t scratch_ev = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int err = TL_OK;
     bool cuda_sticky = false;      // the context is lost: TL_ERR_CUDA cannot be cleared
@@ -213,6 +217,7 @@ static void arena_release(size_t mark)
 
 static void *arena_alloc(size_t bytes)
 {
+    g.scratch_used = true;
     bytes = (bytes + 255) & ~(size_t)255;
     if (bytes == 0) bytes = 256;
     for (size_t i = g.chunks.empty() ? 0 : g.chunks.size() - 1; i < g.chunks.size(); i++) {
@@ -331,6 +336,15 @@ void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
     return d;
 }
 
+// A stream that is set while another one's calls may still be using scratch waits for them (set_stream).  The event is recorded
+// behind the calls, not when the stream changes: the caller may have destroyed the old stream by then.
+static void scratch_mark()
+{
+    if (!g.track_scratch || !g.scratch_used || g.capturing) return;
+    if (!g.scratch_ev && !TL_CUDA(cudaEventCreateWithFlags(&g.scratch_ev, cudaEventDisableTiming))) return;
+    g.scratch_ev_set = TL_CUDA(cudaEventRecord(g.scratch_ev, g.cur_stream));
+}
+
 Scope::~Scope()
 {
     if (staged_) {
@@ -347,7 +361,7 @@ Scope::~Scope()
         if (TL_CUDA(cudaStreamSynchronize(g.cur_stream)))
             for (auto &e : entries_) if (e.write_back && e.pinned) memcpy(e.host, e.pinned, e.bytes);
     }
-    g.scope_depth--;
+    if (--g.scope_depth == 0) scratch_mark();
     arena_release(arena_mark_);
     g_pinned_off = pinned_mark_;
 }
@@ -366,7 +380,22 @@ void trainlib_clear_error(void) { if (!(g.err == TL_ERR_CUDA && g.cuda_sticky) &
 
 int trainlib_init(int device) { return init_device(device); }
 int trainlib_device(void) { return g.device; }
-void trainlib_set_stream(void *s) { if (ready()) { defer_flush(); g.cur_stream = s ? (cudaStream_t)s : g.own_stream; } }
+void trainlib_set_stream(void *s)
+{
+    if (!ready()) return;
+    defer_flush();
+    const cudaStream_t to = s ? (cudaStream_t)s : g.own_stream;
+    if (to != g.cur_stream && !g.capturing) {
+        if (g.scratch_used && !g.track_scratch) {
+            if (g.cur_stream == g.own_stream) { g.track_scratch = true; scratch_mark(); g.track_scratch = false; }
+            else { TL_CUDA(cudaDeviceSynchronize()); g.scratch_ev_set = false; }       // once: from here on events follow the calls
+        }
+        if (g.cur_stream != g.own_stream) g.track_scratch = true;
+        if (g.scratch_ev_set) TL_CUDA(cudaStreamWaitEvent(to, g.scratch_ev, 0));
+        g.scratch_used = false;
+    }
+    g.cur_stream = to;
+}
 void *trainlib_stream(void) { return ready() ? (void *)g.cur_stream : nullptr; }
 static bool g_capturing_now();
 // A tensor-core kernel whose bounded wait gave up returns early and records the wait's id in a device word.  Every
@@ -501,6 +530,8 @@ int trainlib_graph_launch(void *handle)
     TlGraph *t = (TlGraph *)handle;
     if (!t) { set_error(TL_ERR_BAD_ARGS, "trainlib_graph_launch: null graph"); return TL_ERR_BAD_ARGS; }
     if (!TL_CUDA(cudaGraphLaunch(t->exec, g.cur_stream))) return g.err;
+    g.scratch_used = true;
+    scratch_mark();
     g.launches += t->kernels;
     return TL_OK;
 }

@@ -114,6 +114,30 @@ def test_linear_rows_of_any_length(run, oracle, inn, out):
         assert_close(got[k].astype(F).reshape(want[k].shape), want[k], FP16_TOL if run.half else FP32_TOL, k)
 
 
+def test_products_alternating_between_streams(run):
+    """split contractions use scratch and counters of the library: calls of two streams, never synchronised in between"""
+    import torch
+    N, K, M = 16, 2048, 300
+    rng = seeded(5)
+    mats = [(rounded(run, rng.standard_normal((N, K)) / np.sqrt(K)), rounded(run, rng.standard_normal((K, M)))) for _ in range(8)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    args, outs = [], []
+    for A, B in mats:
+        a, b, c = run.t(A), run.t(B), run.zeros(N, M)
+        args.append(run.args(run.sname("matMul_args"), A=a, B=b, C=c, N=N, K=K, M=M, trans_B=0, USE_BIASES=0)); outs.append(c)
+    torch.cuda.synchronize()
+    try:
+        for rep in range(5):
+            for i, a in enumerate(args):
+                run.lib.trainlib_set_stream(streams[i % 2].cuda_stream)
+                run.call("mm_fp16" if run.half else "mm", a)
+        torch.cuda.synchronize()
+    finally:
+        run.lib.trainlib_set_stream(None)
+    for (A, B), c in zip(mats, outs):
+        assert_close(c.get().astype(F), (A.astype(np.float64) @ B.astype(np.float64)).astype(F), FP16_TOL if run.half else FP32_TOL, "mm")
+
+
 @pytest.mark.parametrize("rows,width", [(1, 1), (7, 33), (200, 128), (700, 250), (300, 512), (5, 1024), (9, 1500)])
 def test_layernorm_shapes(run, oracle, rows, width):
     rng = seeded(rows + width)
