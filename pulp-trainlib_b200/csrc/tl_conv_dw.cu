@@ -10,6 +10,11 @@
 
 namespace tl {
 
+// A launch gets 48 KB of shared memory without asking, and the kernel's static arrays count: up to 800 bytes here (the sums of 25
+// taps over eight warps).  Above this the limit is raised for the kernel first.
+static constexpr size_t DW_DEFAULT_SMEM = 48 * 1024 - 8 * 25 * sizeof(float);
+template <class K> static void dw_allow(K kernel, size_t smem) { if (smem > DW_DEFAULT_SMEM) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }
+
 struct DwDiv { uint32_t m; int d; };
 static DwDiv dw_div(int d) { DwDiv r; r.d = d; r.m = d == 1 ? 0u : 0xFFFFFFFFu / (uint32_t)d + 1u; return r; }
 __device__ __forceinline__ int dw_quot(int n, DwDiv d) { return d.m ? (int)__umulhi((uint32_t)n, d.m) : n; }
@@ -255,7 +260,7 @@ static bool dw3_params(const ConvGeom &g, Dw3Params &p, const void *src, const v
     if (p.padU < 0 || p.padL < 0 || p.padL > 2 || p.padU > 2 || (long long)g.n * g.Cin >= (1ll << 31)) return false;
     p.PH = std::max(p.Ho + 2, p.Hs + p.padU); p.O4 = ceil_div(p.Wo, 4); p.W4 = p.Ws / 4;
     p.PW = std::max(4 * p.O4 + 12, 4 + (p.Ws + 3) / 4 * 4);
-    if ((long long)p.PH * p.PW > 12 * 1024) return false;                  // 48 KB of shared memory
+    if ((long long)p.PH * p.PW > 12 * 1024) return false;                  // 48 KB of planes
     p.vec_s = p.Ws % 4 == 0 && ((uintptr_t)src) % (4 * esize) == 0; p.vec_o = p.Wo % 4 == 0 && ((uintptr_t)dst) % (4 * esize) == 0;
     p.dW4 = dw_div(std::max(1, p.W4)); p.dWs = dw_div(p.Ws); p.dRow = dw_div(p.vec_s ? p.Hs * p.W4 : p.Hs * p.Ws); p.dO4 = dw_div(p.Ho * p.O4);
     return true;
@@ -301,10 +306,10 @@ template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T
     while (p.G > 1 && (size_t)p.G * (P + KK) * 4 > 48 * 1024) p.G--;
     const size_t smem = (size_t)p.G * (P + KK) * 4;
     const int grid = ceil_div(p.planes, p.G);
-#define TL_DW(KV)                                                                                                                   \
-    do {                                                                                                                            \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(dw_plane_kernel<T, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        TL_LAUNCH((dw_plane_kernel<T, KV>), grid, 256, smem, p, src, w, dst);                                                       \
+#define TL_DW(KV)                                                             \
+    do {                                                                      \
+        dw_allow(dw_plane_kernel<T, KV>, smem);                               \
+        TL_LAUNCH((dw_plane_kernel<T, KV>), grid, 256, smem, p, src, w, dst); \
     } while (0)
     if (g.Hk == 3 && g.Wk == 3) TL_DW(3); else if (g.Hk == 5 && g.Wk == 5) TL_DW(5); else TL_DW(0);
 #undef TL_DW
@@ -322,9 +327,13 @@ template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy,
         while (q.G > 1 && (size_t)q.G * q.PH * q.PW * 4 > 24 * 1024) q.G--;
         const size_t smem = (size_t)q.G * q.PH * q.PW * 4;
         const dim3 grid(g.Cin, groups);
-        if (q.padL == 1) TL_LAUNCH((dw3_wg_kernel<T, 1>), grid, 128, smem, q, x, dy, part, g.n);
-        else if (q.padL == 0) TL_LAUNCH((dw3_wg_kernel<T, 0>), grid, 128, smem, q, x, dy, part, g.n);
-        else TL_LAUNCH((dw3_wg_kernel<T, 2>), grid, 128, smem, q, x, dy, part, g.n);
+#define TL_DW(PADL)                                                                \
+    do {                                                                           \
+        dw_allow(dw3_wg_kernel<T, PADL>, smem);                                    \
+        TL_LAUNCH((dw3_wg_kernel<T, PADL>), grid, 128, smem, q, x, dy, part, g.n); \
+    } while (0)
+        if (q.padL == 1) TL_DW(1); else if (q.padL == 0) TL_DW(0); else TL_DW(2);
+#undef TL_DW
         return true;
     }
     DwParams p;
@@ -337,10 +346,10 @@ template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy,
     while (p.G > 1 && (size_t)p.G * P * 4 > 48 * 1024) p.G--;
     const size_t smem = (size_t)p.G * P * 4;
     const dim3 grid(g.Cin, groups);
-#define TL_DW(KV)                                                                                                                      \
-    do {                                                                                                                               \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(dw_wg_plane_kernel<T, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        TL_LAUNCH((dw_wg_plane_kernel<T, KV>), grid, 256, smem, p, x, dy, part, g.n);                                                  \
+#define TL_DW(KV)                                                                     \
+    do {                                                                              \
+        dw_allow(dw_wg_plane_kernel<T, KV>, smem);                                    \
+        TL_LAUNCH((dw_wg_plane_kernel<T, KV>), grid, 256, smem, p, x, dy, part, g.n); \
     } while (0)
     if (g.Hk == 3) TL_DW(3); else TL_DW(5);
 #undef TL_DW

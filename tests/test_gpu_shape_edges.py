@@ -55,15 +55,15 @@ def test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n):
 
 
 @pytest.mark.parametrize("c,h,w,k,pad,n", [(5, 9, 7, 3, 1, 3), (64, 28, 28, 3, 1, 4), (3, 33, 18, 3, 0, 2), (8, 6, 6, 5, 2, 9), (2, 40, 41, 3, 2, 1), (7, 4, 4, 3, 1, 700), (4, 12, 12, 4, 1, 2)])
-def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n):
-    g = geom(c, h, w, c, k, pad=pad)
+def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
+    g = geom(c, h, w, c, k, stride=stride, pad=pad)
     Ho, Wo = out_hw(g)
     rng = seeded(c + h + w + n)
     x, wt, dy = rounded(run, rng.standard_normal((n, c, h, w))), rounded(run, rng.standard_normal((c, k, k)) / k), rounded(run, rng.standard_normal((n, c, Ho, Wo)) / 4)
     run.lib.trainlib_set_streams(n)
     X, W_, dY = run.t(x), run.t(wt), run.t(dy)
     Y, dX, dW = run.zeros(n, c, Ho, Wo), run.zeros(*x.shape), run.zeros(*wt.shape)
-    fields = {} if run.half else dict(stride_h=1, stride_w=1)
+    fields = {} if run.half else dict(stride_h=stride, stride_w=stride)
     a = run.args(run.sname("DepthWise_Conv_args"), input=run.blob(X, dX, C=c, H=h, W=w), coeff=run.blob(W_, dW, C=c, H=k, W=k), output=run.blob(Y, dY, C=c, H=Ho, W=Wo),
                  Lpad=pad, Rpad=pad, Upad=pad, Dpad=pad, skip_wg_grad=0, skip_in_grad=0, HWC=0, **fields)
     run.call(run.fname("pulp_conv_dw_fp32_fw_cl"), a); run.call(run.fname("pulp_conv_dw_fp32_bw_cl"), a)
@@ -74,6 +74,17 @@ def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n):
         assert_close(dx[s], oracle.dw_ig(dy[s], wt, g), tol, "ig stream %d" % s)
     want = sum(oracle.dw_wg(x[s], dy[s], g).astype(np.float64) for s in range(n)).astype(F)
     assert_close(dW.get().astype(F), want, tol, "wg")
+
+
+# Planes whose staged windows come to just below, exactly and just above the 48 KB that a launch gets without asking: the weight
+# gradients keep static arrays beside them.  Floats staged: 3x3 with pad 1 11 880, 12 276, 12 288, 11 446 (past that kernel's own
+# limit), with pad 0 and 2 12 288; 5x5 11 881, 12 100, 12 544; stride 2 (fp32 only) 12 285, 12 519.
+@pytest.mark.parametrize("c,h,w,k,pad,stride,n", [(2, 97, 108, 3, 1, 1, 2), (2, 97, 112, 3, 1, 1, 2), (3, 94, 116, 3, 1, 1, 3), (2, 95, 116, 3, 1, 1, 1), (2, 96, 118, 3, 0, 1, 2), (2, 92, 114, 3, 2, 1, 2),
+                                                  (2, 105, 105, 5, 2, 1, 2), (3, 106, 106, 5, 2, 1, 2), (2, 108, 108, 5, 2, 1, 1), (2, 104, 115, 3, 1, 2, 2), (2, 106, 115, 3, 1, 2, 2)])
+def test_depthwise_planes_at_the_shared_memory_limit(run, oracle, c, h, w, k, pad, stride, n):
+    if run.half and stride != 1:
+        pytest.skip("the fp16 argument struct has no stride")
+    test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride)
 
 
 @pytest.mark.parametrize("N,K,M", [(1, 1, 1), (17, 3001, 41), (16, 2048, 300), (33, 64, 31), (130, 7, 130), (64, 129, 65), (500, 40, 333), (1000, 60, 520), (128, 512, 128)])
