@@ -31,7 +31,9 @@ void        trainlib_clear_error(void);
  * so call order is execution order.  trainlib_init is implicit in every entry point. */
 int   trainlib_init(int device);              /* returns TL_OK or an error code */
 int   trainlib_device(void);
-void  trainlib_set_stream(void *cuda_stream); /* NULL = the library's own stream */
+void  trainlib_set_stream(void *cuda_stream); /* NULL = the library's own stream.  Library scratch is shared: what is queued on the new
+                                               * stream waits for the calls of the one before where both use it.  Pending deferred
+                                               * sums run on the stream before: it must still exist. */
 void *trainlib_stream(void);
 void  trainlib_synchronize(void);
 

@@ -120,6 +120,8 @@ private:
 bool is_device_pointer(const void *p);
 bool arena_pinned();                // a captured graph holds addresses of library-owned device memory: it must stay where it is
 bool capturing();                   // between trainlib_graph_begin and _end
+void scratch_touch();               // library-owned memory that calls of two streams share is in use on the current stream
+void scratch_mark();                // behind such a use: what a stream set later waits for
 
 // deferred reductions (tl_defer.cu): partial results kept until one batched launch sums them all
 bool defer_enabled();

@@ -112,6 +112,8 @@ void defer_flush()
     if (d.batch.count > 0) {
         TL_LAUNCH(deferred_reduce_kernel, d.batch.ctas, 1024, 0, d.batch);
         d.batch.count = 0; d.batch.ctas = 0;
+        scratch_touch();
+        scratch_mark();                                             // no Scope need follow: the stream may change next
     }
     // Grow to what the last epoch asked for.  Captured graphs may hold addresses inside the old block: it is then kept beside the
     // new one until the last graph is destroyed.  (A graph of a small network used to freeze the arena at its size, and every
@@ -147,6 +149,7 @@ float *defer_alloc(size_t floats)
     if (d.off + bytes > d.cap) return nullptr;
     float *p = reinterpret_cast<float *>(d.base + d.off);
     d.off += bytes;
+    scratch_touch();
     return p;
 }
 

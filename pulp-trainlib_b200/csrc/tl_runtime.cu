@@ -27,7 +27,7 @@ struct Context {
     int scope_depth = 0;
     int live_graphs = 0;           // captured graphs hold arena addresses: while one lives (or is being recorded) no chunk is freed or merged
     bool capturing = false;
-    bool scratch_used = false;     // since the stream was last set: calls of two streams share the arena and the kernels' ticket counters
+    bool scratch_used = false;     // since the stream was last set: calls of two streams share the arenas (staging, deferred sums) and the kernels' ticket counters
     bool track_scratch = false;    // the caller has changed between streams of its own: every use of scratch is followed by an event
     bool scratch_ev_set = false;
     cudaEvent_t scratch_ev = nullptr;
@@ -217,7 +217,7 @@ static void arena_release(size_t mark)
 
 static void *arena_alloc(size_t bytes)
 {
-    g.scratch_used = true;
+    scratch_touch();
     bytes = (bytes + 255) & ~(size_t)255;
     if (bytes == 0) bytes = 256;
     for (size_t i = g.chunks.empty() ? 0 : g.chunks.size() - 1; i < g.chunks.size(); i++) {
@@ -337,8 +337,10 @@ void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
 }
 
 // A stream that is set while another one's calls may still be using scratch waits for them (set_stream).  The event is recorded
-// behind the calls, not when the stream changes: the caller may have destroyed the old stream by then.
-static void scratch_mark()
+// behind the calls (and behind the batched sum of deferred ones), not when the stream changes: the caller may have destroyed the
+// old stream by then.
+void scratch_touch() { g.scratch_used = true; }
+void scratch_mark()
 {
     if (!g.track_scratch || !g.scratch_used || g.capturing) return;
     if (!g.scratch_ev && !TL_CUDA(cudaEventCreateWithFlags(&g.scratch_ev, cudaEventDisableTiming))) return;
@@ -383,7 +385,7 @@ int trainlib_device(void) { return g.device; }
 void trainlib_set_stream(void *s)
 {
     if (!ready()) return;
-    defer_flush();
+    defer_flush();                                  // on the stream that holds the partial results; `to` waits for it like for any use of scratch
     const cudaStream_t to = s ? (cudaStream_t)s : g.own_stream;
     if (to != g.cur_stream && !g.capturing) {
         if (g.scratch_used && !g.track_scratch) {
@@ -530,7 +532,7 @@ int trainlib_graph_launch(void *handle)
     TlGraph *t = (TlGraph *)handle;
     if (!t) { set_error(TL_ERR_BAD_ARGS, "trainlib_graph_launch: null graph"); return TL_ERR_BAD_ARGS; }
     if (!TL_CUDA(cudaGraphLaunch(t->exec, g.cur_stream))) return g.err;
-    g.scratch_used = true;
+    scratch_touch();
     scratch_mark();
     g.launches += t->kernels;
     return TL_OK;

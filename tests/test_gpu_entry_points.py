@@ -506,3 +506,63 @@ def test_deferred_reductions_give_the_same_bits_in_one_launch(pkg, gpulib):
     for k, (a, b) in enumerate(zip(results[0], results[1])):
         assert np.abs(a).max() > 0 and np.array_equal(a, b), "deferred and immediate sums differ: output %d, %d of %d elements, max |a| %g, max |a - b| %g" % (
             k, int((a != b).sum()), a.size, float(np.abs(a).max()), float(np.abs(a - b).max()))
+
+
+def weight_gradient_calls(r, cases, seed):
+    """Conv2D weight-gradient calls over streams of their own inputs: [(streams, args)], [dW]"""
+    calls, outs = [], []
+    for k, (g, n) in enumerate(cases):
+        Ho, Wo = out_hw(g)
+        rs = np.random.default_rng(seed + k)
+        X, dY = r.t(rs.uniform(-1, 1, (n, g["Cin"], g["Hin"], g["Win"]))), r.t(rs.standard_normal((n, g["Cout"], Ho, Wo)))
+        dW, one = r.zeros(g["Cout"], g["Cin"], g["Hk"], g["Wk"]), r.zeros(1)
+        calls.append((n, r.args("Conv2D_args", input=r.blob(X, one, C=g["Cin"], H=g["Hin"], W=g["Win"]), coeff=r.blob(one, dW, C=g["Cin"], H=g["Hk"], W=g["Wk"], dim=g["Cout"] * g["Cin"] * g["Hk"] * g["Wk"]),
+                                bias=r.blob(one, one), output=r.blob(one, dY, C=g["Cout"], H=Ho, W=Wo), Lpad=g["padL"], Rpad=g["padR"], Upad=g["padU"], Dpad=g["padD"],
+                                stride_h=g["sh"], stride_w=g["sw"], i2c_buffer=one, bt_buffer=one, USE_BIASES=0, USE_IM2COL=1, HWC=0)))
+        outs.append(dW)
+    return calls, outs
+
+
+@pytest.mark.gpu
+def test_deferred_reductions_alternating_between_streams(pkg, gpulib):
+    """The arena of deferred sums is shared between streams: a call on the new stream writes its partial results where the old
+    one's batched sum, still waiting behind a delay, has yet to read"""
+    import torch
+    r = AbiRunner(pkg, gpulib, device=True)
+    calls, outs = weight_gradient_calls(r, [(geom(16, 32, 32, 16, 3, pad=1), 40), (geom(32, 16, 16, 32, 3, pad=1), 300), (geom(16, 16, 16, 16, 3, pad=1), 50)], 31)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def run(i):
+        gpulib.trainlib_set_streams(calls[i][0]); r.call("pulp_conv2d_fp32_bw_param_grads_cl", calls[i][1])
+    try:
+        for i in range(len(calls)):
+            run(i)
+        want = [o.get().copy() for o in outs]
+        gpulib.trainlib_set_deferred_reductions(1)
+        for i in range(len(calls)):                 # sizes the arena
+            run(i)
+        gpulib.trainlib_flush_reductions()
+        before = gpulib.trainlib_kernel_launches()
+        run(0)
+        assert gpulib.trainlib_kernel_launches() - before == 1, "the sum was not deferred"
+        gpulib.trainlib_flush_reductions()
+        for o in outs:
+            gpulib.trainlib_memset(o.dev.ptr, 0, o.dev.nbytes)
+        gpulib.trainlib_synchronize()
+        for rep in range(3):
+            for flush in (False, True):             # summed by the change of stream / by a call of its own before it
+                for i in range(len(calls)):
+                    s = streams[i % 2]
+                    gpulib.trainlib_set_stream(s.cuda_stream)
+                    run(i)
+                    with torch.cuda.stream(s):
+                        torch.cuda._sleep(4000000)  # about two milliseconds
+                    if flush:
+                        gpulib.trainlib_flush_reductions()
+            gpulib.trainlib_set_stream(None)
+            torch.cuda.synchronize()
+            for k, (o, w) in enumerate(zip(outs, want)):
+                assert np.array_equal(o.get(), w), "repetition %d, layer %d" % (rep, k)
+    finally:
+        gpulib.trainlib_set_stream(None); gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
+        r.close()
