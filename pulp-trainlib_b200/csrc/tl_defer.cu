@@ -6,8 +6,8 @@
 // trainlib_set_deferred_reductions(1) the library keeps the partial results of device-resident calls in an arena of its
 // own, notes what is to be summed into which gradient, and runs ALL pending sums as one launch
 //   - when an entry point that reads gradients is called (pulp_gradient_descent_*), on trainlib_synchronize(),
-//     trainlib_memcpy_d2h(), trainlib_graph_end(), trainlib_set_stream(), when the mode is switched off, when the arena or
-//     the job table is full, and
+//     trainlib_memcpy_d2h(), trainlib_timer_stop_ms(), trainlib_graph_begin(), _end() and _launch(), trainlib_set_stream(),
+//     when the mode is switched off, when the job table is full, and
 //   - on trainlib_flush_reductions(), which a caller must issue before anything outside the library (a collective,
 //     its own kernels) reads a gradient.
 // Until then the gradient buffers named by the deferred calls do not hold their values: that is the contract of the

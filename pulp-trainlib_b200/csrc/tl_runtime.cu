@@ -531,6 +531,7 @@ int trainlib_graph_launch(void *handle)
     if (!ready()) return g.err;
     TlGraph *t = (TlGraph *)handle;
     if (!t) { set_error(TL_ERR_BAD_ARGS, "trainlib_graph_launch: null graph"); return TL_ERR_BAD_ARGS; }
+    defer_flush();                                  // the recorded calls may keep partial results where the pending sums have theirs
     if (!TL_CUDA(cudaGraphLaunch(t->exec, g.cur_stream))) return g.err;
     scratch_touch();
     scratch_mark();

@@ -566,3 +566,40 @@ def test_deferred_reductions_alternating_between_streams(pkg, gpulib):
     finally:
         gpulib.trainlib_set_stream(None); gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
         r.close()
+
+
+@pytest.mark.gpu
+def test_a_replay_leaves_pending_deferred_sums_alone(pkg, gpulib):
+    """a graph recorded with deferred sums keeps its partial results where calls outside it keep theirs: what is pending when it
+    is launched must have been summed by then"""
+    r = AbiRunner(pkg, gpulib, device=True)
+    calls, outs = weight_gradient_calls(r, [(geom(16, 32, 32, 16, 3, pad=1), 40), (geom(16, 16, 16, 16, 3, pad=1), 50)], 41)
+    graph = None
+
+    def run(i):
+        gpulib.trainlib_set_streams(calls[i][0]); r.call("pulp_conv2d_fp32_bw_param_grads_cl", calls[i][1])
+    try:
+        for i in range(2):
+            run(i)
+        want = [o.get().copy() for o in outs]
+        gpulib.trainlib_set_deferred_reductions(1)
+        for rep in range(2):                        # the first pass sizes the arena
+            for i in range(2):
+                run(i)
+            gpulib.trainlib_flush_reductions()
+        gpulib.trainlib_graph_begin()
+        run(1)
+        graph = gpulib.trainlib_graph_end()
+        assert graph
+        for o in outs:
+            gpulib.trainlib_memset(o.dev.ptr, 0, o.dev.nbytes)
+        run(0)                                      # pending
+        assert gpulib.trainlib_graph_launch(graph) == 0
+        gpulib.trainlib_flush_reductions()
+        for k, (o, w) in enumerate(zip(outs, want)):
+            assert np.array_equal(o.get(), w), "layer %d" % k
+    finally:
+        gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
+        if graph:
+            gpulib.trainlib_graph_destroy(graph)
+        r.close()
