@@ -129,6 +129,7 @@ float *defer_alloc(size_t floats);
 void defer_plain(const float *part, float *out, long long n, int groups);
 void defer_columns(const float *part, float *out, int rows, int dim, int pairs);
 void defer_wgt(const float *part, float *out, int groups, long long group_floats, int Cin, int Cout, int s2, int xg, int cigs, int ncopy);
+void defer_settle(const void *out); // before a gradient is written again: its pending sum, if there is one, runs first
 void defer_flush();
 void defer_release();               // the last captured graph is gone
 

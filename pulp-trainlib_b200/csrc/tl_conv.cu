@@ -1102,6 +1102,7 @@ template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T 
 
 template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw, T *dbias)
 {
+    defer_settle(dw);
     if (dbias) channel_sum<T>(sc, dy, dbias, g.n, g.Cout, g.Hout * g.Wout);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise) {

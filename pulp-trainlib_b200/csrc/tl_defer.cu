@@ -106,15 +106,27 @@ __global__ void __launch_bounds__(1024) deferred_reduce_kernel(const __grid_cons
 
 bool defer_enabled() { return d.on; }
 
-// all pending sums as one launch; the arena is free again afterwards (stream order: what follows runs after the sums)
+// all pending sums as one launch
+static void run_pending()
+{
+    if (d.batch.count == 0) return;
+    TL_LAUNCH(deferred_reduce_kernel, d.batch.ctas, 1024, 0, d.batch);
+    d.batch.count = 0; d.batch.ctas = 0;
+    scratch_touch();
+    scratch_mark();                                                 // no Scope need follow: the stream may change next
+}
+
+// The jobs of one launch run side by side and later than sums that are taken at once, so a gradient has one pending sum at most.
+void defer_settle(const void *out)
+{
+    for (int j = 0; j < d.batch.count; j++)
+        if (d.batch.job[j].out == out) { run_pending(); return; }
+}
+
+// the pending sums, after which the arena is free again (stream order: what follows runs after the sums)
 void defer_flush()
 {
-    if (d.batch.count > 0) {
-        TL_LAUNCH(deferred_reduce_kernel, d.batch.ctas, 1024, 0, d.batch);
-        d.batch.count = 0; d.batch.ctas = 0;
-        scratch_touch();
-        scratch_mark();                                             // no Scope need follow: the stream may change next
-    }
+    run_pending();
     // Grow to what the last epoch asked for.  Captured graphs may hold addresses inside the old block: it is then kept beside the
     // new one until the last graph is destroyed.  (A graph of a small network used to freeze the arena at its size, and every
     // later sum of a larger one ran at once: 25 launches and 100 us of a 4096-stream step.)

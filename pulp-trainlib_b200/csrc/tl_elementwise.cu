@@ -684,6 +684,7 @@ template <class T>
 void instnorm_bw_param(Scope &sc, const T *x, const T *dy, T *dgb, const T *mean, const T *stdev, int n, int C, int D)
 {
     if (n * C <= 0) return;
+    defer_settle(dgb);
     bool deferred;
     float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
     if (!part) return;
@@ -696,6 +697,7 @@ template <class T>
 void instnorm_bw_both(Scope &sc, const T *x, const T *dy, T *dx, T *dgb, const T *gamma, const T *mean, const T *var, const T *stdev, int n, int C, int D)
 {
     if (n * C <= 0) return;
+    defer_settle(dgb);
     bool deferred;
     float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
     if (!part) return;
@@ -726,6 +728,7 @@ void instnorm_relu_bw(Scope &sc, const T *x, const T *y, T *dy, const T *dy2, T 
                       int n, int C, int D)
 {
     if (n * C <= 0) return;
+    defer_settle(dgb);
     bool deferred;
     float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
     if (!part) return;

@@ -508,14 +508,14 @@ def test_deferred_reductions_give_the_same_bits_in_one_launch(pkg, gpulib):
             k, int((a != b).sum()), a.size, float(np.abs(a).max()), float(np.abs(a - b).max()))
 
 
-def weight_gradient_calls(r, cases, seed):
-    """Conv2D weight-gradient calls over streams of their own inputs: [(streams, args)], [dW]"""
+def weight_gradient_calls(r, cases, seed, one_gradient=False):
+    """Conv2D weight-gradient calls on inputs of their own: [(streams, args)], [dW]; one_gradient: all write the first one's dW"""
     calls, outs = [], []
     for k, (g, n) in enumerate(cases):
         Ho, Wo = out_hw(g)
         rs = np.random.default_rng(seed + k)
         X, dY = r.t(rs.uniform(-1, 1, (n, g["Cin"], g["Hin"], g["Win"]))), r.t(rs.standard_normal((n, g["Cout"], Ho, Wo)))
-        dW, one = r.zeros(g["Cout"], g["Cin"], g["Hk"], g["Wk"]), r.zeros(1)
+        dW, one = outs[0] if one_gradient and outs else r.zeros(g["Cout"], g["Cin"], g["Hk"], g["Wk"]), r.zeros(1)
         calls.append((n, r.args("Conv2D_args", input=r.blob(X, one, C=g["Cin"], H=g["Hin"], W=g["Win"]), coeff=r.blob(one, dW, C=g["Cin"], H=g["Hk"], W=g["Wk"], dim=g["Cout"] * g["Cin"] * g["Hk"] * g["Wk"]),
                                 bias=r.blob(one, one), output=r.blob(one, dY, C=g["Cout"], H=Ho, W=Wo), Lpad=g["padL"], Rpad=g["padR"], Upad=g["padU"], Dpad=g["padD"],
                                 stride_h=g["sh"], stride_w=g["sw"], i2c_buffer=one, bt_buffer=one, USE_BIASES=0, USE_IM2COL=1, HWC=0)))
@@ -602,4 +602,30 @@ def test_a_replay_leaves_pending_deferred_sums_alone(pkg, gpulib):
         gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
         if graph:
             gpulib.trainlib_graph_destroy(graph)
+        r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("streams", [(1, 300), (40, 41)], ids=["second_sums_at_once", "both_deferred"])
+def test_a_gradient_written_twice_before_the_flush_holds_the_last_value(pkg, gpulib, streams):
+    """two calls into one gradient buffer with the first one's sum pending; with 1 and 300 streams (in a process whose arena has not
+    grown otherwise) the second one's partial results do not fit the arena and are summed at once"""
+    r = AbiRunner(pkg, gpulib, device=True)
+    calls, outs = weight_gradient_calls(r, [(geom(16, 32, 32, 16, 3, pad=1), n) for n in streams], 51, one_gradient=True)
+
+    def run(i):
+        gpulib.trainlib_set_streams(calls[i][0]); r.call("pulp_conv2d_fp32_bw_param_grads_cl", calls[i][1])
+    try:
+        run(1)
+        want = outs[0].get().copy()
+        gpulib.trainlib_set_deferred_reductions(1)
+        for rep in range(2):
+            run(0)
+            gpulib.trainlib_flush_reductions()
+        run(0)
+        run(1)
+        gpulib.trainlib_flush_reductions()
+        assert np.array_equal(outs[0].get(), want)
+    finally:
+        gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
         r.close()
