@@ -423,7 +423,13 @@ void *trainlib_malloc(size_t bytes)
     if (!TL_CUDA(cudaMalloc(&p, bytes ? bytes : 256))) return nullptr;
     return p;
 }
-void trainlib_free(void *p) { if (p && ready()) { cudaStreamSynchronize(g.cur_stream); TL_CUDA(cudaFree(p)); } }
+void trainlib_free(void *p)
+{
+    if (!p || !ready()) return;
+    defer_flush();                                  // a pending sum may write this buffer
+    cudaStreamSynchronize(g.cur_stream);
+    TL_CUDA(cudaFree(p));
+}
 void *trainlib_malloc_host(size_t bytes)
 {
     if (!ready()) return nullptr;

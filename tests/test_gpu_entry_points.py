@@ -629,3 +629,27 @@ def test_a_gradient_written_twice_before_the_flush_holds_the_last_value(pkg, gpu
     finally:
         gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
         r.close()
+
+
+@pytest.mark.gpu
+def test_freeing_a_gradient_with_its_sum_pending(pkg, gpulib):
+    """trainlib_free runs pending sums first: one of them may write the buffer that goes"""
+    r = AbiRunner(pkg, gpulib, device=True)
+    calls, outs = weight_gradient_calls(r, [(geom(16, 32, 32, 16, 3, pad=1), 40)], 61)
+    other = pkg.DeviceBuffer(gpulib, nbytes=4096)
+    try:
+        gpulib.trainlib_set_deferred_reductions(1)
+        gpulib.trainlib_set_streams(calls[0][0])
+        for rep in range(2):                        # the first pass sizes the arena
+            r.call("pulp_conv2d_fp32_bw_param_grads_cl", calls[0][1])
+            gpulib.trainlib_flush_reductions()
+        r.call("pulp_conv2d_fp32_bw_param_grads_cl", calls[0][1])
+        before = gpulib.trainlib_kernel_launches()
+        other.free()
+        assert gpulib.trainlib_kernel_launches() - before == 1
+        gpulib.trainlib_flush_reductions()
+        assert gpulib.trainlib_kernel_launches() - before == 1
+        pkg.check(gpulib)
+    finally:
+        gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
+        r.close()
