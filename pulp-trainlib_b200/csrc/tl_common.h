@@ -98,7 +98,9 @@ public:
     template <class T> const T *in(const T *p, size_t n) { return (const T *)map((void *)p, n * sizeof(T), true, false); }
     template <class T> T *out(T *p, size_t n) { return (T *)map((void *)p, n * sizeof(T), false, true); }
     template <class T> T *inout(T *p, size_t n) { return (T *)map((void *)p, n * sizeof(T), true, true); }
-    template <class T> T *scratch(size_t n) { return (T *)alloc(n * sizeof(T)); }   // device-only temporary
+    template <class T> T *scratch(size_t n) { return (T *)alloc(n * sizeof(T), true); }   // device-only temporary
+    // the same for a path that has another one to fall back on: no memory is no error
+    template <class T> T *try_scratch(size_t n) { return (T *)alloc(n * sizeof(T), false); }
     bool ok() const { return ok_; }
     bool staged() const { return staged_; }   // some buffer of this call lives in host memory (mirrored in the arena)
     // a reduction of this call may be deferred: every buffer is the caller's own device memory and the call does not go
@@ -109,7 +111,7 @@ private:
     struct Entry { void *host; void *dev; void *pinned; size_t bytes; bool write_back; bool copied_in; };
     bool upload(Entry &e);
     void *map(void *p, size_t bytes, bool copy_in, bool copy_out);
-    void *alloc(size_t bytes);
+    void *alloc(size_t bytes, bool needed);
     std::vector<Entry> entries_;
     size_t arena_mark_, pinned_mark_;
     bool ok_;

@@ -414,7 +414,7 @@ template <> bool try_tc_ig<float>(Scope &sc, const ConvGeom &g, const float *dy,
     const long long planes = (long long)g.n * g.Cout;
     const long long total = planes * g.Hin * (g.Win / 4);
     if (total >= (1ll << 31)) return false;
-    float *dil = sc.scratch<float>((size_t)planes * g.Hin * g.Win);
+    float *dil = sc.try_scratch<float>((size_t)planes * g.Hin * g.Win);
     if (!dil) return false;
     const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 32);
     TL_LAUNCH(conv_dilate_dy_kernel, blocks, 256, 0, dy, dil, (unsigned)total, g.Hout, g.Wout, g.Hin, g.Win, g.sh, g.sw);
@@ -1047,7 +1047,7 @@ template <> bool try_tc_wg<float>(Scope &sc, const ConvGeom &g, const float *x, 
     if (g.sh == 1 && gemm_path() != 2 && work >= (1ll << 22) && conv_wgy_run(x, dy, nullptr, sm_count(), &small, g.n, g.Cin, g.Cout, g.Hout, g.Wout, true)) {
         const long long nw = (long long)g.Cout * g.Cin * 9;
         bool deferred;
-        float *part = partials_alloc<float>(sc, (size_t)small * nw, deferred);
+        float *part = partials_alloc<float>(sc, (size_t)small * nw, deferred, false);
         if (!part) return false;
         if (!conv_wgy_run(x, dy, part, small, &small, g.n, g.Cin, g.Cout, g.Hout, g.Wout, false)) return false;
         reduce_partials<float>(part, dw, nw, small, deferred);
@@ -1062,7 +1062,7 @@ template <> bool try_tc_wg<float>(Scope &sc, const ConvGeom &g, const float *x, 
     long long group_floats = 0;
     if (!conv_wgt_run(x, dy, nullptr, sm_count(), &groups, &group_floats, g.n, g.Cin, g.Cout, g.Hout, g.Wout, g.sh, true)) return false;
     bool deferred;
-    float *part = partials_alloc<float>(sc, (size_t)groups * (size_t)group_floats, deferred);
+    float *part = partials_alloc<float>(sc, (size_t)groups * (size_t)group_floats, deferred, false);
     if (!part) return false;
     if (!conv_wgt_run(x, dy, part, groups, &groups, &group_floats, g.n, g.Cin, g.Cout, g.Hout, g.Wout, g.sh, false)) return false;
     conv_wgt_reduce(part, dw, groups, g.Cin, g.Cout, g.sh, deferred);
@@ -1077,7 +1077,7 @@ template <> bool try_1x1_wg<float>(Scope &sc, const ConvGeom &g, const float *x,
     if (!conv1x1s_wg(g, x, dy, nullptr, 8 * sm_count(), &groups, true)) return false;
     const long long nw = (long long)g.Cout * g.Cin;
     bool deferred;
-    float *part = partials_alloc<float>(sc, (size_t)groups * nw, deferred);
+    float *part = partials_alloc<float>(sc, (size_t)groups * nw, deferred, false);
     if (!part) return false;
     if (!conv1x1s_wg(g, x, dy, part, groups, &groups, false)) return false;
     reduce_partials<float>(part, dw, nw, groups, deferred);
@@ -1092,7 +1092,7 @@ template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T 
     const int most = (int)std::min<long long>(1 << 20, std::max<long long>(1, (64ll << 20) / nw));     // partial results: 256 MB at most
     if (!conv_mma_wg<T>(g, x, dy, nullptr, most, &groups, true)) return false;
     bool deferred;
-    float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred);
+    float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred, false);
     if (!part) return false;
     if (!conv_mma_wg<T>(g, x, dy, part, most, &groups, false)) return false;
     profile_add_flops(conv_flops(g));
@@ -1109,11 +1109,12 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
         int groups = 0;
         if (dw_wg_planes<T>(g, x, dy, nullptr, groups, true)) {
             bool deferred;
-            float *part = partials_alloc<T>(sc, (size_t)groups * g.Cin * KK, deferred);
-            if (!part) return;
-            dw_wg_planes<T>(g, x, dy, part, groups, false);
-            reduce_partials<T>(part, dw, (long long)g.Cin * KK, groups, deferred);
-            return;
+            float *part = partials_alloc<T>(sc, (size_t)groups * g.Cin * KK, deferred, false);
+            if (part) {
+                dw_wg_planes<T>(g, x, dy, part, groups, false);
+                reduce_partials<T>(part, dw, (long long)g.Cin * KK, groups, deferred);
+                return;
+            }
         }
         TL_LAUNCH((dw_wg_kernel<T>), g.Cin * KK, 256, 0, g, x, dy, dw);
         return;
@@ -1145,7 +1146,7 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
             if (groups > items) groups = (int)items;
             if (groups < 1) groups = 1;
             bool deferred;
-            float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred);
+            float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred, true);
             if (!part) return;
             const int vec = sizeof(T) == 4 && (((uintptr_t)x | (uintptr_t)dy) & 15) == 0;
             dim3 grid(ci_tiles * co_tiles, groups);
@@ -1187,7 +1188,7 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
     if (groups > items) groups = (int)items;
     if (groups < 1) groups = 1;
     bool deferred;
-    float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred);
+    float *part = partials_alloc<T>(sc, (size_t)groups * nw, deferred, true);
     if (!part) return;
     dim3 grid(ci_tiles * co_tiles, groups);
 #define TL_WG_LAUNCH(KH_, KW_)                                                                                        \

@@ -686,7 +686,7 @@ void instnorm_bw_param(Scope &sc, const T *x, const T *dy, T *dgb, const T *mean
     if (n * C <= 0) return;
     defer_settle(dgb);
     bool deferred;
-    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
+    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred, true);
     if (!part) return;
     if (!instnorm_bw_warp(x, dy, (T *)nullptr, part, (const T *)nullptr, mean, (const T *)nullptr, stdev, n, C, D))
         TL_LAUNCH((instnorm_bw_param_kernel<T>), n * C, D >= 256 ? 256 : 64, 0, x, dy, part, mean, stdev, D);
@@ -699,7 +699,7 @@ void instnorm_bw_both(Scope &sc, const T *x, const T *dy, T *dx, T *dgb, const T
     if (n * C <= 0) return;
     defer_settle(dgb);
     bool deferred;
-    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
+    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred, true);
     if (!part) return;
     if (instnorm_bw_warp(x, dy, dx, part, gamma, mean, var, stdev, n, C, D)) {
         instnorm_param_reduce<T>(sc, part, dgb, n, C, deferred);
@@ -730,7 +730,7 @@ void instnorm_relu_bw(Scope &sc, const T *x, const T *y, T *dy, const T *dy2, T 
     if (n * C <= 0) return;
     defer_settle(dgb);
     bool deferred;
-    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred);
+    float *part = partials_alloc<T>(sc, (size_t)2 * n * C, deferred, true);
     if (!part) return;
     if (instnorm_bw_warp(x, dy, dx, part, gb, mean, var, stdev, n, C, D, true, dy2)) {
         instnorm_param_reduce<T>(sc, part, dgb, n, C, deferred);
@@ -1042,7 +1042,7 @@ template <class T> void mse_fw(const T *y, const T *t, T *loss, int dim, int n)
     if (n <= 0) return;
     Scope sc;
     int parts = n <= 64 ? std::min(ceil_div(dim, 1024), 128) : 1;
-    float *part = parts > 1 ? sc.scratch<float>((size_t)n * parts) : nullptr;
+    float *part = parts > 1 ? sc.try_scratch<float>((size_t)n * parts) : nullptr;
     if (!part) parts = 1;
     for (int s0 = 0; s0 < n; s0 += 65535)                   // a grid has 65 535 rows at most
         TL_LAUNCH((mse_fw_kernel<T>), dim3(parts, std::min(n - s0, 65535)), 256, 0, y + (long long)s0 * dim, t + (long long)s0 * dim, loss + s0, part, dim, parts);

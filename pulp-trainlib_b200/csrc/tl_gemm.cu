@@ -333,7 +333,7 @@ template <class T> bool linear_wg_streams(Scope &sc, const T *dy, const T *x, T 
     // worth it when the layer is small against the stream count; large layers keep the GEMM tiles
     if ((long long)out * in > 16384 || n < 64) return false;
     const int per = 32, blocks = ceil_div(n, per), count = out * in;
-    float *part = sc.scratch<float>((size_t)blocks * count);
+    float *part = sc.try_scratch<float>((size_t)blocks * count);
     if (!part) return false;
     dim3 grid(ceil_div(count, 256), blocks);
     TL_LAUNCH((linear_wg_streams_partial_kernel<T>), grid, 256, 0, dy, x, part, n, out, in, per);

@@ -439,9 +439,9 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
                 const int per = ceil_div(p.chunks, (int)s);
                 p.splits = ceil_div(p.chunks, per);
                 if (p.splits > 1) {
-                    p.part = sc.scratch<float>((size_t)tiles * p.splits * BM * BN);
-                    if (!p.part) return;
-                    p.ticket0 = ticket; ticket += (int)tiles;
+                    p.part = sc.try_scratch<float>((size_t)tiles * p.splits * BM * BN);
+                    if (p.part) { p.ticket0 = ticket; ticket += (int)tiles; }
+                    else p.splits = 1;
                 }
             }
         }

@@ -527,7 +527,7 @@ template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int 
     }
 }
 
-// Returns false when the product should go to the other kernels (too small, or no tensor-map encoder).
+// Returns false when the product should go to the other kernels (too small, no tensor-map encoder, no memory for the copies).
 template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
 {
     typedef TmCfg<T> Cfg;
@@ -552,9 +552,9 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
         const bool aligned = sizeof(T) == 2 && ((uintptr_t)src & 15) == 0 && (batch == 1 || bs % EB == 0);
         if (aligned && cs == 1 && rs % EB == 0 && rs >= d.K) { o = {src, nullptr, rs, bs, 0}; return true; }
         if (aligned && rs == 1 && cs % EB == 0 && cs >= rows) { o = {src, nullptr, cs, bs, 1}; return true; }
-        const size_t count = (size_t)batch * rows * Kp;
-        T *hi = sc.scratch<T>(count), *lo = sizeof(T) == 4 ? sc.scratch<T>(count) : nullptr;
-        if (!hi || (sizeof(T) == 4 && !lo)) return false;
+        const size_t count = ((size_t)batch * rows * Kp + 63) & ~(size_t)63;
+        T *hi = sc.try_scratch<T>(Cfg::PARTS * count), *lo = sizeof(T) == 4 ? hi + count : nullptr;
+        if (!hi) return false;
         PackOp<T> &q = pack.op[pack.count++];
         const bool straight = cs == 1;
         q = {src, hi, lo, rs, cs, bs, rows, d.K, Kp, ceil_div(Kp, straight ? 64 : 32), ceil_div(rows, straight ? 32 : 64), blocks, straight, (straight ? rs : rs == 1 ? cs : 1) % EB == 0 && (batch == 1 || bs % EB == 0) && ((uintptr_t)src & 15) == 0};
@@ -576,7 +576,7 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     p.status = status; p.a_mn = a.mn; p.b_mn = b.mn; p.b_one = b_batch < copies;
     p.tiles_m = ceil_div(d.M, p.BN); p.tiles_n = ceil_div(d.N, p.pair ? 2 * TM_BM : TM_BM); p.tiles = p.tiles_m * p.tiles_n * d.batch;
     p.part = nullptr;
-    if (p.splits > 1 && !(p.part = sc.scratch<float>((size_t)p.tiles * p.splits * TM_BM * p.BN))) return false;
+    if (p.splits > 1 && !(p.part = sc.try_scratch<float>((size_t)p.tiles * p.splits * TM_BM * p.BN))) return false;
     const int b_rows = p.pair ? p.BN / 2 : p.BN;
     p.stage_bytes = Cfg::PARTS * (TM_BM * 128u + (uint32_t)b_rows * 128u);
     p.stages = std::min<int>(TM_MAX_STAGES, TM_RING / p.stage_bytes);

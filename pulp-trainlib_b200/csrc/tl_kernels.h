@@ -130,14 +130,15 @@ __device__ __forceinline__ long long wgt_partial_index(long long e, int Cin, int
 
 // Partial results of an fp32 reduction: from the deferred-reduction arena when that mode is on and every buffer of the call
 // is device-resident (`deferred` = true: the caller notes the sum with defer_*), else scratch of the call (the caller sums at once).
-template <class T> inline float *partials_alloc(Scope &sc, size_t floats, bool &deferred)
+// needed: there is no other path, so that no memory is an error.
+template <class T> inline float *partials_alloc(Scope &sc, size_t floats, bool &deferred, bool needed)
 {
     deferred = false;
     if (sizeof(T) == 4 && sc.may_defer()) {
         float *p = defer_alloc(floats);
         if (p) { deferred = true; return p; }
     }
-    return sc.scratch<float>(floats);
+    return needed ? sc.scratch<float>(floats) : sc.try_scratch<float>(floats);
 }
 // 1x1 strided convolutions (tl_conv1x1.cu); false = geometry not covered, nothing launched
 bool conv1x1s_fw(const ConvGeom &g, const float *x, const float *w, const float *bias, float *y);

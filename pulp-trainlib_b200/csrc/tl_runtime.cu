@@ -203,7 +203,8 @@ static void arena_release(size_t mark)
             for (auto &c : g.chunks) { total += c.cap; cudaFree(c.base); }
             g.chunks.clear();
             char *base = nullptr;
-            if (TL_CUDA(cudaMalloc(&base, total))) g.chunks.push_back({base, total, 0});
+            if (cudaMalloc(&base, total) == cudaSuccess) g.chunks.push_back({base, total, 0});
+            else cudaGetLastError();                                 // the next call that needs scratch asks for what it needs
         } else {
             for (auto &c : g.chunks) c.off = 0;
         }
@@ -215,7 +216,8 @@ static void arena_release(size_t mark)
     }
 }
 
-static void *arena_alloc(size_t bytes)
+// needed: the call cannot do without it, so that no memory is an error
+static void *arena_alloc(size_t bytes, bool needed)
 {
     scratch_touch();
     bytes = (bytes + 255) & ~(size_t)255;
@@ -228,7 +230,10 @@ static void *arena_alloc(size_t bytes)
     if (!g.chunks.empty()) cap = g.chunks.back().cap * 2;
     while (cap < bytes) cap *= 2;
     char *base = nullptr;
-    if (!TL_CUDA(cudaMalloc(&base, cap))) return nullptr;
+    cudaError_t e = cudaMalloc(&base, cap);
+    if (e == cudaErrorMemoryAllocation && cap > bytes) { cudaGetLastError(); cap = bytes; e = cudaMalloc(&base, cap); }      // without the room to grow
+    if (e == cudaErrorMemoryAllocation && !needed) { cudaGetLastError(); return nullptr; }
+    if (!cuda_ok(e, "cudaMalloc (scratch)")) return nullptr;
     g.chunks.push_back({base, cap, bytes});
     return base;
 }
@@ -289,10 +294,10 @@ Scope::Scope() : arena_mark_(0), pinned_mark_(g_pinned_off), ok_(true), staged_(
     g.scope_depth++;
 }
 
-void *Scope::alloc(size_t bytes)
+void *Scope::alloc(size_t bytes, bool needed)
 {
-    void *p = arena_alloc(bytes);
-    if (!p) ok_ = false;
+    void *p = arena_alloc(bytes, needed);
+    if (!p && needed) ok_ = false;
     return p;
 }
 
@@ -328,7 +333,7 @@ void *Scope::map(void *p, size_t bytes, bool copy_in, bool copy_out)
             return nullptr;
         }
     }
-    void *d = arena_alloc(bytes);
+    void *d = arena_alloc(bytes, true);
     if (!d) { ok_ = false; return nullptr; }
     staged_ = true;
     entries_.push_back({p, d, pinned_alloc(p, bytes), bytes, copy_out, false});

@@ -653,3 +653,53 @@ def test_freeing_a_gradient_with_its_sum_pending(pkg, gpulib):
     finally:
         gpulib.trainlib_set_deferred_reductions(0); gpulib.trainlib_set_streams(1)
         r.close()
+
+
+def pointwise_call(r, x, w, y, n, cin, cout, h, wd):
+    """pulp_conv_pw_fp32_fw_cl on torch tensors"""
+    one = r.zeros(4)
+    at = lambda t: t.data_ptr()
+    mk = lambda d, C, H, W, dim=None: r.pkg.make_blob(r.keep, at(d), one.arg, C=C, H=H, W=W, dim=dim)
+    args = r.args("PointWise_Conv_args", input=mk(x, cin, h, wd), coeff=mk(w, cin, 1, 1, cout * cin), output=mk(y, cout, h, wd), transpose_buffer=one,
+                  skip_wg_grad=0, skip_in_grad=0, opt_matmul_type_fw=0, opt_matmul_type_wg=0, opt_matmul_type_ig=0, HWC=0)
+    r.lib.trainlib_set_streams(n)
+    r.lib.pulp_conv_pw_fp32_fw_cl(ctypes.byref(args))
+
+
+def check_pointwise(x, w, y, step):
+    """in 64 bits, `step` pixels of a stream at a time; 1e-5 of the result's largest value as everywhere"""
+    import torch
+    top = err = 0.0
+    w64 = w.double()
+    for s in range(x.shape[0]):
+        for p in range(0, x.shape[2], step):
+            want = w64 @ x[s, :, p:p + step].double()
+            top = max(top, float(want.abs().max())); err = max(err, float((y[s, :, p:p + step] - want).abs().max()))
+    assert 0 < top and err <= FP32_TOL * top, (err, top)
+
+
+@pytest.mark.gpu
+def test_a_layer_whose_scratch_does_not_fit_takes_its_other_path_without_an_error(pkg, gpulib):
+    """two streams of 64 -> 64 channels on 2048 x 4096 with 2.5 GB of the device left: the packed copies of the tcgen05 path (4.3 GB a
+    stream) cannot be had, the layer runs on the path without them and no error is latched"""
+    import torch
+    n, c, h, wd = 2, 64, 2048, 4096
+    r = AbiRunner(pkg, gpulib, device=True)
+    gen = torch.Generator("cuda").manual_seed(3)
+    x = torch.randn(n, c, h * wd, device="cuda", generator=gen)
+    w = torch.randn(c, c, device="cuda", generator=gen) / 8
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    hog = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (5 << 29)), dtype=torch.uint8, device="cuda")
+    try:
+        pointwise_call(r, x, w, y, n, c, c, h, wd)
+        gpulib.trainlib_synchronize()
+        code, text = gpulib.trainlib_last_error(), gpulib.trainlib_last_error_string()
+        gpulib.trainlib_clear_error()
+        assert code == 0, text
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        gpulib.trainlib_set_streams(1)
+        r.close()
+    check_pointwise(x, w, y, 1 << 20)
