@@ -527,15 +527,19 @@ template <class T> static void tm_plan(int N, int M, int batch, int ksteps, int 
     }
 }
 
-// Returns false when the product should go to the other kernels (too small, no tensor-map encoder, no memory for the copies).
-template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
+// fp16 operands stay where they are when one index is contiguous (returns 1: the contracted one, 2: the rows) and the other steps in
+// multiples of 16 bytes; 0 = the operand is packed
+template <class T> static int tm_in_place(const T *src, long long rs, long long cs, long long bs, int rows, int K, int batch)
+{
+    constexpr long long EB = 16 / (long long)sizeof(T);
+    if (sizeof(T) != 2 || ((uintptr_t)src & 15) || (batch > 1 && bs % EB)) return 0;
+    return cs == 1 && rs % EB == 0 && rs >= K ? 1 : rs == 1 && cs % EB == 0 && cs >= rows ? 2 : 0;
+}
+
+// false: no tensor-map encoder, no memory for the copies
+template <class T> static bool tm_product(const GemmDesc<T> &d)
 {
     typedef TmCfg<T> Cfg;
-    if (d.N < 1 || d.M < 1 || d.K < 1 || d.batch < 1 || d.segs < 1 || (d.batch > 1 && d.segs > 1)) return false;
-    if (gemm_path() != 3) {      // 3 = forced (tests): every shape, the tails come from the tensor maps' zero fill
-        if (d.segs == 1 && (d.N < TM_BM || d.M < TM_BM / 2 || d.K < (d.batch > 1 ? 1 : 2) * Cfg::BK)) return false;
-        if ((long long)d.N * d.M * d.K * d.batch * d.segs < (1ll << 26)) return false;
-    }
     EncodeTiledFn enc = (EncodeTiledFn)tc_encode_tiled_fn();
     int *status = tc_status_word();
     if (!enc || !status) return false;
@@ -543,15 +547,13 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
     if (!sc.ok()) return false;
     constexpr long long EB = 16 / (long long)sizeof(T);
     const int Kp = (int)(((long long)d.K + EB - 1) / EB * EB);
-    // fp16 operands stay where they are when one index is contiguous and the other steps in multiples of 16 bytes
     struct Op { const T *hi, *lo; long long os, bs; int mn; };
     PackOps<T> pack;
     pack.count = 0;
     int blocks = 0;
     auto prepare = [&](const T *src, long long rs, long long cs, long long bs, int rows, int batch, Op &o) -> bool {
-        const bool aligned = sizeof(T) == 2 && ((uintptr_t)src & 15) == 0 && (batch == 1 || bs % EB == 0);
-        if (aligned && cs == 1 && rs % EB == 0 && rs >= d.K) { o = {src, nullptr, rs, bs, 0}; return true; }
-        if (aligned && rs == 1 && cs % EB == 0 && cs >= rows) { o = {src, nullptr, cs, bs, 1}; return true; }
+        const int where = tm_in_place<T>(src, rs, cs, bs, rows, d.K, batch);
+        if (where) { o = {src, nullptr, where == 1 ? rs : cs, bs, where - 1}; return true; }
         const size_t count = ((size_t)batch * rows * Kp + 63) & ~(size_t)63;
         T *hi = sc.try_scratch<T>(Cfg::PARTS * count), *lo = sizeof(T) == 4 ? hi + count : nullptr;
         if (!hi) return false;
@@ -602,6 +604,34 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
         const long long quads = (long long)p.tiles * TM_BM * p.BN / 4;
         if (p.splits <= 16) TL_LAUNCH((tm_reduce_kernel<T, 1>), (unsigned)(quads / 256), 256, 0, p);
         else TL_LAUNCH((tm_reduce_kernel<T, 8>), (unsigned)(quads / 32), 256, 0, p);
+    }
+    return true;
+}
+
+// The packed copies of a batch are scratch that the library keeps (in fp32 twice the bytes of the operand), so a batch that would need
+// more than this goes out in slices (a block of 512 MB then holds those of the shared operand too); a slice's launches are hundreds of
+// microseconds by then.
+static constexpr long long TM_PACK_BYTES = 480ll << 20;
+
+// Returns false when the product should go to the other kernels (too small, or see tm_product).
+template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
+{
+    typedef TmCfg<T> Cfg;
+    if (d.N < 1 || d.M < 1 || d.K < 1 || d.batch < 1 || d.segs < 1 || (d.batch > 1 && d.segs > 1)) return false;
+    if (gemm_path() != 3) {      // 3 = forced (tests): every shape, the tails come from the tensor maps' zero fill
+        if (d.segs == 1 && (d.N < TM_BM || d.M < TM_BM / 2 || d.K < (d.batch > 1 ? 1 : 2) * Cfg::BK)) return false;
+        if ((long long)d.N * d.M * d.K * d.batch * d.segs < (1ll << 26)) return false;
+    }
+    if (d.batch == 1 || d.accumulate) return tm_product<T>(d);           // (accumulated: a slice that fails could not be taken back)
+    const long long bytes = (long long)sizeof(T) * Cfg::PARTS * d.K;
+    const long long per = (tm_in_place<T>(d.A, d.a_rs, d.a_cs, d.a_bs, d.N, d.K, d.batch) ? 0 : bytes * d.N) +
+                          (d.b_bs == 0 || tm_in_place<T>(d.B, d.b_cs, d.b_rs, d.b_bs, d.M, d.K, d.batch) ? 0 : bytes * d.M);
+    const int slices = ceil_div(d.batch, per ? std::max(1ll, TM_PACK_BYTES / per) : d.batch), each = ceil_div(d.batch, slices);
+    for (int b = 0; b < d.batch; b += each) {
+        GemmDesc<T> s = d;
+        s.batch = std::min(each, d.batch - b);
+        s.A += b * d.a_bs; s.B += b * d.b_bs; s.C += b * d.c_bs;
+        if (!tm_product<T>(s)) return false;
     }
     return true;
 }

@@ -703,3 +703,26 @@ def test_a_layer_whose_scratch_does_not_fit_takes_its_other_path_without_an_erro
         gpulib.trainlib_set_streams(1)
         r.close()
     check_pointwise(x, w, y, 1 << 20)
+
+
+@pytest.mark.gpu
+def test_the_scratch_of_a_pointwise_layer_does_not_grow_with_its_batch(pkg, gpulib):
+    """1201 streams of 64 -> 64 channels on 64 x 64: the packed copies would be 2.5 GB, the layer goes out in slices of 480 MB"""
+    import torch
+    n, c, h = 1201, 64, 64
+    r = AbiRunner(pkg, gpulib, device=True)
+    gen = torch.Generator("cuda").manual_seed(4)
+    x = torch.randn(n, c, h * h, device="cuda", generator=gen)
+    w = torch.randn(c, c, device="cuda", generator=gen) / 8
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize(); torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    try:
+        pointwise_call(r, x, w, y, n, c, c, h, h)
+        gpulib.trainlib_synchronize()
+        pkg.check(gpulib)
+    finally:
+        gpulib.trainlib_set_streams(1)
+        r.close()
+    assert free - torch.cuda.mem_get_info()[0] < 1 << 30
+    check_pointwise(x, w, y, h * h)
