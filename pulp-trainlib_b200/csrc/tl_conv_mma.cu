@@ -20,8 +20,14 @@ namespace tl {
 static constexpr int CM_MAXTAPS = 49;
 static constexpr int CM_SMEM_MAX = 220 * 1024;
 
-// n / d for n, d < 2^16
+// n / d, exact while n d < 2^32: the host checks it for the planes, patches are bounded by shared memory
 struct CmDiv { uint32_t m; int d; };
+// Streams of a tile on planes of P < tile pixels.  Offsets inside a tile are 32 bits wide (bytes of a source, elements of a result): a
+// stream has less than 2^25 elements on either side (checked where the path is chosen), a tile less than 2^29.
+static int cm_streams(int tile, int P, int n, long long stream_elements)
+{
+    return (int)std::max(1ll, std::min<long long>(std::min(tile / P, n), ((1ll << 29) - 1) / stream_elements));
+}
 static CmDiv cm_div(int d) { CmDiv r; r.d = d; r.m = d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); return r; }
 __device__ __forceinline__ CmDiv cm_div_dev(int d) { CmDiv r; r.d = d; r.m = d == 1 ? 0u : 0xFFFFFFFFu / (uint32_t)d + 1u; return r; }
 __device__ __forceinline__ int cm_quot(int n, CmDiv d) { return d.m ? (int)__umulhi((uint32_t)n, d.m) : n; }
@@ -43,7 +49,7 @@ __device__ __forceinline__ uint32_t cm_lds32(uint32_t addr) { uint32_t v; asm vo
 // A patch of the source plane(s), channels-last: `streams` x rows x cols pixels of `chans` channels (a multiple of 8 fp16 / 4
 // fp32; channels at or past c_left read as zero).  One item = one pixel x 16 bytes of channels: neighbouring threads take
 // neighbouring pixels, so the per-channel loads are coalesced and the 16-byte store is conflict-free.  Addresses are a
-// CTA-uniform base plus a 32-bit byte offset (the host keeps a tile's span below 4 GB).
+// CTA-uniform base plus a 32-bit byte offset (cm_streams keeps a tile's span below 2 GB).
 template <class T, int NT>
 __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams, int streams_left, int rows, int cols, CmDiv dcols,
                                          int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch)
@@ -460,7 +466,7 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
     // the largest patch over the classes: streams x rows x cols
     long long pix = 0; int taps = 0, tiles_max = 0; p.st_tile = 1;
     const int P0 = p.cls[0].Hc * p.cls[0].Wc;                              // class 0 has the most pixels
-    if (P0 < BN) p.st_tile = std::max(1, std::min(BN / P0, p.n));
+    if (P0 < BN) p.st_tile = cm_streams(BN, P0, p.n, std::max((long long)p.Cs * p.Hs * p.Ws, (long long)p.Cd * p.oH * p.oW));
     for (int i = 0; i < p.ncls; i++) {
         const CmClass &c = p.cls[i];
         const int P = c.Hc * c.Wc;
@@ -512,8 +518,7 @@ template <class T> static bool conv_mma_dispatch(CmFwd &p)
 {
     constexpr int CK = sizeof(T) == 2 ? 16 : 8;
     const int cpad = ceil_div(p.Cs, CK) * CK;
-    // 32-bit offsets inside a tile
-    if ((long long)p.Cs * p.Hs * p.Ws * 16 >= (1ll << 29) || (long long)p.Cd * p.oH * p.oW * 16 >= (1ll << 29)) return false;
+    if ((long long)p.Cs * p.Hs * p.Ws >= (1ll << 25) || (long long)p.Cd * p.oH * p.oW >= (1ll << 25)) return false;      // cm_streams
     p.linear = p.ncls == 1 && p.osx == 1 && p.osy == 1;
     p.pairs = p.linear && (p.oW * p.oH) % 2 == 0 && ((uintptr_t)p.dst) % (2 * sizeof(T)) == 0;
     long long tiles = 0;                                                   // 128-pixel tiles
@@ -783,7 +788,9 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     p.ci_tiles = ceil_div(p.Ci, CI);
     const int ctiles = p.ci_tiles * ceil_div(p.Co, CO);
     const int slots = std::max(1, std::min(2 * sm_count() / ctiles, part_groups));
-    auto tiles_of = [&](int bn) -> long long { return P < bn ? ceil_div(p.n, std::max(1, std::min(bn / P, p.n))) : p.Wo > bn ? (long long)p.n * p.Ho * ceil_div(p.Wo, bn) : (long long)p.n * ceil_div(P, bn); };
+    const long long stream_elements = (long long)p.Ci * p.H * p.W + (long long)p.Co * P;
+    if (stream_elements >= (1ll << 25)) return false;                      // cm_streams
+    auto tiles_of = [&](int bn) -> long long { return P < bn ? ceil_div(p.n, cm_streams(bn, P, p.n, stream_elements)) : p.Wo > bn ? (long long)p.n * p.Ho * ceil_div(p.Wo, bn) : (long long)p.n * ceil_div(P, bn); };
     // pixels per tile: what makes the fewest pixels of the longest CTA (planes and rounds come out even), halo rows included
     double best = 1e30;
     for (int bn = BN; bn >= BN / 4; bn -= SZ == 2 ? 16 : 8) {
@@ -792,13 +799,13 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
         if (cost < 0.98 * best) { best = cost; p.bn = bn; }
     }
     const int bn = p.bn;
-    p.st_tile = P < bn ? std::max(1, std::min(bn / P, p.n)) : 1;
+    p.st_tile = P < bn ? cm_streams(bn, P, p.n, stream_elements) : 1;
     const bool wide = p.Wo > bn;
     p.tiles_r = ceil_div(p.Wo, bn); p.tiles_s = wide ? p.Ho * p.tiles_r : ceil_div(P, bn);
     if (wide) { p.cols = (bn - 1) * p.S + cols0 - (p.Wo - 1) * p.S; p.dcols = cm_div(p.cols); }
     else if ((long long)P * p.Wo >= (1ll << 32)) return false;
     const long long tiles = tiles_of(bn);
-    if (tiles >= (1 << 30) || ((long long)p.Ci * p.H * p.W + (long long)p.Co * P) * 16 >= (1ll << 29)) return false;      // 32-bit offsets inside a tile
+    if (tiles >= (1 << 30)) return false;
     p.tiles = (int)tiles;
     p.steps = ceil_div(P < bn ? p.st_tile * P : bn, SZ == 2 ? 16 : 8);
     const int rows = (wide ? 0 : P < bn ? p.Ho - 1 : (bn + p.Wo - 2) / p.Wo) * p.S + p.rows_max;

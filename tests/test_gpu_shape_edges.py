@@ -171,3 +171,30 @@ def test_mse_lengths(run, oracle, dim):
     tol = FP16_TOL if run.half else FP32_TOL
     assert_close(np.asarray([loss], F), np.asarray([np.mean((t.astype(np.float64) - y) ** 2)], F), tol, "loss")
     assert_close(dy.astype(F) * dim, (2.0 * (y.astype(np.float64) - t)).astype(F), tol if dim < 5000 or not run.half else 0.1, "dy")
+
+
+def test_conv2d_planes_of_one_pixel_and_millions_of_channels(pkg, gpulib):
+    """128 streams of nine million channels on 1 x 1: the streams that share a tile of the weight gradient lie past 4 GB"""
+    import torch
+    n, c = 128, 9000000
+    r = AbiRunner(pkg, gpulib, device=True)
+    gen = torch.Generator("cuda").manual_seed(6)
+    x, dw, dy = torch.randn(n, c, device="cuda", generator=gen), torch.empty(c, 9, device="cuda"), torch.randn(n, device="cuda", generator=gen)
+    one = r.zeros(4)
+    mk = lambda d, g, C, H, W, dim=None: pkg.make_blob(r.keep, d, g, C=C, H=H, W=W, dim=dim)
+    a = r.args("Conv2D_args", input=mk(x.data_ptr(), one.arg, c, 1, 1), coeff=mk(one.arg, dw.data_ptr(), c, 3, 3, 9 * c), bias=mk(one.arg, one.arg, 1, 1, 1), output=mk(one.arg, dy.data_ptr(), 1, 1, 1),
+               Lpad=1, Rpad=1, Upad=1, Dpad=1, stride_h=1, stride_w=1, i2c_buffer=one, bt_buffer=one, USE_BIASES=0, USE_IM2COL=0, HWC=0)
+    torch.cuda.synchronize()
+    try:
+        gpulib.trainlib_set_streams(n)
+        r.call("pulp_conv2d_fp32_bw_param_grads_cl", a)
+        gpulib.trainlib_synchronize()
+    finally:
+        gpulib.trainlib_set_streams(1)
+        r.close()
+    err = top = 0.0
+    for k in range(0, c, 1000000):
+        want = (x[:, k:k + 1000000].double() * dy.double()[:, None]).sum(0)
+        top = max(top, float(want.abs().max())); err = max(err, float((dw[k:k + 1000000, 4] - want).abs().max()))
+    assert err <= FP32_TOL * top, (err, top)
+    assert float(dw[:, :4].abs().max()) == 0 and float(dw[:, 5:].abs().max()) == 0
