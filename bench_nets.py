@@ -287,7 +287,9 @@ class ResNet8Streams(object):
     FAMILIES = (
         ("conv_fw_ig_tensor", ("conv_mn_kernel", "conv_tc_kernel"), "tensor",
          "forward of the 7 3x3 convolutions and their input gradients as tcgen05 3xTF32 implicit GEMMs (useful FLOP: zeros of a dilated dY are not counted)"),
-        ("conv_wg_tensor", ("conv_wgt_kernel",), "tensor", "weight gradient of the stride-1 3x3 convolutions with 32+ channels as a tcgen05 3xTF32 pixel-contraction GEMM"),
+        ("conv_wg_tensor", ("conv_wgt_kernel", "conv_wgy_kernel"), "tensor",
+         "weight gradient of the 3x3 convolutions as tcgen05 3xTF32 pixel-contraction GEMMs (conv_wgy_kernel: 8 and 16 channels at stride 1)"),
+        ("conv_mma", ("conv_mma_kernel", "conv_mma_wg_kernel"), "tensor", "convolutions of small shards as 3xTF32 on the warp-level tensor-core instructions"),
         ("conv_wg_ffma", ("conv_wg3x3_partial_kernel", "conv_wg_partial_kernel", "conv_wg_direct_kernel"), "ffma", "weight gradient of the other convolutions, fp32 FFMA"),
         ("conv_1x1_strided", ("conv1x1s_mma_kernel", "conv1x1s_wg_kernel", "conv1x1_strided_ig_kernel"), "hbm",
          "forward, weight gradient and in-place input gradient of the two 1x1 stride-2 shortcut convolutions: 2 FLOP per byte, bound by memory traffic and instruction issue"),
@@ -324,7 +326,9 @@ class ResNet8Streams(object):
                 fams.append({"family": fam, "kernels": [m for m in members if m in base], "bound": bound, "launches_per_step": c, "ms_per_step": t, "flops": f, "work": what})
         for key, (c, t, f) in base.items():
             if key not in used:
-                fams.append({"family": key, "kernels": [key], "bound": "hbm", "launches_per_step": c, "ms_per_step": t, "flops": 0.0, "work": "bandwidth-bound"})
+                # (a kernel that multiplies and is in no family: reported with its rate and no peak, not as bandwidth-bound)
+                fams.append({"family": key, "kernels": [key], "bound": "unclassified" if f else "hbm", "launches_per_step": c, "ms_per_step": t, "flops": f,
+                             "work": "unclassified" if f else "bandwidth-bound"})
         # fp32 on the tensor cores is 3xTF32: one third of the TF32 rate, TF32 = half the bf16 rate
         tensor_sus, tensor_burst = pk["bf16_tflops_sustained"] / 6.0, pk["bf16_tflops"] / 6.0
         ffma_peak = 72.8
@@ -334,7 +338,9 @@ class ResNet8Streams(object):
                 continue
             f["achieved"] = f["flops"] / (f["ms_per_step"] * 1e-3) / 1e12 if f["ms_per_step"] > 0 else None
             f["unit"] = "TFLOP/s"
-            if f["bound"] == "tensor":
+            if f["bound"] == "unclassified":
+                f.update({"peak": None, "frac": None, "peak_note": "no peak assigned"})
+            elif f["bound"] == "tensor":
                 f.update({"peak": tensor_sus, "peak_burst": tensor_burst, "frac": f["achieved"] / tensor_sus, "frac_of_burst": f["achieved"] / tensor_burst,
                           "peak_note": "3xTF32-effective fp32 peak = measured bf16 / 6: sustained figure (kernels timed inside a long step), burst beside it"})
             else:

@@ -640,12 +640,15 @@ bool conv_wgy_run(const float *x, const float *dy, float *part, int part_groups,
     p.status = tc_status_word();
     if (!p.status) return false;
     const size_t smem = 1024 + (size_t)p.NC * p.conv_bytes + (size_t)p.NR * p.raw_bytes;
-    auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-        TL_LAUNCH(kern, ctas, WGY_THREADS, smem, tx, tdy, p);
-    };
-    if (cigs == 2) { if (cogs == 2) launch(conv_wgy_kernel<2, 2>); else launch(conv_wgy_kernel<2, 1>); }
-    else { if (cogs == 2) launch(conv_wgy_kernel<1, 2>); else launch(conv_wgy_kernel<1, 1>); }
+    // (a macro, not a function of the kernel: the profile takes its name from the launch)
+#define TL_WGY(CIGS, COGS)                                                                                                     \
+    do {                                                                                                                       \
+        cudaFuncSetAttribute(conv_wgy_kernel<CIGS, COGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);            \
+        TL_LAUNCH((conv_wgy_kernel<CIGS, COGS>), ctas, WGY_THREADS, smem, tx, tdy, p);                                         \
+    } while (0)
+    if (cigs == 2) { if (cogs == 2) TL_WGY(2, 2); else TL_WGY(2, 1); }
+    else { if (cogs == 2) TL_WGY(1, 2); else TL_WGY(1, 1); }
+#undef TL_WGY
     profile_add_flops(2.0 * n * Cout * Cin * 9.0 * H * W);
     return true;
 }

@@ -448,6 +448,8 @@ def test_profile_credits_useful_flops_to_the_kernel_that_ran(pkg, gpulib):
         credited = sum(row[3] for row in table)
         assert abs(credited - 3 * want) <= 1e-6 * want, (credited, 3 * want, table)
         assert all(row[3] == 0.0 for row in table if "reduce" in row[0] or "column" in row[0])
+        assert all("_kernel" in row[0] for row in table), table
+        assert [row[3] for row in table if "conv_wgy_kernel" in row[0]] == [want], table
         r.close()
     finally:
         gpulib.trainlib_set_streams(1)
