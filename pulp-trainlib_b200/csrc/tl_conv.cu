@@ -437,7 +437,7 @@ template <class T> static bool try_pointwise(const ConvGeom &g, const T *src, co
     d.A = src; d.a_rs = 1; d.a_cs = P; d.a_bs = (long long)K * P;
     d.B = w; d.b_rs = ig ? g.Cin : 1; d.b_cs = ig ? 1 : g.Cin;
     d.C = dst; d.c_rs = 1; d.c_cs = P; d.c_bs = (long long)M * P;
-    d.N = P; d.K = K; d.M = M; d.batch = g.n;
+    d.N = P; d.K = K; d.M = M; d.batch = g.n; d.flops = conv_flops(g);
     if (bias) { d.bias = bias; d.bias_mode = 2; }
     return gemm_tensor_core_tma<T>(d);
 }
@@ -453,12 +453,12 @@ template <class T> static bool try_pointwise_wg(const ConvGeom &g, const T *x, c
     d.A = dy; d.a_rs = P; d.a_cs = 1; d.a_ks = (long long)g.Cout * P;
     d.B = x; d.b_rs = 1; d.b_cs = P; d.b_ks = (long long)g.Cin * P;
     d.C = dw; d.c_rs = g.Cin; d.c_cs = 1;
-    d.N = g.Cout; d.K = P; d.M = g.Cin; d.segs = g.n;
+    d.N = g.Cout; d.K = P; d.M = g.Cin; d.segs = g.n; d.flops = conv_flops(g);
     return gemm_tensor_core_tma<T>(d);
 }
 template <class T> void conv_fw(Scope &sc, const ConvGeom &g, const T *x, const T *w, const T *bias, T *y)
 {
-    if (!g.depthwise && try_pointwise<T>(g, x, w, bias, y, false)) { profile_add_flops(conv_flops(g)); return; }
+    if (!g.depthwise && try_pointwise<T>(g, x, w, bias, y, false)) return;
     if (!g.depthwise && try_tc_fw<T>(sc, g, x, w, bias, y)) return;
     if (!g.depthwise && conv_mma_fw<T>(g, x, w, bias, y)) { profile_add_flops(conv_flops(g)); return; }
     if (g.depthwise) {
@@ -584,7 +584,7 @@ template <class T> void conv_ig_accumulate(Scope &sc, const ConvGeom &g, const T
 }
 template <class T> void conv_ig(Scope &sc, const ConvGeom &g, const T *dy, const T *w, T *dx)
 {
-    if (!g.depthwise && try_pointwise<T>(g, dy, w, nullptr, dx, true)) { profile_add_flops(conv_flops(g)); return; }
+    if (!g.depthwise && try_pointwise<T>(g, dy, w, nullptr, dx, true)) return;
     if (!g.depthwise && try_tc_ig<T>(sc, g, dy, w, dx)) return;
     if (!g.depthwise && conv_mma_ig<T>(g, dy, w, dx)) { profile_add_flops(conv_flops(g)); return; }
     if (g.depthwise) {
@@ -1122,7 +1122,7 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
     const long long nw = (long long)g.Cout * g.Cin * KK;
     const int ci_tiles = ceil_div(g.Cin, 16), co_tiles = ceil_div(g.Cout, 16);
     const bool k3 = g.Hk == 3 && g.Wk == 3 && g.padL == 1, k1 = g.Hk == 1 && g.Wk == 1 && g.padL == 0 && g.padU == 0;
-    if (try_pointwise_wg<T>(g, x, dy, dw)) { profile_add_flops(conv_flops(g)); return; }
+    if (try_pointwise_wg<T>(g, x, dy, dw)) return;
     if (try_tc_wg<T>(sc, g, x, dy, dw)) return;
     if (try_1x1_wg<T>(sc, g, x, dy, dw)) return;
     // the register-tiled FFMA kernel below keeps stride-1 3x3 fp32 layers with few input channels on 8, 16 and 32 pixel rows (ten streams of 16 -> 32 on

@@ -599,8 +599,9 @@ template <class T> static bool tm_product(const GemmDesc<T> &d)
     }
     if (p.pair) TL_LAUNCH_CLUSTER((gemm_tma_kernel<T, true>), (unsigned)(2 * std::min(p.tiles, sm_count() / 2)), TM_THREADS, smem, 2, ma0, ma1, mb0, mb1, p);
     else if (p.splits == 1) TL_LAUNCH((gemm_tma_kernel<T, false>), (unsigned)std::min(p.tiles, sm_count()), TM_THREADS, smem, ma0, ma1, mb0, mb1, p);
-    else {
-        TL_LAUNCH((gemm_tma_kernel<T, false>), (unsigned)(p.tiles * p.splits), TM_THREADS, smem, ma0, ma1, mb0, mb1, p);
+    else TL_LAUNCH((gemm_tma_kernel<T, false>), (unsigned)(p.tiles * p.splits), TM_THREADS, smem, ma0, ma1, mb0, mb1, p);
+    profile_add_flops(d.flops);
+    if (p.splits > 1) {
         const long long quads = (long long)p.tiles * TM_BM * p.BN / 4;
         if (p.splits <= 16) TL_LAUNCH((tm_reduce_kernel<T, 1>), (unsigned)(quads / 256), 256, 0, p);
         else TL_LAUNCH((tm_reduce_kernel<T, 8>), (unsigned)(quads / 32), 256, 0, p);
@@ -631,6 +632,7 @@ template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d)
         GemmDesc<T> s = d;
         s.batch = std::min(each, d.batch - b);
         s.A += b * d.a_bs; s.B += b * d.b_bs; s.C += b * d.c_bs;
+        s.flops = d.flops * s.batch / d.batch;
         if (!tm_product<T>(s)) return false;
     }
     return true;

@@ -19,6 +19,7 @@ template <class T> struct GemmDesc {
     bool accumulate = false;        // C += result instead of C = result
     const T *bias = nullptr;        // added after the product
     int bias_mode = 0;              // 1: bias[i] (per row), 2: bias[j] (per column)
+    double flops = 0;               // gemm_tensor_core_tma only: what the profile credits the product's launch with (convolutions)
 };
 template <class T> void gemm(const GemmDesc<T> &d);
 template <class T> bool gemm_tensor_core_tma(const GemmDesc<T> &d);      // false: not a product for it, nothing launched

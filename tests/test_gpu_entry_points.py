@@ -728,3 +728,24 @@ def test_the_scratch_of_a_pointwise_layer_does_not_grow_with_its_batch(pkg, gpul
         r.close()
     assert free - torch.cuda.mem_get_info()[0] < 1 << 30
     check_pointwise(x, w, y, h * h)
+
+
+@pytest.mark.gpu
+def test_profile_credits_a_split_product_not_its_sum(pkg, gpulib):
+    """fp16 pointwise layer over streams: its weight gradient is one product split over the pixels, summed by a second kernel"""
+    n, cin, cout, h = 64, 64, 128, 28
+    r = AbiRunner(pkg, gpulib, device=True, half=True)
+    X, W_, dY, Y, dX, dW, tr = (r.zeros(*s) for s in ((n, cin, h, h), (cout, cin), (n, cout, h, h), (n, cout, h, h), (n, cin, h, h), (cout, cin), (4,)))
+    a = r.args("PointWise_Conv_args_fp16", input=r.blob(X, dX, C=cin, H=h, W=h), coeff=r.blob(W_, dW, C=cin, dim=cout * cin), output=r.blob(Y, dY, C=cout, H=h, W=h), transpose_buffer=tr,
+               skip_wg_grad=0, skip_in_grad=0, opt_matmul_type_fw=0, opt_matmul_type_wg=0, opt_matmul_type_ig=0, HWC=0)
+    gpulib.trainlib_set_streams(n)
+    try:
+        gpulib.trainlib_profile(1)
+        r.call("pulp_conv_pw_fp16_fw_cl", a); r.call("pulp_conv_pw_fp16_bw_cl", a)
+    finally:
+        gpulib.trainlib_profile(0); gpulib.trainlib_set_streams(1)
+    table = pkg.profile_table(gpulib, flops=True)
+    assert any("tm_reduce_kernel" in row[0] for row in table), table
+    assert all(row[3] == 0.0 for row in table if "gemm_tma_kernel" not in row[0]), table
+    assert sum(row[3] for row in table) == 3 * 2.0 * n * cin * cout * h * h, table
+    r.close()
