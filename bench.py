@@ -231,7 +231,7 @@ class MmSweep(object):
         big = shapes[-1]
         peak = pk["bf16_tflops_sustained"] if self.half else pk["bf16_tflops_sustained"] / 6.0
         return {"bound": "tensor", "achieved": big["tflops"], "peak": peak, "unit": "TFLOP/s", "frac": big["tflops"] / peak, "traffic": None,
-                "peak_source": pk["source"], "kernel": "gemm_tma_kernel + pack_kmajor_kernel, %d^3" % big["n"], "algorithmic_flops": 2.0 * big["n"] ** 3,
+                "peak_source": pk["source"], "kernel": ("gemm_tma_kernel, %d^3" if self.half else "gemm_tma_kernel + pack_kmajor_kernel, %d^3") % big["n"], "algorithmic_flops": 2.0 * big["n"] ** 3,
                 "per_shape": shapes, "sweep_tflops": self.flops / (ms * 1e-3) / 1e12,
                 "peak_note": "measured sustained bf16 (fp16 operands)" if self.half else "3xTF32-effective fp32 peak = measured sustained bf16 / 6"}
 

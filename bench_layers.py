@@ -99,7 +99,7 @@ class ConvStep(_Layer):
         tf = self.flops / (ms * 1e-3) / 1e12
         peak = pk["bf16_tflops_sustained"] / 6.0
         return {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak, "traffic": None, "peak_source": pk["source"],
-                "kernel": "conv FW + WG + IG + SGD (whole step, 7 launches)", "algorithmic_flops": self.flops, "algorithmic_bytes": self.bytes,
+                "kernel": "conv FW + WG + IG + SGD (whole step, 5 launches)", "algorithmic_flops": self.flops, "algorithmic_bytes": self.bytes,
                 "us_per_step": 1e3 * ms, "hbm_frac": self.bytes / (ms * 1e-3) / 1e9 / pk["hbm_gbs"],
                 "peak_note": "3xTF32-effective fp32 peak = measured sustained bf16 / 6; at 28 MFLOP and 0.5 MB the step is bound by launch latency, "
                              "neither by the tensor cores nor by HBM"}
@@ -173,7 +173,7 @@ class MhsaStep(_Layer):
     def roofline(self, ms, pk):
         tf = self.flops / (ms * 1e-3) / 1e12
         return {"bound": "ffma", "achieved": tf, "peak": 72.8, "unit": "TFLOP/s", "frac": tf / 72.8, "traffic": None, "peak_source": pk["source"],
-                "kernel": "attention forward + backward: 11 launches (fused score-softmax-value kernel and its two backward kernels, projections and weight gradients as strided FFMA GEMMs)", "algorithmic_flops": self.flops,
+                "kernel": "attention forward + backward: 7 launches (fused score-softmax-value kernel and its two backward kernels, projections and weight gradients as four groups of FFMA products)", "algorithmic_flops": self.flops,
                 "algorithmic_bytes": self.bytes, "us_per_step": 1e3 * ms,
                 "peak_note": "FFMA peak measured on this part (125 MAC/clk/SM); the 256^3 products stay on the FFMA tiles because their summation "
                              "order keeps the backward inside 1e-5 of the reference"}

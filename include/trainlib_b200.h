@@ -44,7 +44,8 @@ void  trainlib_synchronize(void);
  *   - a host address: the bytes the call reads are copied to a device staging arena
  *     first, the bytes it writes are copied back before the call returns.
  * TL_MEM_AUTO asks the driver per pointer; TL_MEM_DEVICE / TL_MEM_HOST assert that all
- * pointers are of one kind and skip the query. */
+ * pointers are of one kind and skip the query, except that TL_MEM_HOST still asks about buffers of
+ * up to 384 KB: those are copied by the host, which a device address would bring down. */
 enum { TL_MEM_AUTO = 0, TL_MEM_DEVICE = 1, TL_MEM_HOST = 2 };
 void  trainlib_set_memory_mode(int mode);
 int   trainlib_memory_mode(void);

@@ -99,7 +99,6 @@ __device__ __forceinline__ void rows_times_tile(const T *__restrict__ M, const f
     }
 }
 
-// a_tile[d][t] = A[d][t0 + t] (zero beyond the last token)
 // four neighbours from a 4-element-aligned address
 __device__ __forceinline__ void ld4(const float *p, float (&v)[4]) { const float4 x = *reinterpret_cast<const float4 *>(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
 __device__ __forceinline__ void ld4(const __half *p, float (&v)[4])
@@ -108,6 +107,7 @@ __device__ __forceinline__ void ld4(const __half *p, float (&v)[4])
     const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&x.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&x.y));
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
+// a_tile[d][t] = A[d][t0 + t] (zero beyond the last token)
 template <class T>
 __device__ __forceinline__ void load_a_tile(const T *__restrict__ A, float *a_tile, int H, int L, int t0)
 {

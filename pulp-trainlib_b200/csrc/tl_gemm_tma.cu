@@ -6,15 +6,16 @@
 // A producer warp issues cp.async.bulk.tensor (128-byte swizzle; out-of-range rows and k read as zero, so no tail code) into
 // a ring of shared-memory stages and runs ahead across tiles; an issuer warp runs tcgen05.mma from shared-memory descriptors
 // into tensor memory and releases each stage with tcgen05.commit; four warps read finished accumulators with tcgen05.ld and
-// write C (any strides).  What bounds it is the way from L2 into the SM: 48 KB per 512 tensor cycles of a 128 x 256 fp16 tile.
+// write C (any strides).  What bounds single CTAs is the way from L2 into the SM: 48 KB per 512 tensor cycles of a 128 x 256 fp16 tile.
 //   PAIR: two CTAs share a 256 x BN tile (cta_group::2): each holds its 128 rows of A and half of B's rows, 32 KB instead of 48.
+//         fp16 4096^3 so: tensor pipe active 89 % of the cycles, 102 us at the 1.25 GHz that the power limit leaves it.
 //   fp16: kind::f16, operands in place whichever index is contiguous: K-major tiles ([row][64 k]) or MN-major ones ([k][64 rows],
 //         the majorness bits of the instruction descriptor).  Packing B of a plain product into K-major scratch took 43 of the
 //         155 us of a 4096^3 product.  BN = 256 with two accumulators: a tile's epilogue runs under the next tile's products.
 //   fp32: 3xTF32 on packed (hi, lo) pairs.  B_hi and B_lo lie behind each other: D0 += A_hi [B_hi | B_lo]^T is one instruction of
 //         N = 2 BN (A_hi is read once), D1 += A_lo B_hi^T a second one; the epilogue adds the three parts, whose accumulation
 //         chains are a third as long as one common chain (the accumulator truncates).
-// Measured, whole call: fp16 4096^3 173 -> 101 us, fp16 2048^3 29 -> 17.5 us, fp32 2048^3 118 -> 89 us, fp32 1000 x 600 x 1300
+// Measured, whole call: fp16 4096^3 173 -> 120 us over seconds (101 us in short runs), fp16 2048^3 29 -> 17.5 us, fp32 2048^3 118 -> 89 us, fp32 1000 x 600 x 1300
 // (B transposed) 31 -> 20.3 us, fp32 300 x 2050 x 914 67 -> 26 us.
 // Few tiles: `splits` CTAs share the K steps of a tile and write partial tiles; tm_reduce_kernel adds them in order.  A contraction
 // may run over several segments (the streams of a batch), which the tensor maps' third index selects, as it selects a batch.

@@ -36,7 +36,7 @@ def elementwise_err(a, b):
 
 def assert_close(a, b, tol, what="", elem_tol=None):
     """both bars of the training-step path: max|a-b| / max|b| <= tol for the tensor, and
-    |a-b| <= tol * max(|b|, 1e-2 max|b|) for every element"""
+    |a-b| <= ELEMENTWISE_FACTOR * tol * max(|b|, 1e-2 max|b|) for every element"""
     assert np.all(np.isfinite(np.asarray(a, np.float64))), "%s: non-finite values" % what
     e = rel_err(a, b)
     assert e <= tol, "%s: rel err %.3e > %.1e" % (what, e, tol)
