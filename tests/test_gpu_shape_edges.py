@@ -54,6 +54,20 @@ def test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n):
     assert_close(dB.get().astype(F), dy.astype(np.float64).sum(axis=(0, 2, 3)).astype(F), tol, "bias gradient")
 
 
+# the half-precision kernels on runs of slots (tl_conv_px.cu): loads of one, two and four pixels, planes smaller and larger than a run, runs
+# that start inside a row, channel counts at and off multiples of 16, slices of result channels, groups of source channels,
+# windows of 1 to 49 taps, strides 2 and 3 with parities that no tap reaches, a bias gradient in a spare channel and on its own
+SLOTS = [(24, 28, 28, 48, 3, 1, 130), (5, 27, 43, 23, 3, 1, 70), (64, 6, 6, 96, 3, 1, 60), (3, 48, 46, 90, 3, 1, 20), (32, 9, 14, 17, 5, 1, 40), (16, 31, 33, 33, 5, 1, 9), (6, 40, 40, 20, 7, 1, 12), (90, 19, 21, 70, 1, 1, 40),
+         (40, 41, 41, 80, 5, 1, 3), (96, 15, 17, 96, 1, 1, 90), (34, 10, 23, 55, 1, 2, 210), (43, 23, 34, 22, 3, 2, 60), (7, 39, 39, 58, 3, 2, 280), (20, 30, 31, 40, 3, 3, 110), (13, 33, 32, 24, 5, 2, 40), (1, 1, 300, 128, 3, 1, 40)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", SLOTS)
+def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
+    if not run.half:
+        pytest.skip("half precision only")
+    test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+
+
 @pytest.mark.parametrize("c,h,w,k,pad,n", [(5, 9, 7, 3, 1, 3), (64, 28, 28, 3, 1, 4), (3, 33, 18, 3, 0, 2), (8, 6, 6, 5, 2, 9), (2, 40, 41, 3, 2, 1), (7, 4, 4, 3, 1, 700), (4, 12, 12, 4, 1, 2)])
 def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
     g = geom(c, h, w, c, k, stride=stride, pad=pad)
