@@ -665,13 +665,14 @@ static bool px_covers(const ConvGeom &g)
 //   forward, stride 2 (one load a pixel): 54 of 43 -> 22 on 23 x 34 (152) 11.7 / 18.7; 335 of 3 -> 6 on 36 x 37 (264) 17.7 / 20.7; 321 of
 //     7 -> 58 on 39 x 39 (1183) 32.2 / 24.4
 //   input gradient, stride 2 (a class per parity): 51 of 14 -> 5 on 32 x 30 (28) 7.8 / 8.1; 54 of 43 -> 22 on 23 x 34 (152) 21.2 / 12.3
-//   1 x 1 (stride 1: what the products of tl_gemm_tma.cu decline): 70 of 20 -> 70 on 19 x 21 (72) 18.8 / 8.0; stride 2: 42 of 8 -> 59
+//   1 x 1 (stride 1: what the products of tl_gemm_tma.cu decline): 70 of 20 -> 70 on 19 x 21 (72) 18.8 / 8.0, on even planes, which
+//     mma.sync stages two pixels at a time, 72 of 13 -> 126 on 26 x 22 (84) 1.4 us slower for the two directions; stride 2: 42 of 8 -> 59
 //     on 39 x 42 (18) 6.8 / 6.2 and 12.3 / 11.0, 207 of 34 -> 55 on 10 x 23 (38) 11.8 / 7.5 and 18.7 / 9.9
 static double px_work(const ConvGeom &g) { return (double)g.n * g.Hout * g.Wout * g.Hk * g.Wk * (ceil_div(g.Cin, 16) * 16) * (ceil_div(g.Cout, 16) * 16); }
 static bool px_pays(const ConvGeom &g, bool ig)
 {
     const double w = px_work(g);
-    if (g.Hk * g.Wk == 1) return w >= (g.sh == 1 ? 5e7 : 1.5e7);
+    if (g.Hk * g.Wk == 1) return w >= (g.sh > 1 ? 1.5e7 : g.Hin * g.Win % 2 ? 5e7 : 1.5e8);
     if (g.sh == 1) return w >= ((ig ? g.Cout : g.Cin) > 32 ? (ig ? 5e8 : 4e8) : 1e8);
     return w >= (ig ? 6e7 : 1e9);
 }
