@@ -9,7 +9,9 @@
 // asynchronous copies at once, and the K steps of a chunk dealt to the WARPS of the CTA (every warp owns the whole tile for
 // its share of K; the partial tiles meet in shared memory in warp order).  Outputs with fewer tiles than SMs are further
 // split along K over CTAs; the CTA of a tile that finishes last adds the splits in order, so results do not depend on
-// scheduling.
+// scheduling.  Where a 128 x 128 x 512 product of one chunk spends its 3500 cycles (clock counters, fp16): 1000 in front of the first
+// copy (1600 with divisions by variables), 800 issuing copies, 250 waiting, 680 multiplying, 120 exchanging, 600 storing (1050
+// with the parameters of the end first read there).
 //   fp32: FFMA (full fp32 products and sums), 4 x 4 results per lane, operands read as 16-byte vectors along
 //         whichever of k / row is contiguous in memory: no transposition on the way into shared memory.
 //   fp16: mma.sync.m16n8k16 with fp32 accumulation, fragments by ldmatrix (plain for K-contiguous operands, .trans for
@@ -24,19 +26,29 @@ namespace tl {
 
 static constexpr int GG_MAX = 6;
 
+// n / d by multiplication, exact while n d < 2^32; m = 1: by division, where n may be larger than that (a division by a variable costs
+// a warp about a hundred cycles, and the chain of them in front of the first copy was a third of a small product's time)
+struct GgDiv { uint32_t m; int d; };
+static GgDiv gg_div(int d, long long n_max) { GgDiv r; r.d = d; r.m = d == 1 ? 0u : n_max * d < (1ll << 32) ? (uint32_t)(((1ull << 32) + d - 1) / d) : 1u; return r; }
+__device__ __forceinline__ int gg_quot(int n, GgDiv d) { return d.m > 1u ? (int)__umulhi((uint32_t)n, d.m) : d.m ? n / d.d : n; }
+
 template <class T> struct GgProb {
     const T *A[3], *B[3]; T *C; const T *bias;
     int N, M, K, segs, seg_list;                // seg_list: segment s uses A[s], B[s]; else A[0] + s * a_ss, B[0] + s * b_ss
     int a_kc, b_kc;                             // 1: k is the contiguous (or nearest) index of the operand, 0: its row
-    int a_vw, b_vw;                             // elements per copy (16 bytes, 4 bytes or one element)
-    int tiles_m, tiles_nm, splits, first, chunks;   // column tiles, tiles per matrix, CTAs per tile, first CTA, K chunks in all
+    int a_vl, b_vl;                             // log2 of the elements per copy (16 bytes, 4 bytes or one element)
+    GgDiv tiles_m, tiles_nm, splits;            // column tiles, tiles per matrix, CTAs per tile
+    GgDiv cps;                                  // K chunks of a segment
+    int chunks, per;                            // K chunks in all, of one CTA
+    int quads, plain;                           // four neighbouring results may be stored at once / and nothing is added to them
     long long a_cs, a_ss_, b_cs, b_ss_;         // strides of the contiguous-side and the other index (a_cs: usually 1)
     long long a_bs, b_bs, c_bs, a_ks, b_ks;     // batch strides, segment strides
     long long c_rs, c_cs;
     float alpha; int accumulate, bias_mode, ticket0;
     float *part;                                // [tile][split][BM * BN]
 };
-template <class T> struct GgParams { GgProb<T> p[GG_MAX]; int count; };
+// G: room for so many products (a launch of one product has its parameters at fixed addresses); first: the first CTA of each (past the grid: none)
+template <class T, int G> struct GgParams { int first[G]; GgProb<T> p[G]; };
 
 static __device__ unsigned gg_tickets[16384];   // one per tile of a K-split product; zero between launches
 
@@ -59,16 +71,14 @@ template <class T, int ROWS, int KC, int PAD, int NT> struct GgLoader {
     long long pass, chunk;      // bytes from one piece of the thread to the next, from one chunk to the next
     uint32_t sm, sm_pass;       // byte offset of the first piece in the stage, step
     int s, s_step, c, kc, vw, lim_c, lim_s;    // strided / contiguous index of the first piece; limits of the non-k index
-    long long cs_b;             // bytes between neighbours along the contiguous index (4-byte copies of any stride)
 
-    __device__ __forceinline__ void init(const T *src, int kc_, int vw_, int row0, int k0, int rows, long long cs, long long ss)
+    static constexpr int log2c(int n) { return n <= 1 ? 0 : 1 + log2c(n / 2); }
+    __device__ __forceinline__ void init(const T *src, int kc_, int vl, int row0, int k0, int rows, long long cs, long long ss)
     {
-        kc = kc_; vw = vw_;
-        const int tc = kc ? KC : ROWS;
-        const int v = vw == V16 ? V16 : (SZ == 4 || vw == V4) ? V4 : 1;
-        const int pc = tc / v;                                             // pieces per shared-memory row: powers of two
+        kc = kc_; vw = 1 << vl;
+        const int tc = kc ? KC : ROWS, pl = (kc ? log2c(KC) : log2c(ROWS)) - vl;       // pieces per shared-memory row: powers of two
         const int tid = threadIdx.x;
-        s = tid / pc; c = (tid % pc) * v; s_step = NT / pc;
+        s = tid >> pl; c = (tid & ((1 << pl) - 1)) << vl; s_step = NT >> pl;
         const int pitch = tc + PAD;
         sm = (uint32_t)((s * pitch + c) * SZ); sm_pass = (uint32_t)(s_step * pitch * SZ);
         const long long c0 = kc ? k0 : row0, s0 = kc ? row0 : k0;
@@ -76,7 +86,6 @@ template <class T, int ROWS, int KC, int PAD, int NT> struct GgLoader {
         ptr = safe + ((s0 + s) * ss + (c0 + c) * cs) * SZ;
         pass = (long long)s_step * ss * SZ; chunk = (kc ? (long long)KC * cs : (long long)KC * ss) * SZ;
         lim_c = rows - row0; lim_s = rows - row0;
-        cs_b = cs * SZ;
     }
     // k_left: rows of k from this chunk's start to the end of the segment
     __device__ __forceinline__ void fetch(uint32_t stage, int k_left)
@@ -197,10 +206,9 @@ template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST> struc
     static constexpr size_t SMEM = SMEM_OP > SMEM_RED ? SMEM_OP : SMEM_RED;
 };
 
-template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC>
-__global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(const __grid_constant__ GgParams<T> g)
+template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC, int G>
+__global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(const __grid_constant__ GgParams<T, G> g)
 {
-    pdl_wait();
     typedef GgCfg<T, BM, BN, WM, WN, WK, KC, ST> Cfg;
     constexpr int NT = Cfg::NT, PAD = Cfg::PAD, PK = Cfg::PK, PA_R = Cfg::PA_R, PB_R = Cfg::PB_R;
     extern __shared__ __align__(16) unsigned char gg_smem[];
@@ -208,28 +216,37 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     int pi = 0;
-    while (pi + 1 < g.count && (int)blockIdx.x >= g.p[pi + 1].first) pi++;
-    const GgProb<T> &p = g.p[pi];
-    const int local = (int)blockIdx.x - p.first;
-    const int split = local % p.splits, tile = local / p.splits;
-    const int b = tile / p.tiles_nm, t2 = tile % p.tiles_nm;
-    const int i0 = (t2 / p.tiles_m) * BM, j0 = (t2 % p.tiles_m) * BN;
+#pragma unroll
+    for (int i = 1; i < G; i++) pi += (int)blockIdx.x >= g.first[i];
+    const GgProb<T> &p = g.p[G == 1 ? 0 : pi];
+    const int local = (int)blockIdx.x - (G == 1 ? 0 : g.first[pi]);
+    const int tile = gg_quot(local, p.splits), split = local - tile * p.splits.d;
+    const int b = gg_quot(tile, p.tiles_nm), t2 = tile - b * p.tiles_nm.d, trow = gg_quot(t2, p.tiles_m);
+    const int i0 = trow * BM, j0 = (t2 - trow * p.tiles_m.d) * BN;
     const int a_kc = p.a_kc, b_kc = p.b_kc;
-    const int per = (p.chunks + p.splits - 1) / p.splits, ch0 = split * per, nch = min(p.chunks - ch0, per);
-    const int K = p.K, cps = p.chunks / p.segs;                            // chunks of a segment
+    const int ch0 = split * p.per, nch = min(p.chunks - ch0, p.per);
+    const int K = p.K, cps = p.cps.d;                                      // chunks of a segment
 
     // walk of the copies: chunk within its segment, segment
     GgLoader<T, BM, KC, PAD, NT> la;
     GgLoader<T, BN, KC, PAD, NT> lb;
-    int f_seg = ch0 / cps, f_c = ch0 % cps, f_left = nch;
+    int f_seg = gg_quot(ch0, p.cps), f_c = ch0 - f_seg * cps, f_left = nch;
+    const int c_first = f_c;
     auto open_segment = [&]() {
         const T *A, *B;
         if (p.seg_list) { A = f_seg == 0 ? p.A[0] : f_seg == 1 ? p.A[1] : p.A[2]; B = f_seg == 0 ? p.B[0] : f_seg == 1 ? p.B[1] : p.B[2]; }
         else { A = p.A[0] + f_seg * p.a_ks; B = p.B[0] + f_seg * p.b_ks; }
-        la.init(A + b * p.a_bs, a_kc, p.a_vw, i0, f_c * KC, p.N, p.a_cs, p.a_ss_);
-        lb.init(B + b * p.b_bs, b_kc, p.b_vw, j0, f_c * KC, p.M, p.b_cs, p.b_ss_);
+        la.init(A + b * p.a_bs, a_kc, p.a_vl, i0, f_c * KC, p.N, p.a_cs, p.a_ss_);
+        lb.init(B + b * p.b_bs, b_kc, p.b_vl, j0, f_c * KC, p.M, p.b_cs, p.b_ss_);
     };
     open_segment();
+    // what the end of the kernel reads of its parameters: a first read of one misses the constant cache
+    T *C = p.C + b * p.c_bs;
+    const long long c_rs = p.c_rs, c_cs = p.c_cs;
+    const float alpha = p.alpha;
+    const int plain = p.plain, nsplits = p.splits.d;
+    asm volatile("" ::"l"(C), "l"(c_rs), "l"(c_cs), "f"(alpha), "r"(plain));
+    pdl_wait();                                                            // everything above reads parameters only
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(gg_smem);
     auto fetch = [&](int stage) {
         if (f_left > 0) {
@@ -263,7 +280,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
     }
 
     for (int s = 0; s < ST - 1; s++) fetch(s);
-    int cur = 0, c_c = ch0 % cps;
+    int cur = 0, c_c = c_first;
     for (int ch = 0; ch < nch; ch++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncthreads();
@@ -315,9 +332,9 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
     __syncthreads();
 
     constexpr int Q = BN / 4, QUADS = BM * Q;                              // four neighbouring columns per thread
-    if (p.splits > 1) {
+    if (nsplits > 1) {
         __shared__ unsigned ticket_s;
-        float *part = p.part + ((size_t)tile * p.splits + split) * (BM * BN);
+        float *part = p.part + ((size_t)tile * nsplits + split) * (BM * BN);
         for (int e = tid; e < QUADS; e += NT) {
             const int i = e / Q, j = (e % Q) * 4;
             float4 v = *reinterpret_cast<const float4 *>(red + i * Cfg::RED_P + j);
@@ -329,72 +346,77 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
         __syncthreads();
         if (tid == 0) ticket_s = atomicAdd(&gg_tickets[p.ticket0 + tile], 1u);
         __syncthreads();
-        if (ticket_s != (unsigned)(p.splits - 1)) return;
+        if (ticket_s != (unsigned)(nsplits - 1)) return;
         __threadfence();
         if (tid == 0) gg_tickets[p.ticket0 + tile] = 0;
     }
-    T *C = p.C + b * p.c_bs;
-    const bool pair = p.c_cs == 1 && (p.c_rs & 3) == 0 && (((uintptr_t)C) & (4 * sizeof(T) - 1)) == 0;
     for (int e = tid; e < QUADS; e += NT) {
         const int i = e / Q, j = (e % Q) * 4;
         if (i0 + i >= p.N || j0 + j >= p.M) continue;
         float4 v;
-        if (p.splits > 1) {
-            const float4 *src = reinterpret_cast<const float4 *>(p.part + (size_t)tile * p.splits * (BM * BN)) + e;
+        if (nsplits > 1) {
+            const float4 *src = reinterpret_cast<const float4 *>(p.part + (size_t)tile * nsplits * (BM * BN)) + e;
             v = __ldcg(src);
 #pragma unroll 4
-            for (int s = 1; s < p.splits; s++) { const float4 u = __ldcg(src + (size_t)s * QUADS); v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w; }
+            for (int s = 1; s < nsplits; s++) { const float4 u = __ldcg(src + (size_t)s * QUADS); v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w; }
         } else {
             v = *reinterpret_cast<const float4 *>(red + i * Cfg::RED_P + j);
 #pragma unroll
             for (int w = 1; w < WK; w++) { const float4 u = *reinterpret_cast<const float4 *>(red + (w * BM + i) * Cfg::RED_P + j); v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w; }
         }
-        float r[4] = {v.x * p.alpha, v.y * p.alpha, v.z * p.alpha, v.w * p.alpha};
-        T *dst = C + (long long)(i0 + i) * p.c_rs + (long long)(j0 + j) * p.c_cs;
+        float r[4] = {v.x * alpha, v.y * alpha, v.z * alpha, v.w * alpha};
+        T *dst = C + (long long)(i0 + i) * c_rs + (long long)(j0 + j) * c_cs;
         const int live = min(4, p.M - j0 - j);
-        const float brow = p.bias_mode == 1 ? ld(p.bias + i0 + i) : 0.f;
+        bool whole = plain && live == 4;
+        if (!whole) {
+            const float brow = p.bias_mode == 1 ? ld(p.bias + i0 + i) : 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (q >= live) break;
-            if (p.accumulate) r[q] += ld(dst + q * p.c_cs);
-            if (p.bias_mode == 1) r[q] += brow; else if (p.bias_mode == 2) r[q] += ld(p.bias + j0 + j + q);
-        }
-        if (pair && live == 4) {
-            if constexpr (HALF) {
-                __half2 h0 = __floats2half2_rn(r[0], r[1]), h1 = __floats2half2_rn(r[2], r[3]);
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<uint32_t *>(&h0), *reinterpret_cast<uint32_t *>(&h1));
-            } else *reinterpret_cast<float4 *>(dst) = make_float4(r[0], r[1], r[2], r[3]);
-        } else {
+            for (int q = 0; q < 4; q++) {
+                if (q >= live) break;
+                if (p.accumulate) r[q] += ld(dst + q * c_cs);
+                if (p.bias_mode == 1) r[q] += brow; else if (p.bias_mode == 2) r[q] += ld(p.bias + j0 + j + q);
+            }
+            whole = p.quads && live == 4;
+            if (!whole) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) if (q < live) st(dst + q * p.c_cs, r[q]);
+                for (int q = 0; q < 4; q++) if (q < live) st(dst + q * c_cs, r[q]);
+            }
         }
+        if (!whole) continue;
+        if constexpr (HALF) {
+            __half2 h0 = __floats2half2_rn(r[0], r[1]), h1 = __floats2half2_rn(r[2], r[3]);
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<uint32_t *>(&h0), *reinterpret_cast<uint32_t *>(&h1));
+        } else *reinterpret_cast<float4 *>(dst) = make_float4(r[0], r[1], r[2], r[3]);
     }
 }
 
 // ---------------------------------------------------------------- host side
 // Which of an operand's two indices runs along shared-memory rows, and how wide its copies may be.
 template <class T> static void gg_operand(const T *const *ptrs, int nptr, long long rs, long long ks, long long bs, int batch, long long seg, int segs, bool list,
-                                          int &kc, int &vw, long long &cs, long long &ss)
+                                          int &kc, int &vl, long long &cs, long long &ss)
 {
     kc = ks == 1 || (rs != 1 && std::llabs(ks) <= std::llabs(rs));
     cs = kc ? ks : rs; ss = kc ? rs : ks;
     constexpr int V16 = 16 / (int)sizeof(T), V4 = 4 / (int)sizeof(T);
-    vw = 1;
+    vl = 0;                                                                // one element
     if (cs != 1) return;
     auto fits = [&](int v) {
         const size_t mask = (size_t)v * sizeof(T) - 1;
         for (int i = 0; i < nptr; i++) if (((uintptr_t)ptrs[i]) & mask) return false;
         return ss % v == 0 && (batch == 1 || bs % v == 0) && (list || segs == 1 || seg % v == 0);
     };
-    if (fits(V16)) vw = V16; else if (V4 > 1 && fits(V4)) vw = V4;
+    if (fits(V16)) vl = sizeof(T) == 4 ? 2 : 3; else if (V4 > 1 && fits(V4)) vl = 1;
 }
 
-template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC>
+// CYC: cycles of one K chunk in a CTA (measured with the SMs about as full as such products make them), in units of those of a split:
+// writing the partial tile, the ticket and the last CTA's sum cost 2500 cycles, and 150 more per split.
+template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC, int CYC, int G>
 static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
 {
     typedef GgCfg<T, BM, BN, WM, WN, WK, KC, ST> Cfg;
-    GgParams<T> g;
-    g.count = count;
+    GgParams<T, G> g;
+    for (int i = 0; i < G; i++) g.first[i] = 0x7fffffff;
+    int tiles_of[GG_MAX];
     long long tiles_all = 0, tile_steps = 0;
     int shortest = 1 << 30;
     for (int i = 0; i < count; i++) {
@@ -409,49 +431,56 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
         p.a_ks = tr ? s.b_ks : s.a_ks; p.b_ks = tr ? s.a_ks : s.b_ks;
         p.c_rs = tr ? s.c_cs : s.c_rs; p.c_cs = tr ? s.c_rs : s.c_cs;
         const int np = s.seg_list ? s.segs : 1;
-        gg_operand<T>(p.A, np, a_rs, a_ks_, p.a_bs, s.batch, p.a_ks, s.segs, s.seg_list != 0, p.a_kc, p.a_vw, p.a_cs, p.a_ss_);
-        gg_operand<T>(p.B, np, b_rs_, b_ks_, p.b_bs, s.batch, p.b_ks, s.segs, s.seg_list != 0, p.b_kc, p.b_vw, p.b_cs, p.b_ss_);
+        gg_operand<T>(p.A, np, a_rs, a_ks_, p.a_bs, s.batch, p.a_ks, s.segs, s.seg_list != 0, p.a_kc, p.a_vl, p.a_cs, p.a_ss_);
+        gg_operand<T>(p.B, np, b_rs_, b_ks_, p.b_bs, s.batch, p.b_ks, s.segs, s.seg_list != 0, p.b_kc, p.b_vl, p.b_cs, p.b_ss_);
         p.alpha = s.alpha; p.accumulate = s.accumulate ? 1 : 0;
         p.bias_mode = s.bias ? (tr && s.bias_mode ? 3 - s.bias_mode : s.bias_mode) : 0;
-        p.tiles_m = ceil_div(p.M, BN); p.tiles_nm = p.tiles_m * ceil_div(p.N, BM);
-        p.chunks = p.segs * ceil_div(p.K, KC);
-        p.splits = 1; p.part = nullptr; p.ticket0 = 0;
-        tiles_all += (long long)p.tiles_nm * s.batch;
+        const int tiles_m = ceil_div(p.M, BN);
+        tiles_of[i] = tiles_m * ceil_div(p.N, BM);
+        p.tiles_m = gg_div(std::max(1, tiles_m), tiles_of[i]); p.tiles_nm = gg_div(tiles_of[i], (long long)tiles_of[i] * s.batch);
+        p.chunks = p.segs * ceil_div(p.K, KC); p.cps = gg_div(std::max(1, ceil_div(p.K, KC)), p.chunks);
+        p.quads = p.c_cs == 1 && (p.c_rs & 3) == 0 && (s.batch == 1 || (p.c_bs & 3) == 0) && (((uintptr_t)p.C) & (4 * sizeof(T) - 1)) == 0;
+        p.plain = p.quads && !p.accumulate && !p.bias_mode;
+        p.part = nullptr; p.ticket0 = 0;
+        tiles_all += (long long)tiles_of[i] * s.batch;
         shortest = std::min(shortest, p.chunks);
-        tile_steps += (long long)p.tiles_nm * s.batch * p.chunks;
+        tile_steps += (long long)tiles_of[i] * s.batch * p.chunks;
     }
-    // Split K over CTAs while the group leaves SMs idle: enough CTAs for two per SM, never less than 256 of K each (a
-    // split costs a round trip through L2 and the sum of the last CTA).
-    constexpr int MIN_CH = KC >= 256 ? 1 : 256 / KC;
+    // Split K over CTAs while the group leaves SMs idle, up to enough CTAs for two per SM, and only as far as the chunks saved are worth it
+    // (128 x 512 x 128 in fp16, 32 tiles: two splits 6300 cycles, none 4700).
     const long long want = 2ll * sm_count();
     int ticket = 0;
     long long first = 0;
     for (int i = 0; i < count; i++) {
         GgProb<T> &p = g.p[i];
-        const long long tiles = (long long)p.tiles_nm * list[i].batch;
+        const long long tiles = (long long)tiles_of[i] * list[i].batch;
+        int splits = 1;
         // this product's share of the wanted CTAs, per tile; in a group that fills the SMs, a contraction much longer than the
         // shortest one (three segments beside products of one) is cut to about that length
-        long long s = tiles_all < sm_count() ? (want * p.chunks + tile_steps - 1) / tile_steps
-                                             : (tiles_all < 4 * sm_count() && p.chunks >= 2 * shortest ? p.chunks / std::max(shortest, MIN_CH) : 1);
-        if (s > 1 && p.chunks >= 2 * MIN_CH) {
-            s = std::min<long long>(std::min<long long>(s, p.chunks / MIN_CH), 64);
-            if (s > 1 && ticket + tiles <= 16384) {
-                const int per = ceil_div(p.chunks, (int)s);
-                p.splits = ceil_div(p.chunks, per);
-                if (p.splits > 1) {
-                    p.part = sc.try_scratch<float>((size_t)tiles * p.splits * BM * BN);
-                    if (p.part) { p.ticket0 = ticket; ticket += (int)tiles; }
-                    else p.splits = 1;
-                }
+        const bool filled = tiles_all >= sm_count();
+        const long long most = !filled ? (want * p.chunks + tile_steps - 1) / std::max(1ll, tile_steps) : (tiles_all < 4 * sm_count() && p.chunks >= 2 * shortest ? p.chunks / std::max(shortest, 1) : 1);
+        if (most > 1 && p.chunks >= 2) {
+            const int cap = (int)std::min<long long>(std::min<long long>(most, p.chunks), 64);
+            long long best = (long long)p.chunks * CYC;
+            for (int s = 2; s <= cap; s++) {
+                const int per = ceil_div(p.chunks, s);
+                const long long cost = (long long)per * CYC + 2500 + 150 * s;
+                if (cost < best) { best = cost; splits = ceil_div(p.chunks, per); }
+            }
+            if (splits > 1) {
+                if (ticket + tiles <= 16384) p.part = sc.try_scratch<float>((size_t)tiles * splits * BM * BN);
+                if (p.part) { p.ticket0 = ticket; ticket += (int)tiles; }
+                else splits = 1;
             }
         }
-        p.first = (int)first;
-        first += tiles * p.splits;
+        p.splits = gg_div(splits, tiles * splits); p.per = ceil_div(p.chunks, splits);
+        g.first[i] = (int)first;
+        first += tiles * splits;
     }
-    auto kern = gemm_group_kernel<T, BM, BN, WM, WN, WK, KC, ST, OCC>;
+    auto kern = gemm_group_kernel<T, BM, BN, WM, WN, WK, KC, ST, OCC, G>;
     static bool attr_set = false;
     if (!attr_set) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM); attr_set = true; }
-    TL_LAUNCH((gemm_group_kernel<T, BM, BN, WM, WN, WK, KC, ST, OCC>), (unsigned)first, Cfg::NT, Cfg::SMEM, g);
+    TL_LAUNCH((gemm_group_kernel<T, BM, BN, WM, WN, WK, KC, ST, OCC, G>), (unsigned)first, Cfg::NT, Cfg::SMEM, g);
 }
 
 template <class T> void gemm_group(const GemmGroup<T> *list, int count)
@@ -474,14 +503,16 @@ template <class T> void gemm_group(const GemmGroup<T> *list, int count)
     // fp32, us: 256^3 4.8 with 16 x 32 tiles, 6.1 with 32 x 32; 2000x50x2000 46 and 35.  fp16: 128x512x128 4.9 with 16 x 32,
     // 5.7 with 32 x 32, 9.7 with 64 x 64; 1000x60x1000 11.8, 10.3, 6.4.  Four warps per CTA, several CTAs per SM: eight warps
     // on one 32 x 32 fp32 tile cost 20 to 40 % more (shorter runs of FMAs between barriers).
+#define GG_LAUNCH(...) do { if (n == 1) gg_launch<T, __VA_ARGS__, 1>(sc, live, n); else gg_launch<T, __VA_ARGS__, GG_MAX>(sc, live, n); } while (0)
     if constexpr (sizeof(T) == 2) {
-        if (tiles64 >= sm_count()) gg_launch<T, 64, 64, 2, 2, 1, 64, 3, 3>(sc, live, n);
-        else if (tiles32 >= sm_count()) gg_launch<T, 32, 32, 1, 1, 4, 128, 3, 4>(sc, live, n);
-        else gg_launch<T, 16, 32, 1, 1, 4, 128, 3, 4>(sc, live, n);
+        if (tiles64 >= sm_count()) GG_LAUNCH(64, 64, 2, 2, 1, 64, 3, 3, 900);
+        else if (tiles32 >= sm_count()) GG_LAUNCH(32, 32, 1, 1, 4, 128, 3, 4, 700);
+        else GG_LAUNCH(16, 32, 1, 1, 4, 128, 3, 4, 500);
     } else {
-        if (2 * tiles32 >= 3 * sm_count()) gg_launch<T, 32, 32, 2, 1, 2, 64, 3, 4>(sc, live, n);
-        else gg_launch<T, 16, 32, 1, 1, 4, 64, 3, 4>(sc, live, n);
+        if (2 * tiles32 >= 3 * sm_count()) GG_LAUNCH(32, 32, 2, 1, 2, 64, 3, 4, 2500);
+        else GG_LAUNCH(16, 32, 1, 1, 4, 64, 3, 4, 1200);
     }
+#undef GG_LAUNCH
 }
 template void gemm_group<float>(const GemmGroup<float> *, int);
 template void gemm_group<__half>(const GemmGroup<__half> *, int);
