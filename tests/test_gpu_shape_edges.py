@@ -68,6 +68,45 @@ def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
     test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
 
 
+# half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
+# tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
+# for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
+@pytest.mark.parametrize("L,E,Fd,heads", [(203, 24, 96, 8), (400, 16, 64, 4), (97, 16, 544, 16), (512, 8, 24, 3), (333, 12, 1280, 5)])
+def test_half_precision_attention_core(pkg, gpulib, L, E, Fd, heads):
+    gpulib.trainlib_set_streams(1)
+    rng = seeded(L + E + Fd)
+    half = lambda *s: rng.standard_normal(s).astype(np.float16).astype(F)
+    x, dy = half(E, L), half(E, L)
+    ws = [(half(E, Fd) / np.sqrt(E)).astype(np.float16).astype(F) for _ in range(3)] + [(half(E, Fd) / np.sqrt(Fd)).astype(np.float16).astype(F)]
+    zb = np.zeros(Fd, F)
+    r = AbiRunner(pkg, gpulib, device=True, half=True)
+    gpulib.trainlib_profile(1)
+    got = {k: v.astype(np.float64) for k, v in r.mhsa(x, ws[0], ws[1], ws[2], zb, zb, zb, ws[3], dy, L, E, Fd, heads).items()}
+    gpulib.trainlib_profile(0)
+    assert sum("mma_attn" in t[0] for t in pkg.profile_table(gpulib)) == 3
+    r.close()
+    H = Fd // heads
+    hd = lambda k: got[k].reshape(heads, H, L)
+    P, dP, scale = got["softmax"].reshape(heads, L, L), got["dsoftmax"].reshape(heads, L, L), 1 / np.sqrt(H)
+    u = 2.0 ** -11
+    def close(a, b, terms, what):
+        # the error bound of a sum is that of its terms' absolute values; the largest of them against the largest result
+        assert np.abs(a - b).max() <= 1.05 * terms, "%s: %.2e of %.2e" % (what, np.abs(a - b).max(), terms)
+    att = np.einsum("hdk,hqk->hdq", hd("v"), P)
+    close(hd("att"), att, u * (np.abs(att).max() + np.einsum("hdk,hqk->hdq", np.abs(hd("v")), P).max()), "att")
+    want = np.einsum("hdq,hdk->hqk", hd("datt"), hd("v"))
+    close(dP, want, u * np.abs(want).max() + 2.0 ** -24, "dP")
+    dv = np.einsum("hdq,hqk->hdk", hd("datt"), P)
+    close(hd("dv"), dv, u * (np.abs(dv).max() + np.einsum("hdq,hqk->hdk", np.abs(hd("datt")), P).max()) + 2.0 ** -24, "dv")
+    # dS = (dP - sum dP P) P from the rounded dP and P, as the kernels form it
+    dS = (dP - (dP * P).sum(-1, keepdims=True)) * P
+    dq, dk = scale * np.einsum("hdk,hqk->hdq", hd("k"), dS), scale * np.einsum("hdq,hqk->hdk", hd("q"), dS)
+    for k, w, m in (("dq", dq, np.einsum("hdk,hqk->hdq", np.abs(hd("k")), np.abs(dS)).max()), ("dk", dk, np.einsum("hdq,hqk->hdk", np.abs(hd("q")), np.abs(dS)).max())):
+        close(hd(k), w, u * np.abs(w).max() + 2.0 ** -18 * scale * m + 2.0 ** -24 + 2e-3 * np.abs(w).max(), k)      # (the layer's 1/sqrt is one Newton step: 1.8e-3)
+    # the probabilities sum to one up to their rounding
+    assert np.abs(P.sum(-1) - 1).max() <= u * (1 + 1e-3) + L * 2.0 ** -25
+
+
 @pytest.mark.parametrize("c,h,w,k,pad,n", [(5, 9, 7, 3, 1, 3), (64, 28, 28, 3, 1, 4), (3, 33, 18, 3, 0, 2), (8, 6, 6, 5, 2, 9), (2, 40, 41, 3, 2, 1), (7, 4, 4, 3, 1, 700), (4, 12, 12, 4, 1, 2)])
 def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
     g = geom(c, h, w, c, k, stride=stride, pad=pad)
