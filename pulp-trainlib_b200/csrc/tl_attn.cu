@@ -40,8 +40,18 @@ __device__ __forceinline__ void tile_from_rows(const float *a_tile, const T *__r
         float acc[ATT_TQ] = {0.f, 0.f, 0.f, 0.f};
         for (int d0 = 0; d0 < H; d0 += B) {
             float m[B];
+            if constexpr (sizeof(T) == 4) {
 #pragma unroll
-            for (int u = 0; u < B; u++) m[u] = d0 + u < H ? ld(M + (size_t)(d0 + u) * L + j) : 0.f;
+                for (int u = 0; u < B; u++) m[u] = d0 + u < H ? M[(size_t)(d0 + u) * L + j] : 0.f;
+            } else {
+                // rows past the last are fetched from it and replaced by zero: under a condition, a load and its conversion from half
+                // precision were waited for one by one (16 x 240 cycles); in fp32 the clamps cost more than they save
+                T raw[B];
+#pragma unroll
+                for (int u = 0; u < B; u++) raw[u] = M[(size_t)min(d0 + u, H - 1) * L + j];
+#pragma unroll
+                for (int u = 0; u < B; u++) m[u] = d0 + u < H ? __half2float(raw[u]) : 0.f;
+            }
 #pragma unroll
             for (int u = 0; u < B; u++) {
                 const float4 a = *reinterpret_cast<const float4 *>(a_tile + min(d0 + u, H - 1) * ATT_TQ);
@@ -69,10 +79,22 @@ __device__ __forceinline__ void rows_times_tile(const T *__restrict__ M, const f
         for (int i = 0; i < R * ATT_TQ; i++) acc[i] = 0.f;
         for (int j0 = 0; j0 < L; j0 += 32 * U) {
             float m[U][R];
+            if constexpr (sizeof(T) == 4) {
 #pragma unroll
-            for (int u = 0; u < U; u++)
+                for (int u = 0; u < U; u++)
 #pragma unroll
-                for (int r = 0; r < R; r++) m[u][r] = j0 + 32 * u + lane < L ? ld(row[r] + j0 + 32 * u + lane) : 0.f;
+                    for (int r = 0; r < R; r++) m[u][r] = j0 + 32 * u + lane < L ? row[r][j0 + 32 * u + lane] : 0.f;
+            } else {
+                T raw[U][R];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int r = 0; r < R; r++) raw[u][r] = row[r][min(j0 + 32 * u + lane, L - 1)];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int r = 0; r < R; r++) m[u][r] = j0 + 32 * u + lane < L ? __half2float(raw[u][r]) : 0.f;
+            }
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 if (j0 + 32 * u >= L) break;
