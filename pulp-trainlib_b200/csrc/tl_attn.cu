@@ -136,7 +136,7 @@ __device__ __forceinline__ void load_a_tile(const T *__restrict__ A, float *a_ti
 {
     for (int i = threadIdx.x; i < H * ATT_TQ; i += ATT_THREADS) {
         const int d = i / ATT_TQ, t = i % ATT_TQ;
-        a_tile[i] = (t0 + t < L) ? ld(A + (size_t)d * L + t0 + t) : 0.f;
+        a_tile[i] = ld0(t0 + t < L, A + (size_t)d * L + t0 + t);
     }
 }
 
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_query_kernel(const T *__r
         for (int j0 = 0; j0 < L; j0 += 256) {
             float p[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) p[u] = j0 + 32 * u + lane < L ? ld(P + roff + j0 + 32 * u + lane) : 0.f;
+            for (int u = 0; u < 8; u++) p[u] = ld0(j0 + 32 * u + lane < L, P + roff + j0 + 32 * u + lane);
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int j = j0 + 32 * u + lane;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_query_kernel(const T *__r
         for (int j0 = 0; j0 < L; j0 += 256) {
             float p[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) p[u] = j0 + 32 * u + lane < L ? ld(P + roff + j0 + 32 * u + lane) : 0.f;
+            for (int u = 0; u < 8; u++) p[u] = ld0(j0 + 32 * u + lane < L, P + roff + j0 + 32 * u + lane);
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int j = j0 + 32 * u + lane;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_key_kernel(const T *__res
         if (vec) { ld4(P + off, p); ld4(dP + off, g); }
         else {
 #pragma unroll
-            for (int kk = 0; kk < ATT_TQ; kk++) { p[kk] = kk < nk ? ld(P + off + kk) : 0.f; g[kk] = kk < nk ? ld(dP + off + kk) : 0.f; }
+            for (int kk = 0; kk < ATT_TQ; kk++) { p[kk] = ld0(kk < nk, P + off + kk); g[kk] = ld0(kk < nk, dP + off + kk); }
         }
 #pragma unroll
         for (int kk = 0; kk < ATT_TQ; kk++) { p_tile[kk * Lp + query] = p[kk]; ds_tile[kk * Lp + query] = __fmul_rn(__fsub_rn(g[kk], dot), p[kk]); }
@@ -292,7 +292,7 @@ __device__ __forceinline__ void am_ld4(const __half *p, int left, bool vec, floa
 {
     if (vec && left >= 4) { ld4(p, v); return; }
 #pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = i < left ? ld(p + i) : 0.f;
+    for (int i = 0; i < 4; i++) v[i] = ld0(i < left, p + i);
 }
 
 // tile[row][j] = alpha * sum_d cols[d][row] M[d][j] for the sixteen rows and j < L, zero for L <= j < the next multiple of 16
@@ -316,7 +316,7 @@ __device__ __forceinline__ void am_scores(const float *cols, const __half *__res
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const int d = d0 + 8 * u + t + 4 * h, n = n0 + 8 * i + g;
-                        m[u][i][h] = d < H && n < L ? ld(M + (size_t)d * L + n) : 0.f;
+                        m[u][i][h] = ld0(d < H && n < L, M + (size_t)d * L + n);
                     }
 #pragma unroll
             for (int i = 0; i < NTL; i++)
@@ -424,7 +424,7 @@ template <int NT> __device__ __forceinline__ void am_columns(const __half *__res
 {
     for (int i = threadIdx.x; i < ((H + 31) & ~31) * AM_Q; i += NT) {
         const int d = i / AM_Q, c = i % AM_Q;
-        cols[d * AM_AP + c] = d < H && t0 + c < L ? ld(A + (size_t)d * L + t0 + c) : 0.f;
+        cols[d * AM_AP + c] = ld0(d < H && t0 + c < L, A + (size_t)d * L + t0 + c);
     }
 }
 
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(NT) mma_attn_bw_query_kernel(const __half *__r
         for (int j0 = 0; j0 < L; j0 += 256) {
             float p[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) p[u] = j0 + 32 * u + lane < L ? ld(P + roff + j0 + 32 * u + lane) : 0.f;
+            for (int u = 0; u < 8; u++) p[u] = ld0(j0 + 32 * u + lane < L, P + roff + j0 + 32 * u + lane);
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int j = j0 + 32 * u + lane;
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(NT) mma_attn_bw_query_kernel(const __half *__r
         for (int j0 = 0; j0 < L; j0 += 256) {
             float p[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) p[u] = j0 + 32 * u + lane < L ? ld(P + roff + j0 + 32 * u + lane) : 0.f;
+            for (int u = 0; u < 8; u++) p[u] = ld0(j0 + 32 * u + lane < L, P + roff + j0 + 32 * u + lane);
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int j = j0 + 32 * u + lane;

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) dw_plane_kernel(const __grid_constant__ D
     for (int e = threadIdx.x; e < np * P; e += 256) {
         const int g = dw_quot(e, p.dP), rc = e - g * P, r = dw_quot(rc, p.dPW), c = rc - r * p.PW;
         const int h = r + p.r0, x = c + p.c0;
-        win[e] = ((unsigned)h < (unsigned)p.Hs && (unsigned)x < (unsigned)p.Ws) ? ld(s0 + (g * p.Hs + h) * p.Ws + x) : 0.f;
+        win[e] = ld0((unsigned)h < (unsigned)p.Hs && (unsigned)x < (unsigned)p.Ws, s0 + (g * p.Hs + h) * p.Ws + x);
     }
     for (int e = threadIdx.x; e < np * KK; e += 256) {
         const int g = e / KK, t = e - g * KK;
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) dw_wg_plane_kernel(const __grid_constant_
         for (int e = threadIdx.x; e < ns * P; e += 256) {
             const int g = dw_quot(e, p.dP), rc = e - g * P, r = dw_quot(rc, p.dPW), c = rc - r * p.PW;
             const int h = r + p.r0, xx = c + p.c0;
-            dw_smem[e] = ((unsigned)h < (unsigned)p.Hs && (unsigned)xx < (unsigned)p.Ws) ? ld(x + (((long long)(s + g) * p.C + ch) * p.Hs + h) * p.Ws + xx) : 0.f;
+            dw_smem[e] = ld0((unsigned)h < (unsigned)p.Hs && (unsigned)xx < (unsigned)p.Ws, x + (((long long)(s + g) * p.C + ch) * p.Hs + h) * p.Ws + xx);
         }
         __syncthreads();
 #pragma unroll 2
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(128) dw3_wg_kernel(const __grid_constant__ Dw3
             if (p.vec_o) { const float4 t = dw_ld4(dp); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
             else {
 #pragma unroll
-                for (int k = 0; k < 4; k++) d[k] = 4 * j4 + k < p.Wo ? ld(dp + k) : 0.f;
+                for (int k = 0; k < 4; k++) d[k] = ld0(4 * j4 + k < p.Wo, dp + k);
             }
             const float *b = dw_smem + g * P + i * p.PW + 4 * j4;
 #pragma unroll

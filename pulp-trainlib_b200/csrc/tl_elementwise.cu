@@ -781,7 +781,7 @@ template <class T> void batchnorm_fw(const T *x, T *y, const T *w, const T *b, i
 template <class T, int NV> __device__ __forceinline__ void ln_load(const T *__restrict__ p, int width, int lane, float (&v)[NV])
 {
 #pragma unroll
-    for (int k = 0; k < NV; k++) { const int j = lane + 32 * k; v[k] = j < width ? ld(p + j) : 0.f; }
+    for (int k = 0; k < NV; k++) { const int j = lane + 32 * k; v[k] = ld0(j < width, p + j); }
 }
 // mean and standard deviation of a row  [ref: lib/sources/pulp_layernorm_fp32.c:60-77]
 __device__ __forceinline__ void ln_stats(float s1, float s2, int width, float eps, float &mean, float &sv)

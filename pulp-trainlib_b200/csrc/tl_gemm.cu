@@ -49,14 +49,14 @@ gemm_ffma_kernel(GemmDesc<T> d)
             const int e = tid + q * NT;
             int i, k;
             if (a_k_contig) { i = e / BK; k = e % BK; } else { k = e / BM; i = e % BM; }
-            ra[q] = (i0 + i < d.N && k0 + k < d.K) ? ld(A + (long long)(i0 + i) * d.a_rs + (long long)(k0 + k) * d.a_cs) : 0.f;
+            ra[q] = ld0(i0 + i < d.N && k0 + k < d.K, A + (long long)(i0 + i) * d.a_rs + (long long)(k0 + k) * d.a_cs);
         }
 #pragma unroll
         for (int q = 0; q < BE; q++) {
             const int e = tid + q * NT;
             int j, k;
             if (b_k_contig) { j = e / BK; k = e % BK; } else { k = e / BN; j = e % BN; }
-            rb[q] = (j0 + j < d.M && k0 + k < d.K) ? ld(B + (long long)(k0 + k) * d.b_rs + (long long)(j0 + j) * d.b_cs) : 0.f;
+            rb[q] = ld0(j0 + j < d.M && k0 + k < d.K, B + (long long)(k0 + k) * d.b_rs + (long long)(j0 + j) * d.b_cs);
         }
     };
     auto stash = [&](int stage) {
@@ -467,7 +467,7 @@ template <class T, int V> __device__ __forceinline__ void linear_bw_body(LBW_PAR
         for (int o = slab * rows_per_slab + (int)threadIdx.x; o < o_end; o += LBW_STRIPS * LBW_LANES) db[o] = dy[o];
     float acc[V], xv[V];
 #pragma unroll
-    for (int q = 0; q < V; q++) { acc[q] = 0.f; xv[q] = live ? ld(x + col0 + q) : 0.f; }
+    for (int q = 0; q < V; q++) { acc[q] = 0.f; xv[q] = ld0(live, x + col0 + q); }
     if (live && V <= 2) {
         // narrow strips: the elements of sixteen rows are on their way before the first is used
         constexpr int U = 16;
@@ -480,7 +480,7 @@ template <class T, int V> __device__ __forceinline__ void linear_bw_body(LBW_PAR
                 const T *p = W + (long long)min(o, o_end - 1) * in + col0;
                 if constexpr (V == 2 && sizeof(T) == 2) *reinterpret_cast<__half2 *>(w[u]) = __ldcs(reinterpret_cast<const __half2 *>(p));
                 else w[u][0] = __ldcs(p);
-                g[u] = o < o_end ? ld(dy + o) : 0.f;
+                g[u] = ld0(o < o_end, dy + o);
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {

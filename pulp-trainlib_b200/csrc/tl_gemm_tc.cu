@@ -90,7 +90,7 @@ __device__ __forceinline__ void gt_stage(const T *__restrict__ base, long long r
             float t[KC];
 #pragma unroll
             for (int j = 0; j < KC; j++)
-                t[j] = (row0 + r < rows_valid && k + j < K) ? ld(base + (long long)(row0 + r) * rs + (long long)(k + j) * cs) : 0.f;
+                t[j] = ld0(row0 + r < rows_valid && k + j < K, base + (long long)(row0 + r) * rs + (long long)(k + j) * cs);
             const uint32_t off = (uint32_t)c * LBO + (uint32_t)(r >> 3) * 128u + (uint32_t)(r & 7) * 16u;
             if constexpr (sizeof(T) == 2) {
                 uint32_t w[4];

@@ -113,7 +113,7 @@ template <class T> __device__ __forceinline__ void tm_store4(const TmParams &p, 
     const T *bias = reinterpret_cast<const T *>(p.bias);
     const int live = min(4, p.M - col);
     float r[4];
-    const float brow = p.bias_mode == 1 ? ld(bias + row) : 0.f;
+    const float brow = ld0(p.bias_mode == 1, bias + row);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         r[q] = p.alpha * in[q] + brow;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(TM_THREADS) gemm_tma_kernel(const __grid_const
                     const bool whole = !p.accumulate && col0 + c0 + 32 <= p.M;
                     if (whole && (vec || p.c_rs == 1)) {
                         const T *bias = reinterpret_cast<const T *>(p.bias);
-                        const float brow = p.bias_mode == 1 ? ld(bias + row) : 0.f;
+                        const float brow = ld0(p.bias_mode == 1, bias + row);
 #pragma unroll
                         for (int j = 0; j < 32; j++) v[j] = __float_as_uint(p.alpha * __uint_as_float(v[j]) + brow);
                         if (p.bias_mode == 2) {
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(const __grid_constant_
             const T *p = s + (long long)rr * o.rs + (long long)(k0 + kk) * o.cs;
             float v[8];
 #pragma unroll
-            for (int q = 0; q < 8; q++, p += 4 * o.cs) v[q] = rr < left && k0 + kk + 4 * q < o.K ? ld(p) : 0.f;
+            for (int q = 0; q < 8; q++, p += 4 * o.cs) v[q] = ld0(rr < left && k0 + kk + 4 * q < o.K, p);
 #pragma unroll
             for (int q = 0; q < 8; q++) tile[kk + 4 * q][rr] = v[q];
         }
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(const __grid_constant_
             }
         } else {
 #pragma unroll
-            for (int q = 0; q < 8; q++) v[q] = (r0 + r < o.rows && k0 + kq + q < o.K) ? ld(p + q) : 0.f;
+            for (int q = 0; q < 8; q++) v[q] = ld0(r0 + r < o.rows && k0 + kq + q < o.K, p + q);
         }
     }
     if (r0 + r >= o.rows || k0 + kq >= o.Kp) return;

@@ -253,6 +253,15 @@ template <class T> void mhsa_bw(Scope &sc, const MhsaDims &d, const T *x, const 
 // ---------------------------------------------------------------- device scalar helpers
 __device__ __forceinline__ float ld(const float *p) { return *p; }
 __device__ __forceinline__ float ld(const __half *p) { return __half2float(*p); }
+// *p, or zero where ok is false.  The half-precision form loads under the condition and converts outside of it: `ok ? ld(p) : 0` puts the
+// conversion under the condition too, and each load of a batch is then waited for where it stands (240 cycles each).
+__device__ __forceinline__ float ld0(bool ok, const float *p) { return ok ? *p : 0.f; }
+__device__ __forceinline__ float ld0(bool ok, const __half *p)
+{
+    unsigned short r = 0;
+    if (ok) r = *reinterpret_cast<const unsigned short *>(p);
+    return __half2float(__ushort_as_half(r));
+}
 __device__ __forceinline__ void st(float *p, float v) { *p = v; }
 __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
 
