@@ -216,6 +216,12 @@ def test_layernorm_shapes(run, oracle, rows, width):
             assert_close(got[k].astype(F), v, tol, k)
 
 
+# the backward pass of a few rows as one cluster: fewest and most rows and columns, and just past them
+@pytest.mark.parametrize("rows,width", [(9, 1), (128, 129), (129, 257), (512, 512), (513, 512), (512, 513), (17, 31)])
+def test_layernorm_of_one_cluster(run, oracle, rows, width):
+    test_layernorm_shapes(run, oracle, rows, width)
+
+
 @pytest.mark.parametrize("dim", [1, 5, 1023, 1025, 70001, 400000])
 def test_mse_lengths(run, oracle, dim):
     rng = seeded(dim)
