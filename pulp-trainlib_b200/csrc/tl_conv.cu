@@ -1089,6 +1089,7 @@ template <> bool try_1x1_wg<float>(Scope &sc, const ConvGeom &g, const float *x,
 // weight gradient on mma.sync: per-CTA partials + the fixed-order reduction
 template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw)
 {
+    if (conv_mma_wg_cluster<T>(g, x, dy, dw)) { profile_add_flops(conv_flops(g)); return true; }
     int groups = 0;
     const long long nw = (long long)g.Cout * g.Cin * g.Hk * g.Wk;
     const int most = (int)std::min<long long>(1 << 20, std::max<long long>(1, (64ll << 20) / nw));     // partial results: 256 MB at most
@@ -1105,7 +1106,7 @@ template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T 
 template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw, T *dbias)
 {
     defer_settle(dw);
-    if constexpr (sizeof(T) == 2) if (conv_px_wg(sc, g, x, dy, dw, dbias)) return;
+    if constexpr (sizeof(T) == 2) if (!conv_mma_wg_cluster_first(g) && conv_px_wg(sc, g, x, dy, dw, dbias)) return;
     if (dbias) channel_sum<T>(sc, dy, dbias, g.n, g.Cout, g.Hout * g.Wout);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise) {

@@ -49,10 +49,12 @@ __device__ __forceinline__ uint32_t cm_lds32(uint32_t addr) { uint32_t v; asm vo
 // A patch of the source plane(s), channels-last: `streams` x rows x cols pixels of `chans` channels (a multiple of 8 fp16 / 4
 // fp32; channels at or past c_left read as zero).  One item = one pixel x 16 bytes of channels: neighbouring threads take
 // neighbouring pixels, so the per-channel loads are coalesced and the 16-byte store is conflict-free.  Addresses are a
-// CTA-uniform base plus a 32-bit byte offset (cm_streams keeps a tile's span below 2 GB).
+// CTA-uniform base plus a 32-bit byte offset (cm_streams keeps a tile's span below 2 GB).  `warp`: this warp's place in the deal;
+// a caller that stages two things at once counts the second one's warps from the other end, so that on small tiles both are loaded
+// at the same time by different warps.
 template <class T, int NT>
 __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams, int streams_left, int rows, int cols, CmDiv dcols,
-                                         int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch)
+                                         int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch, int warp)
 {
     constexpr int SZ = (int)sizeof(T);
     const char *base = reinterpret_cast<const char *>(src);
@@ -66,7 +68,7 @@ __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams,
         const int w_even = col0 & ~1, half = (col0 + cols + 1 - w_even) >> 1, rc_n = rows * half, items = streams * rc_n;
         const CmDiv dhalf = cm_div_dev(half);
         const int blocks = (items + 31) >> 5;
-        int g = 0, blk = threadIdx.x >> 5;
+        int g = 0, blk = warp;
         while (blk >= blocks) { blk -= blocks; g++; }
         for (; g < groups;) {
             const int p = blk * 32 + lane;
@@ -102,7 +104,7 @@ __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams,
         return;
     }
     const int rc_n = rows * cols, pix = streams * rc_n, blocks = (pix + 31) >> 5;
-    int g = 0, blk = threadIdx.x >> 5;
+    int g = 0, blk = warp;
     while (blk >= blocks) { blk -= blocks; g++; }
     while (g < groups) {
         const int p = blk * 32 + lane;
@@ -138,12 +140,12 @@ __device__ __forceinline__ void cm_stage(uint32_t sm, const T *src, int streams,
 // multiplied.  The caller commits and waits.
 template <int NT>
 __device__ __forceinline__ void cm_stage_async(uint32_t sm, const float *src, int streams, int streams_left, int rows, int cols, CmDiv dcols,
-                                               int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch)
+                                               int row0, int col0, int H, int W, int chans, int c_left, uint32_t cstride, uint32_t sstride, uint32_t pitch, int warp)
 {
     const char *base = reinterpret_cast<const char *>(src);
     const int groups = chans >> 3, lane = threadIdx.x & 31, rc_n = rows * cols, pix = streams * rc_n, blocks = (pix + 31) >> 5;
     const uint32_t cs = cstride * 4;
-    int g = 0, blk = threadIdx.x >> 5;
+    int g = 0, blk = warp;
     while (blk >= blocks) { blk -= blocks; g++; }
     while (g < groups) {
         const int p = blk * 32 + lane;
@@ -188,7 +190,9 @@ template <class T, int WM> constexpr int cm_ctas() { return sizeof(T) == 2 && WM
 template <class T, int MT, int WM, int WN, int WK, int BN>
 __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_kernel(const __grid_constant__ CmFwd p)
 {
-    pdl_wait();
+    // a first read of a parameter misses the constant cache, one after the other where an index depends on another one: all lines at once
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(CmFwd) / 4); i += 16) asm volatile("" ::"r"(reinterpret_cast<const uint32_t *>(&p)[i]));
     constexpr int NT = 32 * WM * WN * WK, BM = 16 * MT * WM, TN = BN / WN, N8 = TN / 8;
     constexpr int CK = sizeof(T) == 2 ? 16 : 8, SZ = (int)sizeof(T);
     constexpr bool HALF = sizeof(T) == 2;
@@ -206,8 +210,9 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
     const int tiles_s = P < BN ? 1 : wide ? c.Hc * tiles_r : (P + BN - 1) / BN;      // tiles of one stream
     const int cols = wide ? c.wide_cols : c.cols;
     const int tiles = (P < BN ? (p.n + p.st_tile - 1) / p.st_tile : p.n * tiles_s);
-    if ((int)blockIdx.x >= tiles) return;
+    if ((int)blockIdx.x >= tiles) { pdl_wait(); return; }
 
+    // the tables come from the arguments alone: they are made before the wait for the kernel in front
     for (int t = tid; t < p.KK; t += NT) tap_of[t] = -1;
     __syncthreads();
     for (int t = tid; t < ntaps; t += NT) {
@@ -215,6 +220,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
         tap_of[p.widx[c.tap0 + t]] = t;
     }
     __syncthreads();
+    pdl_wait();
 
     // Weights of channels k0 .. k0 + kc as [tap][BM][wpitch].  A thread takes one (m, k) pair (fp16: two neighbouring k), walks
     // its taps, which are contiguous in memory, nine loads in flight, and stores each to its tap's matrix: one or two
@@ -254,8 +260,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
                 }
             }
         }
-        if constexpr (!HALF) asm volatile("cp.async.wait_all;" ::: "memory");
-    };
+    };                                                                             // (fp32: copies in flight, the caller waits)
     if (p.resident) load_weights(0, p.groups * p.CKS);
 
     const CmDiv dcols = wide ? cm_div_dev(cols) : c.dcols, dW = c.dW;
@@ -281,11 +286,11 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
         if constexpr (!HALF)
             if (async) {
                 cm_stage_async<NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
-                                   (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
+                                   (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch, NT / 32 - 1 - warp);
                 return;
             }
         cm_stage<T, NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
-                        (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch);
+                        (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch, NT / 32 - 1 - warp);
     };
     // two patches (fp32, weights resident): the next tile's channels are on their way while this tile is multiplied
     const bool two = !HALF && p.patch2 != 0;
@@ -328,6 +333,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
                 __syncthreads();                                                    // the patch (and the weights) are free again
                 if (!p.resident) load_weights(k0, p.CKS);
                 stage(geo, g, patch, false);
+                if constexpr (!HALF) asm volatile("cp.async.wait_all;" ::: "memory");       // the weights
                 __syncthreads();
             }
             const uint32_t wg = wsm + (uint32_t)(p.resident ? k0 * SZ : 0);
@@ -597,17 +603,65 @@ INST(__half)
 // its tap group in registers; WK warps share the pixels of a tile.  Every CTA leaves one partial dW, summed in CTA order by the
 // reduction that the other weight-gradient kernels use.
 struct CmWg {
-    const void *x, *dy; float *part;
+    const void *x, *dy; float *part; void *dw;       // partial results per CTA, or (cluster kernel) the result
     int n, Ci, H, W, Co, Ho, Wo, S, KK, Wk, padU, padL, tap0, ntaps;
-    int bn, st_tile, tiles, tiles_s, tiles_r, rows_max, cols, ci_tiles, steps;       // tiles_r: tiles of a row longer than a tile
+    int bn, st_tile, tiles, tiles_s, tiles_r, rows_max, cols, ci_tiles, steps, shares;       // tiles_r: tiles of a row longer than a tile
     CmDiv dW, dcols;
     uint32_t xpitch, dpitch, d_off, t_off, buf2;    // bytes: pixel of X / of dY; offsets of the dY tile, of the address tables, of the second tiles (0: none)
 };
 
+// One tile of output pixels: its first stream, first pixel, first row and column, the end of its pixels, the rows of X it needs.
+struct CmWgTile { int s0, p0, i0, col_t, last, rows; };
+__device__ __forceinline__ CmWgTile cm_wg_tile(const CmWg &p, int tile)
+{
+    const int P = p.Ho * p.Wo;
+    const bool multi = P < p.bn, wide = p.Wo > p.bn;
+    CmWgTile t;
+    t.s0 = multi ? tile * p.st_tile : tile / p.tiles_s;
+    const int ts = tile - (multi ? tile : t.s0 * p.tiles_s), row_t = wide ? ts / p.tiles_r : 0;
+    t.col_t = wide ? (ts - row_t * p.tiles_r) * p.bn : 0;                                               // a tile within one long row
+    t.p0 = multi ? 0 : wide ? row_t * p.Wo + t.col_t : ts * p.bn;
+    t.i0 = wide ? row_t : cm_quot(t.p0, p.dW);
+    t.last = multi ? P - 1 : wide ? t.p0 + min(p.bn, p.Wo - t.col_t) - 1 : min(t.p0 + p.bn, P) - 1;
+    t.rows = ((wide ? t.i0 : cm_quot(t.last, p.dW)) - t.i0) * p.S + p.rows_max;
+    return t;
+}
+// pixel q of the tile -> its bytes from the first pixel of the staged X (pixels without a value: that of pixel 0)
+__device__ __forceinline__ int cm_wg_pixel(const CmWg &p, const CmWgTile &t, int q)
+{
+    const int P = p.Ho * p.Wo;
+    const bool multi = P < p.bn, wide = p.Wo > p.bn;
+    if (q >= (multi ? p.st_tile * P : t.last + 1 - t.p0)) q = 0;
+    int st = 0, pp = t.p0 + q;
+    if (multi) { st = q / P; pp = q - st * P; }
+    const int i = wide ? t.i0 : cm_quot(pp, p.dW), j = pp - i * p.Wo - t.col_t;
+    return ((st * t.rows + (i - t.i0) * p.S) * p.cols + j * p.S) * (int)p.xpitch;
+}
+// X and dY of a tile into shared memory (ASYNC: by copies that the caller waits for)
+template <class T, int NT, int CI, int CO, bool ASYNC>
+__device__ __forceinline__ void cm_wg_stage(const CmWg &p, const CmWgTile &t, uint32_t xs, uint32_t ds, int ci0, int co0, int warp)
+{
+    const int P = p.Ho * p.Wo;
+    const bool multi = P < p.bn;
+    const long long xplane = (long long)p.H * p.W;
+    const T *xp = reinterpret_cast<const T *>(p.x) + ((long long)t.s0 * p.Ci + ci0) * xplane, *dp = reinterpret_cast<const T *>(p.dy) + ((long long)t.s0 * p.Co + co0) * P;
+    const int st_n = multi ? p.st_tile : 1, run = multi ? P : p.bn, row0 = t.i0 * p.S - p.padU, col0 = t.col_t * p.S - p.padL, d_end = multi ? P : t.last + 1;
+    const CmDiv drun = cm_div_dev(run);
+    if constexpr (ASYNC) {
+        cm_stage_async<NT>(xs, xp, st_n, p.n - t.s0, t.rows, p.cols, p.dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch, warp);
+        cm_stage_async<NT>(ds, dp, st_n, p.n - t.s0, 1, run, drun, 0, t.p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch, NT / 32 - 1 - warp);
+    } else {
+        cm_stage<T, NT>(xs, xp, st_n, p.n - t.s0, t.rows, p.cols, p.dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch, warp);
+        cm_stage<T, NT>(ds, dp, st_n, p.n - t.s0, 1, run, drun, 0, t.p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch, NT / 32 - 1 - warp);
+    }
+}
+
 template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK>
 __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const __grid_constant__ CmWg p)
 {
-    pdl_wait();
+    // a first read of a parameter misses the constant cache, one after the other where an index depends on another one: all lines at once
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(CmWg) / 4); i += 16) asm volatile("" ::"r"(reinterpret_cast<const uint32_t *>(&p)[i]));
     constexpr int NT = 32 * WM * WN * WK, BN = 128;
     constexpr bool HALF = sizeof(T) == 2;
     constexpr int KS = HALF ? 16 : 8, STEPS = BN / KS;
@@ -619,10 +673,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     const int ci0 = ((int)blockIdx.x % p.ci_tiles) * CI, co0 = ((int)blockIdx.x / p.ci_tiles) * CO;
     const uint32_t xs = (uint32_t)__cvta_generic_to_shared(cm_smem), ds = xs + p.d_off;
     int *table = reinterpret_cast<int *>(cm_smem + p.t_off);
-    const int P = p.Ho * p.Wo, cols = p.cols;
-    const int bn = p.bn;                                                   // pixels of a tile, at most BN
-    const bool multi = P < bn, wide = p.Wo > bn;
-    const CmDiv dW = p.dW, dcols = p.dcols;
+    const int cols = p.cols;
 
     float acc[TAPS][MI][NI][4];
 #pragma unroll
@@ -643,36 +694,17 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     }
 
     const int t_begin = (int)((long long)p.tiles * blockIdx.y / gridDim.y), t_end = (int)((long long)p.tiles * (blockIdx.y + 1) / gridDim.y);
-    const long long xplane = (long long)p.H * p.W;
-    const int st_n = multi ? p.st_tile : 1;
     auto stage = [&](int tile, uint32_t buf, bool async) {
-        const int s0 = multi ? tile * p.st_tile : tile / p.tiles_s, ts = tile % p.tiles_s;
-        const int row_t = wide ? ts / p.tiles_r : 0, col_t = wide ? (ts - row_t * p.tiles_r) * bn : 0;      // a tile within one long row
-        const int p0 = multi ? 0 : wide ? row_t * p.Wo + col_t : ts * bn;
-        const int i0 = wide ? row_t : cm_quot(p0, dW), last = multi ? P - 1 : wide ? p0 + min(bn, p.Wo - col_t) - 1 : min(p0 + bn, P) - 1;
-        const int rows = ((wide ? i0 : cm_quot(last, dW)) - i0) * p.S + p.rows_max;
-        if (tid < BN) {
-            const int live = multi ? st_n * P : last + 1 - p0, q = tid < live ? tid : 0;
-            int st = 0, pp = p0 + q;
-            if (multi) { st = q / P; pp = q - st * P; }
-            const int i = wide ? i0 : cm_quot(pp, dW), j = pp - i * p.Wo - col_t;
-            table[(buf ? BN : 0) + tid] = ((st * rows + (i - i0) * p.S) * cols + j * p.S) * (int)p.xpitch;
-        }
-        const T *xp = reinterpret_cast<const T *>(p.x) + ((long long)s0 * p.Ci + ci0) * xplane, *dp = reinterpret_cast<const T *>(p.dy) + ((long long)s0 * p.Co + co0) * P;
-        const int run = multi ? P : bn, row0 = i0 * p.S - p.padU, col0 = col_t * p.S - p.padL, d_end = multi ? P : last + 1;
-        const CmDiv drun = cm_div_dev(run);
+        const CmWgTile t = cm_wg_tile(p, tile);
+        if (tid < BN) table[(buf ? BN : 0) + tid] = cm_wg_pixel(p, t, tid);
         if constexpr (!HALF)
-            if (async) {
-                cm_stage_async<NT>(xs + buf, xp, st_n, p.n - s0, rows, cols, dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
-                cm_stage_async<NT>(ds + buf, dp, st_n, p.n - s0, 1, run, drun, 0, p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
-                return;
-            }
-        cm_stage<T, NT>(xs + buf, xp, st_n, p.n - s0, rows, cols, dcols, row0, col0, p.H, p.W, CI, p.Ci - ci0, (uint32_t)xplane, (uint32_t)(p.Ci * xplane), p.xpitch);
-        cm_stage<T, NT>(ds + buf, dp, st_n, p.n - s0, 1, run, drun, 0, p0, 1, d_end, CO, p.Co - co0, (uint32_t)P, (uint32_t)(p.Co * P), p.dpitch);
+            if (async) { cm_wg_stage<T, NT, CI, CO, true>(p, t, xs + buf, ds + buf, ci0, co0, warp); return; }
+        cm_wg_stage<T, NT, CI, CO, false>(p, t, xs + buf, ds + buf, ci0, co0, warp);
     };
     // two sets of tiles (fp32): the next tile arrives by asynchronous copies while this one is multiplied
     const bool two = !HALF && p.buf2 != 0;
     uint32_t cur = 0;
+    pdl_wait();
     __syncthreads();                                                       // the zeros of the dY tiles are in place
     if (two && t_begin < t_end) stage(t_begin, 0, true);
     for (int tile = t_begin; tile < t_end; tile++) {
@@ -781,19 +813,161 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, 2) conv_mma_wg_kernel(const
     }
 }
 
-template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool conv_mma_wg_launch(CmWg &p, int part_groups, int *groups_out, bool dry)
+// Few pixels (single streams).  What bounds these layers is the way from one launch to the next: the kernel above left one partial dW
+// per CTA for a reduction of its own, gave half of its warps no pixels and wrote 72 accumulators a thread through shared memory.  Here
+// the CTAs of one 16 x 16 channel tile are one cluster that shares the pixels, each of nine warps has filter taps of its own (fewer
+// taps than warps: the warps share the pixels), and the cluster adds its results through distributed shared memory in rank order, so
+// that no partial results and no second launch exist.
+// Measured with the reduction, before and after: one stream of 16 -> 32 channels on 32 x 32 pixels 8.4 -> 5.9 us (fp16 7.3 -> 4.8), 2 -> 61
+// on 33 x 46 with stride 2 8.6 -> 5.1, 48 -> 48 on 28 x 28 with 5 x 5 windows 27.1 -> 12.5 (three launches before).
+static constexpr int CMC_NW = 9, CMC_TILE = 16, CMC_MAX = 16;
+template <class T, int TPW>
+__global__ void __launch_bounds__(32 * CMC_NW, 2) conv_mma_wg_cluster_kernel(const __grid_constant__ CmWg p)
 {
-    constexpr int BN = 128, SZ = (int)sizeof(T), CO = 16 * MI * WM, CI = 8 * NI * WN, PAD = SZ == 2 ? 16 : 32;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(CmWg) / 4); i += 16) asm volatile("" ::"r"(reinterpret_cast<const uint32_t *>(&p)[i]));
+    constexpr int NT = 32 * CMC_NW, BN = 128, KS = sizeof(T) == 2 ? 16 : 8, KCH = 2;                    // KCH k-steps per chain
+    constexpr bool HALF = sizeof(T) == 2;
+    extern __shared__ __align__(16) unsigned char cm_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = blockIdx.x, ranks = gridDim.x;                        // (the cluster is a row of the grid)
+    const int co_t = (int)blockIdx.y / p.ci_tiles, ci0 = ((int)blockIdx.y - co_t * p.ci_tiles) * CMC_TILE, co0 = co_t * CMC_TILE;
+    const uint32_t xs = (uint32_t)__cvta_generic_to_shared(cm_smem), ds = xs + p.d_off;
+    int *table = reinterpret_cast<int *>(cm_smem + p.t_off);
+    const int KK = p.KK, shares = p.shares, share = shares > 1 ? warp / KK : 0, tap = warp - share * KK;
+    const int t_begin = p.tiles * rank / ranks, t_end = p.tiles * (rank + 1) / ranks;
+    float acc[TPW][2][4] = {};
+    int toff[TPW];
+#pragma unroll
+    for (int u = 0; u < TPW; u++) { const int t = min(tap + u * CMC_NW, KK - 1); toff[u] = ((t / p.Wk) * p.cols + t % p.Wk) * (int)p.xpitch; }
+    // pixels of the tile that no stream covers are zero in the dY tile
+    const int covered = p.Ho * p.Wo < p.bn ? p.st_tile * p.Ho * p.Wo : p.bn;
+    for (uint32_t e = covered * p.dpitch + tid * 16; e < BN * p.dpitch; e += NT * 16) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(ds + e), "r"(0) : "memory");
+    pdl_wait();
+    for (int tile = t_begin; tile < t_end; tile++) {
+        if (tile > t_begin) __syncthreads();
+        const CmWgTile t = cm_wg_tile(p, tile);
+        cm_wg_stage<T, NT, CMC_TILE, CMC_TILE, false>(p, t, xs, ds, ci0, co0, warp);
+        if (tid < BN) table[tid] = cm_wg_pixel(p, t, tid);
+        __syncthreads();
+        if (share >= shares) continue;
+        for (int s = share * KCH; s < p.steps; s += shares * KCH) {
+            uint32_t a[KCH][4], al[HALF ? 1 : KCH][4], xa[KCH][HALF ? 1 : 2];
+#pragma unroll
+            for (int c = 0; c < KCH; c++) {
+                const int k0 = (s + c) * KS;
+                if constexpr (HALF) {
+                    xa[c][0] = xs + (uint32_t)table[k0 + (lane & 15)] + (uint32_t)(lane >> 4) * 16u;
+                    cm_ldsm_t(a[c], ds + (uint32_t)(k0 + (lane & 7) + (lane >> 4) * 8) * p.dpitch + (uint32_t)((lane >> 3) & 1) * 16u);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) xa[c][h] = xs + (uint32_t)table[k0 + (lane & 3) + 4 * h] + (uint32_t)(lane >> 2) * 4u;
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        tc::split_tf32_fast(__uint_as_float(cm_lds32(ds + (uint32_t)(k0 + (lane & 3) + (q >> 1) * 4) * p.dpitch + (uint32_t)((lane >> 2) + (q & 1) * 8) * 4u)), a[c][q], al[c][q]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < TPW; u++) {
+                if (u > 0 && tap + u * CMC_NW >= KK) break;
+                float tmp[2][4] = {};
+#pragma unroll
+                for (int c = 0; c < KCH; c++) {
+                    if constexpr (HALF) {
+                        uint32_t b[4];
+                        cm_ldsm_t(b, xa[c][0] + toff[u]);
+                        cm_hmma(tmp[0], a[c], b[0], b[1]);
+                        cm_hmma(tmp[1], a[c], b[2], b[3]);
+                    } else {
+                        uint32_t bh[2][2], bl[2][2];
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+#pragma unroll
+                            for (int h = 0; h < 2; h++) tc::split_tf32_fast(__uint_as_float(cm_lds32(xa[c][h] + toff[u] + j * 32u)), bh[j][h], bl[j][h]);
+#pragma unroll
+                        for (int term = 0; term < 3; term++)
+#pragma unroll
+                            for (int j = 0; j < 2; j++) cm_tmma(tmp[j], term == 0 ? al[c] : a[c], term == 1 ? bl[j][0] : bh[j][0], term == 1 ? bl[j][1] : bh[j][1]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) acc[u][j][q] += tmp[j][q];
+            }
+        }
+    }
+    // the CTA's dW, rows of one output channel in memory order (taps innermost)
+    const int cols = CMC_TILE * KK, RP = cols + 4;
+    float *red = reinterpret_cast<float *>(cm_smem);
+    __syncthreads();
+    if (share < shares)
+#pragma unroll
+        for (int u = 0; u < TPW; u++) {
+            if (tap + u * CMC_NW >= KK) break;
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    red[(share * CMC_TILE + (lane >> 2) + (q >> 1) * 8) * RP + (j * 8 + 2 * (lane & 3) + (q & 1)) * KK + tap + u * CMC_NW] = acc[u][j][q];
+        }
+    if (shares > 1) {
+        __syncthreads();
+        for (int e = tid; e < CMC_TILE * RP; e += NT) {
+            float v = red[e];
+            for (int k = 1; k < shares; k++) v += red[k * CMC_TILE * RP + e];
+            red[e] = v;
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    // a CTA adds 16 / ranks rows: 16 loads an element whatever the cluster's size, all on their way at once
+    const int live = min(CMC_TILE, p.Ci - ci0) * KK, co_left = p.Co - co0;
+    T *dw = reinterpret_cast<T *>(p.dw) + ((long long)co0 * p.Ci + ci0) * KK;
+    auto remote = [&](int row, int e, int k) {
+        uint32_t at; float v;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(xs + (uint32_t)(row * RP + e) * 4u), "r"(k));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+        return v;
+    };
+    for (int e = tid; e < live; e += NT) {
+        float v[CMC_MAX], sum = 0.f;
+        if (ranks == CMC_MAX) {
+            if (rank >= co_left) break;
+#pragma unroll
+            for (int k = 0; k < CMC_MAX; k++) v[k] = remote(rank, e, k);
+#pragma unroll
+            for (int k = 0; k < CMC_MAX; k++) sum += v[k];
+            st(dw + (long long)rank * p.Ci * KK + e, sum);
+        } else {
+            const int rmask = ranks - 1;                                    // (a power of two)
+#pragma unroll
+            for (int q = 0; q < CMC_MAX; q++) v[q] = remote(rank + (q & ~rmask), e, q & rmask);
+#pragma unroll
+            for (int q = 0; q < CMC_MAX; q++) {
+                sum += v[q];
+                if ((q & rmask) == rmask) {
+                    const int r = rank + (q & ~rmask);
+                    if (r < co_left) st(dw + (long long)r * p.Ci * KK + e, sum);
+                    sum = 0.f;
+                }
+            }
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");      // no CTA leaves while its sums are read
+}
+
+// Pixels per tile and their layout in shared memory (X, then dY), for `slots` CTAs that share the pixels.  false = not covered.
+template <class T> static bool cm_wg_plan(CmWg &p, int CI, int CO, int slots, size_t &xb, size_t &db)
+{
+    constexpr int SZ = (int)sizeof(T), PAD = SZ == 2 ? 16 : 32;
     const int P = p.Ho * p.Wo, cols0 = p.cols;
     p.ci_tiles = ceil_div(p.Ci, CI);
-    const int ctiles = p.ci_tiles * ceil_div(p.Co, CO);
-    const int slots = std::max(1, std::min(2 * sm_count() / ctiles, part_groups));
     const long long stream_elements = (long long)p.Ci * p.H * p.W + (long long)p.Co * P;
     if (stream_elements >= (1ll << 25)) return false;                      // cm_streams
     auto tiles_of = [&](int bn) -> long long { return P < bn ? ceil_div(p.n, cm_streams(bn, P, p.n, stream_elements)) : p.Wo > bn ? (long long)p.n * p.Ho * ceil_div(p.Wo, bn) : (long long)p.n * ceil_div(P, bn); };
     // pixels per tile: what makes the fewest pixels of the longest CTA (planes and rounds come out even), halo rows included
     double best = 1e30;
-    for (int bn = BN; bn >= BN / 4; bn -= SZ == 2 ? 16 : 8) {
+    for (int bn = 128; bn >= 32; bn -= SZ == 2 ? 16 : 8) {
         const int halo = bn + 2 * std::min(p.Wo, bn) * (p.rows_max - 1) / 3;
         const double cost = (double)ceil_div(tiles_of(bn), slots) * halo;
         if (cost < 0.98 * best) { best = cost; p.bn = bn; }
@@ -810,8 +984,28 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     p.steps = ceil_div(P < bn ? p.st_tile * P : bn, SZ == 2 ? 16 : 8);
     const int rows = (wide ? 0 : P < bn ? p.Ho - 1 : (bn + p.Wo - 2) / p.Wo) * p.S + p.rows_max;
     p.xpitch = CI * SZ + PAD; p.dpitch = CO * SZ + PAD;
-    const size_t xb = ((size_t)p.st_tile * rows * p.cols * p.xpitch + 15) & ~(size_t)15, db = (size_t)BN * p.dpitch;
+    xb = ((size_t)p.st_tile * rows * p.cols * p.xpitch + 15) & ~(size_t)15; db = (size_t)128 * p.dpitch;
     p.d_off = (uint32_t)xb;
+    return true;
+}
+
+template <class T, int TPW> static void conv_mma_wg_cluster_launch(const CmWg &p, int ranks, size_t smem)
+{
+    static bool set = false;
+    if (!set) {
+        cudaFuncSetAttribute(conv_mma_wg_cluster_kernel<T, TPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM_MAX);
+        cudaFuncSetAttribute(conv_mma_wg_cluster_kernel<T, TPW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        set = true;
+    }
+    TL_LAUNCH_CLUSTER((conv_mma_wg_cluster_kernel<T, TPW>), dim3(ranks, p.ci_tiles * ceil_div(p.Co, CMC_TILE)), 32 * CMC_NW, smem, ranks, p);
+}
+
+template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool conv_mma_wg_launch(CmWg &p, int part_groups, int *groups_out, bool dry)
+{
+    constexpr int BN = 128, SZ = (int)sizeof(T), CO = 16 * MI * WM, CI = 8 * NI * WN;
+    const int ctiles = ceil_div(p.Ci, CI) * ceil_div(p.Co, CO);
+    size_t xb, db;
+    if (!cm_wg_plan<T>(p, CI, CO, std::max(1, std::min(2 * sm_count() / ctiles, part_groups)), xb, db)) return false;
     const bool two = SZ == 4 && 2 * (xb + db) + 8 * BN <= 110 * 1024;
     p.buf2 = two ? (uint32_t)(xb + db) : 0u; p.t_off = (uint32_t)((xb + db) * (two ? 2 : 1));
     const size_t smem = std::max((size_t)p.t_off + 8 * BN, (size_t)WK * CO * (CI * TAPS + 4) * 4);
@@ -830,15 +1024,64 @@ template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool
     return true;
 }
 
-// Partial results per CTA into `part`; false = geometry not covered.  dry_run: only the number of groups.
-template <class T> bool conv_mma_wg(const ConvGeom &geom, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry)
+template <class T> static bool cm_wg_params(const ConvGeom &geom, const T *x, const T *dy, CmWg &p)
 {
     const ConvGeom g = cm_flat(geom);
     const int KK = g.Hk * g.Wk;
     if (g.depthwise || gemm_path() == 1 || KK > CM_MAXTAPS || g.sh != g.sw || (long long)g.Hin * g.Win >= (1ll << 31)) return false;
-    CmWg p;
-    p.x = x; p.dy = dy; p.part = part; p.n = g.n; p.Ci = g.Cin; p.H = g.Hin; p.W = g.Win; p.Co = g.Cout; p.Ho = g.Hout; p.Wo = g.Wout; p.S = g.sh;
+    p = CmWg();
+    p.x = x; p.dy = dy; p.n = g.n; p.Ci = g.Cin; p.H = g.Hin; p.W = g.Win; p.Co = g.Cout; p.Ho = g.Hout; p.Wo = g.Wout; p.S = g.sh;
     p.KK = KK; p.Wk = g.Wk; p.padU = g.padU; p.padL = g.padL; p.rows_max = g.Hk; p.cols = (g.Wout - 1) * g.sw + g.Wk; p.dW = cm_div(g.Wout); p.dcols = cm_div(p.cols);
+    return true;
+}
+
+// Where it pays: while every CTA has an SM (a cluster of 16 needs most of a GPC, and 16 x 16 tiles read more per product than the kernel
+// above: one stream of 64 -> 64 on 32 x 32, 256 CTAs, fp32 12.1 us against 9.4 there) and up to 2048 pixels (32 -> 32 on 64 x 64:
+// 11.7 against 10.7; 32 -> 64 on two planes of 32 x 32, 9.6 against 9.8, is about where they meet).  Very few pixels under many channels
+// leave the kernel above one partial result to write and read again per CTA: there up to eight CTAs an SM (256 -> 256 on 8 x 8
+// 15.5 -> 11.4 us, 512 -> 512 on 4 x 4 37.1 -> 20.7), except for 1 x 1 windows (512 -> 512 on 4 x 4: 8.9 against 19.3).
+template <class T> static bool cm_wg_cluster_plan(const ConvGeom &g, const T *x, const T *dy, CmWg &p, int &ranks, size_t &smem)
+{
+    size_t xb, db;
+    if ((long long)g.n * g.Hout * g.Wout > CMC_MAX * 128 || !cm_wg_params(g, x, dy, p) || !cm_wg_plan<T>(p, CMC_TILE, CMC_TILE, CMC_MAX, xb, db)) return false;
+    p.t_off = (uint32_t)(xb + db);
+    p.shares = std::max(1, CMC_NW / p.KK);
+    smem = std::max((size_t)p.t_off + 4 * 128, (size_t)p.shares * CMC_TILE * (CMC_TILE * p.KK + 4) * 4);
+    for (ranks = 1; ranks < std::min(p.tiles, CMC_MAX);) ranks *= 2;
+    const long long pixels = (long long)p.n * p.Ho * p.Wo, ctas = (long long)p.ci_tiles * ceil_div(p.Co, CMC_TILE) * ranks;
+    return smem <= CM_SMEM_MAX && (ctas <= sm_count() || (p.KK > 1 && pixels <= 64 && ctas <= 8ll * sm_count()));
+}
+template <class T> bool conv_mma_wg_cluster(const ConvGeom &g, const T *x, const T *dy, T *dw)
+{
+    CmWg p;
+    int ranks;
+    size_t smem;
+    if (!cm_wg_cluster_plan<T>(g, x, dy, p, ranks, smem)) return false;
+    p.dw = dw;
+    const int tpw = ceil_div(p.KK, CMC_NW);
+    if (tpw <= 1) conv_mma_wg_cluster_launch<T, 1>(p, ranks, smem);
+    else if (tpw <= 3) conv_mma_wg_cluster_launch<T, 3>(p, ranks, smem);
+    else conv_mma_wg_cluster_launch<T, 6>(p, ranks, smem);
+    return true;
+}
+// fp16: in front of the tcgen05 kernel over slots, whose launch and reduction cost about 10 us at any size, while the products of a CTA
+// are few (48 -> 48 on 28 x 28, 5 x 5: 8.6 us against 13.3; with 7 x 7 windows 16.6 against 15.5)
+bool conv_mma_wg_cluster_first(const ConvGeom &g)
+{
+    CmWg p;
+    int ranks;
+    size_t smem;
+    return cm_wg_cluster_plan<__half>(g, nullptr, nullptr, p, ranks, smem) && (long long)ranks * p.ci_tiles * ceil_div(p.Co, CMC_TILE) * p.KK * p.steps <= 100ll * sm_count();
+}
+
+// Partial results per CTA into `part`; false = geometry not covered.  dry_run: only the number of groups.
+template <class T> bool conv_mma_wg(const ConvGeom &geom, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry)
+{
+    CmWg p;
+    if (!cm_wg_params(geom, x, dy, p)) return false;
+    const ConvGeom g = cm_flat(geom);
+    const int KK = p.KK;
+    p.part = part;
     if (KK == 1) {
         if (g.Cin > 32 && g.Cout > 16) return conv_mma_wg_launch<T, 1, 2, 4, 2, 2, 2>(p, part_groups, groups_out, dry);
         return conv_mma_wg_launch<T, 1, 1, 4, 2, 1, 4>(p, part_groups, groups_out, dry);
@@ -850,7 +1093,7 @@ template <class T> bool conv_mma_wg(const ConvGeom &geom, const T *x, const T *d
     if (g.Cin > 16) return conv_mma_wg_launch<T, 9, 1, 2, 1, 2, 4>(p, part_groups, groups_out, dry);
     return conv_mma_wg_launch<T, 9, 1, 2, 1, 1, 8>(p, part_groups, groups_out, dry);
 }
-#define INST(T) template bool conv_mma_wg<T>(const ConvGeom &, const T *, const T *, float *, int, int *, bool);
+#define INST(T) template bool conv_mma_wg<T>(const ConvGeom &, const T *, const T *, float *, int, int *, bool); template bool conv_mma_wg_cluster<T>(const ConvGeom &, const T *, const T *, T *);
 INST(float)
 INST(__half)
 #undef INST

@@ -153,6 +153,8 @@ bool conv_px_wg(Scope &sc, const ConvGeom &g, const __half *x, const __half *dy,
 template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, const T *bias, T *y);
 template <class T> bool conv_mma_ig(const ConvGeom &g, const T *dy, const T *w, T *dx);
 template <class T> bool conv_mma_wg(const ConvGeom &g, const T *x, const T *dy, float *part, int part_groups, int *groups_out, bool dry_run);
+template <class T> bool conv_mma_wg_cluster(const ConvGeom &g, const T *x, const T *dy, T *dw);
+bool conv_mma_wg_cluster_first(const ConvGeom &g);
 // depthwise planes through shared memory (tl_conv_dw.cu)
 template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T *dst, bool ig);
 template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy, float *part, int &groups, bool dry_run);

@@ -68,6 +68,21 @@ def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
     test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
 
 
+# weight gradients of few pixels, one cluster per 16 x 16 channel tile (conv_mma_wg_cluster_kernel): one to sixteen CTAs of a cluster, ranks
+# without pixels, a last tile cut short, several streams in a tile, rows longer than a tile, channel remainders, windows of fewer taps
+# than the nine warps (which then share the pixels), of more, and of several rounds, strides, odd planes
+FEW_PIXELS = [(16, 32, 32, 32, 3, 1, 1), (17, 9, 9, 17, 5, 2, 1), (2, 33, 46, 61, 3, 2, 1), (60, 13, 18, 8, 3, 1, 1), (5, 3, 300, 20, 3, 1, 1), (33, 5, 5, 31, 2, 2, 1), (1, 1, 1, 1, 1, 1, 1), (24, 40, 40, 24, 1, 1, 1),
+              (48, 28, 28, 48, 5, 1, 1), (7, 11, 13, 9, 7, 1, 5), (20, 3, 3, 20, 3, 1, 30), (20, 7, 5, 20, 3, 1, 40), (96, 4, 4, 96, 3, 1, 1), (3, 64, 64, 12, 5, 2, 1), (12, 21, 19, 40, 3, 3, 3), (9, 6, 7, 30, 4, 1, 2)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", FEW_PIXELS)
+def test_conv2d_of_few_pixels(run, oracle, cin, h, w, cout, k, stride, n):
+    run.lib.trainlib_profile(1)
+    test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+    run.lib.trainlib_profile(0)
+    assert any("wg_cluster" in t[0] for t in run.pkg.profile_table(run.lib))
+
+
 # half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
 # tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
 # for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
