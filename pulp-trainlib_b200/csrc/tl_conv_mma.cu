@@ -181,13 +181,14 @@ struct CmFwd {
     int CKS, groups, cblk, resident;         // channels staged at a time, how often, k-steps per chain; weights loaded once per CTA
     uint32_t pitch, wpitch, w_off, patch2;   // bytes: pixel, weight row; offset of the weights behind the patch; of the second patch (0: none)
     int rows_max, linear, pairs;
+    int ksplit, kshare;                      // CTAs of a cluster that share the source channels, channels of each
 };
 
 // CTAs per SM.  What bounds these kernels is issue at few warps, so a third one helps where the registers allow it without loss: fp16
 // tiles of 16 and 32 channels (400 streams of 8 -> 20 on 9 x 11: 12.4 -> 10.0 us a direction; 50 of 30 -> 13, 5 x 5: 19.5 -> 16.7).
 // The 64-channel tiles lose the overlap of their fragment loads (88 -> 96 us), the fp32 ones up to 6 %.
 template <class T, int WM> constexpr int cm_ctas() { return sizeof(T) == 2 && WM == 1 ? 3 : 2; }
-template <class T, int MT, int WM, int WN, int WK, int BN>
+template <class T, int MT, int WM, int WN, int WK, int BN, bool KS = false>
 __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_kernel(const __grid_constant__ CmFwd p)
 {
     // a first read of a parameter misses the constant cache, one after the other where an index depends on another one: all lines at once
@@ -210,7 +211,15 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
     const int tiles_s = P < BN ? 1 : wide ? c.Hc * tiles_r : (P + BN - 1) / BN;      // tiles of one stream
     const int cols = wide ? c.wide_cols : c.cols;
     const int tiles = (P < BN ? (p.n + p.st_tile - 1) / p.st_tile : p.n * tiles_s);
-    if ((int)blockIdx.x >= tiles) { pdl_wait(); return; }
+    // KS: one cluster per tile, whose CTAs have a share of the source channels each
+    int bx = blockIdx.x, gx = gridDim.x, rank = 0;
+    if constexpr (KS) {
+        asm("mov.u32 %0, %%clusterid.x;" : "=r"(bx));
+        asm("mov.u32 %0, %%nclusterid.x;" : "=r"(gx));
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    }
+    const int koff = KS ? rank * p.kshare : 0, Cs = KS ? min(p.kshare, p.Cs - koff) : p.Cs;
+    if (bx >= tiles) { pdl_wait(); return; }
 
     // the tables come from the arguments alone: they are made before the wait for the kernel in front
     for (int t = tid; t < p.KK; t += NT) tap_of[t] = -1;
@@ -234,8 +243,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
         const T *w = reinterpret_cast<const T *>(p.w);
         for (int e = tid; e < items; e += NT) {
             const int eq = cm_quot(e, dq), er = e - eq * dq.d, m = m_first ? er : eq, k = (m_first ? eq : er) * V;
-            const bool ok0 = m0 + m < p.Cd && k0 + k < p.Cs, ok1 = ok0 && k0 + k + 1 < p.Cs;
-            const T *src = ok0 ? w + (long long)(m0 + m) * p.wm + (long long)(k0 + k) * p.wk : w;
+            const bool ok0 = m0 + m < p.Cd && k0 + k < Cs, ok1 = ok0 && k0 + k + 1 < Cs;
+            const T *src = ok0 ? w + (long long)(m0 + m) * p.wm + (long long)(koff + k0 + k) * p.wk : w;
             const uint32_t to = wsm + (uint32_t)m * p.wpitch + (uint32_t)(k * SZ);
             for (int t0 = 0; t0 < KK; t0 += 9) {
                 if constexpr (HALF) {
@@ -282,22 +291,22 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
     };
     auto stage = [&](const Geo &q, int g, uint32_t to, bool async) {
         const int k0 = g * p.CKS;
-        const T *src = reinterpret_cast<const T *>(p.src) + ((long long)q.s0 * p.Cs + k0) * src_plane;
+        const T *src = reinterpret_cast<const T *>(p.src) + ((long long)q.s0 * p.Cs + koff + k0) * src_plane;
         if constexpr (!HALF)
             if (async) {
-                cm_stage_async<NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
+                cm_stage_async<NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, Cs - k0,
                                    (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch, NT / 32 - 1 - warp);
                 return;
             }
-        cm_stage<T, NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, p.Cs - k0,
+        cm_stage<T, NT>(to, src, st_n, p.n - q.s0, q.rows, cols, dcols, q.i0 * p.S + c.dr_min, q.col_t * p.S + c.dc_min, p.Hs, p.Ws, p.CKS, Cs - k0,
                         (uint32_t)src_plane, (uint32_t)(p.Cs * src_plane), p.pitch, NT / 32 - 1 - warp);
     };
     // two patches (fp32, weights resident): the next tile's channels are on their way while this tile is multiplied
     const bool two = !HALF && p.patch2 != 0;
     uint32_t cur = 0;
-    if (two) stage(geometry(blockIdx.x), 0, patch, true);
+    if (two) stage(geometry(bx), 0, patch, true);
 
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (int tile = bx; tile < tiles; tile += gx) {
         const Geo geo = geometry(tile);
         const int s0 = geo.s0, p0 = geo.p0, i0 = geo.i0, col_t = geo.col_t, live = geo.live, rows = geo.rows;
         // start addresses (in the patch) of the pixels this lane supplies fragments for
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
                 __syncthreads();                                                    // this patch has landed, the other one is free
                 poff = cur; cur ^= p.patch2;
                 if (g + 1 < p.groups) stage(geo, g + 1, patch + cur, true);
-                else if (tile + (int)gridDim.x < tiles) stage(geometry(tile + gridDim.x), 0, patch + cur, true);
+                else if (tile + gx < tiles) stage(geometry(tile + gx), 0, patch + cur, true);
             } else {
                 __syncthreads();                                                    // the patch (and the weights) are free again
                 if (!p.resident) load_weights(k0, p.CKS);
@@ -416,6 +425,35 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
                         for (int j = 0; j < N8; j++)
 #pragma unroll
                             for (int q = 0; q < 4; q++) acc[i][j][q] += red[((((k - 1) * WM * WN + wmn) * MT + i) * N8 + j) * 128 + q * 32 + lane];
+            if constexpr (KS) {
+                // then those of the cluster (which has one tile only) in the memory of its first CTA, in rank order
+                float *own = red + (WK - 1) * WM * WN * MT * N8 * 128;
+                if (wk == 0)
+#pragma unroll
+                    for (int i = 0; i < MT; i++)
+#pragma unroll
+                        for (int j = 0; j < N8; j++)
+#pragma unroll
+                            for (int q = 0; q < 4; q++) own[((wmn * MT + i) * N8 + j) * 128 + q * 32 + lane] = acc[i][j][q];
+                asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+                if (wk == 0 && rank == 0) {
+                    const uint32_t at = (uint32_t)__cvta_generic_to_shared(own) + (uint32_t)(wmn * MT * N8 * 128 + lane) * 4u;
+                    for (int r = 1; r < p.ksplit; r++) {
+                        uint32_t there;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(r));
+                        float v[MT * N8 * 4];
+#pragma unroll
+                        for (int q = 0; q < MT * N8 * 4; q++) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(there + 128u * q) : "memory");
+#pragma unroll
+                        for (int i = 0; i < MT; i++)
+#pragma unroll
+                            for (int j = 0; j < N8; j++)
+#pragma unroll
+                                for (int q = 0; q < 4; q++) acc[i][j][q] += v[(i * N8 + j) * 4 + q];
+                    }
+                }
+                if (rank > 0) continue;
+            }
             if (wk > 0) continue;
         }
         // results: a lane holds pixel pairs of two rows (output channels) per 16 x 8 fragment
@@ -464,9 +502,10 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, cm_ctas<T, WM>()) conv_mma_
                 }
         }
     }
+    if constexpr (KS) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");      // no CTA leaves while its sums are read
 }
 
-template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_launch(CmFwd &p, int cpad, bool dry)
+template <class T, int MT, int WM, int WN, int WK, int BN, bool KS = false> static bool conv_mma_launch(CmFwd &p, int cpad, bool dry)
 {
     constexpr int CK = sizeof(T) == 2 ? 16 : 8, SZ = (int)sizeof(T), BM = 16 * MT * WM;
     // the largest patch over the classes: streams x rows x cols
@@ -484,7 +523,7 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
         taps = std::max(taps, c.ntaps);
         tiles_max = std::max(tiles_max, P < BN ? ceil_div(p.n, p.st_tile) : (int)std::min<long long>((long long)p.n * (wide ? (long long)c.Hc * ceil_div(c.Wc, BN) : ceil_div(P, BN)), 1 << 30));
     }
-    const size_t red = WK > 1 ? (size_t)(WK - 1) * WM * WN * MT * (BN / WN / 8) * 512 : 0;
+    const size_t red = WK > 1 ? (size_t)(KS ? WK : WK - 1) * WM * WN * MT * (BN / WN / 8) * 512 : 0;
     auto plan = [&](int cks, bool resident, size_t limit, bool two) {
         p.CKS = cks; p.groups = ceil_div(cpad, cks); p.resident = resident;
         p.pitch = (uint32_t)(cks * SZ + 16); p.wpitch = (uint32_t)((resident ? p.groups * cks : cks) * SZ + 16);
@@ -510,13 +549,14 @@ template <class T, int MT, int WM, int WN, int WK, int BN> static bool conv_mma_
     p.cblk = std::min(nck, 16);
     while (WK > 1 && p.cblk > 1 && taps * ceil_div(nck, p.cblk) < 2 * WK) p.cblk = (p.cblk + 1) / 2;
     const size_t smem = p.w_off + (size_t)taps * BM * p.wpitch;
-    auto kern = conv_mma_kernel<T, MT, WM, WN, WK, BN>;
+    auto kern = conv_mma_kernel<T, MT, WM, WN, WK, BN, KS>;
     static size_t attr = 0;
     if (smem > attr) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM_MAX); attr = CM_SMEM_MAX; }
     const int co_tiles = ceil_div(p.Cd, BM);
     // every CTA slot taken: co-resident CTAs share an SM, so a last round that only some of them have costs less than idle slots
     const int gx = std::min(tiles_max, std::max(1, sm_count() * (cm_ctas<T, WM>() == 3 && smem <= 74 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls)));
-    TL_LAUNCH((conv_mma_kernel<T, MT, WM, WN, WK, BN>), dim3(gx, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p);
+    if (KS) TL_LAUNCH_CLUSTER((conv_mma_kernel<T, MT, WM, WN, WK, BN, KS>), dim3(tiles_max * p.ksplit, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p.ksplit, p);
+    else TL_LAUNCH((conv_mma_kernel<T, MT, WM, WN, WK, BN, KS>), dim3(gx, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p);
     return true;
 }
 
@@ -531,7 +571,28 @@ template <class T> static bool conv_mma_dispatch(CmFwd &p)
     for (int i = 0; i < p.ncls; i++) tiles += ((long long)p.n * p.cls[i].Hc * p.cls[i].Wc + 127) / 128;
     // Few tiles (single streams): 16 x 32 result tiles whose taps and channels are dealt to four warps each, so that a layer of
     // 32 channels on 32 x 32 pixels still occupies 64 CTAs; otherwise 128 pixels by 16, 32 or 64 channels.
-    if (2 * tiles * ceil_div(p.Cd, p.Cd > 32 ? 64 : 32) < sm_count()) return conv_mma_launch<T, 1, 1, 2, 4, 32>(p, cpad, false);
+    if (2 * tiles * ceil_div(p.Cd, p.Cd > 32 ? 64 : 32) < sm_count()) {
+        // Long sums under few tiles run at the speed of one CTA's chain of taps and channels.  A cluster that shares the channels costs
+        // about 1 us more and pays from 48 products of 16 (fp32: 8) channels a pixel, with three CTAs or more and two per SM at most:
+        // one stream of 96 -> 96 on 9 x 13 with stride 2, fp32, 13.4 -> 6.8 us forward and 8.9 -> 7.1 back, 256 -> 256 on 8 x 8 25.8 -> 9.3,
+        // 512 -> 500 on 4 x 4 with 1 x 1 windows, whose weights bound it, fp16, 15.8 -> 8.1; but 32 -> 16 on 32 x 32 (36) 6.0 -> 6.2 and
+        // 64 -> 64 on 32 x 32 with two CTAs 8.6 -> 8.9.
+        const int nck = cpad / CK;
+        int ctas = 0, taps = 0;
+        for (int i = 0; i < p.ncls; i++) {
+            const int P = p.cls[i].Hc * p.cls[i].Wc;
+            ctas += P < 32 ? ceil_div(p.n * P, 32) : p.n * ceil_div(P, 32);
+            taps = std::max(taps, p.cls[i].ntaps);
+        }
+        ctas *= ceil_div(p.Cd, 16);
+        const int most = std::min(std::min(8, nck), 2 * sm_count() / ctas);
+        if (most >= 3 && (taps * nck >= 48 || (taps == 1 && nck >= 24))) {
+            p.kshare = ceil_div(nck, most) * CK;
+            p.ksplit = ceil_div(cpad, p.kshare);
+            if (conv_mma_launch<T, 1, 1, 2, 4, 32, true>(p, p.kshare, false)) return true;
+        }
+        return conv_mma_launch<T, 1, 1, 2, 4, 32>(p, cpad, false);
+    }
     if (p.Cd > 32) return conv_mma_launch<T, 2, 2, 4, 1, 128>(p, cpad, false) || conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
     if (p.Cd > 16) return conv_mma_launch<T, 2, 1, 8, 1, 128>(p, cpad, false) || conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);
     return conv_mma_launch<T, 1, 1, 8, 1, 128>(p, cpad, false);

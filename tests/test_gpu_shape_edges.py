@@ -83,6 +83,16 @@ def test_conv2d_of_few_pixels(run, oracle, cin, h, w, cout, k, stride, n):
     assert any("wg_cluster" in t[0] for t in run.pkg.profile_table(run.lib))
 
 
+# long sums under few pixels, one cluster per result tile whose CTAs share the source channels: channel counts that divide into unequal
+# shares, a last share of few channels, strides whose parities have different taps (some none), more streams in a tile, 1 x 1 windows
+LONG_SUMS = [(96, 9, 13, 96, 3, 2, 1), (60, 13, 18, 8, 3, 1, 1), (130, 7, 9, 100, 3, 1, 1), (400, 4, 4, 390, 1, 1, 1), (50, 5, 5, 52, 5, 1, 3), (75, 3, 3, 66, 3, 3, 7), (200, 5, 7, 17, 2, 1, 1), (48, 28, 28, 40, 5, 1, 1)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", LONG_SUMS)
+def test_conv2d_of_long_sums(run, oracle, cin, h, w, cout, k, stride, n):
+    test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+
+
 # half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
 # tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
 # for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
