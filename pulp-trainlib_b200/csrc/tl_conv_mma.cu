@@ -1098,7 +1098,8 @@ template <class T> static bool cm_wg_params(const ConvGeom &geom, const T *x, co
 
 // Where it pays: while every CTA has an SM (a cluster of 16 needs most of a GPC, and 16 x 16 tiles read more per product than the kernel
 // above: one stream of 64 -> 64 on 32 x 32, 256 CTAs, fp32 12.1 us against 9.4 there) and up to 2048 pixels (32 -> 32 on 64 x 64:
-// 11.7 against 10.7; 32 -> 64 on two planes of 32 x 32, 9.6 against 9.8, is about where they meet).  Very few pixels under many channels
+// 11.7 against 10.7; 32 -> 64 on two planes of 32 x 32, 9.6 against 9.8, is about where they meet) that every CTA stages at once (33 -> 27,
+// 1 x 1, on 14 planes of 7 x 20, two tiles a CTA, fp16: 8.1 against 7.1).  Very few pixels under many channels
 // leave the kernel above one partial result to write and read again per CTA: there up to eight CTAs an SM (256 -> 256 on 8 x 8
 // 15.5 -> 11.4 us, 512 -> 512 on 4 x 4 37.1 -> 20.7), except for 1 x 1 windows (512 -> 512 on 4 x 4: 8.9 against 19.3).
 template <class T> static bool cm_wg_cluster_plan(const ConvGeom &g, const T *x, const T *dy, CmWg &p, int &ranks, size_t &smem)
@@ -1110,7 +1111,7 @@ template <class T> static bool cm_wg_cluster_plan(const ConvGeom &g, const T *x,
     smem = std::max((size_t)p.t_off + 4 * 128, (size_t)p.shares * CMC_TILE * (CMC_TILE * p.KK + 4) * 4);
     for (ranks = 1; ranks < std::min(p.tiles, CMC_MAX);) ranks *= 2;
     const long long pixels = (long long)p.n * p.Ho * p.Wo, ctas = (long long)p.ci_tiles * ceil_div(p.Co, CMC_TILE) * ranks;
-    return smem <= CM_SMEM_MAX && (ctas <= sm_count() || (p.KK > 1 && pixels <= 64 && ctas <= 8ll * sm_count()));
+    return p.tiles <= CMC_MAX && smem <= CM_SMEM_MAX && (ctas <= sm_count() || (p.KK > 1 && pixels <= 64 && ctas <= 8ll * sm_count()));
 }
 template <class T> bool conv_mma_wg_cluster(const ConvGeom &g, const T *x, const T *dy, T *dw)
 {

@@ -102,10 +102,18 @@ template <class T, int ROWS, int KC, int PAD, int NT> struct GgLoader {
         } else if (SZ == 4 || vw == V4) {
             const int cb = min(max(lc, 0), V4) * SZ;
             constexpr int Q = ROWS * KC / V4 / NT;
+            const char *from = ptr;
+            uint32_t to = stage + sm;
+            if (__all_sync(0xffffffffu, s + (Q - 1) * s_step < ls && lc >= V4)) {
+                // all of a warp's pieces inside the matrix: half the instructions of a piece are its limits
 #pragma unroll 8
-            for (int q = 0; q < Q; q++) {
-                const int b = s + q * s_step < ls ? cb : 0;
-                gg_cp4(stage + sm + q * sm_pass, b ? ptr + q * pass : safe, b);
+                for (int q = 0; q < Q; q++, from += pass, to += sm_pass) gg_cp4(to, from, 4);
+            } else {
+#pragma unroll 8
+                for (int q = 0; q < Q; q++, from += pass, to += sm_pass) {
+                    const int b = s + q * s_step < ls ? cb : 0;
+                    gg_cp4(to, b ? from : safe, b);
+                }
             }
         } else {
             constexpr int Q = ROWS * KC / NT, U = 8;
@@ -241,11 +249,8 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
     };
     open_segment();
     // what the end of the kernel reads of its parameters: a first read of one misses the constant cache
-    T *C = p.C + b * p.c_bs;
-    const long long c_rs = p.c_rs, c_cs = p.c_cs;
-    const float alpha = p.alpha;
-    const int plain = p.plain, nsplits = p.splits.d;
-    asm volatile("" ::"l"(C), "l"(c_rs), "l"(c_cs), "f"(alpha), "r"(plain));
+    asm volatile("" ::"l"(p.C), "l"(p.c_bs), "l"(p.c_rs), "l"(p.c_cs), "f"(p.alpha), "r"(p.plain));
+    const int nsplits = p.splits.d;
     pdl_wait();                                                            // everything above reads parameters only
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(gg_smem);
     auto fetch = [&](int stage) {
@@ -350,6 +355,10 @@ __global__ void __launch_bounds__(32 * WM * WN * WK, OCC) gemm_group_kernel(cons
         __threadfence();
         if (tid == 0) gg_tickets[p.ticket0 + tile] = 0;
     }
+    T *C = p.C + b * p.c_bs;
+    const long long c_rs = p.c_rs, c_cs = p.c_cs;
+    const float alpha = p.alpha;
+    const int plain = p.plain;
     for (int e = tid; e < QUADS; e += NT) {
         const int i = e / Q, j = (e % Q) * 4;
         if (i0 + i >= p.N || j0 + j >= p.M) continue;
@@ -408,6 +417,14 @@ template <class T> static void gg_operand(const T *const *ptrs, int nptr, long l
     if (fits(V16)) vl = sizeof(T) == 4 ? 2 : 3; else if (V4 > 1 && fits(V4)) vl = 1;
 }
 
+// What a chunk of an operand costs beyond that of 16-byte copies: more of them, and single halves come by way of registers, eight loads in
+// flight at a time (175 x 869 x 60 with rows of 869 halves: 10.1 us with no split, 5.8 with the ones that this asks for).
+template <class T, int ROWS, int KC, int NT> static constexpr int gg_copy_cycles(int vl)
+{
+    constexpr int V16 = 16 / (int)sizeof(T), V4 = 4 / (int)sizeof(T);
+    return (1 << vl) == V16 ? 0 : (1 << vl) == V4 ? ROWS * KC / V4 / NT * 8 : ROWS * KC / NT / 8 * 200;
+}
+
 // CYC: cycles of one K chunk in a CTA (measured with the SMs about as full as such products make them), in units of those of a split:
 // writing the partial tile, the ticket and the last CTA's sum cost 2500 cycles, and 150 more per split.
 template <class T, int BM, int BN, int WM, int WN, int WK, int KC, int ST, int OCC, int CYC, int G>
@@ -461,10 +478,11 @@ static void gg_launch(Scope &sc, const GemmGroup<T> *list, int count)
         const long long most = !filled ? (want * p.chunks + tile_steps - 1) / std::max(1ll, tile_steps) : (tiles_all < 4 * sm_count() && p.chunks >= 2 * shortest ? p.chunks / std::max(shortest, 1) : 1);
         if (most > 1 && p.chunks >= 2) {
             const int cap = (int)std::min<long long>(std::min<long long>(most, p.chunks), 64);
-            long long best = (long long)p.chunks * CYC;
+            const long long cyc = CYC + gg_copy_cycles<T, BM, KC, Cfg::NT>(p.a_vl) + gg_copy_cycles<T, BN, KC, Cfg::NT>(p.b_vl);
+            long long best = p.chunks * cyc;
             for (int s = 2; s <= cap; s++) {
                 const int per = ceil_div(p.chunks, s);
-                const long long cost = (long long)per * CYC + 2500 + 150 * s;
+                const long long cost = per * cyc + 2500 + 150 * s;
                 if (cost < best) { best = cost; splits = ceil_div(p.chunks, per); }
             }
             if (splits > 1) {
