@@ -458,6 +458,7 @@ template <class T> static bool try_pointwise_wg(const ConvGeom &g, const T *x, c
 }
 template <class T> void conv_fw(Scope &sc, const ConvGeom &g, const T *x, const T *w, const T *bias, T *y)
 {
+    if constexpr (sizeof(T) == 4) if (conv_pw_fw(g, x, w, bias, y)) return;
     if (!g.depthwise && try_pointwise<T>(g, x, w, bias, y, false)) return;
     if constexpr (sizeof(T) == 2) if (conv_px_fw(g, x, w, bias, y)) { profile_add_flops(conv_flops(g)); return; }
     if (!g.depthwise && try_tc_fw<T>(sc, g, x, w, bias, y)) return;
@@ -585,6 +586,7 @@ template <class T> void conv_ig_accumulate(Scope &sc, const ConvGeom &g, const T
 }
 template <class T> void conv_ig(Scope &sc, const ConvGeom &g, const T *dy, const T *w, T *dx)
 {
+    if constexpr (sizeof(T) == 4) if (conv_pw_ig(g, dy, w, dx)) return;
     if (!g.depthwise && try_pointwise<T>(g, dy, w, nullptr, dx, true)) return;
     if constexpr (sizeof(T) == 2) if (conv_px_ig(g, dy, w, dx)) { profile_add_flops(conv_flops(g)); return; }
     if (!g.depthwise && try_tc_ig<T>(sc, g, dy, w, dx)) return;

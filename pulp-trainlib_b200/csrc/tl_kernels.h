@@ -149,6 +149,9 @@ bool conv1x1s_wg(const ConvGeom &g, const float *x, const float *dy, float *part
 bool conv_px_fw(const ConvGeom &g, const __half *x, const __half *w, const __half *bias, __half *y);
 bool conv_px_ig(const ConvGeom &g, const __half *dy, const __half *w, __half *dx);
 bool conv_px_wg(Scope &sc, const ConvGeom &g, const __half *x, const __half *dy, __half *dw, __half *db);   // db: the bias gradient too, or null
+// fp32 pointwise layers over many pixels on tcgen05 (tl_conv_pw.cu); false = not covered, nothing launched
+bool conv_pw_fw(const ConvGeom &g, const float *x, const float *w, const float *bias, float *y);
+bool conv_pw_ig(const ConvGeom &g, const float *dy, const float *w, float *dx);
 // any-shape convolutions on mma.sync, fp16 and 3xTF32 (tl_conv_mma.cu); false = geometry not covered, nothing launched
 template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, const T *bias, T *y);
 template <class T> bool conv_mma_ig(const ConvGeom &g, const T *dy, const T *w, T *dx);

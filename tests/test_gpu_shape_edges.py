@@ -93,6 +93,23 @@ def test_conv2d_of_long_sums(run, oracle, cin, h, w, cout, k, stride, n):
     test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
 
 
+# single-precision pointwise layers over many pixels (tl_conv_pw.cu): CTAs whose last 128 pixels are cut short, planes smaller than that, odd
+# ones, one and many pieces of channels, channel counts off multiples of 8 and 16, more than 128 result channels (three products, one
+# accumulator), weights that leave room for two, three or four stages, weights that do not fit (another kernel), the GEMM's layers
+POINTWISE = [(64, 28, 28, 128, 13), (33, 17, 19, 70, 40), (7, 4, 4, 20, 700), (1, 30, 31, 40, 11), (20, 23, 23, 200, 20), (40, 25, 25, 256, 16), (96, 16, 17, 160, 37), (72, 100, 100, 72, 1), (96, 30, 30, 120, 8), (5, 47, 48, 17, 30),
+             (256, 20, 20, 256, 25), (12, 97, 98, 9, 9)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,n", POINTWISE)
+def test_pointwise_over_many_pixels(run, oracle, cin, h, w, cout, n):
+    if run.half:
+        pytest.skip("single precision only")
+    run.lib.trainlib_profile(1)
+    test_conv2d_shapes(run, oracle, cin, h, w, cout, 1, 1, n)
+    run.lib.trainlib_profile(0)
+    assert any("conv_pw_kernel" in t[0] for t in run.pkg.profile_table(run.lib)) == (cin < 256)
+
+
 # half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
 # tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
 # for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
