@@ -1088,6 +1088,21 @@ template <> bool try_1x1_wg<float>(Scope &sc, const ConvGeom &g, const float *x,
     return true;
 }
 
+// weight gradient of a pointwise layer over many pixels: per-CTA partials + the fixed-order reduction
+template <class T> static bool try_pw_wg(Scope &, const ConvGeom &, const T *, const T *, T *) { return false; }
+template <> bool try_pw_wg<float>(Scope &sc, const ConvGeom &g, const float *x, const float *dy, float *dw)
+{
+    int groups = 0;
+    if (!conv_pw_wg(g, x, dy, nullptr, &groups, true)) return false;
+    const long long nw = (long long)g.Cout * g.Cin;
+    bool deferred;
+    float *part = partials_alloc<float>(sc, (size_t)groups * nw, deferred, false);
+    if (!part) return false;
+    if (!conv_pw_wg(g, x, dy, part, &groups, false)) return false;
+    reduce_partials<float>(part, dw, nw, groups, deferred);
+    return true;
+}
+
 // weight gradient on mma.sync: per-CTA partials + the fixed-order reduction
 template <class T> static bool try_mma_wg(Scope &sc, const ConvGeom &g, const T *x, const T *dy, T *dw)
 {
@@ -1128,6 +1143,7 @@ template <class T> void conv_wg(Scope &sc, const ConvGeom &g, const T *x, const 
     const long long nw = (long long)g.Cout * g.Cin * KK;
     const int ci_tiles = ceil_div(g.Cin, 16), co_tiles = ceil_div(g.Cout, 16);
     const bool k3 = g.Hk == 3 && g.Wk == 3 && g.padL == 1, k1 = g.Hk == 1 && g.Wk == 1 && g.padL == 0 && g.padU == 0;
+    if (try_pw_wg<T>(sc, g, x, dy, dw)) return;
     if (try_pointwise_wg<T>(g, x, dy, dw)) return;
     if (try_tc_wg<T>(sc, g, x, dy, dw)) return;
     if (try_1x1_wg<T>(sc, g, x, dy, dw)) return;

@@ -1,4 +1,5 @@
-// Single-precision pointwise layers (1 x 1, stride 1) over many pixels in one launch: forward and input gradient as 3xTF32 products on tcgen05
+// Single-precision pointwise layers (1 x 1, stride 1) over many pixels as 3xTF32 products on tcgen05, each direction in one launch: forward and input
+// gradient
 //     dst[s][m][p] = sum over k of w[m][k] * src[s][k][p] (+ bias[m])          (input gradient: w transposed)
 // [ref: lib/sources/pulp_conv_pw_fp32.c:27 (FW), :233 (IG)]
 //
@@ -246,5 +247,254 @@ static bool pw_covers(const ConvGeom &g, int sources, int results)
 // false = not covered, nothing launched
 bool conv_pw_fw(const ConvGeom &g, const float *x, const float *w, const float *bias, float *y) { return pw_covers(g, g.Cin, g.Cout) && pw_run(g, x, w, bias, y, false); }
 bool conv_pw_ig(const ConvGeom &g, const float *dy, const float *w, float *dx) { return pw_covers(g, g.Cout, g.Cin) && pw_run(g, dy, w, nullptr, dx, true); }
+
+// ---------------------------------------------------------------- weight gradient
+//     dW[co][ci] = sum over the pixels of all streams of dY[co][p] * X[ci][p]          [ref: lib/sources/pulp_conv_pw_fp32.c:121]
+// The contraction runs over the pixels, which are contiguous in memory: four of them are a 16-byte piece of the K-major layout as they
+// come.  A CTA takes one stretch of the pixels, 32 at a time (three groups of four converter warps, each with a stage of its own): rows of
+// X in hi and lo, rows of dY in hi and lo.  The tensor core truncates what it accumulates, so a chain is four k-steps long: each piece has a
+// fresh accumulator (two banks), and eight warps add it to sums that they hold in registers.  Lanes are source channels, so that a
+// CTA's partial result is written coalesced in the layout of dW; a second launch adds the partial results.
+static constexpr int PWW_GROUPS = 3, PWW_STAGES = 2 * PWW_GROUPS, PWW_CONV = PWW_GROUPS * 128, PWW_ISSUERS = 2, PWW_THREADS = PWW_CONV + PWW_ISSUERS * 32 + 256;
+
+struct PwWgParams {
+    const float *x, *dy; float *part; int *status;
+    int P, Cin, Cout, total, per;               // plane, channels, pixels of all streams, of a CTA
+    int N, co_slices, RA, la, fold, lbo, cols;  // result channels of a slice, slices of them; source channels of a slice, padded; rows to their lo parts; pieces of four pixels
+    uint32_t stage_bytes;
+};
+
+// Rows u = 0, 1, ... of a lane, a step apart: of X up to nx, of dY from there to nu (the same in all lanes of a warp); `have`: those that exist.
+template <bool VEC> __device__ __forceinline__ void pw_wg_load(const float *f, const float *fy, long long step, float (&v)[8][4], int nx, int nu, uint32_t have,
+                                                               int left, int wrap, long long next_x, long long next_y)
+{
+#pragma unroll
+    for (int u = 0; u < 8; u++, f += step) {
+        if (u >= nu) break;
+        if (u == nx) f = fy;
+        const bool ok = (have >> u) & 1;
+        if (VEC) {
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ok) q = *reinterpret_cast<const float4 *>(f);
+            v[u][0] = q.x; v[u][1] = q.y; v[u][2] = q.z; v[u][3] = q.w;
+        } else {
+            const long long next = u < nx ? next_x : next_y;                                   // from the end of a plane to the next stream's
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[u][e] = ok && e < left ? f[e + (e >= wrap ? next : 0)] : 0.f;
+        }
+    }
+}
+__device__ __forceinline__ void pw_wg_store(const float (&v)[8][4], uint32_t to, uint32_t to_y, uint32_t lo_x, uint32_t lo_y, uint32_t step, int nx, int nu)
+{
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        if (u >= nu) break;
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) pw_split(v[u][e], h[e], l[e]);
+        const uint32_t at = (u < nx ? to : to_y) + (uint32_t)u * step;
+        pw_sts(at, h);
+        pw_sts(at + (u < nx ? lo_x : lo_y), l);
+    }
+}
+
+template <bool VEC, int PX> __global__ void __launch_bounds__(PWW_THREADS, 1) conv_pw_wg_kernel(const __grid_constant__ PwWgParams p)
+{
+    constexpr int KG = PX / 4, RS = 128 / KG, IB = 32 / PX;                 // pieces of four pixels, rows that a group of warps loads at once, pieces of an accumulator
+    extern __shared__ __align__(1024) unsigned char pw_smem[];
+    __shared__ __align__(8) uint64_t full[PWW_STAGES], empty[PWW_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int lo = blockIdx.x * p.per, hi = min(p.total, lo + p.per), pieces = (hi - lo + PX - 1) / PX, N = p.N, P = p.P;
+    const int co0 = ((int)blockIdx.y % p.co_slices) * N, ci0 = ((int)blockIdx.y / p.co_slices) * p.RA;
+    volatile int *abort_flag = &abort_s;
+    const uint32_t sm = tc::smem_u32(pw_smem);
+    if (warp == 0) { tc::tmem_alloc(&tmem_s, (uint32_t)p.cols); tc::tmem_relinquish(); }
+    if (tid == 32) {
+        for (int i = 0; i < PWW_STAGES; i++) { tc::mbar_init(&full[i], 4); tc::mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; i++) { tc::mbar_init(&acc_full[i], 1); tc::mbar_init(&acc_empty[i], 8); }
+        tc::fence_barrier_init();
+        abort_s = 0;
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tmem_s;
+    pdl_wait();
+
+    if (warp < PWW_CONV / 32) {
+        const int group = warp >> 2, kg = lane % KG, wq = RS / 4 * (warp & 3), r0 = lane / KG + wq;
+        const int nx = (p.RA - wq + RS - 1) / RS, nu = (p.RA + N - wq + RS - 1) / RS;
+        uint32_t have = 0;
+        for (int u = 0; u < nu; u++) have |= (uint32_t)(u < nx ? ci0 + r0 + RS * u < p.Cin : co0 + r0 + RS * u - p.RA < p.Cout) << u;
+        int g = lo + group * PX + kg * 4, s = g / P, pp = g - s * P;
+        const float *x = p.x + ((long long)s * p.Cin + ci0 + r0) * P + pp, *y = p.dy + ((long long)s * p.Cout + co0 + r0 + RS * nx - p.RA) * P + pp;
+        const long long step = (long long)RS * P, next_x = (long long)(p.Cin - 1) * P, next_y = (long long)(p.Cout - 1) * P;
+        const uint32_t to = sm + (uint32_t)group * p.stage_bytes + (uint32_t)(kg * p.lbo + r0) * 16u, lo_x = (uint32_t)p.la * 16u, lo_y = (uint32_t)N * 16u;
+        float v[8][4];
+        for (int c = group, t = 0; c < pieces; c += PWW_GROUPS, t++) {
+            pw_wg_load<VEC>(x, y, step, v, nx, nu, g < hi ? have : 0u, hi - g, P - pp, next_x, next_y);
+            const int st = group + (t & 1) * PWW_GROUPS;
+            if (!tc::warp_wait_or_abort(&empty[st], (uint32_t)(~t >> 1) & 1u, abort_flag, p.status, 59, 20u, lane)) break;
+            const uint32_t at = to + (uint32_t)((t & 1) * PWW_GROUPS) * p.stage_bytes;
+            pw_wg_store(v, at, at + (uint32_t)(2 * p.la - p.RA) * 16u, lo_x, lo_y, RS * 16u, nx, nu);
+            tc::fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&full[st]);
+            g += PWW_GROUPS * PX; pp += PWW_GROUPS * PX; x += PWW_GROUPS * PX; y += PWW_GROUPS * PX;
+            while (pp >= P) { pp -= P; x += next_x; y += next_y; }
+        }
+    } else if (warp < PWW_CONV / 32 + PWW_ISSUERS) {
+        // ---- the products: 32 pixels for an accumulator, each issuing warp one of the two (a wait, a commit and a product cost one warp 100 to
+        // 150 cycles each whatever their size)
+        const uint64_t d0 = tc::smem_desc_kmajor(0u, (uint32_t)p.lbo * 16u, 128u);
+        const uint32_t hw = (uint32_t)(d0 >> 32), lw0 = (uint32_t)d0 + (sm >> 4);
+        const uint32_t id1 = tc::mma_idesc(tc::FMT_TF32, 128, (uint32_t)N), id2 = tc::mma_idesc(tc::FMT_TF32, 128, (uint32_t)(2 * N));
+        const int bank = warp - PWW_CONV / 32;
+        const uint32_t d = tmem + (uint32_t)(bank * 2 * N);
+        int st = IB * bank; uint32_t ph = 0, use = 0;
+        bool ok = true;
+        for (int c0 = IB * bank; c0 < pieces && ok; c0 += IB * PWW_ISSUERS, use++) {
+            if (use && !tc::warp_wait_or_abort(&acc_empty[bank], (use - 1) & 1u, abort_flag, p.status, 60, 0u, lane)) break;
+            for (int c = c0; c < min(pieces, c0 + IB); c++, st++) {
+                if (!tc::warp_wait_or_abort(&full[st], ph, abort_flag, p.status, 61, 0u, lane)) { ok = false; break; }
+                tc::tc_fence_after();
+                uint32_t aw = lw0 + (uint32_t)st * (p.stage_bytes / 16);
+#pragma unroll
+                for (int k = 0; k < PX / 8; k++, aw += 2u * (uint32_t)p.lbo) {
+                    const uint64_t ah = ((uint64_t)hw << 32) | aw, al = ah + (uint32_t)p.la, bh = ah + (uint32_t)(2 * p.la);
+                    if (tc::elect_one()) {
+                        tc::mma_tf32_ss(d, ah, bh, id2, (uint32_t)(c > c0 || k > 0));
+                        if (!p.fold) tc::mma_tf32_ss(d + (uint32_t)N, al, bh, id1, 1u);
+                    }
+                }
+                if (tc::elect_one()) tc::mma_commit(&empty[st]);
+                __syncwarp();
+            }
+            if (!ok) break;
+            if (tc::elect_one()) tc::mma_commit(&acc_full[bank]);
+            __syncwarp();
+            st += IB * (PWW_ISSUERS - 1);
+            if (st >= PWW_STAGES) { st -= PWW_STAGES; ph ^= 1; }
+        }
+    } else {
+        // ---- sums: a lane has a source channel, each set of four warps half of the result channels
+        const int quad = warp & 3, set = (warp - PWW_CONV / 32 - PWW_ISSUERS) >> 2, ng = N / 16, half = (ng + 1) / 2, first = set * half, count = min(half, ng - first);
+        float acc[4][16];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int j = 0; j < 16; j++) acc[q][j] = 0.f;
+        bool ok = true;
+        for (int c = 0; c < (pieces + IB - 1) / IB; c++) {
+            const int bank = c & 1;
+            if (!tc::warp_wait_or_abort(&acc_full[bank], (uint32_t)(c >> 1) & 1u, abort_flag, p.status, 62, 20u, lane)) { ok = false; break; }
+            tc::tc_fence_after();
+            const uint32_t d = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(bank * 2 * N + first * 16);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (q < count) {
+#pragma unroll
+                    for (int e = 0; e < 16; e += 8) {
+                        uint32_t a[8], b[8];
+                        tc::tmem_ld8(d + (uint32_t)(q * 16 + e), a);
+                        tc::tmem_ld8(d + (uint32_t)(N + q * 16 + e), b);
+                        tc::tmem_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 8; j++) acc[q][e + j] += __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                    }
+                }
+            }
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&acc_empty[bank]);
+        }
+        const int row = quad * 32 + lane, ci = ci0 + row;
+        if (p.fold) {                                                       // the products of X_lo, in lanes 64 .. 127
+            float *other = reinterpret_cast<float *>(pw_smem) + (set * 64) * 64 + (row & 63);
+            if (row >= 64) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int j = 0; j < 16; j++) other[(q * 16 + j) * 64] = acc[q][j];
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (row < 64) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int j = 0; j < 16; j++) acc[q][j] += other[(q * 16 + j) * 64];
+            }
+        }
+        if (ok && row < p.RA && ci < p.Cin) {
+            float *to = p.part + (long long)blockIdx.x * p.Cin * p.Cout + ci;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int co = co0 + (first + q) * 16 + j;
+                    if (q < count && co < p.Cout) to[(long long)co * p.Cin] = acc[q][j];
+                }
+        }
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, (uint32_t)p.cols); }
+}
+
+// One partial result per CTA into `part`, their number into *groups; dry_run: only that; false = not covered.
+// What bounds it: the converter warps' chain of load, split, store and hand-over at three pieces in flight (64 -> 64 channels, a piece of 32 pixels:
+// 1200 cycles, where its bytes take 650); loading the next piece's first half between the stores of this one was slower (the proxy
+// fence waits for loads in flight), 16 pixels at a time took 1.3 times as long for up to 128 rows.  Measured with the sum of the
+// partial results over eighty random layers (us, mma.sync / here):
+//   64 streams of 64 -> 128 on 28 x 28 32.6 / 19.6;  64 of 160 -> 96 on 20 x 20 58.5 / 17.0;  512 of 64 -> 64 on 32 x 32 130 / 77;  256 of 128 -> 64
+//     on 28 x 28 126 / 51;  45402 pixels of 14 -> 24 14.5 / 13.7
+// The error against 64 bits is 0.65 to 1.08 times that of mma.sync's (the mean 0.95; shorter sums in registers, from more CTAs, cost
+// 3 to 30 us at 200 to 500 thousand pixels and did not change it).
+//   few pixels: 7161 of 72 -> 72 14.7 / 11.8, 9976 of 8 -> 95 9.7 / 11.8, 4797 of 6 -> 16 7.6 / 8.5, 2400 of 52 -> 66 10.0 / 10.5
+bool conv_pw_wg(const ConvGeom &g, const float *x, const float *dy, float *part, int *groups, bool dry_run)
+{
+    if (g.depthwise || gemm_path() != 0 || g.Hk != 1 || g.Wk != 1 || g.sh != 1 || g.sw != 1 || g.padU != 0 || g.padL != 0 || g.Hin != g.Hout || g.Win != g.Wout) return false;
+    const long long total = (long long)g.n * g.Hin * g.Win;
+    if (total >= (1ll << 30) || g.Hin * g.Win < 16) return false;
+    if (total < 72ll * sm_count() && !(total >= 48ll * sm_count() && g.Cin >= 32 && g.Cout >= 32)) return false;
+    PwWgParams p = {};
+    p.P = g.Hin * g.Win; p.Cin = g.Cin; p.Cout = g.Cout; p.total = (int)total;
+    p.co_slices = ceil_div(g.Cout, 128);
+    p.N = ceil_div(ceil_div(g.Cout, p.co_slices), 16) * 16;
+    const int ci_slices = ceil_div(g.Cin, 128), slices = p.co_slices * ci_slices;
+    p.RA = ceil_div(ceil_div(g.Cin, ci_slices), 16) * 16;
+    if (slices > sm_count() / 8) return false;
+    p.fold = p.RA <= 64; p.la = p.fold ? 64 : p.RA;
+    const int px = p.RA + p.N <= 128 && PWW_STAGES * 8u * (2 * (p.la + p.N) + 1) * 16 + 2048 <= PW_SMEM ? 32 : 16;      // pixels of a piece: eight 16-byte loads a lane
+    p.lbo = 2 * (p.la + p.N) + (px == 32 ? 1 : 2);                         // an odd number: eight groups of pixels store to all banks; two past a multiple of eight: four groups x two rows do
+    p.stage_bytes = (uint32_t)(px / 4 * p.lbo) * 16u;
+    p.per = std::max(128, ceil_div(ceil_div(total, sm_count() / slices), 32) * 32);
+    *groups = ceil_div(total, p.per);
+    if (dry_run) return true;
+    p.cols = 32;
+    while (p.cols < 4 * p.N) p.cols *= 2;
+    p.x = x; p.dy = dy; p.part = part; p.status = tc_status_word();
+    if (!p.status) return false;
+    // the products read 128 rows whatever X has: rows past the last are not used, but have to lie in shared memory
+    const size_t smem = PWW_STAGES * (size_t)p.stage_bytes + 128 * 16;
+    const bool vec = p.P % 4 == 0 && (((uintptr_t)x | (uintptr_t)dy) & 15) == 0;
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(conv_pw_wg_kernel<true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        cudaFuncSetAttribute(conv_pw_wg_kernel<false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        cudaFuncSetAttribute(conv_pw_wg_kernel<true, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        cudaFuncSetAttribute(conv_pw_wg_kernel<false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        attr = true;
+    }
+    const dim3 grid(*groups, slices);
+    if (px == 32 && vec) TL_LAUNCH((conv_pw_wg_kernel<true, 32>), grid, PWW_THREADS, smem, p);
+    else if (px == 32) TL_LAUNCH((conv_pw_wg_kernel<false, 32>), grid, PWW_THREADS, smem, p);
+    else if (vec) TL_LAUNCH((conv_pw_wg_kernel<true, 16>), grid, PWW_THREADS, smem, p);
+    else TL_LAUNCH((conv_pw_wg_kernel<false, 16>), grid, PWW_THREADS, smem, p);
+    profile_add_flops(2.0 * total * g.Cin * g.Cout);
+    return true;
+}
 
 } // namespace tl

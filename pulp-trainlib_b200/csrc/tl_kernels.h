@@ -152,6 +152,7 @@ bool conv_px_wg(Scope &sc, const ConvGeom &g, const __half *x, const __half *dy,
 // fp32 pointwise layers over many pixels on tcgen05 (tl_conv_pw.cu); false = not covered, nothing launched
 bool conv_pw_fw(const ConvGeom &g, const float *x, const float *w, const float *bias, float *y);
 bool conv_pw_ig(const ConvGeom &g, const float *dy, const float *w, float *dx);
+bool conv_pw_wg(const ConvGeom &g, const float *x, const float *dy, float *part, int *groups, bool dry_run);
 // any-shape convolutions on mma.sync, fp16 and 3xTF32 (tl_conv_mma.cu); false = geometry not covered, nothing launched
 template <class T> bool conv_mma_fw(const ConvGeom &g, const T *x, const T *w, const T *bias, T *y);
 template <class T> bool conv_mma_ig(const ConvGeom &g, const T *dy, const T *w, T *dx);

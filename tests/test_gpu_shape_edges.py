@@ -110,6 +110,21 @@ def test_pointwise_over_many_pixels(run, oracle, cin, h, w, cout, n):
     assert any("conv_pw_kernel" in t[0] for t in run.pkg.profile_table(run.lib)) == (cin < 256)
 
 
+# their weight gradient: lanes with hi and lo rows of X (up to 64 source channels) and without, slices of either side's channels, pieces of 16 and
+# of 32 pixels, planes that no 16-byte load fits, a last piece cut short
+POINTWISE_WG = [(64, 28, 28, 128, 15), (33, 17, 19, 70, 40), (7, 4, 4, 20, 700), (1, 30, 31, 40, 13), (20, 23, 23, 200, 21), (160, 20, 20, 96, 27), (96, 31, 30, 33, 9), (130, 25, 25, 140, 18), (5, 47, 48, 17, 80), (64, 40, 41, 8, 98)]
+
+
+@pytest.mark.parametrize("cin,h,w,cout,n", POINTWISE_WG)
+def test_pointwise_weight_gradient_over_many_pixels(run, oracle, cin, h, w, cout, n):
+    if run.half:
+        pytest.skip("single precision only")
+    run.lib.trainlib_profile(1)
+    test_conv2d_shapes(run, oracle, cin, h, w, cout, 1, 1, n)
+    run.lib.trainlib_profile(0)
+    assert any("conv_pw_wg_kernel" in t[0] for t in run.pkg.profile_table(run.lib))
+
+
 # half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
 # tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
 # for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
