@@ -1,5 +1,6 @@
-// Depthwise convolution, one filter per channel [ref: lib/sources/pulp_conv_naive_fp32.c:29,113,153], for planes that fit
-// shared memory.  The layer does nine multiply-adds per value read, so nothing may be read twice from HBM.  A CTA stages whole planes of one or more
+// Depthwise convolution, one filter per channel [ref: lib/sources/pulp_conv_naive_fp32.c:29,113,153].  The layer does nine multiply-adds per
+// value read, so nothing may be read twice from HBM.  3 x 3 filters with stride 1 work in registers (the strips below).  For the others, on planes
+// that fit shared memory, a CTA stages whole planes of one or more
 // (stream, channel) pairs with their zero border once (coalesced, each value read once from HBM), and every window is then
 // read from shared memory without bounds checks.  64 channels of 28 x 28 x 64 streams, fp32 (25.7 MB per pass): forward 45 us
 // and input gradient 92 us with one bounds-checked global read per tap; 145 us for the weight gradient, which ran one CTA per
@@ -112,22 +113,6 @@ __global__ void __launch_bounds__(256) dw_wg_plane_kernel(const __grid_constant_
     }
 }
 
-// ---------------------------------------------------------------- 3 x 3, stride 1
-// The common case with four neighbouring results per thread: a window row of six values serves four results (two or three
-// shared loads per twelve multiply-adds instead of one per multiply-add), the filter sits in registers, and rows of whole
-// 16-byte groups (8 bytes in fp16) move as vectors.  Shared-memory rows hold image column w at index 4 + w between zero columns.
-// What bounds it is the shared-memory pipe: busy 88 % of the cycles of a forward pass of the layer above (11 us by itself), half of
-// its wavefronts bank conflicts.
-template <class T> struct DwVec;
-template <> struct DwVec<float> { typedef float4 V; };
-template <> struct DwVec<__half> { typedef uint2 V; };
-__device__ __forceinline__ float4 dw_ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ float4 dw_ld4(const __half *p)
-{
-    const uint2 u = *reinterpret_cast<const uint2 *>(p);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-}
 __device__ __forceinline__ void dw_st4(float *p, const float (&v)[4]) { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void dw_st4(__half *p, const float (&v)[4])
 {
@@ -135,116 +120,108 @@ __device__ __forceinline__ void dw_st4(__half *p, const float (&v)[4])
     *reinterpret_cast<uint2 *>(p) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
 }
 
-struct Dw3Params {
+// A thread has V neighbouring columns of a strip of up to R rows of one plane: every row of the source is read once per strip (its
+// neighbours' columns come from L1), straight into registers, all rows of the strip in flight together, with no shared memory, no
+// zero border and no barrier.  V = 4: rows of whole 16-byte groups (8 in fp16) and one column of padding.  Staging planes in shared
+// memory with a zero border was bound by that memory's pipe, half of its wavefronts bank conflicts; now it is the loads: 25.7 MB in
+// 6.7 us of the layer above (3.8 TB/s), and with rows of odd lengths, three 4-byte loads a value, their issue.  us, staged / here, forward and both
+// gradients: 64 channels of 28 x 28 x 64 streams 10.4 / 6.7 and 24.6 / 16.7 (fp16 10.0 / 6.1, 23.3 / 14.8); 64 of 112 x 112 x 4 16.0 / 5.1, 36.9 / 13.0;
+// 48 of 27 x 33 x 100 15.1 / 13.5, 36.1 / 31.0; planes of one stream as before, by their launches (3.2 / 3.0).  Strips of eight rows instead of
+// four change nothing in the weight gradient.
+struct Dw3Strip {
     int C, planes, G, Hs, Ws, Ho, Wo, padU, padL, flip;
-    int PH, PW, W4, O4, vec_s, vec_o;            // staged rows, floats per staged row, quads per source row / result row, vector access
-    DwDiv dW4, dWs, dRow, dO4;                   // dRow: quads (or values) of a source plane
+    int strips, rows, cols;                      // strips of a plane, rows of a strip, threads of a row
+    DwDiv dPer, dCols;
 };
-// one plane group of the source into shared memory (the zero border is already there)
-template <class T, int NT> __device__ __forceinline__ void dw3_stage(const Dw3Params &p, const T *src, int np, float *win, long long plane_step)
+__device__ __forceinline__ float4 dw_ld4_0(bool ok, const float *p) { float4 v = make_float4(0.f, 0.f, 0.f, 0.f); if (ok) v = *reinterpret_cast<const float4 *>(p); return v; }
+__device__ __forceinline__ float4 dw_ld4_0(bool ok, const __half *p)
 {
-    const int P = p.PH * p.PW;
-    if (p.vec_s) {
-        const int per = p.Hs * p.W4;
-#pragma unroll 2
-        for (int e = threadIdx.x; e < np * per; e += NT) {
-            const int g = dw_quot(e, p.dRow), q = e - g * per, r = dw_quot(q, p.dW4), c4 = q - r * p.W4;
-            *reinterpret_cast<float4 *>(win + g * P + (r + p.padU) * p.PW + 4 + 4 * c4) = dw_ld4(src + g * plane_step + r * p.Ws + 4 * c4);
-        }
-    } else {
-        const int per = p.Hs * p.Ws;
-#pragma unroll 4
-        for (int e = threadIdx.x; e < np * per; e += NT) {
-            const int g = dw_quot(e, p.dRow), q = e - g * per, r = dw_quot(q, p.dWs), c = q - r * p.Ws;
-            win[g * P + (r + p.padU) * p.PW + 4 + c] = ld(src + g * plane_step + q);
-        }
-    }
+    uint2 u = make_uint2(0u, 0u);
+    if (ok) u = *reinterpret_cast<const uint2 *>(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
 }
-// the six window values that four neighbouring results need from one row
-template <int PADL> __device__ __forceinline__ void dw3_row(const float *row, float (&v)[6])
+// rows h0 .. h0 + R + 1 of a plane, `need` of them, the V + 2 columns around result column V j
+template <class T, int V, int R> __device__ __forceinline__ void dw3_strip_load(const Dw3Strip &p, const T *s, int h0, int need, int j, float (&v)[R + 2][V + 2])
 {
-    if constexpr (PADL == 1) {
-        const float4 m = *reinterpret_cast<const float4 *>(row + 4);
-        v[0] = row[3]; v[1] = m.x; v[2] = m.y; v[3] = m.z; v[4] = m.w; v[5] = row[8];
-    } else {
 #pragma unroll
-        for (int k = 0; k < 6; k++) v[k] = row[4 - PADL + k];
+    for (int r = 0; r < R + 2; r++) {
+        const bool ok = r < need && (unsigned)(h0 + r) < (unsigned)p.Hs;
+        const T *row = s + (h0 + r) * p.Ws;
+        if constexpr (V == 4) {
+            const float4 m = dw_ld4_0(ok && 4 * j < p.Ws, row + 4 * j);
+            v[r][0] = ld0(ok && j > 0 && 4 * j - 1 < p.Ws, row + 4 * j - 1); v[r][1] = m.x; v[r][2] = m.y; v[r][3] = m.z; v[r][4] = m.w;
+            v[r][5] = ld0(ok && 4 * j + 4 < p.Ws, row + 4 * j + 4);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) v[r][k] = ld0(ok && (unsigned)(j - p.padL + k) < (unsigned)p.Ws, row + j - p.padL + k);
+        }
     }
 }
-template <class T, int PADL>
-__global__ void __launch_bounds__(128) dw3_kernel(const __grid_constant__ Dw3Params p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
+template <class T, int V, int R>
+__global__ void __launch_bounds__(256, 2) dw3_strip_kernel(const __grid_constant__ Dw3Strip p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
 {
     pdl_wait();
-    extern __shared__ __align__(16) float dw_smem[];
-    const int P = p.PH * p.PW, pl0 = blockIdx.x * p.G, np = min(p.G, p.planes - pl0), O = p.Ho * p.Wo, per = p.Ho * p.O4;
-    float *ws = dw_smem + p.G * P;
-    for (int e = threadIdx.x; e < np * P / 4; e += 128) reinterpret_cast<float4 *>(dw_smem)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int e = threadIdx.x; e < np * 9; e += 128) { const int g = e / 9, t = e - 9 * g; ws[e] = ld(w + (long long)((pl0 + g) % p.C) * 9 + (p.flip ? 8 - t : t)); }
-    __syncthreads();
-    dw3_stage<T, 128>(p, src + (long long)pl0 * p.Hs * p.Ws, np, dw_smem, (long long)p.Hs * p.Ws);
-    __syncthreads();
-    T *d0 = dst + (long long)pl0 * O;
-    for (int e = threadIdx.x; e < np * per; e += 128) {
-        const int g = p.G == 1 ? 0 : dw_quot(e, p.dO4), q = e - g * per, i = q / p.O4, j4 = q - i * p.O4;
-        const float *b = dw_smem + g * P + i * p.PW + 4 * j4, *wp = ws + g * 9;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const int pl0 = blockIdx.x * p.G, np = min(p.G, p.planes - pl0), per = p.strips * p.cols, c0 = pl0 % p.C;
+    for (int e = threadIdx.x; e < np * per; e += 256) {
+        const int g = p.G == 1 ? 0 : dw_quot(e, p.dPer), q = e - g * per, strip = dw_quot(q, p.dCols), j = q - strip * p.cols, i0 = strip * p.rows, rows = min(p.rows, p.Ho - i0);
+        int c = c0 + g;
+        while (c >= p.C) c -= p.C;
+        float wv[9], v[R + 2][V + 2];
 #pragma unroll
-        for (int kh = 0; kh < 3; kh++) {
-            float v[6];
-            dw3_row<PADL>(b + kh * p.PW, v);
+        for (int t = 0; t < 9; t++) wv[t] = ld(w + (long long)c * 9 + (p.flip ? 8 - t : t));
+        dw3_strip_load<T, V, R>(p, src + (long long)(pl0 + g) * p.Hs * p.Ws, i0 - p.padU, rows + 2, j, v);
+        T *o = dst + (long long)(pl0 + g) * p.Ho * p.Wo + (long long)i0 * p.Wo + V * j;
 #pragma unroll
-            for (int kw = 0; kw < 3; kw++) {
-                const float wv = wp[kh * 3 + kw];
+        for (int r = 0; r < R; r++, o += p.Wo) {
+            if (r >= rows) break;
+            float acc[V];
 #pragma unroll
-                for (int k = 0; k < 4; k++) acc[k] = fmaf(wv, v[k + kw], acc[k]);
-            }
-        }
-        T *o = d0 + (long long)g * O + i * p.Wo + 4 * j4;
-        if (p.vec_o) dw_st4(o, acc);
-        else {
+            for (int k = 0; k < V; k++) acc[k] = 0.f;
 #pragma unroll
-            for (int k = 0; k < 4; k++) if (4 * j4 + k < p.Wo) st(o + k, acc[k]);
+            for (int t = 0; t < 9; t++)
+#pragma unroll
+                for (int k = 0; k < V; k++) acc[k] = fmaf(wv[t], v[r + t / 3][k + t % 3], acc[k]);
+            if constexpr (V == 4) dw_st4(o, acc);
+            else st(o, acc[0]);
         }
     }
 }
-template <class T, int PADL>
-__global__ void __launch_bounds__(128) dw3_wg_kernel(const __grid_constant__ Dw3Params p, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part, int n)
+template <class T, int V, int R>
+__global__ void __launch_bounds__(128, 4) dw3_strip_wg_kernel(const __grid_constant__ Dw3Strip p, const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ part, int n)
 {
     pdl_wait();
-    extern __shared__ __align__(16) float dw_smem[];
     __shared__ float red[4][9];
-    const int ch = blockIdx.x, P = p.PH * p.PW, O = p.Ho * p.Wo, per = p.Ho * p.O4;
+    const int ch = blockIdx.x, per = p.strips * p.cols;
     const int s_begin = (int)((long long)n * blockIdx.y / gridDim.y), s_end = (int)((long long)n * (blockIdx.y + 1) / gridDim.y);
-    for (int e = threadIdx.x; e < p.G * P / 4; e += 128) reinterpret_cast<float4 *>(dw_smem)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     float acc[9];
 #pragma unroll
     for (int t = 0; t < 9; t++) acc[t] = 0.f;
-    for (int s = s_begin; s < s_end; s += p.G) {
-        const int ns = min(p.G, s_end - s);
-        __syncthreads();
-        dw3_stage<T, 128>(p, x + ((long long)s * p.C + ch) * p.Hs * p.Ws, ns, dw_smem, (long long)p.C * p.Hs * p.Ws);
-        __syncthreads();
-#pragma unroll 2
-        for (int e = threadIdx.x; e < ns * per; e += 128) {
-            const int g = p.G == 1 ? 0 : dw_quot(e, p.dO4), q = e - g * per, i = q / p.O4, j4 = q - i * p.O4;
-            const T *dp = dy + ((long long)(s + g) * p.C + ch) * O + i * p.Wo + 4 * j4;
-            float d[4];
-            if (p.vec_o) { const float4 t = dw_ld4(dp); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
-            else {
+    int s = s_begin, q = threadIdx.x;
+    while (q >= per) { q -= per; s++; }
+    while (s < s_end) {
+        const int strip = dw_quot(q, p.dCols), j = q - strip * p.cols, i0 = strip * p.rows, rows = min(p.rows, p.Ho - i0);
+        const long long pl = (long long)s * p.C + ch;
+        const T *dp = dy + pl * p.Ho * p.Wo + (long long)i0 * p.Wo + V * j;
+        float d[R][V], v[R + 2][V + 2];
 #pragma unroll
-                for (int k = 0; k < 4; k++) d[k] = ld0(4 * j4 + k < p.Wo, dp + k);
-            }
-            const float *b = dw_smem + g * P + i * p.PW + 4 * j4;
-#pragma unroll
-            for (int kh = 0; kh < 3; kh++) {
-                float v[6];
-                dw3_row<PADL>(b + kh * p.PW, v);
-#pragma unroll
-                for (int kw = 0; kw < 3; kw++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) acc[kh * 3 + kw] = fmaf(d[k], v[k + kw], acc[kh * 3 + kw]);
-            }
+        for (int r = 0; r < R; r++, dp += p.Wo) {
+            if constexpr (V == 4) { const float4 t = dw_ld4_0(r < rows, dp); d[r][0] = t.x; d[r][1] = t.y; d[r][2] = t.z; d[r][3] = t.w; }
+            else d[r][0] = ld0(r < rows, dp);
         }
+        dw3_strip_load<T, V, R>(p, x + pl * p.Hs * p.Ws, i0 - p.padU, rows + 2, j, v);
+        // a strip's own sum first: short chains, which the longer ones of a thread then add up
+#pragma unroll
+        for (int t = 0; t < 9; t++) {
+            float sum = 0.f;
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int k = 0; k < V; k++) sum = fmaf(d[r][k], r < rows ? v[r + t / 3][k + t % 3] : 0.f, sum);
+            acc[t] += sum;
+        }
+        q += 128;
+        while (q >= per) { q -= per; s++; }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -252,20 +229,19 @@ __global__ void __launch_bounds__(128) dw3_wg_kernel(const __grid_constant__ Dw3
     __syncthreads();
     if (threadIdx.x < 9) part[((long long)blockIdx.y * p.C + ch) * 9 + threadIdx.x] = ((red[0][threadIdx.x] + red[1][threadIdx.x]) + red[2][threadIdx.x]) + red[3][threadIdx.x];
 }
-
-static bool dw3_params(const ConvGeom &g, Dw3Params &p, const void *src, const void *dst, int esize, bool ig)
+// V of the strips; 0: not covered
+static int dw3_strip(const ConvGeom &g, Dw3Strip &p, const void *src, const void *dst, int esize, bool ig, int R)
 {
-    if (g.Hk != 3 || g.Wk != 3 || g.sh != 1 || g.sw != 1) return false;
+    if (g.Hk != 3 || g.Wk != 3 || g.sh != 1 || g.sw != 1) return 0;
     p.C = g.Cin; p.planes = g.n * g.Cin; p.flip = ig;
     p.Hs = ig ? g.Hout : g.Hin; p.Ws = ig ? g.Wout : g.Win; p.Ho = ig ? g.Hin : g.Hout; p.Wo = ig ? g.Win : g.Wout;
     p.padU = ig ? 2 - g.padU : g.padU; p.padL = ig ? 2 - g.padL : g.padL;
-    if (p.padU < 0 || p.padL < 0 || p.padL > 2 || p.padU > 2 || (long long)g.n * g.Cin >= (1ll << 31)) return false;
-    p.PH = std::max(p.Ho + 2, p.Hs + p.padU); p.O4 = ceil_div(p.Wo, 4); p.W4 = p.Ws / 4;
-    p.PW = std::max(4 * p.O4 + 12, 4 + (p.Ws + 3) / 4 * 4);
-    if ((long long)p.PH * p.PW > 12 * 1024) return false;                  // 48 KB of planes
-    p.vec_s = p.Ws % 4 == 0 && ((uintptr_t)src) % (4 * esize) == 0; p.vec_o = p.Wo % 4 == 0 && ((uintptr_t)dst) % (4 * esize) == 0;
-    p.dW4 = dw_div(std::max(1, p.W4)); p.dWs = dw_div(p.Ws); p.dRow = dw_div(p.vec_s ? p.Hs * p.W4 : p.Hs * p.Ws); p.dO4 = dw_div(p.Ho * p.O4);
-    return true;
+    if ((long long)g.n * g.Cin >= (1ll << 31) || (long long)p.Hs * p.Ws >= (1ll << 24) || (long long)p.Ho * p.Wo >= (1ll << 24)) return 0;
+    const int V = p.padL == 1 && p.Ws % 4 == 0 && p.Wo % 4 == 0 && ((uintptr_t)src | (uintptr_t)dst) % (4 * esize) == 0 ? 4 : 1;
+    p.cols = p.Wo / V; p.strips = ceil_div(p.Ho, R); p.rows = ceil_div(p.Ho, p.strips); p.strips = ceil_div(p.Ho, p.rows);
+    if ((long long)p.strips * p.cols * p.cols >= (1ll << 32)) return 0;     // (exact quotients)
+    p.dPer = dw_div(p.strips * p.cols); p.dCols = dw_div(p.cols);
+    return V;
 }
 
 static bool dw_window(const ConvGeom &g, DwParams &p, bool ig)
@@ -286,19 +262,14 @@ static bool dw_window(const ConvGeom &g, DwParams &p, bool ig)
 // forward and stride-1 input gradient; false = not covered
 template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T *dst, bool ig)
 {
-    Dw3Params q;
-    if (dw3_params(g, q, src, dst, (int)sizeof(T), ig)) {
-        // about two quads per thread, fewer planes per CTA when that would leave SMs idle
-        q.G = std::max(1, std::min(256 / (q.Ho * q.O4), q.planes / (4 * sm_count())));
-        while (q.G > 1 && (size_t)q.G * (q.PH * q.PW + 9) * 4 > 48 * 1024 - 16) q.G--;
-        const size_t smem = (size_t)q.G * (q.PH * q.PW + 9) * 4;
-        const int grid = ceil_div(q.planes, q.G);
-        if (smem <= 48 * 1024) {
-            if (q.padL == 1) TL_LAUNCH((dw3_kernel<T, 1>), grid, 128, smem, q, src, w, dst);
-            else if (q.padL == 0) TL_LAUNCH((dw3_kernel<T, 0>), grid, 128, smem, q, src, w, dst);
-            else TL_LAUNCH((dw3_kernel<T, 2>), grid, 128, smem, q, src, w, dst);
-            return true;
-        }
+    Dw3Strip t;
+    if (const int V = dw3_strip(g, t, src, dst, (int)sizeof(T), ig, 8)) {
+        const int per = t.strips * t.cols;
+        t.G = std::max(1, std::min(per >= 4096 ? 1 : per >= 256 ? 4 : 256 / per, t.planes / (2 * sm_count())));
+        const int grid = ceil_div(t.planes, t.G);
+        if (V == 4) TL_LAUNCH((dw3_strip_kernel<T, 4, 8>), grid, 256, 0, t, src, w, dst);
+        else TL_LAUNCH((dw3_strip_kernel<T, 1, 8>), grid, 256, 0, t, src, w, dst);
+        return true;
     }
     DwParams p;
     if (!dw_window(g, p, ig)) return false;
@@ -320,22 +291,13 @@ template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T
 // partial weight gradients [groups][C][K*K]; 3 x 3 and 5 x 5 filters.  dry: only the number of groups
 template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy, float *part, int &groups, bool dry)
 {
-    Dw3Params q;
-    if (dw3_params(g, q, x, dy, (int)sizeof(T), false)) {
+    Dw3Strip t;
+    if (const int V = dw3_strip(g, t, x, dy, (int)sizeof(T), false, 4)) {
         groups = std::max(1, std::min(ceil_div(8 * sm_count(), g.Cin), g.n));
         if (dry) return true;
-        // all planes of a CTA at once while eight CTAs fit an SM's shared memory: one wait for memory instead of one per plane
-        q.G = ceil_div(g.n, groups);
-        while (q.G > 1 && (size_t)q.G * q.PH * q.PW * 4 > 24 * 1024) q.G--;
-        const size_t smem = (size_t)q.G * q.PH * q.PW * 4;
         const dim3 grid(g.Cin, groups);
-#define TL_DW(PADL)                                                                \
-    do {                                                                           \
-        dw_allow(dw3_wg_kernel<T, PADL>, smem);                                    \
-        TL_LAUNCH((dw3_wg_kernel<T, PADL>), grid, 128, smem, q, x, dy, part, g.n); \
-    } while (0)
-        if (q.padL == 1) TL_DW(1); else if (q.padL == 0) TL_DW(0); else TL_DW(2);
-#undef TL_DW
+        if (V == 4) TL_LAUNCH((dw3_strip_wg_kernel<T, 4, 4>), grid, 128, 0, t, x, dy, part, g.n);
+        else TL_LAUNCH((dw3_strip_wg_kernel<T, 1, 4>), grid, 128, 0, t, x, dy, part, g.n);
         return true;
     }
     DwParams p;

@@ -186,6 +186,13 @@ def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
     assert_close(dW.get().astype(F), want, tol, "wg")
 
 
+# 3 x 3 with stride 1 in register strips: rows of whole 16-byte groups and not, one row, one column, strips of unequal rows, many planes in a CTA
+# (more than there are channels), several rounds of a CTA's threads, padding of two columns beside whole groups
+@pytest.mark.parametrize("c,h,w,pad,n", [(6, 31, 20, 1, 5), (3, 1, 8, 1, 2), (2, 9, 1, 1, 40), (1, 1, 1, 1, 3), (3, 6, 8, 1, 900), (200, 9, 12, 1, 3), (2, 130, 131, 1, 1), (4, 17, 12, 2, 6), (5, 18, 16, 0, 4), (1, 300, 260, 1, 1)])
+def test_depthwise_in_register_strips(run, oracle, c, h, w, pad, n):
+    test_depthwise_shapes(run, oracle, c, h, w, 3, pad, n)
+
+
 # Planes whose staged windows come to just below, exactly and just above the 48 KB that a launch gets without asking: the weight
 # gradients keep static arrays beside them.  Floats staged: 3x3 with pad 1 11 880, 12 276, 12 288, 11 446 (past that kernel's own
 # limit), with pad 0 and 2 12 288; 5x5 11 881, 12 100, 12 544; stride 2 (fp32 only) 12 285, 12 519.
