@@ -122,11 +122,12 @@ __device__ __forceinline__ void dw_st4(__half *p, const float (&v)[4])
 
 // A thread has V neighbouring columns of a strip of up to R rows of one plane: every row of the source is read once per strip (its
 // neighbours' columns come from L1), straight into registers, all rows of the strip in flight together, with no shared memory, no
-// zero border and no barrier.  V = 4: rows of whole 16-byte groups (8 in fp16) and one column of padding.  Staging planes in shared
+// zero border and no barrier.  V = 4: rows of whole 16-byte groups (8 in fp16) and one column of padding.  Six CTAs of 128 threads fit an SM (two of 256 left a
+// wave half empty at 4096 planes of 28 x 28: 6.6 / 6.2 us, fp16 6.1 / 5.0).  Staging planes in shared
 // memory with a zero border was bound by that memory's pipe, half of its wavefronts bank conflicts; now it is the loads: 25.7 MB in
-// 6.7 us of the layer above (3.8 TB/s), and with rows of odd lengths, three 4-byte loads a value, their issue.  us, staged / here, forward and both
-// gradients: 64 channels of 28 x 28 x 64 streams 10.4 / 6.7 and 24.6 / 16.7 (fp16 10.0 / 6.1, 23.3 / 14.8); 64 of 112 x 112 x 4 16.0 / 5.1, 36.9 / 13.0;
-// 48 of 27 x 33 x 100 15.1 / 13.5, 36.1 / 31.0; planes of one stream as before, by their launches (3.2 / 3.0).  Strips of eight rows instead of
+// 6.2 us of the layer above (4.1 TB/s), and with rows of odd lengths, three 4-byte loads a value, their issue.  us, staged / here, forward and both
+// gradients: 64 channels of 28 x 28 x 64 streams 10.4 / 6.2 and 24.6 / 16.7 (fp16 10.0 / 5.0, 23.3 / 13.8); 64 of 112 x 112 x 4 16.0 / 5.5, 36.9 / 13.7;
+// 48 of 27 x 33 x 100 15.1 / 13.1, 36.1 / 30.4; planes of one stream as before, by their launches (3.2 / 3.0).  Strips of eight rows instead of
 // four change nothing in the weight gradient.
 struct Dw3Strip {
     int C, planes, G, Hs, Ws, Ho, Wo, padU, padL, flip;
@@ -159,11 +160,11 @@ template <class T, int V, int R> __device__ __forceinline__ void dw3_strip_load(
     }
 }
 template <class T, int V, int R>
-__global__ void __launch_bounds__(256, 2) dw3_strip_kernel(const __grid_constant__ Dw3Strip p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
+__global__ void __launch_bounds__(128, 6) dw3_strip_kernel(const __grid_constant__ Dw3Strip p, const T *__restrict__ src, const T *__restrict__ w, T *__restrict__ dst)
 {
     pdl_wait();
     const int pl0 = blockIdx.x * p.G, np = min(p.G, p.planes - pl0), per = p.strips * p.cols, c0 = pl0 % p.C;
-    for (int e = threadIdx.x; e < np * per; e += 256) {
+    for (int e = blockIdx.y * 128 + threadIdx.x; e < np * per; e += 128 * gridDim.y) {
         const int g = p.G == 1 ? 0 : dw_quot(e, p.dPer), q = e - g * per, strip = dw_quot(q, p.dCols), j = q - strip * p.cols, i0 = strip * p.rows, rows = min(p.rows, p.Ho - i0);
         int c = c0 + g;
         while (c >= p.C) c -= p.C;
@@ -265,10 +266,19 @@ template <class T> bool dw_planes(const ConvGeom &g, const T *src, const T *w, T
     Dw3Strip t;
     if (const int V = dw3_strip(g, t, src, dst, (int)sizeof(T), ig, 8)) {
         const int per = t.strips * t.cols;
-        t.G = std::max(1, std::min(per >= 4096 ? 1 : per >= 256 ? 4 : 256 / per, t.planes / (2 * sm_count())));
-        const int grid = ceil_div(t.planes, t.G);
-        if (V == 4) TL_LAUNCH((dw3_strip_kernel<T, 4, 8>), grid, 256, 0, t, src, w, dst);
-        else TL_LAUNCH((dw3_strip_kernel<T, 1, 8>), grid, 256, 0, t, src, w, dst);
+        // planes of a CTA: up to two rounds of its threads, as full as they get, fewer where that would leave SMs idle; the rounds are CTAs of
+        // their own while SMs are
+        const int most = std::max(1, std::min(per >= 4096 ? 1 : per >= 256 ? 2 : 256 / per, t.planes / (4 * sm_count())));
+        double full = 0.0;
+        t.G = 1;
+        for (int G = 1; G <= most; G++) {
+            const double f = (double)(G * per) / (ceil_div(G * per, 128) * 128);
+            if (f > full + 0.01) { full = f; t.G = G; }
+        }
+        const int groups = ceil_div(t.planes, t.G);
+        const dim3 grid(groups, std::max(1, std::min(ceil_div(t.G * per, 128), 6 * sm_count() / groups)));
+        if (V == 4) TL_LAUNCH((dw3_strip_kernel<T, 4, 8>), grid, 128, 0, t, src, w, dst);
+        else TL_LAUNCH((dw3_strip_kernel<T, 1, 8>), grid, 128, 0, t, src, w, dst);
         return true;
     }
     DwParams p;
