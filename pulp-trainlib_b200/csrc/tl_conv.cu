@@ -427,8 +427,9 @@ template <> bool try_tc_ig<float>(Scope &sc, const ConvGeom &g, const float *dy,
 // A pointwise layer of stride 1 as products of the tcgen05 GEMM, one per stream, with the pixels as rows (the contiguous index of
 // the results).  What mma.sync pays for these layers is not the arithmetic but its staging: every element is copied by itself
 // into a channels-last patch, once per 64 output channels.  The GEMM declines planes of less than 128 pixels, less than 64
-// output channels and small layers, which stay there.  Measured, 64 streams of 64 -> 128 on 28 x 28: fp32 35.5 -> 24 us (9 of it
-// the packing), fp16 21.5 -> 9.9 us; 100 streams of 96 -> 160 on 15 x 17 in fp16 (packed: odd rows) 33.5 -> 15.6 us.
+// output channels and small layers, which stay there.  Measured, 64 streams of 64 -> 128 on 28 x 28 in fp16 21.5 -> 9.9 us; 100 streams of
+// 96 -> 160 on 15 x 17 in fp16 (packed: odd rows) 33.5 -> 15.6 us.  fp32 layers come here with few pixels or with weights past shared
+// memory only (tl_conv_pw.cu takes the others).
 template <class T> static bool try_pointwise(const ConvGeom &g, const T *src, const T *w, const T *bias, T *dst, bool ig)
 {
     if (g.Hk != 1 || g.Wk != 1 || g.sh != 1 || g.sw != 1 || g.padU != 0 || g.padL != 0 || g.Hin != g.Hout || g.Win != g.Wout || gemm_path() == 1) return false;
@@ -443,7 +444,7 @@ template <class T> static bool try_pointwise(const ConvGeom &g, const T *src, co
 }
 // Its weight gradient in fp16: dW = sum over the streams of dY X^T, one product whose contraction runs over the pixels of all
 // streams (64 streams of 64 -> 128 on 28 x 28: 35.0 -> 11.8 us with the sum of the partial results; 100 of 96 -> 160 on 15 x 17,
-// packed, 43.4 -> 20.5).  fp32 operands would have to be split into two copies of three times the activations' bytes (39 -> 47 us).
+// packed, 43.4 -> 20.5).  fp32 operands would have to be split into two copies of three times the activations' bytes: conv_pw_wg_kernel.
 template <class T> static bool try_pointwise_wg(const ConvGeom &g, const T *x, const T *dy, T *dw)
 {
     if (g.Hk != 1 || g.Wk != 1 || g.sh != 1 || g.sw != 1 || g.padU != 0 || g.padL != 0 || g.Hin != g.Hout || g.Win != g.Wout || gemm_path() == 1) return false;

@@ -6,8 +6,8 @@
 // A product of the GEMM in tl_gemm_tma.cu needs its fp32 operands as packed (hi, lo) copies: three times the activations' bytes written
 // and read again, and a launch of its own.  Here the split happens on the way into shared memory.  The pixels of all streams are one
 // line of rows, of which each CTA takes one stretch (equal shares: no last wave), 128 rows of D at a time:
-//   20 converter warps read 32 channels x 128 pixels at a time (lanes along the pixels; four warps take a piece of 32 loads a lane, five pieces are in flight), split and
-//      store them as [hi, lo][4 channels][pixel][16 bytes], which is the tensor core's K-major layout without swizzle;
+//   20 converter warps: four at a time read a piece of 32 channels x 128 pixels (lanes along the pixels, 32 loads a lane in flight), five
+//      pieces at once, split it and store it as [hi, lo][4 channels][pixel][16 bytes], which is the tensor core's K-major layout without swizzle;
 //   one warp issues D_hi += A_hi B_hi, D_lo += A_hi B_lo + A_lo B_hi (the weights lie behind each other, so that A_hi takes one instruction);
 //   four warps add the two parts and store: a lane has a pixel, so a warp stores 32 neighbouring ones of a channel.
 // The weights are split once per CTA and stay.  What bounds it: the activations' bytes, from L2 or HBM; figures at pw_covers.
