@@ -126,7 +126,7 @@ __device__ __forceinline__ void dw_st4(__half *p, const float (&v)[4])
 // wave half empty at 4096 planes of 28 x 28: 6.6 / 6.2 us, fp16 6.1 / 5.0).  Staging planes in shared
 // memory with a zero border was bound by that memory's pipe, half of its wavefronts bank conflicts; now it is the loads: 25.7 MB in
 // 6.2 us of the layer above (4.1 TB/s), and with rows of odd lengths, three 4-byte loads a value, their issue.  us, staged / here, forward and both
-// gradients: 64 channels of 28 x 28 x 64 streams 10.4 / 6.2 and 24.6 / 16.7 (fp16 10.0 / 5.0, 23.3 / 13.8); 64 of 112 x 112 x 4 16.0 / 5.5, 36.9 / 13.7;
+// gradients: 64 channels of 28 x 28 x 64 streams 10.4 / 6.2 and 24.6 / 14.6 (fp16 10.0 / 5.0, 23.3 / 12.6); 64 of 112 x 112 x 4 16.0 / 5.5, 36.9 / 13.7;
 // 48 of 27 x 33 x 100 15.1 / 13.1, 36.1 / 30.4; planes of one stream as before, by their launches (3.2 / 3.0).  Strips of eight rows instead of
 // four change nothing in the weight gradient.
 struct Dw3Strip {
@@ -303,7 +303,8 @@ template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy,
 {
     Dw3Strip t;
     if (const int V = dw3_strip(g, t, x, dy, (int)sizeof(T), false, 4)) {
-        groups = std::max(1, std::min(ceil_div(8 * sm_count(), g.Cin), g.n));
+        // one wave of the four CTAs that fit an SM (two waves and a bit: 17.1 us for both gradients of 64 channels of 28 x 28 x 64, 14.6 so)
+        groups = std::max(1, std::min(4 * sm_count() / g.Cin, g.n));
         if (dry) return true;
         const dim3 grid(g.Cin, groups);
         if (V == 4) TL_LAUNCH((dw3_strip_wg_kernel<T, 4, 4>), grid, 128, 0, t, x, dy, part, g.n);
