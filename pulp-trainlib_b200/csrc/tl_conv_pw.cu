@@ -30,11 +30,6 @@ struct PwParams {
     int N, kc, chunks, kpad, stages, accs, cols; // result channels padded; channels of a piece, pieces, channels padded; accumulators
 };
 
-__device__ __forceinline__ void pw_split(float x, uint32_t &hi, uint32_t &lo)
-{
-    tc::split_tf32_fast(x, hi, lo);
-    lo += 0x1000u;                              // the tensor core cuts it off
-}
 __device__ __forceinline__ void pw_sts(uint32_t to, const uint32_t *x) { asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]) : "memory"); }
 
 __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_constant__ PwParams p)
@@ -88,7 +83,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int k = c * 4 + j;
-                pw_split(m < p.Cd && k < p.C ? p.w[(long long)m * p.wm + (long long)k * p.wk] : 0.f, h[j], l[j]);
+                tc::split_tf32_rn(m < p.Cd && k < p.C ? p.w[(long long)m * p.wm + (long long)k * p.wk] : 0.f, h[j], l[j]);
             }
             pw_sts(b_sm + (uint32_t)c * b_lbo + (uint32_t)m * 16u, h);
             pw_sts(b_sm + (uint32_t)c * b_lbo + (uint32_t)(N + m) * 16u, l);
@@ -114,7 +109,7 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
                 if (c % 2 == 0 && c * 4 >= p.kc) break;
                 uint32_t h[4], l[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) pw_split(v[c * 4 + j], h[j], l[j]);
+                for (int j = 0; j < 4; j++) tc::split_tf32_rn(v[c * 4 + j], h[j], l[j]);
                 pw_sts(to + (uint32_t)c * 2048u, h);
                 pw_sts(to + PW_HALF + (uint32_t)c * 2048u, l);
             }
@@ -291,7 +286,7 @@ __device__ __forceinline__ void pw_wg_store(const float (&v)[8][4], uint32_t to,
         if (u >= nu) break;
         uint32_t h[4], l[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++) pw_split(v[u][e], h[e], l[e]);
+        for (int e = 0; e < 4; e++) tc::split_tf32_rn(v[u][e], h[e], l[e]);
         const uint32_t at = (u < nx ? to : to_y) + (uint32_t)u * step;
         pw_sts(at, h);
         pw_sts(at + (u < nx ? lo_x : lo_y), l);

@@ -277,6 +277,15 @@ __device__ __forceinline__ void split_tf32_fast(float x, uint32_t &hi, uint32_t 
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
+// The same with the low part rounded to the 19 bits that the tensor core reads, to nearest: half a unit of the last place that stays is
+// 2^-11 of lo's power of two, and the sum is exact.  (Added to the bits, as for hi, it turns the NaN of the GPU's own operations, 0x7FFFFFFF,
+// into a zero.  hi loses that NaN here too: lo, which is NaN for every NaN and infinity, has to keep it.)
+__device__ __forceinline__ void split_tf32_rn(float x, uint32_t &hi, uint32_t &lo)
+{
+    split_tf32_fast(x, hi, lo);
+    lo = __float_as_uint(fmaf(__uint_as_float(lo & 0xFF800000u), 0x1p-11f, __uint_as_float(lo)));
+}
+
 // Split that leaves the rounding of the big part to the tensor core: kind::tf32 reads the top 19 bits of an
 // fp32 operand, i.e. it uses trunc(x) when handed x itself, so only lo = x - trunc(x) has to be computed (exact
 // in fp32, same sign as x, below 2^-10 |x|).

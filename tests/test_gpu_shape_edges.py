@@ -125,6 +125,50 @@ def test_pointwise_weight_gradient_over_many_pixels(run, oracle, cin, h, w, cout
     assert any("conv_pw_wg_kernel" in t[0] for t in run.pkg.profile_table(run.lib))
 
 
+def conv_outputs(run, x, wt, dy, k, stride=1, bias=False):
+    """Y, dX, dW (and dB) of one layer with padding k // 2, and the names of the kernels that ran"""
+    n, cin, h, w = x.shape
+    cout, Ho, Wo = dy.shape[1:]
+    run.lib.trainlib_set_streams(n)
+    Y, dX, dW, dB, B, one = run.zeros(*dy.shape), run.zeros(*x.shape), run.zeros(*wt.shape), run.zeros(cout), run.zeros(cout), run.zeros(4)
+    a = run.args(run.sname("Conv2D_args"), input=run.blob(run.t(x), dX, C=cin, H=h, W=w), coeff=run.blob(run.t(wt), dW, C=cin, H=k, W=k, dim=wt.size), bias=run.blob(B, dB, dim=cout, W=cout),
+                 output=run.blob(Y, run.t(dy), C=cout, H=Ho, W=Wo), Lpad=k // 2, Rpad=k // 2, Upad=k // 2, Dpad=k // 2, stride_h=stride, stride_w=stride,
+                 i2c_buffer=one, bt_buffer=one, USE_BIASES=int(bias), USE_IM2COL=0, HWC=0)
+    run.lib.trainlib_profile(1)
+    for f in ("fw", "bw_param_grads", "bw_input_grads"):
+        run.call(run.fname("pulp_conv2d_fp32_%s_cl" % f), a)
+    run.lib.trainlib_profile(0)
+    return [t.get().astype(F) for t in (Y, dX, dW, dB)[:3 + bias]], [t[0] for t in run.pkg.profile_table(run.lib)]
+
+
+# NaN and infinity reach every result that they are a factor of, and no other one.  The bits: what operations of the GPU produce and its negative,
+# the host's, one whose payload lies below the bits that the tensor core reads, infinity (which the split into two parts turns into NaN)
+@pytest.mark.parametrize("bits", [0x7FFFFFFF, 0xFFFFFFFF, 0x7FC00000, 0x7F800001, 0x7F800000])
+@pytest.mark.parametrize("cin,cout", [(64, 32), (100, 140)])
+def test_pointwise_layers_keep_what_is_no_number(run, cin, cout, bits):
+    if run.half:
+        pytest.skip("single precision only")
+    n, h, w = 26, 28, 28
+    rng = seeded(cin)
+    bad = np.array([bits], np.uint32).view(F)[0]
+    x, wt, dy = (rng.standard_normal(s).astype(F) for s in ((n, cin, h, w), (cout, cin, 1, 1), (n, cout, h, w)))
+    clean, names = conv_outputs(run, x, wt, dy, 1)
+    assert sum("conv_pw_kernel" in t for t in names) == 1 and any("conv_pw_wg_kernel" in t for t in names)
+    with np.errstate(invalid="ignore"):
+        for where in ("x", "w", "dy"):
+            v = dict(x=x.copy(), w=wt.copy(), dy=dy.copy())
+            touched = [np.zeros(t.shape, bool) for t in clean]
+            if where == "x":
+                v["x"][3, 5, 7, 9] = bad; touched[0][3, :, 7, 9] = True; touched[2][:, 5] = True
+            elif where == "w":
+                v["w"][6, 2] = bad; touched[0][:, 6] = True; touched[1][:, 2] = True
+            else:
+                v["dy"][25, 31, 27, 27] = bad; touched[1][25, :, 27, 27] = True; touched[2][31] = True
+            got, _ = conv_outputs(run, v["x"], v["w"], v["dy"], 1)
+            for g, c, t in zip(got, clean, touched):
+                assert not np.isfinite(g[t]).any() and np.array_equal(g[~t], c[~t])
+
+
 # half-precision attention with enough blocks of sixteen queries for the mma.sync kernels: every core product against 64 bits from the
 # tensors that the layer leaves behind.  A result is rounded to 2^-11 of itself, and where the stored probabilities or dP stand in
 # for the unrounded ones the kernels used, each term by as much again: att and dv two such errors, dq and dk four
