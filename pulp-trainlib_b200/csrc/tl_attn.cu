@@ -264,9 +264,11 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_bw_key_kernel(const T *__res
 // ---------------------------------------------------------------- the same three kernels on mma.sync
 // For half precision: sixteen queries (keys) per CTA, every product as m16n8k8 TF32 instructions, some 40 instructions for 4096
 // multiply-adds where the kernels above take 220, and a quarter of what they fetch from L2.  fp16 values are TF32 values; the fp32
-// tile of probabilities is split into two TF32 parts (small term first), and the accumulators of four k-steps are added to fp32
-// registers with ordinary rounding: the accumulation of mma.sync truncates.  (fp32 operands, split the same way, gave three times
-// the FFMA kernels' error against 64 bits, 2.2e-7 against 7.5e-8, so they stay there.)
+// tile of probabilities (or dS) is split into two TF32 parts, both rounded to nearest (|x - hi - lo| <= 2^-23 |x|, small term first).  The accumulation
+// of mma.sync truncates, so that chains are short: the sums of four k-steps of scores, of two k-steps of both parts of a tile are added
+// to fp32 registers with ordinary rounding.  Of 262 144 dq and dk (4 heads x 512 x 64) 130 are not the half nearest to the 64-bit value, of the
+// kernels above 146; with four k-steps a chain and the low part cut off they were 228.  (fp32 operands, split the same way, gave
+// three times the FFMA kernels' error against 64 bits, 2.2e-7 against 7.5e-8, so they stay there.)
 //   scores:        A = the sixteen columns in shared memory, B = rows of M straight from memory (each is used by one warp only)
 //   rows of M x tile: A = rows of M from memory, four neighbouring tokens per lane (the order of k within a step is free as long as
 //                  both operands follow it), B = the tile; warps that the rows leave over share the tokens
@@ -360,7 +362,7 @@ __device__ __forceinline__ void am_rows(const __half *__restrict__ M, const floa
             const __half *r0 = M + (size_t)min(d0 + g, H - 1) * L + 4 * t, *r1 = M + (size_t)min(d0 + g + 8, H - 1) * L + 4 * t;
             const float *b0 = tile + g * Lp + 4 * t, *b1 = b0 + 8 * Lp;
             for (int s = s0; s < s1; s += U) {
-                float m[U][2][4], tmp[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                float m[U][2][4];
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int left = s + u < s1 ? L - 16 * (s + u) - 4 * t : 0;
@@ -370,26 +372,29 @@ __device__ __forceinline__ void am_rows(const __half *__restrict__ M, const floa
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     if (s + u >= s1) break;
-                    float bv[2][4];
+                    float bv[2][4], tmp[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                    uint32_t a4[2][4], bh[2][4], bl[2][4];
                     *reinterpret_cast<float4 *>(bv[0]) = *reinterpret_cast<const float4 *>(b0 + 16 * (s + u));
                     *reinterpret_cast<float4 *>(bv[1]) = *reinterpret_cast<const float4 *>(b1 + 16 * (s + u));
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {                          // tokens 4 t + 2 h and 4 t + 2 h + 1 are k = t and t + 4
-                        const uint32_t a4[4] = {__float_as_uint(m[u][0][2 * h]), __float_as_uint(m[u][1][2 * h]), __float_as_uint(m[u][0][2 * h + 1]), __float_as_uint(m[u][1][2 * h + 1])};
+                    for (int h = 0; h < 2; h++)                            // tokens 4 t + 2 h and 4 t + 2 h + 1 are k = t and t + 4
 #pragma unroll
-                        for (int n = 0; n < 2; n++) {
-                            uint32_t bh[2], bl[2];
+                        for (int q = 0; q < 4; q++) a4[h][q] = __float_as_uint(m[u][q & 1][2 * h + (q >> 1)]);
 #pragma unroll
-                            for (int q = 0; q < 2; q++) tc::split_tf32_fast(bv[n][2 * h + q], bh[q], bl[q]);
-                            am_mma(tmp[n], a4, bl[0], bl[1]);
-                            am_mma(tmp[n], a4, bh[0], bh[1]);
-                        }
-                    }
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) tc::split_tf32_rn(bv[n][q], bh[n][q], bl[n][q]);
+#pragma unroll
+                    for (int part = 0; part < 2; part++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++)
+#pragma unroll
+                            for (int n = 0; n < 2; n++) am_mma(tmp[n], a4[h], part ? bh[n][2 * h] : bl[n][2 * h], part ? bh[n][2 * h + 1] : bl[n][2 * h + 1]);
+#pragma unroll
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) acc[n][q] += tmp[n][q];
                 }
-#pragma unroll
-                for (int n = 0; n < 2; n++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) acc[n][q] += tmp[n][q];
             }
             if (sp.js > 1) {
 #pragma unroll

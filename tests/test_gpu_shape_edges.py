@@ -208,6 +208,49 @@ def test_half_precision_attention_core(pkg, gpulib, L, E, Fd, heads):
     assert np.abs(P.sum(-1) - 1).max() <= u * (1 + 1e-3) + L * 2.0 ** -25
 
 
+# dq and dk of those kernels are as exact as fp32 sums in fused multiply-adds, 32 partial sums a result: what either lets fall on the wrong side of a
+# rounding to half precision is counted, some 150 of 262 144 results.  1.2 times as many is two and a half standard deviations (sqrt(150) = 12); a low
+# part cut off and chains of four k-steps, in which the tensor core truncates, gave 1.5 times as many
+@pytest.mark.parametrize("L,E,Fd,heads", [(512, 128, 256, 4), (256, 256, 512, 8)])
+def test_half_precision_attention_core_rounds_like_fp32_sums(pkg, gpulib, L, E, Fd, heads):
+    gpulib.trainlib_set_streams(1)
+    rng = seeded(L + E + Fd)
+    x, dy = (rng.standard_normal((E, L)).astype(np.float16).astype(F) for _ in range(2))
+    ws = [(rng.standard_normal((E, Fd)) / np.sqrt(E)).astype(np.float16).astype(F) for _ in range(4)]
+    zb = np.zeros(Fd, F)
+    r = AbiRunner(pkg, gpulib, device=True, half=True)
+    gpulib.trainlib_profile(1)
+    got = r.mhsa(x, ws[0], ws[1], ws[2], zb, zb, zb, ws[3], dy, L, E, Fd, heads)
+    gpulib.trainlib_profile(0)
+    assert sum("mma_attn_bw" in t[0] for t in pkg.profile_table(gpulib)) == 2
+    r.close()
+    H = Fd // heads
+    P, dP = (got[k].astype(F).reshape(heads, L, L) for k in ("softmax", "dsoftmax"))
+
+    def fma_sum(a, b):
+        """sum over the last axis of a * b (broadcast): 32 partial sums, then added in pairs, every step rounded to fp32"""
+        acc = np.zeros(np.broadcast_shapes(a.shape, b.shape)[:-1] + (32,), F)
+        for j in range(0, L, 32):
+            acc = (acc.astype(np.float64) + a[..., j:j + 32].astype(np.float64) * b[..., j:j + 32]).astype(F)
+        while acc.shape[-1] > 1:
+            acc = acc[..., :acc.shape[-1] // 2] + acc[..., acc.shape[-1] // 2:]
+        return acc[..., 0]
+
+    y = F(H)
+    y = (np.int32(0x5f3759df) - (y.view(np.int32) >> 1)).view(F)
+    scale = y * (F(1.5) - F(H) * F(0.5) * y * y)
+    dS = (dP - fma_sum(dP, P)[..., None]) * P
+    dS64 = (dP.astype(np.float64) - (dP.astype(np.float64) * P).sum(-1, keepdims=True)) * P
+    wrong = wrong_fma = 0
+    for name, other, t in (("dq", "k", dS), ("dk", "q", dS.transpose(0, 2, 1))):
+        M = got[other].astype(F).reshape(heads, H, L)
+        exact = (float(scale) * np.einsum("hdj,hnj->hdn", M.astype(np.float64), dS64 if name == "dq" else dS64.transpose(0, 2, 1))).astype(np.float16)
+        fma = np.stack([np.stack([fma_sum(M[h, d], t[h]) for d in range(H)]) for h in range(heads)]) * scale
+        wrong += int((got[name].astype(np.float16).reshape(exact.shape) != exact).sum())
+        wrong_fma += int((fma.astype(np.float16) != exact).sum())
+    assert wrong <= 1.2 * wrong_fma, "%d and %d of %d" % (wrong, wrong_fma, 2 * heads * H * L)
+
+
 @pytest.mark.parametrize("c,h,w,k,pad,n", [(5, 9, 7, 3, 1, 3), (64, 28, 28, 3, 1, 4), (3, 33, 18, 3, 0, 2), (8, 6, 6, 5, 2, 9), (2, 40, 41, 3, 2, 1), (7, 4, 4, 3, 1, 700), (4, 12, 12, 4, 1, 2)])
 def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
     g = geom(c, h, w, c, k, stride=stride, pad=pad)
