@@ -374,26 +374,54 @@ __global__ void __launch_bounds__(PX_THREADS, 3) conv_px_kernel(const __grid_con
 // ---------------------------------------------------------------- weight gradient
 // dW[co][ci][t] = sum over slots of dY[slot][co] X[slot + shift_t][ci]: the same runs of slots, read MN-major (a core matrix is eight slots of
 // eight channels either way), dY with zeros on the slots that are no pixel, so that the contraction runs over whole runs and a
-// tap is again a start address.  Every tap has its accumulators in tensor memory for the life of the CTA, and so has, as a
-// product with a column of ones, the bias gradient.  Twelve warps stage runs into two buffers while ten issue products, the
-// taps dealt to them (a warp starts a product of these sizes every 200 cycles, ten of them one every 22).  Every CTA leaves one partial dW as [tap][ci][co] (neighbouring lanes of tensor memory are neighbouring
-// co), which px_wg_reduce_kernel adds in CTA order.
+// tap is again a start address.  Every tap has its accumulators in tensor memory, and so has, as a product with a column of ones, the
+// bias gradient.  Twelve warps stage runs into two buffers while eight issue products, the taps dealt to them (a warp starts a
+// product of these sizes every 200 cycles, ten of them one every 22).  Every CTA leaves one partial dW as [tap][four ci][co][ci] (neighbouring
+// lanes of tensor memory are neighbouring co), which px_wg_reduce_kernel adds in CTA order.
+// The tensor core truncates what it accumulates, so a chain of steps ends after about PXW_CHAIN of them: four more warps add its sums to a partial
+// result, with ordinary rounding where they lie, sixteen bytes an instruction (four bytes an instruction made the kernel up to 1.8 times as
+// slow).  The last chain is stored as a partial result of its own.  One chain for the life of a CTA (48 steps at 128 streams of
+// 24 -> 48 on 28 x 28, 500 at 512 of 16 -> 39 on 48 x 48) left 0.4 and 3.5 % of the results beside the half nearest to the 64-bit value (mma.sync 0.1 %)
+// and up to 9 % where all terms have one sign; so it is 0.2, 0.3 and 0.5 %, and the error against 64 bits that of the rounding to half
+// precision to five digits.  Time before and after: 24.4 -> 24.9 us and 148 -> 129 there, 74 -> 78 at 300 of 64 -> 64 on 28 x 28, 191 -> 210 at 512
+// of 7 -> 30, 5 x 5, on 48 x 47.
 struct PxWg {
     PxGeo geo; PxSrc x, dy;
     float *part; int *status;
     int KK, tap0[4], ntaps[4];                  // taps of a slice of the grid (ntaps: products, of `copies` taps each)
     int at[PX_MAXTAPS];                         // a tap's start within the run of X, in 16-byte pieces
-    int smin, ts, slx, sly, tiles;              // slots of a tile; of a run of X, of dY
+    int smin, ts, slx, sly, tiles, chains;      // slots of a tile; of a run of X, of dY; chains of a CTA
     int M, N, lgx, copies, ci_slices, tmem_cols, bias;  // lgx: rows of X are 2^lgx pieces
     long long group;                            // floats of one partial result
     uint32_t x_off, buf, ones_off;              // bytes: the run of X behind that of dY, the second pair of runs, 512 bytes of ones
 };
-static constexpr int PXW_STAGERS = 12, PXW_ISSUERS = 10, PXW_THREADS = 32 * (PXW_STAGERS + PXW_ISSUERS);
+static constexpr int PXW_STAGERS = 12, PXW_ISSUERS = 8, PXW_DRAINERS = 4, PXW_THREADS = 32 * (PXW_STAGERS + PXW_ISSUERS + PXW_DRAINERS), PXW_CHAIN = 32;
+
+// Chains of about PXW_CHAIN steps, at most a quarter more: how many a CTA's steps make, and the step before which chain f of issuer i ends.
+// The issuers end theirs in turn, spread over half a chain, so that the others keep the tensor cores busy.
+static int px_wg_chains(int steps) { return steps <= PXW_CHAIN * 5 / 4 ? 1 : (steps + PXW_CHAIN - 1) / PXW_CHAIN; }
+__device__ __forceinline__ int px_wg_chain_end(int f, int i, int issuers, int chains, int steps)
+{
+    const int turn = issuers > 1 ? 64 * i / (issuers - 1) : 32;                                    // 0 .. 64
+    return f + 1 < chains ? (int)(((long long)steps * (128 * (f + 1) + turn - 32)) / (128 * chains)) : steps;
+}
+// Sixteen accumulators of a lane, neighbouring source channels, to the partial result, of which the first `left` exist: a CTA's first ones are
+// stored, later ones added where they lie
+__device__ __forceinline__ void px_wg_out(float *o, int step, int left, const uint32_t (&v)[16], bool first)
+{
+#pragma unroll
+    for (int i = 0; i < 16; i += 4, o += step) {
+        if (i >= left) break;
+        if (first) asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(o), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
+        else asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(o), "f"(__uint_as_float(v[i])), "f"(__uint_as_float(v[i + 1])),
+                          "f"(__uint_as_float(v[i + 2])), "f"(__uint_as_float(v[i + 3])) : "memory");
+    }
+}
 
 __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid_constant__ PxWg p)
 {
     extern __shared__ __align__(1024) unsigned char px_smem[];
-    __shared__ __align__(8) uint64_t full[2], empty[2], done;
+    __shared__ __align__(8) uint64_t full[2], empty[2], done, chain_full[PXW_ISSUERS], chain_empty[PXW_ISSUERS];
     __shared__ uint32_t tmem_s;
     __shared__ int abort_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (one value per warp, and known to be)
@@ -413,6 +441,7 @@ __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid
         tc::fence_barrier_init();
         abort_s = 0;
     }
+    if (tid >= 96 && tid < 96 + PXW_ISSUERS) { tc::mbar_init(&chain_full[tid - 96], 1); tc::mbar_init(&chain_empty[tid - 96], PXW_DRAINERS); tc::fence_barrier_init(); }
     const uint32_t base_sm = tc::smem_u32(px_smem), ones = base_sm + p.ones_off;
     if (tid >= 64 && tid < 96) px_sts(ones + (uint32_t)(tid - 64) * 16u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
     tc::fence_proxy_async();
@@ -423,6 +452,34 @@ __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid
     pdl_wait();
 
     const int t_begin = (int)((long long)p.tiles * blockIdx.x / gridDim.x), t_end = (int)((long long)p.tiles * (blockIdx.x + 1) / gridDim.x);
+    const int steps = (t_end - t_begin) * (ts / 16), chains = p.chains, ncg = N / 16, bias_issuer = fold ? 0 : ntaps % issuers;
+    // M = 64: sixteen rows in the first lanes of every quarter of tensor memory
+    const int q = warp & 3, co = M == 64 ? q * 16 + lane : q * 32 + lane;
+    const bool live = co < p.dy.C && (M == 128 || lane < 16);
+    const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+    const int c4 = (p.x.C + 3) / 4;
+    // the last chain has a partial result of its own: added to the others' it would be waited for
+    float *out = p.part + (long long)(blockIdx.x + (chains > 1 && warp < PXW_STAGERS ? gridDim.x : 0u)) * p.group, *out_bias = out + (long long)p.KK * c4 * p.dy.C * 4 + co;
+    // taps t .. t_last of the slice from column group cg on (sixteen columns: source channels), every by-th group
+    auto drain = [&](int t, int cg, int t_last, int by, bool first) {
+        const int step = p.dy.C * 4;
+        while (cg >= ncg) { cg -= ncg; t++; }
+        while (t <= t_last) {
+            uint32_t v[16];
+            tc::tmem_ld16w(tq + (uint32_t)((t * ncg + cg) * 16), v);
+            float *o = out + (long long)((tap0 + t) * c4 + ci0 / 4 + cg * 4) * step + co * 4;
+            tc::tmem_wait_ld();
+            if (live) px_wg_out(o, step, p.x.C - ci0 - cg * 16, v, first);
+            cg += by;
+            while (cg >= ncg) { cg -= ncg; t++; }
+        }
+    };
+    auto drain_bias = [&](bool first) {
+        uint32_t v[16];
+        tc::tmem_ld16w(tq + (uint32_t)(fold ? N - 16 : ntaps * NC), v);
+        tc::tmem_wait_ld();
+        if (live) { if (first) *out_bias = __uint_as_float(v[15]); else atomicAdd(out_bias, __uint_as_float(v[15])); }
+    };
     if (warp < PXW_STAGERS) {
         for (int tile = t_begin, it = 0; tile < t_end; tile++, it++) {
             const uint32_t buf = base_sm + (it & 1 ? p.buf : 0u);
@@ -448,51 +505,56 @@ __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid
         const uint32_t idesc = tc::mma_idesc(tc::FMT_F16, (uint32_t)M, (uint32_t)NC) | tc::IDESC_A_MN_MAJOR | tc::IDESC_B_MN_MAJOR;
         const uint32_t idesc1 = tc::mma_idesc(tc::FMT_F16, (uint32_t)M, 16u) | tc::IDESC_A_MN_MAJOR | tc::IDESC_B_MN_MAJOR;
         bool ok = true;
-        for (int tile = t_begin, it = 0; tile < t_end; tile++, it++) {
+        int step = 0, chain = 0, chain_end = px_wg_chain_end(0, wi, issuers, chains, steps);
+        uint32_t more = 0;
+        for (int tile = t_begin, it = 0; ok && tile < t_end; tile++, it++) {
             const uint32_t buf = (base_sm + (it & 1 ? p.buf : 0u)) >> 4;
             if (!tc::warp_wait_or_abort(&full[it & 1], (uint32_t)(it >> 1) & 1u, abort_flag, p.status, 53, 20u, lane)) { ok = false; break; }
             tc::tc_fence_after();
             uint32_t aw = (uint32_t)da + buf;
             const uint32_t bw0 = (uint32_t)db + buf + (p.x_off >> 4);
-            for (int k = 0; k < ts; k += 16, aw += 128u) {
-                const uint32_t more = it > 0 || k > 0;
+            for (int k = 0; k < ts; k += 16, aw += 128u, step++, more = 1u) {
+                if (step == chain_end) {                                   // its sums are read before the next chain starts from zero
+                    if (tc::elect_one()) tc::mma_commit(&chain_full[wi]);
+                    __syncwarp();
+                    if (!tc::warp_wait_or_abort(&chain_empty[wi], (uint32_t)chain & 1u, abort_flag, p.status, 63, 20u, lane)) { ok = false; break; }
+                    tc::tc_fence_after();
+                    chain_end = px_wg_chain_end(++chain, wi, issuers, chains, steps);
+                    more = 0u;
+                }
                 const uint64_t ad = ((uint64_t)a_hw << 32) | aw;
                 for (int t = wi; t < ntaps; t += issuers)
                     if (tc::elect_one()) tc::mma_f16_ss(tmem + (uint32_t)(t * NC), ad, ((uint64_t)b_hw << 32) | (bw0 + (uint32_t)(p.at[tap0 + t * copies] + (k << p.lgx))), idesc, more);
-                if (bias && !fold && wi == ntaps % issuers && tc::elect_one()) tc::mma_f16_ss(tmem + (uint32_t)(ntaps * NC), ad, d1, idesc1, more);
+                if (bias && !fold && wi == bias_issuer && tc::elect_one()) tc::mma_f16_ss(tmem + (uint32_t)(ntaps * NC), ad, d1, idesc1, more);
                 __syncwarp();
             }
+            if (!ok) break;
             if (tc::elect_one()) tc::mma_commit(&empty[it & 1]);
             __syncwarp();
         }
         if (ok && tc::elect_one()) tc::mma_commit(&done);
         __syncwarp();
+    } else if (warp >= PXW_STAGERS + PXW_ISSUERS) {
+        // ---- all chains but the last, in the order in which they end
+        bool ok = true;
+        for (int f = 0; ok && f + 1 < chains; f++)
+            for (int i = 0; i < issuers; i++) {
+                ok = tc::warp_wait_or_abort(&chain_full[i], (uint32_t)f & 1u, abort_flag, p.status, 64, 20u, lane);
+                if (!ok) break;
+                tc::tc_fence_after();
+                for (int t = i; t < ntaps; t += issuers)
+                    drain(t * copies, 0, (t + 1) * copies - 1, 1, f == 0);
+                if (bias && i == bias_issuer) drain_bias(f == 0);
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&chain_empty[i]);
+            }
     }
-    if (warp < 8) {                                                        // two warps per quarter of tensor memory
-        const bool ok = t_begin < t_end && tc::warp_wait_or_abort(&done, 0u, abort_flag, p.status, 54, 20u, lane);
-        if (ok) {
+    if (warp < PXW_STAGERS) {                                              // the last chains: three warps per quarter of tensor memory
+        if (t_begin < t_end && tc::warp_wait_or_abort(&done, 0u, abort_flag, p.status, 54, 20u, lane)) {
             tc::tc_fence_after();
-            // M = 64: sixteen rows in the first lanes of every quarter of tensor memory
-            const int q = warp & 3, co = M == 64 ? q * 16 + lane : q * 32 + lane;
-            const bool live = co < p.dy.C && (M == 128 || lane < 16);
-            const int ncg = N / 16, units = ntaps * copies * ncg;
-            float *out = p.part + (long long)blockIdx.x * p.group;
-            for (int u = warp >> 2; u < units; u += 2) {
-                const int t = u / ncg, cg = u - t * ncg;
-                uint32_t v[16];
-                tc::tmem_ld16w(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * 16), v);
-                tc::tmem_wait_ld();
-                const int ci = ci0 + cg * 16;
-                float *o = out + ((long long)(tap0 + t) * p.x.C + ci) * p.dy.C + co;
-#pragma unroll
-                for (int i = 0; i < 16; i++) if (live && ci + i < p.x.C) o[(long long)i * p.dy.C] = __uint_as_float(v[i]);
-            }
-            if (bias && warp < 4) {
-                uint32_t v[16];
-                tc::tmem_ld16w(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(fold ? N - 16 : ntaps * NC), v);
-                tc::tmem_wait_ld();
-                if (live) out[(long long)p.KK * p.x.C * p.dy.C + co] = __uint_as_float(v[15]);
-            }
+            drain(0, warp >> 2, ntaps * copies - 1, PXW_STAGERS / 4, true);
+            if (bias && warp < 4) drain_bias(true);
         }
         tc::tc_fence_before();
     }
@@ -500,27 +562,28 @@ __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid
     if (warp == PXW_STAGERS) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, (uint32_t)p.tmem_cols); }
 }
 
-// 32 neighbouring elements x 8 slices of the partial results per CTA; the slices are added in order
-__global__ void __launch_bounds__(256) px_wg_reduce_kernel(const float *part, __half *dw, __half *db, int groups, long long group, int Co, int Ci, int KK, int total)
+// 32 neighbouring elements x SL slices of the partial results per CTA; the slices are added in order
+template <int SL>
+__global__ void __launch_bounds__(32 * SL) px_wg_reduce_kernel(const float *part, __half *dw, __half *db, int groups, long long group, int Co, int Ci, int KK, int total)
 {
     pdl_wait();
-    __shared__ float sums[8][32];
+    __shared__ float sums[SL][32];
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
     float acc = 0.f;
     if (e < total) {
         const float *src = part + e;
 #pragma unroll 8
-        for (int g = sl; g < groups; g += 8) acc += __ldcg(src + (long long)g * group);
+        for (int g = sl; g < groups; g += SL) acc += __ldcg(src + (long long)g * group);
     }
     sums[sl][lane] = acc;
     __syncthreads();
     if (sl || e >= total) return;
 #pragma unroll
-    for (int s = 1; s < 8; s++) acc += sums[s][lane];
-    const int q = e / Co, co = e - q * Co, nw = Ci * KK;
-    if (q >= nw) { db[co] = __float2half_rn(acc); return; }
-    const int t = q / Ci, ci = q - t * Ci;
-    dw[((long long)co * Ci + ci) * KK + t] = __float2half_rn(acc);
+    for (int s = 1; s < SL; s++) acc += sums[s][lane];
+    const int c4 = (Ci + 3) / 4, q = (e >> 2) / Co, co = (e >> 2) - q * Co;
+    if (q >= c4 * KK) { db[e - c4 * KK * Co * 4] = __float2half_rn(acc); return; }
+    const int t = q / c4, ci = (q - t * c4) * 4 + (e & 3);
+    if (ci < Ci) dw[((long long)co * Ci + ci) * KK + t] = __float2half_rn(acc);
 }
 
 // ---------------------------------------------------------------- host side
@@ -761,7 +824,7 @@ bool conv_px_wg(Scope &sc, const ConvGeom &geom, const __half *x, const __half *
         const int lgx = N % 64 == 0 ? 3 : N % 32 == 0 ? 2 : 1, copies = g.sh == 1 && N == 8 << lgx && N * g.Wk <= 256 ? g.Wk : 1, prods = p.KK / copies;
         const int tmax = (512 - 16) / (N * copies), tsl = tmax ? ceil_div(prods, tmax) : 5, per = ceil_div(prods, std::max(tsl, 1));
         if (tsl > 4) continue;
-        const int slices = cis * tsl, gx_max = (int)std::max<long long>(1, std::min<long long>(sm_count() / slices, (64ll << 20) / nw));       // (partial results: 256 MB at most)
+        const int slices = cis * tsl, gx_max = (int)std::max<long long>(1, std::min<long long>(sm_count() / slices, (32ll << 20) / nw));       // (partial results: 256 MB at most)
         for (int ts = 512; ts >= 64; ts -= 16) {
             const int slx = (ts + span + 31) & ~31, sly = (ts + 31) & ~31;
             const uint32_t yb = (uint32_t)ceil_div(k8y, 8) * sly * 128u, xb = (uint32_t)(p.x.nsub * ((N / 8) >> lgx) * copies) * slx * (16u << lgx), buf = yb + xb;
@@ -786,15 +849,18 @@ bool conv_px_wg(Scope &sc, const ConvGeom &geom, const __half *x, const __half *
         }
     }
     if (best >= 1e30) return false;
-    const int total = (int)(nw + (db ? g.Cout : 0));
-    bp.group = total;
-    bp.part = sc.try_scratch<float>((size_t)bgx * total);
+    bp.chains = px_wg_chains(ceil_div(bp.tiles, bgx) * (bp.ts / 16));
+    const int total = p.KK * ceil_div(g.Cin, 4) * 4 * g.Cout + (db ? g.Cout : 0);
+    bp.group = ceil_div(total, 4) * 4;
+    const int groups = bp.chains > 1 ? 2 * bgx : bgx;
+    bp.part = sc.try_scratch<float>((size_t)groups * bp.group);
     if (!bp.part) return false;
     static bool attr = false;
     if (!attr) { cudaFuncSetAttribute(conv_px_wg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); attr = true; }
     TL_LAUNCH(conv_px_wg_kernel, dim3(bgx, bslices), PXW_THREADS, bsmem, bp);
     profile_add_flops(2.0 * g.n * g.Hout * g.Wout * nw);
-    TL_LAUNCH(px_wg_reduce_kernel, ceil_div(total, 32), 256, 0, bp.part, dw, db, bgx, bp.group, g.Cout, g.Cin, p.KK, total);
+    if (groups <= 160) TL_LAUNCH(px_wg_reduce_kernel<8>, ceil_div(total, 32), 256, 0, bp.part, dw, db, groups, bp.group, g.Cout, g.Cin, p.KK, total);
+    else TL_LAUNCH(px_wg_reduce_kernel<16>, ceil_div(total, 32), 512, 0, bp.part, dw, db, groups, bp.group, g.Cout, g.Cin, p.KK, total);
     return true;
 }
 

@@ -24,6 +24,22 @@ def rounded(r, a):
     return a.astype(r.dt).astype(F)
 
 
+def conv_outputs(run, x, wt, dy, k, stride=1, bias=False):
+    """Y, dX, dW (and dB) of one layer with padding k // 2, and the names of the kernels that ran"""
+    n, cin, h, w = x.shape
+    cout, Ho, Wo = dy.shape[1:]
+    run.lib.trainlib_set_streams(n)
+    Y, dX, dW, dB, B, one = run.zeros(*dy.shape), run.zeros(*x.shape), run.zeros(*wt.shape), run.zeros(cout), run.zeros(cout), run.zeros(4)
+    a = run.args(run.sname("Conv2D_args"), input=run.blob(run.t(x), dX, C=cin, H=h, W=w), coeff=run.blob(run.t(wt), dW, C=cin, H=k, W=k, dim=wt.size), bias=run.blob(B, dB, dim=cout, W=cout),
+                 output=run.blob(Y, run.t(dy), C=cout, H=Ho, W=Wo), Lpad=k // 2, Rpad=k // 2, Upad=k // 2, Dpad=k // 2, stride_h=stride, stride_w=stride,
+                 i2c_buffer=one, bt_buffer=one, USE_BIASES=int(bias), USE_IM2COL=0, HWC=0)
+    run.lib.trainlib_profile(1)
+    for f in ("fw", "bw_param_grads", "bw_input_grads"):
+        run.call(run.fname("pulp_conv2d_fp32_%s_cl" % f), a)
+    run.lib.trainlib_profile(0)
+    return [t.get().astype(F) for t in (Y, dX, dW, dB)[:3 + bias]], [t[0] for t in run.pkg.profile_table(run.lib)]
+
+
 CONV = [(28, 14, 45, 28, 3, 1, 1), (3, 33, 41, 70, 5, 2, 3), (6, 42, 13, 81, 5, 1, 1), (40, 9, 11, 64, 3, 1, 5), (16, 5, 5, 8, 3, 1, 40), (20, 3, 200, 24, 3, 1, 2),
         (17, 12, 130, 33, 3, 2, 2), (64, 7, 7, 96, 1, 1, 30), (24, 28, 28, 48, 3, 1, 60), (33, 11, 12, 17, 3, 3, 2), (1, 6, 6, 4, 1, 1, 2), (70, 10, 10, 12, 7, 1, 1),
         (12, 8, 9, 16, 1, 2, 3), (64, 12, 12, 64, 5, 1, 4), (16, 7, 8, 8, 3, 1, 150), (8, 10, 16, 16, 3, 1, 63), (16, 32, 32, 16, 3, 1, 9), (8, 12, 32, 8, 3, 1, 30), (64, 16, 17, 64, 1, 1, 70), (36, 13, 15, 100, 1, 1, 100), (64, 40, 40, 72, 1, 1, 10), (72, 12, 12, 64, 1, 1, 110), (33, 9, 8, 130, 1, 1, 230)]
@@ -66,6 +82,28 @@ def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
     if not run.half:
         pytest.skip("half precision only")
     test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+
+
+# Long sums of the weight and bias gradient, terms of one sign: the tensor core truncates what it accumulates, up to 2^-23 of the sum at every k-step and half of that in
+# the mean.  Over a chain of 32 steps from zero that is 32 / 2 * 2^-24 = 1e-6 of a result, to which the rounding to half precision adds 2^-11 / 1.7
+# for one result and 1 / sqrt(results) of it for their mean, 4e-6.  (One chain of all steps of a CTA: 5e-5.)
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", [(16, 48, 48, 39, 3, 1, 512), (7, 48, 47, 30, 5, 1, 512), (20, 31, 33, 100, 3, 2, 500)])
+def test_long_weight_gradients_on_runs_of_slots_do_not_drift(run, cin, h, w, cout, k, stride, n):
+    if not run.half:
+        pytest.skip("half precision only")
+    import torch
+    gen = torch.Generator("cuda").manual_seed(cin)
+    Ho, Wo = (h - 1) // stride + 1, (w - 1) // stride + 1
+    x = torch.rand(n, cin, h, w, device="cuda", generator=gen).half()
+    dy = (torch.rand(n, cout, Ho, Wo, device="cuda", generator=gen) / 256).half()
+    (_, _, dW, dB), names = conv_outputs(run, x.float().cpu().numpy(), np.ones((cout, cin, k, k), F), dy.float().cpu().numpy(), k, stride, bias=True)
+    assert any("conv_px_wg_kernel" in t for t in names)
+    d64 = dy.double().permute(1, 0, 2, 3).reshape(cout, -1)
+    xp = torch.nn.functional.pad(x.double(), (k // 2,) * 4)
+    want = torch.stack([d64 @ xp[:, :, i:i + stride * Ho:stride, j:j + stride * Wo:stride][:, :, :Ho, :Wo].permute(0, 2, 3, 1).reshape(-1, cin) for i in range(k) for j in range(k)], -1)
+    rel = lambda got, want: (torch.from_numpy(got.reshape(want.shape)).cuda().double() / want - 1).cpu().numpy()
+    e, eb = rel(dW.reshape(cout, cin, k * k), want), rel(dB, d64.sum(1))
+    assert abs(e.mean()) <= 1e-5 and np.abs(e).max() <= 2.0 ** -11 * 1.02 and np.abs(eb).max() <= 2.0 ** -11 * 1.02, (e.mean(), np.abs(e).max(), np.abs(eb).max())
 
 
 # weight gradients of few pixels, one cluster per 16 x 16 channel tile (conv_mma_wg_cluster_kernel): one to sixteen CTAs of a cluster, ranks
@@ -123,22 +161,6 @@ def test_pointwise_weight_gradient_over_many_pixels(run, oracle, cin, h, w, cout
     test_conv2d_shapes(run, oracle, cin, h, w, cout, 1, 1, n)
     run.lib.trainlib_profile(0)
     assert any("conv_pw_wg_kernel" in t[0] for t in run.pkg.profile_table(run.lib))
-
-
-def conv_outputs(run, x, wt, dy, k, stride=1, bias=False):
-    """Y, dX, dW (and dB) of one layer with padding k // 2, and the names of the kernels that ran"""
-    n, cin, h, w = x.shape
-    cout, Ho, Wo = dy.shape[1:]
-    run.lib.trainlib_set_streams(n)
-    Y, dX, dW, dB, B, one = run.zeros(*dy.shape), run.zeros(*x.shape), run.zeros(*wt.shape), run.zeros(cout), run.zeros(cout), run.zeros(4)
-    a = run.args(run.sname("Conv2D_args"), input=run.blob(run.t(x), dX, C=cin, H=h, W=w), coeff=run.blob(run.t(wt), dW, C=cin, H=k, W=k, dim=wt.size), bias=run.blob(B, dB, dim=cout, W=cout),
-                 output=run.blob(Y, run.t(dy), C=cout, H=Ho, W=Wo), Lpad=k // 2, Rpad=k // 2, Upad=k // 2, Dpad=k // 2, stride_h=stride, stride_w=stride,
-                 i2c_buffer=one, bt_buffer=one, USE_BIASES=int(bias), USE_IM2COL=0, HWC=0)
-    run.lib.trainlib_profile(1)
-    for f in ("fw", "bw_param_grads", "bw_input_grads"):
-        run.call(run.fname("pulp_conv2d_fp32_%s_cl" % f), a)
-    run.lib.trainlib_profile(0)
-    return [t.get().astype(F) for t in (Y, dX, dW, dB)[:3 + bias]], [t[0] for t in run.pkg.profile_table(run.lib)]
 
 
 # NaN and infinity reach every result that they are a factor of, and no other one.  The bits: what operations of the GPU produce and its negative,
