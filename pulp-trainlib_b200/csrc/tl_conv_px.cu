@@ -562,28 +562,57 @@ __global__ void __launch_bounds__(PXW_THREADS, 1) conv_px_wg_kernel(const __grid
     if (warp == PXW_STAGERS) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, (uint32_t)p.tmem_cols); }
 }
 
-// 32 neighbouring elements x SL slices of the partial results per CTA; the slices are added in order
+// 32 neighbouring elements x SL slices of the partial results per CTA; the slices are added in order.
+// The products above also multiply the zeros of dY with pixels of X (on slots that are no result) and dY with zeros of X (the padding), which an
+// infinite or NaN factor makes NaN.  So a sum that is no finite number is formed again by the whole CTA, from the pairs of pixels that the
+// operator has; it is the only case in which X and dY are read.
+struct PxWgSum { const float *part; const __half *x, *dy; __half *dw, *db; long long group; int groups, n, Ci, H, W, Co, Ho, Wo, S, padU, padL, Wk, KK, total; };
 template <int SL>
-__global__ void __launch_bounds__(32 * SL) px_wg_reduce_kernel(const float *part, __half *dw, __half *db, int groups, long long group, int Co, int Ci, int KK, int total)
+__global__ void __launch_bounds__(32 * SL) px_wg_reduce_kernel(const __grid_constant__ PxWgSum p)
 {
     pdl_wait();
     __shared__ float sums[SL][32];
-    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+    __shared__ uint32_t again_s;
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, e = blockIdx.x * 32 + lane, c4 = (p.Ci + 3) / 4;
     float acc = 0.f;
-    if (e < total) {
-        const float *src = part + e;
+    if (e < p.total) {
+        const float *src = p.part + e;
 #pragma unroll 8
-        for (int g = sl; g < groups; g += SL) acc += __ldcg(src + (long long)g * group);
+        for (int g = sl; g < p.groups; g += SL) acc += __ldcg(src + (long long)g * p.group);
     }
     sums[sl][lane] = acc;
     __syncthreads();
-    if (sl || e >= total) return;
+    bool again = false;
+    if (sl == 0) {
 #pragma unroll
-    for (int s = 1; s < SL; s++) acc += sums[s][lane];
-    const int c4 = (Ci + 3) / 4, q = (e >> 2) / Co, co = (e >> 2) - q * Co;
-    if (q >= c4 * KK) { db[e - c4 * KK * Co * 4] = __float2half_rn(acc); return; }
-    const int t = q / c4, ci = (q - t * c4) * 4 + (e & 3);
-    if (ci < Ci) dw[((long long)co * Ci + ci) * KK + t] = __float2half_rn(acc);
+        for (int s = 1; s < SL; s++) acc += sums[s][lane];
+        const int q = (e >> 2) / p.Co, co = (e >> 2) - q * p.Co, t = q / c4, ci = (q - t * c4) * 4 + (e & 3);
+        if (e < p.total && q >= c4 * p.KK) p.db[e - c4 * p.KK * p.Co * 4] = __float2half_rn(acc);
+        else if (e < p.total && ci < p.Ci) { p.dw[((long long)co * p.Ci + ci) * p.KK + t] = __float2half_rn(acc); again = !isfinite(acc); }
+        const uint32_t mask = __ballot_sync(0xffffffffu, again);
+        if (lane == 0) again_s = mask;
+    }
+    if (!__syncthreads_or(again)) return;
+    for (uint32_t left = again_s; left; left &= left - 1) {
+        const int el = blockIdx.x * 32 + __ffs(left) - 1, q = (el >> 2) / p.Co, co = (el >> 2) - q * p.Co, t = q / c4, ci = (q - t * c4) * 4 + (el & 3);
+        const int dh = t / p.Wk - p.padU, dw = t % p.Wk - p.padL, P = p.Ho * p.Wo;
+        acc = 0.f;
+        for (int i = threadIdx.x; i < p.n * P && !isnan(acc); i += 32 * SL) {
+            const int s = i / P, r = (i - s * P) / p.Wo, h = r * p.S + dh, w = (i - s * P - r * p.Wo) * p.S + dw;
+            if ((unsigned)h < (unsigned)p.H && (unsigned)w < (unsigned)p.W)
+                acc = fmaf(__half2float(p.x[((long long)s * p.Ci + ci) * p.H * p.W + (long long)h * p.W + w]), __half2float(p.dy[((long long)s * p.Co + co) * P + (i - s * P)]), acc);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        __syncthreads();
+        if (lane == 0) sums[sl][0] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int s = 1; s < SL; s++) acc += sums[s][0];
+            p.dw[((long long)co * p.Ci + ci) * p.KK + t] = __float2half_rn(acc);
+        }
+    }
 }
 
 // ---------------------------------------------------------------- host side
@@ -859,8 +888,9 @@ bool conv_px_wg(Scope &sc, const ConvGeom &geom, const __half *x, const __half *
     if (!attr) { cudaFuncSetAttribute(conv_px_wg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024); attr = true; }
     TL_LAUNCH(conv_px_wg_kernel, dim3(bgx, bslices), PXW_THREADS, bsmem, bp);
     profile_add_flops(2.0 * g.n * g.Hout * g.Wout * nw);
-    if (groups <= 160) TL_LAUNCH(px_wg_reduce_kernel<8>, ceil_div(total, 32), 256, 0, bp.part, dw, db, groups, bp.group, g.Cout, g.Cin, p.KK, total);
-    else TL_LAUNCH(px_wg_reduce_kernel<16>, ceil_div(total, 32), 512, 0, bp.part, dw, db, groups, bp.group, g.Cout, g.Cin, p.KK, total);
+    const PxWgSum r = {bp.part, x, dy, dw, db, bp.group, groups, g.n, g.Cin, g.Hin, g.Win, g.Cout, g.Hout, g.Wout, g.sh, g.padU, g.padL, g.Wk, p.KK, total};
+    if (groups <= 160) TL_LAUNCH(px_wg_reduce_kernel<8>, ceil_div(total, 32), 256, 0, r);
+    else TL_LAUNCH(px_wg_reduce_kernel<16>, ceil_div(total, 32), 512, 0, r);
     return true;
 }
 

@@ -84,6 +84,39 @@ def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
     test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
 
 
+# An infinite or NaN pixel reaches the weight gradients of the taps that pair it with a pixel of the other tensor, and no other one: corners, an
+# edge, an even and an odd place of a strided layer, and a pixel inside
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", [(24, 14, 14, 48, 3, 1, 60), (17, 13, 11, 33, 5, 1, 30), (20, 16, 15, 40, 3, 2, 110), (40, 9, 7, 34, 1, 1, 400)])
+def test_weight_gradients_on_runs_of_slots_keep_what_is_no_number_apart(run, cin, h, w, cout, k, stride, n, bad):
+    if not run.half:
+        pytest.skip("half precision only")
+    rng = seeded(cin + k)
+    Ho, Wo, pad = (h - 1) // stride + 1, (w - 1) // stride + 1, k // 2
+    x, wt, dy = (rounded(run, rng.uniform(-1, 1, s)) for s in ((n, cin, h, w), (cout, cin, k, k), (n, cout, Ho, Wo)))
+    clean, names = conv_outputs(run, x, wt, dy, k, stride)
+    if k > 1:
+        assert any("conv_px_wg_kernel" in t for t in names)
+    for s, c, r, q in ((0, 0, 0, 0), (n - 1, cin - 1, h - 1, w - 1), (n // 2, 3, 0, w // 2), (3, 2, h // 2, w // 2)):
+        v = x.copy(); v[s, c, r, q] = bad
+        got = conv_outputs(run, v, wt, dy, k, stride)[0][2]
+        touched = np.zeros(got.shape, bool)
+        for kh in range(k):
+            for kw in range(k):
+                i, j = r + pad - kh, q + pad - kw
+                touched[:, c, kh, kw] = i % stride == 0 and j % stride == 0 and 0 <= i // stride < Ho and 0 <= j // stride < Wo
+        assert not np.isfinite(got[touched]).any()
+        assert_close(got[~touched], clean[2][~touched], FP16_TOL, "x %s" % ((s, c, r, q),))
+        v = dy.copy(); v[s, min(c, cout - 1), min(r, Ho - 1), min(q, Wo - 1)] = bad
+        got = conv_outputs(run, x, wt, v, k, stride)[0][2]
+        touched = np.zeros(got.shape, bool)
+        for kh in range(k):
+            for kw in range(k):
+                touched[min(c, cout - 1), :, kh, kw] = 0 <= min(r, Ho - 1) * stride + kh - pad < h and 0 <= min(q, Wo - 1) * stride + kw - pad < w
+        assert not np.isfinite(got[touched]).any()
+        assert_close(got[~touched], clean[2][~touched], FP16_TOL, "dy %s" % ((s, c, r, q),))
+
+
 # Long sums of the weight and bias gradient, terms of one sign: the tensor core truncates what it accumulates, up to 2^-23 of the sum at every k-step and half of that in
 # the mean.  Over a chain of 32 steps from zero that is 32 / 2 * 2^-24 = 1e-6 of a result, to which the rounding to half precision adds 2^-11 / 1.7
 # for one result and 1 / sqrt(results) of it for their mean, 4e-6.  (One chain of all steps of a CTA: 5e-5.)
