@@ -101,7 +101,7 @@ public:
     template <class T> T *scratch(size_t n) { return (T *)alloc(n * sizeof(T), true); }   // device-only temporary
     // the same for a path that has another one to fall back on: no memory is no error
     template <class T> T *try_scratch(size_t n) { return (T *)alloc(n * sizeof(T), false); }
-    bool ok() const { return ok_; }
+    bool ok() const;                // also sends the uploads that wait: asked in front of a call's kernels
     bool staged() const { return staged_; }   // some buffer of this call lives in host memory (mirrored in the arena)
     // a reduction of this call may be deferred: every buffer is the caller's own device memory and the call does not go
     // on to read the result itself
@@ -114,6 +114,7 @@ private:
     void *alloc(size_t bytes, bool needed);
     std::vector<Entry> entries_;
     size_t arena_mark_, pinned_mark_;
+    unsigned stage_mark_;
     bool ok_;
     bool staged_;
     bool no_defer_ = false;

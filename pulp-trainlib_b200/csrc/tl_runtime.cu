@@ -297,7 +297,8 @@ static void stage_add(StageJobs &s, int &blocks, const void *src, void *dst, siz
     blocks += ceil_div(count, 256 * STAGE_U);
 }
 
-Scope::Scope() : arena_mark_(0), pinned_mark_(g_pinned_off), ok_(true), staged_(false)
+static unsigned g_stage_failures = 0;                    // uploads that could not be launched
+Scope::Scope() : arena_mark_(0), pinned_mark_(g_pinned_off), stage_mark_(g_stage_failures), ok_(true), staged_(false)
 {
     ok_ = ready();
     arena_mark_ = arena_mark();
@@ -313,13 +314,19 @@ void *Scope::alloc(size_t bytes, bool needed)
 
 // The uploads of a call wait for the first use of the library's stream (stream(), which every launch and copy of a call goes
 // through), so that one kernel fetches them all: a launch of its own for each buffer cost the GPU 5 to 7 us whatever its size.
+// A call asks ok() in front of its kernels, which sends them; where that fails its kernels do not run, and nothing is written back.
 static StageJobs g_stage_in = {};
 static int g_stage_blocks = 0;
 static void stage_flush()
 {
     g_stage_waiting = false;                    // (the launch below asks for the stream, too)
-    stage_run(g_stage_in, g_stage_blocks);
+    if (!stage_run(g_stage_in, g_stage_blocks)) g_stage_failures++;
     g_stage_blocks = 0;
+}
+bool Scope::ok() const
+{
+    if (ok_ && g_stage_waiting) stage_flush();
+    return ok_ && stage_mark_ == g_stage_failures;
 }
 
 bool Scope::upload(Entry &e)
@@ -378,14 +385,15 @@ Scope::~Scope()
         if (g_stage_waiting) stage_flush();
         StageJobs s = {};
         int blocks = 0;
+        bool good = ok();                       // (what the mirrors hold is no result otherwise)
         for (auto &e : entries_) {
-            if (!e.write_back) continue;
+            if (!e.write_back || !good) continue;
             if (!e.pinned) { TL_CUDA(cudaMemcpyAsync(e.host, e.dev, e.bytes, cudaMemcpyDeviceToHost, g.cur_stream)); continue; }
-            if (s.jobs == 8) { stage_run(s, blocks); blocks = 0; }
+            if (s.jobs == 8) { good = stage_run(s, blocks); blocks = 0; }
             stage_add(s, blocks, e.dev, e.pinned, e.bytes);
         }
-        stage_run(s, blocks);
-        if (TL_CUDA(cudaStreamSynchronize(g.cur_stream)))
+        if (good) good = stage_run(s, blocks);
+        if (TL_CUDA(cudaStreamSynchronize(g.cur_stream)) && good)
             for (auto &e : entries_) if (e.write_back && e.pinned) memcpy(e.host, e.pinned, e.bytes);
     }
     if (--g.scope_depth == 0) scratch_mark();

@@ -1,0 +1,53 @@
+"""CPU: the library's host code on a CUDA runtime without a device (fake_cudart.c), where launches can be made to fail."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+HEAD = r'''
+import ctypes, sys
+sys.path.insert(0, %r)
+import numpy as np
+from conftest import load_pkg
+pkg = load_pkg()
+fake = ctypes.CDLL(%r)
+lib = pkg.load()
+assert lib.trainlib_init(0) == 0
+'''
+
+
+@pytest.fixture(scope="module")
+def on_fake_runtime(tmp_path_factory):
+    if not os.path.exists(os.path.join(INCLUDE, "cuda_runtime_api.h")):
+        pytest.skip("no CUDA headers")
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.check_call(["gcc", "-O1", "-Wall", "-shared", "-fPIC", "-I" + INCLUDE, os.path.join(HERE, "fake_cudart.c"), "-o", so])
+
+    def run(program):
+        r = subprocess.run([sys.executable, "-c", HEAD % (HERE, so) + program], env=dict(os.environ, LD_PRELOAD=so), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_a_failed_upload_stops_its_call(on_fake_runtime):
+    """host arrays: without its inputs no kernel of the call runs and no output is written; a failed download writes none either"""
+    on_fake_runtime(r'''
+rng = np.random.default_rng(0)
+A, B = rng.standard_normal((9, 8)).astype(np.float32), rng.standard_normal((8, 7)).astype(np.float32)
+def call(fail):
+    keep = pkg.Keep()
+    C = np.full((9, 7), 3.0, np.float32)
+    a = pkg.make_args(keep, "matMul_args", A=A, B=B, C=C, N=9, K=8, M=7, trans_B=0, USE_BIASES=0)
+    lib.trainlib_clear_error()
+    fake.fake_reset(fail)
+    lib.mm(ctypes.byref(a))
+    return fake.fake_launches(), lib.trainlib_last_error(), bool((C == 3.0).all())
+n, err, same = call(0)
+assert n >= 3 and err == pkg.TL_OK and not same, (n, err, same)             # uploads, products, downloads
+assert call(1) == (1, 2, True), call(1)
+assert call(n)[1:] == (2, True), call(n)
+assert call(0) == (n, pkg.TL_OK, False)
+''')
