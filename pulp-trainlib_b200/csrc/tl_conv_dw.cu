@@ -303,8 +303,12 @@ template <class T> bool dw_wg_planes(const ConvGeom &g, const T *x, const T *dy,
 {
     Dw3Strip t;
     if (const int V = dw3_strip(g, t, x, dy, (int)sizeof(T), false, 4)) {
-        // one wave of the four CTAs that fit an SM (two waves and a bit: 17.1 us for both gradients of 64 channels of 28 x 28 x 64, 14.6 so)
-        groups = std::max(1, std::min(4 * sm_count() / g.Cin, g.n));
+        // One wave of the four CTAs that fit an SM (two waves and a bit: 17.1 us for both gradients of 64 channels of 28 x 28 x 64, 14.6 so) while
+        // that is two CTAs a channel.  From 297 channels on it would be one, half of the CTA slots empty or a second wave of few: about a
+        // wave and a half there (us, one / two / three CTAs a channel: 300 channels of 28 x 28 x 64 37.2 / 34.4 / 29.8; 384 38.8 / 38.1 / 33.1; 512 of
+        // 14 x 14 x 64 27.3 / 23.5 / 24.6; 600 32.7 / 28.8 / 28.1; 650 of 14 x 14 x 32 18.3 / 16.6 / 17.7; 960 of 7 x 7 x 64 15.0 / 14.7 / 16.1;
+        // little work, 400 of 7 x 7 x 16, 5.7 / 5.8 / 5.8; below: 256 of 28 x 28 x 64 30.8 / 23.5 / 25.9)
+        groups = std::max(1, std::min(g.Cin > 2 * sm_count() ? ceil_div(6 * sm_count(), g.Cin) : 4 * sm_count() / g.Cin, g.n));
         if (dry) return true;
         const dim3 grid(g.Cin, groups);
         if (V == 4) TL_LAUNCH((dw3_strip_wg_kernel<T, 4, 4>), grid, 128, 0, t, x, dy, part, g.n);

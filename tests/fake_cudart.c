@@ -6,12 +6,13 @@
 
 static struct { char *p; size_t n; } blocks[256];
 static cudaError_t last = cudaSuccess;
-static int launches, fail_at, max_cluster, cluster_limit = 16;
+static int launches, fail_at, max_cluster, max_blocks, cluster_limit = 16;
 
-void fake_reset(int fail) { launches = 0; fail_at = fail; max_cluster = 0; }          /* fail: number of the launch that fails, from 1; 0: none */
+void fake_reset(int fail) { launches = max_cluster = max_blocks = 0; fail_at = fail; }   /* fail: number of the launch that fails, from 1; 0: none */
 void fake_cluster_limit(int n) { cluster_limit = n; }
 int fake_launches(void) { return launches; }
 int fake_max_cluster(void) { return max_cluster; }
+int fake_max_blocks(void) { return max_blocks; }           /* of a launch, along x and y */
 
 cudaError_t cudaGetLastError(void) { cudaError_t e = last; last = cudaSuccess; return e; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "made by the test"; }
@@ -60,8 +61,9 @@ cudaError_t cudaGetDriverEntryPoint(const char *s, void **p, unsigned long long 
     if (r) *r = cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }
-static cudaError_t launch(int cluster)
+static cudaError_t launch(int cluster, dim3 grid)
 {
+    if ((int)(grid.x * grid.y) > max_blocks) max_blocks = (int)(grid.x * grid.y);
     if (cluster > max_cluster) max_cluster = cluster;
     if (++launches == fail_at || cluster > cluster_limit) return last = cudaErrorLaunchOutOfResources;
     return cudaSuccess;
@@ -71,6 +73,6 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void
     int cluster = 1;
     (void)f; (void)args;
     for (unsigned i = 0; i < c->numAttrs; i++) if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = (int)c->attrs[i].val.clusterDim.x;
-    return launch(cluster);
+    return launch(cluster, c->gridDim);
 }
-cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t n, cudaStream_t s) { (void)f; (void)g; (void)b; (void)args; (void)n; (void)s; return launch(1); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **args, size_t n, cudaStream_t s) { (void)f; (void)b; (void)args; (void)n; (void)s; return launch(1, g); }

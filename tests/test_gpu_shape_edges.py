@@ -329,8 +329,9 @@ def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
 
 
 # 3 x 3 with stride 1 in register strips: rows of whole 16-byte groups and not, one row, one column, strips of unequal rows, many planes in a CTA
-# (more than there are channels), several rounds of a CTA's threads, padding of two columns beside whole groups
-@pytest.mark.parametrize("c,h,w,pad,n", [(6, 31, 20, 1, 5), (3, 1, 8, 1, 2), (2, 9, 1, 1, 40), (1, 1, 1, 1, 3), (3, 6, 8, 1, 900), (200, 9, 12, 1, 3), (2, 130, 131, 1, 1), (4, 17, 12, 2, 6), (5, 18, 16, 0, 4), (1, 300, 260, 1, 1)])
+# (more than there are channels), several rounds of a CTA's threads, padding of two columns beside whole groups, so many channels that the
+# weight gradient takes more than one wave of CTAs
+@pytest.mark.parametrize("c,h,w,pad,n", [(6, 31, 20, 1, 5), (3, 1, 8, 1, 2), (2, 9, 1, 1, 40), (1, 1, 1, 1, 3), (3, 6, 8, 1, 900), (200, 9, 12, 1, 3), (2, 130, 131, 1, 1), (4, 17, 12, 2, 6), (5, 18, 16, 0, 4), (1, 300, 260, 1, 1), (297, 6, 8, 1, 7), (600, 5, 7, 1, 2)])
 def test_depthwise_in_register_strips(run, oracle, c, h, w, pad, n):
     test_depthwise_shapes(run, oracle, c, h, w, 3, pad, n)
 

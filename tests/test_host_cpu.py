@@ -51,3 +51,22 @@ assert call(1) == (1, 2, True), call(1)
 assert call(n)[1:] == (2, True), call(n)
 assert call(0) == (n, pkg.TL_OK, False)
 ''')
+
+
+def test_depthwise_weight_gradients_occupy_the_chip(on_fake_runtime):
+    """3 x 3 layers with 64 streams on 148 SMs that hold four CTAs each: up to 296 channels one wave at most and two thirds of one at least (where there are
+    as many planes), beyond a wave and a half and less than a CTA a channel more"""
+    on_fake_runtime(r"""
+x = lib.trainlib_malloc(1 << 22)
+lib.trainlib_set_streams(64)
+keep = pkg.Keep()
+for c in list(range(1, 800, 7)) + [296, 297, 592, 593]:
+    b = lambda ch, h: pkg.make_blob(keep, x, x, C=ch, H=h, W=h)
+    a = pkg.make_args(keep, "DepthWise_Conv_args", input=b(c, 8), coeff=b(c, 3), output=b(c, 8), Lpad=1, Rpad=1, Upad=1, Dpad=1, stride_h=1, stride_w=1, HWC=0)
+    fake.fake_reset(0)
+    lib.pulp_conv_dw_fp32_bw_param_grads_cl(ctypes.byref(a))
+    n = fake.fake_max_blocks()
+    assert lib.trainlib_last_error() == 0
+    if c <= 296: assert min(c * 64, 592 * 2 // 3) <= n <= 592, (c, n)
+    else: assert 888 <= n < 888 + c, (c, n)
+""")
