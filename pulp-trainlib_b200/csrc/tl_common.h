@@ -68,6 +68,17 @@ template <class... P, class... A> inline void launch_clusters(void (*kernel)(P..
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream(); cfg.attrs = attr; cfg.numAttrs = 2;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+// Whether the device can place one cluster of that size (more than eight blocks are not portable).
+template <class... P> inline bool clusters_fit(void (*kernel)(P...), int threads, size_t smem, int cluster)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cluster; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+}
 #define TL_LAUNCH_CLUSTER(kernel, grid, block, smem, cluster, ...)                  \
     do {                                                                            \
         const bool tl_prof_ = ::tl::profiling();                                    \

@@ -1050,15 +1050,20 @@ template <class T> static bool cm_wg_plan(CmWg &p, int CI, int CO, int slots, si
     return true;
 }
 
-template <class T, int TPW> static void conv_mma_wg_cluster_launch(const CmWg &p, int ranks, size_t smem)
+// false: a cluster of more than eight CTAs, which not every device (or part of one) can place
+template <class T, int TPW> static bool conv_mma_wg_cluster_launch(const CmWg &p, int ranks, size_t smem)
 {
-    static bool set = false;
+    static bool set = false, sixteen = false;
     if (!set) {
         cudaFuncSetAttribute(conv_mma_wg_cluster_kernel<T, TPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, CM_SMEM_MAX);
-        cudaFuncSetAttribute(conv_mma_wg_cluster_kernel<T, TPW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (cudaFuncSetAttribute(conv_mma_wg_cluster_kernel<T, TPW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+            sixteen = clusters_fit(conv_mma_wg_cluster_kernel<T, TPW>, 32 * CMC_NW, CM_SMEM_MAX, CMC_MAX);
+        cudaGetLastError();
         set = true;
     }
+    if (ranks > 8 && !sixteen) return false;
     TL_LAUNCH_CLUSTER((conv_mma_wg_cluster_kernel<T, TPW>), dim3(ranks, p.ci_tiles * ceil_div(p.Co, CMC_TILE)), 32 * CMC_NW, smem, ranks, p);
+    return true;
 }
 
 template <class T, int TAPS, int MI, int NI, int WM, int WN, int WK> static bool conv_mma_wg_launch(CmWg &p, int part_groups, int *groups_out, bool dry)
@@ -1121,10 +1126,7 @@ template <class T> bool conv_mma_wg_cluster(const ConvGeom &g, const T *x, const
     if (!cm_wg_cluster_plan<T>(g, x, dy, p, ranks, smem)) return false;
     p.dw = dw;
     const int tpw = ceil_div(p.KK, CMC_NW);
-    if (tpw <= 1) conv_mma_wg_cluster_launch<T, 1>(p, ranks, smem);
-    else if (tpw <= 3) conv_mma_wg_cluster_launch<T, 3>(p, ranks, smem);
-    else conv_mma_wg_cluster_launch<T, 6>(p, ranks, smem);
-    return true;
+    return tpw <= 1 ? conv_mma_wg_cluster_launch<T, 1>(p, ranks, smem) : tpw <= 3 ? conv_mma_wg_cluster_launch<T, 3>(p, ranks, smem) : conv_mma_wg_cluster_launch<T, 6>(p, ranks, smem);
 }
 // fp16: in front of the tcgen05 kernel over slots, whose launch and reduction cost about 10 us at any size, while the products of a CTA
 // are few (48 -> 48 on 28 x 28, 5 x 5: 8.6 us against 13.3; with 7 x 7 windows 16.6 against 15.5)

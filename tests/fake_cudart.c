@@ -61,6 +61,13 @@ cudaError_t cudaGetDriverEntryPoint(const char *s, void **p, unsigned long long 
     if (r) *r = cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }
+cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *f, const cudaLaunchConfig_t *c)
+{
+    (void)f;
+    *n = 9;
+    for (unsigned i = 0; i < c->numAttrs; i++) if (c->attrs[i].id == cudaLaunchAttributeClusterDimension && (int)c->attrs[i].val.clusterDim.x > cluster_limit) *n = 0;
+    return cudaSuccess;
+}
 static cudaError_t launch(int cluster, dim3 grid)
 {
     if ((int)(grid.x * grid.y) > max_blocks) max_blocks = (int)(grid.x * grid.y);

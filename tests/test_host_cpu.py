@@ -70,3 +70,24 @@ for c in list(range(1, 800, 7)) + [296, 297, 592, 593]:
     if c <= 296: assert min(c * 64, 592 * 2 // 3) <= n <= 592, (c, n)
     else: assert 888 <= n < 888 + c, (c, n)
 """)
+
+
+@pytest.mark.parametrize("limit", [8, 16])
+def test_clusters_of_sixteen_only_where_they_can_be_placed(on_fake_runtime, limit):
+    """weight gradients of few pixels run as clusters of up to sixteen CTAs, on a device that places eight at most as smaller ones or on another kernel"""
+    on_fake_runtime(r"""
+fake.fake_cluster_limit(%d)
+x = lib.trainlib_malloc(1 << 22)
+keep = pkg.Keep()
+most = 0
+for half in ("", "_fp16"):
+    for cin, h, k in ((16, 32, 3), (16, 45, 3), (24, 40, 1), (12, 44, 5), (5, 41, 7), (8, 12, 3)):
+        b = lambda ch, hh, dim=None: pkg.make_blob(keep, x, x, C=ch, H=hh, W=hh, dim=dim, half=bool(half))
+        a = pkg.make_args(keep, "Conv2D_args" + half, input=b(cin, h), coeff=b(cin, k, 32 * cin * k * k), bias=b(32, 1), output=b(32, h), Lpad=k // 2, Rpad=k // 2, Upad=k // 2, Dpad=k // 2,
+                          stride_h=1, stride_w=1, i2c_buffer=x, bt_buffer=x, USE_BIASES=0, USE_IM2COL=0, HWC=0)
+        fake.fake_reset(0)
+        getattr(lib, "pulp_conv2d_fp%%s_bw_param_grads_cl" %% ("16" if half else "32"))(ctypes.byref(a))
+        assert fake.fake_launches() >= 1 and lib.trainlib_last_error() == 0, (half, cin, h, k)
+        most = max(most, fake.fake_max_cluster())
+assert most == %d, most
+""" % (limit, limit))
