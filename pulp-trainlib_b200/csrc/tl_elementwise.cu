@@ -903,10 +903,12 @@ __global__ void __launch_bounds__(256) layernorm_bw_warp_kernel(const T *__restr
     }
     if (threadIdx.x == 0) ln_ticket = 0;
 }
-// Few rows (up to 512 of up to 512 elements): one cluster of eight CTAs of sixteen warps, a warp per row while there are that many.  The
+// Few rows (up to 512 of up to 512 elements, 384 of up to 128): one cluster of eight CTAs of sixteen warps, a warp per row while there are that many.  The
 // CTAs' column sums stay in shared memory and every CTA adds its share of the columns over the eight of them in order, through
 // distributed shared memory: two cluster barriers take the place of a round trip through L2, a ticket and the last CTA's sums,
-// which were half of the kernel above at these sizes (128 rows of 128 in fp16 4.9 -> 3.9 us, of 512 9.0 -> 6.1).
+// which were half of the kernel above at these sizes.  us, that kernel / here: 128 rows of 128 4.2 / 3.7 (fp16 4.4 / 3.8), of 512 7.8 / 5.4 (8.4 / 5.4);
+// 384 of 64 5.0 / 4.6, of 128 5.3 / 4.9, of 512 13.1 / 9.0; 512 of 256 9.4 / 7.4, of 512 15.6 / 10.8 (16.2 / 11.5), and from DRAM 20.5 / 18.4.  More narrow
+// rows are too many for eight SMs: 448 of 64 5.2 / 5.4 (fp16 5.3 / 5.6, from DRAM 10.2 / 12.3), of 128 5.6 / 5.7 (5.8 / 6.0).
 static constexpr int LN_CL = 8, LN_CW = 16;
 template <class T, int NV>
 __global__ void __launch_bounds__(32 * LN_CW) layernorm_bw_cluster_kernel(const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ dy, T *__restrict__ dx,
@@ -1009,7 +1011,7 @@ template <class T> void layernorm_bw(Scope &sc, const T *x, const T *w, const T 
     if (width <= 1024) {
         // a warp per row while that gives at most one CTA per two SMs (the last CTA adds that many sums), more rows per warp beyond
         const int rows_per_cta = std::max(8, ceil_div(ceil_div(rows, sm_count() / 2), 8) * 8), ctas = ceil_div(rows, rows_per_cta);
-        if (ctas > 1 && rows <= 512 && width <= 512) {
+        if (ctas > 1 && rows <= (width <= 128 ? 384 : 512) && width <= 512) {
 #define TL_LN_BW(NV) TL_LAUNCH_CLUSTER((layernorm_bw_cluster_kernel<T, NV>), LN_CL, 32 * LN_CW, 0, LN_CL, x, w, dy, dx, dw, db, rows, width, eps)
             if (width <= 128) TL_LN_BW(4); else if (width <= 256) TL_LN_BW(8); else TL_LN_BW(16);
 #undef TL_LN_BW

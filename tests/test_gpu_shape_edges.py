@@ -24,6 +24,14 @@ def rounded(r, a):
     return a.astype(r.dt).astype(F)
 
 
+def kernels_of(run, call, *args):
+    """names of the kernels that a call launches"""
+    run.lib.trainlib_profile(1)
+    call(run, *args)
+    run.lib.trainlib_profile(0)
+    return [t[0] for t in run.pkg.profile_table(run.lib)]
+
+
 def conv_outputs(run, x, wt, dy, k, stride=1, bias=False):
     """Y, dX, dW (and dB) of one layer with padding k // 2, and the names of the kernels that ran"""
     n, cin, h, w = x.shape
@@ -424,9 +432,10 @@ def test_layernorm_shapes(run, oracle, rows, width):
 
 
 # the backward pass of a few rows as one cluster: fewest and most rows and columns, and just past them
-@pytest.mark.parametrize("rows,width", [(9, 1), (128, 129), (129, 257), (512, 512), (513, 512), (512, 513), (17, 31)])
+@pytest.mark.parametrize("rows,width", [(9, 1), (128, 129), (129, 257), (512, 512), (513, 512), (512, 513), (17, 31), (384, 128), (385, 128), (385, 129), (8, 40)])
 def test_layernorm_of_one_cluster(run, oracle, rows, width):
-    test_layernorm_shapes(run, oracle, rows, width)
+    names = kernels_of(run, test_layernorm_shapes, oracle, rows, width)
+    assert any("layernorm_bw_cluster" in t for t in names) == (8 < rows <= (512 if width > 128 else 384) and width <= 512), names
 
 
 @pytest.mark.parametrize("dim", [1, 5, 1023, 1025, 70001, 400000])
