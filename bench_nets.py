@@ -289,7 +289,9 @@ class ResNet8Streams(object):
          "forward of the 7 3x3 convolutions and their input gradients as tcgen05 3xTF32 implicit GEMMs (useful FLOP: zeros of a dilated dY are not counted)"),
         ("conv_wg_tensor", ("conv_wgt_kernel", "conv_wgy_kernel"), "tensor",
          "weight gradient of the 3x3 convolutions as tcgen05 3xTF32 pixel-contraction GEMMs (conv_wgy_kernel: 8 and 16 channels at stride 1)"),
-        ("conv_mma", ("conv_mma_kernel", "conv_px_kernel", "conv_pw_kernel", "conv_mma_wg_kernel", "conv_mma_wg_cluster_kernel", "conv_px_wg_kernel", "conv_pw_wg_kernel"), "tensor", "convolutions of small shards as 3xTF32 on the warp-level tensor-core instructions"),
+        ("conv_mma", ("conv_mma_kernel", "conv_mma_wg_kernel", "conv_mma_wg_cluster_kernel"), "tensor", "convolutions of small shards on the warp-level tensor-core instructions (fp32 as 3xTF32)"),
+        ("conv_px_pw", ("conv_px_kernel", "conv_px_wg_kernel", "conv_pw_kernel", "conv_pw_wg_kernel"), "tensor",
+         "fp16 convolutions over runs of slots and fp32 pointwise layers (3xTF32) as products on tcgen05"),
         ("conv_wg_ffma", ("conv_wg3x3_partial_kernel", "conv_wg_partial_kernel", "conv_wg_direct_kernel"), "ffma", "weight gradient of the other convolutions, fp32 FFMA"),
         ("conv_1x1_strided", ("conv1x1s_mma_kernel", "conv1x1s_wg_kernel", "conv1x1_strided_ig_kernel"), "hbm",
          "forward, weight gradient and in-place input gradient of the two 1x1 stride-2 shortcut convolutions: 2 FLOP per byte, bound by memory traffic and instruction issue"),

@@ -555,7 +555,7 @@ template <class T, int MT, int WM, int WN, int WK, int BN, bool KS = false> stat
     const int co_tiles = ceil_div(p.Cd, BM);
     // every CTA slot taken: co-resident CTAs share an SM, so a last round that only some of them have costs less than idle slots
     const int gx = std::min(tiles_max, std::max(1, sm_count() * (cm_ctas<T, WM>() == 3 && smem <= 74 * 1024 ? 3 : smem <= 110 * 1024 ? 2 : 1) / (co_tiles * p.ncls)));
-    if (KS) TL_LAUNCH_CLUSTER((conv_mma_kernel<T, MT, WM, WN, WK, BN, KS>), dim3(tiles_max * p.ksplit, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p.ksplit, p);
+    if constexpr (KS) TL_LAUNCH_CLUSTER((conv_mma_kernel<T, MT, WM, WN, WK, BN, true>), dim3(tiles_max * p.ksplit, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p.ksplit, p);
     else TL_LAUNCH((conv_mma_kernel<T, MT, WM, WN, WK, BN, KS>), dim3(gx, co_tiles, p.ncls), 32 * WM * WN * WK, smem, p);
     return true;
 }

@@ -25,11 +25,11 @@ def rounded(r, a):
 
 
 def kernels_of(run, call, *args):
-    """names of the kernels that a call launches"""
+    """launches of a call by the kernels' names"""
     run.lib.trainlib_profile(1)
     call(run, *args)
     run.lib.trainlib_profile(0)
-    return [t[0] for t in run.pkg.profile_table(run.lib)]
+    return {t[0]: t[1] for t in run.pkg.profile_table(run.lib)}
 
 
 def conv_outputs(run, x, wt, dy, k, stride=1, bias=False):
@@ -80,16 +80,18 @@ def test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n):
 
 # the half-precision kernels on runs of slots (tl_conv_px.cu): loads of one, two and four pixels, planes smaller and larger than a run, runs
 # that start inside a row, channel counts at and off multiples of 16, slices of result channels, groups of source channels,
-# windows of 1 to 49 taps, strides 2 and 3 with parities that no tap reaches, a bias gradient in a spare channel and on its own
-SLOTS = [(24, 28, 28, 48, 3, 1, 130), (5, 27, 43, 23, 3, 1, 70), (64, 6, 6, 96, 3, 1, 60), (3, 48, 46, 90, 3, 1, 20), (32, 9, 14, 17, 5, 1, 40), (16, 31, 33, 33, 5, 1, 9), (6, 40, 40, 20, 7, 1, 12), (90, 19, 21, 70, 1, 1, 40),
-         (40, 41, 41, 80, 5, 1, 3), (96, 15, 17, 96, 1, 1, 90), (34, 10, 23, 55, 1, 2, 210), (43, 23, 34, 22, 3, 2, 60), (7, 39, 39, 58, 3, 2, 280), (20, 30, 31, 40, 3, 3, 110), (13, 33, 32, 24, 5, 2, 40), (1, 1, 300, 128, 3, 1, 40)]
+# windows of 1 to 49 taps, strides 2 and 3 with parities that no tap reaches, a bias gradient in a spare channel and on its own.
+# The last number: of forward and input gradient, how many run there (the others have too little work, or are products of the GEMM)
+SLOTS = [(24, 28, 28, 48, 3, 1, 130, 2), (5, 27, 43, 23, 3, 1, 70, 2), (64, 6, 6, 96, 3, 1, 60, 0), (3, 48, 46, 90, 3, 1, 20, 2), (32, 9, 14, 17, 5, 1, 40, 2), (16, 31, 33, 33, 5, 1, 9, 1), (6, 40, 40, 20, 7, 1, 12, 2), (90, 19, 21, 70, 1, 1, 40, 0),
+         (40, 41, 41, 80, 5, 1, 3, 1), (96, 15, 17, 96, 1, 1, 90, 0), (34, 10, 23, 55, 1, 2, 210, 2), (43, 23, 34, 22, 3, 2, 60, 1), (7, 39, 39, 58, 3, 2, 280, 2), (20, 30, 31, 40, 3, 3, 110, 1), (13, 33, 32, 24, 5, 2, 40, 1), (1, 1, 300, 128, 3, 1, 40, 1)]
 
 
-@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", SLOTS)
-def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n):
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n,directions", SLOTS)
+def test_conv2d_on_runs_of_slots(run, oracle, cin, h, w, cout, k, stride, n, directions):
     if not run.half:
         pytest.skip("half precision only")
-    test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+    launches = kernels_of(run, test_conv2d_shapes, oracle, cin, h, w, cout, k, stride, n)
+    assert launches.get("conv_px_kernel", 0) == directions and launches.get("conv_px_wg_kernel") == 1, launches
 
 
 # An infinite or NaN pixel reaches the weight gradients of the taps that pair it with a pixel of the other tensor, and no other one: corners, an
@@ -163,13 +165,15 @@ def test_conv2d_of_few_pixels(run, oracle, cin, h, w, cout, k, stride, n):
 
 
 # long sums under few pixels, one cluster per result tile whose CTAs share the source channels: channel counts that divide into unequal
-# shares, a last share of few channels, strides whose parities have different taps (some none), more streams in a tile, 1 x 1 windows
-LONG_SUMS = [(96, 9, 13, 96, 3, 2, 1), (60, 13, 18, 8, 3, 1, 1), (130, 7, 9, 100, 3, 1, 1), (400, 4, 4, 390, 1, 1, 1), (50, 5, 5, 52, 5, 1, 3), (75, 3, 3, 66, 3, 3, 7), (200, 5, 7, 17, 2, 1, 1), (48, 28, 28, 40, 5, 1, 1)]
+# shares, a last share of few channels, strides whose parities have different taps (some none), more streams in a tile, 1 x 1 windows.
+# The last numbers: of forward and input gradient, how many run there in fp32 and in fp16 (the others have shorter sums)
+LONG_SUMS = [(96, 9, 13, 96, 3, 2, 1, 2, 1), (60, 13, 18, 8, 3, 1, 1, 1, 0), (130, 7, 9, 100, 3, 1, 1, 2, 2), (400, 4, 4, 390, 1, 1, 1, 2, 2), (50, 5, 5, 52, 5, 1, 3, 2, 2), (75, 3, 3, 66, 3, 3, 7, 1, 0), (200, 5, 7, 17, 2, 1, 1, 1, 1), (48, 28, 28, 40, 5, 1, 1, 2, 2)]
 
 
-@pytest.mark.parametrize("cin,h,w,cout,k,stride,n", LONG_SUMS)
-def test_conv2d_of_long_sums(run, oracle, cin, h, w, cout, k, stride, n):
-    test_conv2d_shapes(run, oracle, cin, h, w, cout, k, stride, n)
+@pytest.mark.parametrize("cin,h,w,cout,k,stride,n,fp32,fp16", LONG_SUMS)
+def test_conv2d_of_long_sums(run, oracle, cin, h, w, cout, k, stride, n, fp32, fp16):
+    launches = kernels_of(run, test_conv2d_shapes, oracle, cin, h, w, cout, k, stride, n)
+    assert launches.get("(conv_mma_kernel<T, MT, WM, WN, WK, BN, true>)", 0) == (fp16 if run.half else fp32), launches
 
 
 # single-precision pointwise layers over many pixels (tl_conv_pw.cu): CTAs whose last 128 pixels are cut short, planes smaller than that, odd
@@ -341,7 +345,8 @@ def test_depthwise_shapes(run, oracle, c, h, w, k, pad, n, stride=1):
 # weight gradient takes more than one wave of CTAs
 @pytest.mark.parametrize("c,h,w,pad,n", [(6, 31, 20, 1, 5), (3, 1, 8, 1, 2), (2, 9, 1, 1, 40), (1, 1, 1, 1, 3), (3, 6, 8, 1, 900), (200, 9, 12, 1, 3), (2, 130, 131, 1, 1), (4, 17, 12, 2, 6), (5, 18, 16, 0, 4), (1, 300, 260, 1, 1), (297, 6, 8, 1, 7), (600, 5, 7, 1, 2)])
 def test_depthwise_in_register_strips(run, oracle, c, h, w, pad, n):
-    test_depthwise_shapes(run, oracle, c, h, w, 3, pad, n)
+    launches = kernels_of(run, test_depthwise_shapes, oracle, c, h, w, 3, pad, n)
+    assert sum(v for t, v in launches.items() if "dw3_strip_kernel" in t) == 2 and sum(v for t, v in launches.items() if "dw3_strip_wg_kernel" in t) == 1, launches
 
 
 # Planes whose staged windows come to just below, exactly and just above the 48 KB that a launch gets without asking: the weight
