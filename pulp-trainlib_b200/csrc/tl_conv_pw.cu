@@ -20,19 +20,22 @@ namespace tl {
 
 int *tc_status_word();          // tl_conv_tc.cu
 
-static constexpr int PW_STAGES = 5, PW_CONV = PW_STAGES * 128, PW_THREADS = PW_CONV + 160, PW_KC = 32;
+static constexpr int PW_STAGES = 5, PW_CONV = PW_STAGES * 128, PW_THREADS = PW_CONV + 160, PW_KC = 32, PW_MAX_SOURCES = 512;
 static constexpr uint32_t PW_HALF = PW_KC / 4 * 128 * 16, PW_STAGE = 2 * PW_HALF, PW_SMEM = 225 * 1024;
 
 struct PwParams {
     const float *src, *w, *bias; float *dst; int *status;
     int P, C, Cd, wm, wk;                       // plane, source and result channels; weight index = m * wm + k * wk
     int total, per;                             // pixels of all streams, of a CTA
-    int N, kc, chunks, kpad, stages, accs, cols; // result channels padded; channels of a piece, pieces, channels padded; accumulators
+    int N, kc, chunks, kpad, stages, accs, cols; // result channels padded; channels of a piece, pieces, channels padded; sets of accumulators
+    int chain, chains;                          // pieces that share an accumulator, accumulators of a set (pairs of hi and lo)
 };
 
 __device__ __forceinline__ void pw_sts(uint32_t to, const uint32_t *x) { asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to), "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]) : "memory"); }
 
-__global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_constant__ PwParams p)
+// CHAINS: several accumulators for the source channels (pw_chains).  Layers with one have a kernel without the loop over them: 1.1 us less for the two
+// directions of 64 streams of 64 -> 128 on 28 x 28.
+template <bool CHAINS> __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_constant__ PwParams p)
 {
     extern __shared__ __align__(1024) unsigned char pw_smem[];
     __shared__ __align__(8) uint64_t full[PW_STAGES], empty[PW_STAGES], acc_full[2], acc_empty[2];
@@ -131,16 +134,17 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
             const int buf = p.accs == 2 ? t & 1 : 0, use = p.accs == 2 ? t >> 1 : t;
             if (use && !tc::warp_wait_or_abort(&acc_empty[buf], (uint32_t)(use - 1) & 1u, abort_flag, p.status, 56, 20u, lane)) break;
             tc::tc_fence_after();
-            const uint32_t d = tmem + (uint32_t)(buf * 2 * N), dl = d + (uint32_t)N;
-            uint32_t bw = b_lw0;
+            uint32_t d = tmem + (uint32_t)(buf * (CHAINS ? p.chains : 1) * 2 * N), dl = d + (uint32_t)N, bw = b_lw0;
+            int first = 0;                                                 // piece with which the chain begins
             for (int c = 0; c < p.chunks; c++) {
+                if (CHAINS && c - first == p.chain) { first = c; d += (uint32_t)(2 * N); dl += (uint32_t)(2 * N); }
                 if (!tc::warp_wait_or_abort(&full[st], ph, abort_flag, p.status, 57, 0u, lane)) { ok = false; break; }
                 tc::tc_fence_after();
                 uint32_t aw = a_lw0 + (uint32_t)st * (PW_STAGE / 16);
                 const int ks = min(p.kc, p.kpad - c * p.kc) / 8;
                 for (int k = 0; k < ks; k++, aw += 256u, bw += 2u * (b_lbo / 16)) {
                     const uint64_t ah = ((uint64_t)a_hw << 32) | aw, al = ((uint64_t)a_hw << 32) | (aw + PW_HALF / 16), bh = ((uint64_t)b_hw << 32) | bw;
-                    const uint32_t more = c > 0 || k > 0;
+                    const uint32_t more = c > first || k > 0;
                     if (tc::elect_one()) {
                         tc::mma_tf32_ss(d, ah, bh, id2, more);
                         if (!both) tc::mma_tf32_ss(dl, ah, ((uint64_t)b_hw << 32) | (bw + (uint32_t)N), id1, more);
@@ -163,14 +167,24 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
             const int buf = p.accs == 2 ? t & 1 : 0, use = p.accs == 2 ? t >> 1 : t;
             if (!tc::warp_wait_or_abort(&acc_full[buf], (uint32_t)use & 1u, abort_flag, p.status, 58, 20u, lane)) break;
             tc::tc_fence_after();
-            const uint32_t d = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 2 * N);
+            const uint32_t d = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * (CHAINS ? p.chains : 1) * 2 * N);
             float *to = p.dst + (long long)so * p.Cd * P + po;
             const bool live = x < hi;
             for (int m = 0; m < N; m += 16) {
                 uint32_t a[16], b[16];
+                float v[16];
                 tc::tmem_ld16(d + (uint32_t)m, a);
                 tc::tmem_ld16(d + (uint32_t)(N + m), b);
                 tc::tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                for (int q = 1; CHAINS && q < p.chains; q++) {
+                    tc::tmem_ld16(d + (uint32_t)(q * 2 * N + m), a);
+                    tc::tmem_ld16(d + (uint32_t)(q * 2 * N + N + m), b);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] += __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                }
                 if (m + 16 >= N) {                                          // read: the next tile's products may start
                     tc::tc_fence_before();
                     __syncwarp();
@@ -179,11 +193,11 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
                 float *y = to + (long long)m * P;
                 if (live && m + 16 <= p.Cd) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++, y += P) *y = __uint_as_float(a[j]) + __uint_as_float(b[j]) + bias_s[m + j];
+                    for (int j = 0; j < 16; j++, y += P) *y = v[j] + bias_s[m + j];
                 } else if (live) {
 #pragma unroll
                     for (int j = 0; j < 16; j++, y += P)
-                        if (m + j < p.Cd) *y = __uint_as_float(a[j]) + __uint_as_float(b[j]) + bias_s[m + j];
+                        if (m + j < p.Cd) *y = v[j] + bias_s[m + j];
                 }
             }
             x += 128; po += 128;
@@ -193,6 +207,25 @@ __global__ void __launch_bounds__(PW_THREADS, 1) conv_pw_kernel(const __grid_con
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0) { tc::tc_fence_after(); tc::tmem_dealloc(tmem, (uint32_t)p.cols); }
+}
+
+// The tensor core truncates what it accumulates, so that a chain of steps is as long as those of the kernel that would take the layer
+// otherwise.  gemm: one chain, as there (the errors against 64 bits are equal to three digits, 1.69e-6 in both at 300 channels of one sign).
+// Else mma.sync, whose chains are at most 16 steps, most of them shorter: two pieces (eight steps), where tensor memory has no
+// room for so many accumulators three, and the storing warps add the sums with ordinary rounding.  The error against 64 bits, 30 streams on
+// 20 x 20, in units of 1e-7, mma.sync / one chain / here: normal 96 -> 32 3.6 / 2.7 / 1.8, 256 -> 32 4.7 / 6.4 / 2.0, 400 -> 16 4.1 / 9.7 / 2.0, 420 -> 48 7.8 /
+// 10.4 / 2.6; terms of one sign 3.6 / 4.3 / 2.3, 4.8 / 14.0 / 2.7, 4.2 / 23.0 / 2.7, 8.9 / 24.4 / 4.0.  From some 500 channels on mma.sync loads its weights
+// piece by piece, in chains as short as those (620 -> 32: 2.2 and 1.7; one chain 15 and 38), and takes the layers.
+static bool pw_chains(PwParams &p, bool gemm)
+{
+    p.chain = p.chunks; p.chains = 1;
+    if (gemm) return true;
+    if (p.C > PW_MAX_SOURCES) return false;
+    for (p.chain = 2; p.chain <= 3; p.chain++) {
+        p.chains = ceil_div(p.chunks, p.chain);
+        if (2 * p.N * p.chains <= 512) return true;
+    }
+    return false;
 }
 
 static bool pw_run(const ConvGeom &g, const float *src, const float *w, const float *bias, float *dst, bool ig)
@@ -209,16 +242,23 @@ static bool pw_run(const ConvGeom &g, const float *src, const float *w, const fl
     p.stages = (int)std::min<size_t>(PW_STAGES, (PW_SMEM - weights) / PW_STAGE);
     p.status = tc_status_word();
     if (!p.status) return false;
-    p.accs = 4 * p.N <= 512 ? 2 : 1;
+    if (!pw_chains(p, p.P >= 128 && p.Cd >= 64 && total * p.C * p.Cd >= (1ll << 26))) return false;
+    p.accs = 4 * p.N * p.chains <= 512 ? 2 : 1;
     p.cols = 32;
-    while (p.cols < 2 * p.N * p.accs) p.cols *= 2;
+    while (p.cols < 2 * p.N * p.chains * p.accs) p.cols *= 2;
     p.src = src; p.w = w; p.bias = bias; p.dst = dst;
     p.wm = ig ? 1 : g.Cin; p.wk = ig ? g.Cin : 1;
     p.total = (int)total;
     p.per = ceil_div(ceil_div(total, sm_count()), 32) * 32;
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(conv_pw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM); attr = true; }
-    TL_LAUNCH(conv_pw_kernel, ceil_div(total, p.per), PW_THREADS, weights + (size_t)p.stages * PW_STAGE, p);
+    if (!attr) {
+        cudaFuncSetAttribute(conv_pw_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        cudaFuncSetAttribute(conv_pw_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PW_SMEM);
+        attr = true;
+    }
+    const size_t smem = weights + (size_t)p.stages * PW_STAGE;
+    if (p.chains > 1) TL_LAUNCH(conv_pw_kernel<true>, ceil_div(total, p.per), PW_THREADS, smem, p);
+    else TL_LAUNCH(conv_pw_kernel<false>, ceil_div(total, p.per), PW_THREADS, smem, p);
     profile_add_flops(2.0 * total * g.Cin * g.Cout);
     return true;
 }

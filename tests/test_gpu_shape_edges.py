@@ -193,6 +193,30 @@ def test_pointwise_over_many_pixels(run, oracle, cin, h, w, cout, n):
     assert any("conv_pw_kernel" in t[0] for t in run.pkg.profile_table(run.lib)) == (cin < 256)
 
 
+# Terms of one sign show what the tensor core cuts off: half of 2^-23 of the sum in the mean at every step.  Chains of at most twelve steps of eight channels,
+# whose sums are added to fp32 registers, leave 12 / 2 * 2^-24 = 3.6e-7 of a result, the three terms of a product and the sum of the chains some
+# 1e-7 more (one chain for all channels: 1.4e-6 at 256, 2.3e-6 at 400).  Two sets of accumulators and one, chains of two and of three pieces,
+# more than 64 results on small planes, so many channels that the layer runs elsewhere
+@pytest.mark.parametrize("cin,h,w,cout,n,here", [(256, 20, 20, 32, 30, 1), (400, 19, 21, 16, 30, 1), (310, 20, 20, 63, 25, 1), (330, 21, 20, 48, 25, 1), (180, 10, 11, 80, 100, 1), (512, 20, 20, 30, 30, 1), (600, 20, 20, 30, 25, 0)])
+def test_pointwise_layers_of_many_channels_do_not_drift(run, cin, h, w, cout, n, here):
+    if run.half:
+        pytest.skip("single precision only")
+    rng = seeded(cin)
+    x, wt = (rng.uniform(0, 1, s).astype(F) for s in ((n, cin, h, w), (cout, cin, 1, 1)))
+    run.lib.trainlib_set_streams(n)
+    Y, B, one = run.zeros(n, cout, h, w), run.zeros(cout), run.zeros(4)
+    a = run.args("Conv2D_args", input=run.blob(run.t(x), one, C=cin, H=h, W=w), coeff=run.blob(run.t(wt), one, C=cin, H=1, W=1, dim=wt.size), bias=run.blob(B, B, dim=cout, W=cout),
+                 output=run.blob(Y, Y, C=cout, H=h, W=w), stride_h=1, stride_w=1, i2c_buffer=one, bt_buffer=one, USE_BIASES=0, USE_IM2COL=0, HWC=0)
+    run.lib.trainlib_profile(1)
+    run.call("pulp_conv2d_fp32_fw_cl", a)
+    run.lib.trainlib_profile(0)
+    names = [t[0] for t in run.pkg.profile_table(run.lib)]
+    assert any("conv_pw_kernel" in t for t in names) == bool(here), names
+    want = np.einsum("oc,nchw->nohw", wt[:, :, 0, 0].astype(np.float64), x[:4].astype(np.float64))
+    drift = (Y.get()[:4] / want - 1).mean()
+    assert abs(drift) <= 6e-7, drift
+
+
 # their weight gradient: lanes with hi and lo rows of X (up to 64 source channels) and without, slices of either side's channels, pieces of 16 and
 # of 32 pixels, planes that no 16-byte load fits, a last piece cut short
 POINTWISE_WG = [(64, 28, 28, 128, 15), (33, 17, 19, 70, 40), (7, 4, 4, 20, 700), (1, 30, 31, 40, 13), (20, 23, 23, 200, 21), (160, 20, 20, 96, 27), (96, 31, 30, 33, 9), (130, 25, 25, 140, 18), (5, 47, 48, 17, 80), (64, 40, 41, 8, 98)]
