@@ -768,7 +768,7 @@ static bool px_pays(const ConvGeom &g, bool ig)
     if (g.sh == 1) return w >= ((ig ? g.Cout : g.Cin) > 32 ? (ig ? 5e8 : 4e8) : 1e8);
     return w >= (ig ? 6e7 : 1e9);
 }
-// The weight gradient, with the bias gradient (a kernel and its sum less where there is one): 128 of 24 -> 48 on 28 x 28 36.0 / 22.0; 30 of
+// The weight gradient, with the bias gradient (a kernel and its sum less where there is one): 128 of 24 -> 48 on 28 x 28 36.0 / 23.9; 30 of
 // 40 -> 80, 5 x 5, on 41 x 41 182 / 45; 1 of 24 -> 45 on 39 x 27 (15) 11.5 / 9.9; 56 of 11 -> 8 on 8 x 15 (15) 8.4 / 10.1.  Sixteen result
 // channels fill a quarter of the rows of a product: 3 x 3 layers stay (262 of 27 -> 11 on 27 x 35 34.8 / 39.8), larger windows do
 // not (30 of 42 -> 6, 5 x 5, on 29 x 25 37.2 / 19.1).  1 x 1: only where the products of tl_gemm_tma.cu would have to pack odd planes
